@@ -77,10 +77,11 @@ __device__ __forceinline__ bool term_slots(const BondedTable& t, const int* atom
 
 // One thread per term, the four kinds one after the other in the index space. contrib holds three doubles per (term,
 // atom of the term): bonds, then angles, torsions and specials; a term that is skipped writes zeros.
-// partials: {PE, W, Wxx, Wyy, Wzz} per block.
+// scalars: {PE, W, Wxx, Wyy, Wzz}.
 __global__ void k_bonded_terms(BondedTable t, const double* __restrict__ x, const double* __restrict__ y,
                                const double* __restrict__ z, const double* __restrict__ charge,
-                               double* __restrict__ contrib, double* __restrict__ partials, unsigned* __restrict__ missing) {
+                               double* __restrict__ contrib, double* __restrict__ partials, unsigned* __restrict__ ticket,
+                               double* __restrict__ scalars, unsigned* __restrict__ missing) {
     const long long id = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     double sums[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
     const long long first_angle = t.n_bonds, first_torsion = first_angle + t.n_angles;
@@ -226,7 +227,7 @@ __global__ void k_bonded_terms(BondedTable t, const double* __restrict__ x, cons
         }
         for (int c = 0; c < 3; ++c) { out[c] = f[c]; out[3 + c] = -f[c]; }
     }
-    block_sum_to_partials<5>(sums, partials);
+    sum_over_grid<5>(sums, partials, ticket, scalars, false);
 }
 
 // One thread per owned atom: adds up, in table order, the contributions of the terms the atom takes part in.

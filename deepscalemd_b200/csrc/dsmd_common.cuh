@@ -33,21 +33,20 @@ struct Grid {
     float cellw[3];     // cell width per axis (length units); the x cells are finer than the y and z cells
     float r_pad;        // list radius plus a rounding margin: the reach used to prune cell rows
     float x_reach;      // widest half window along x (stencil * width of an unrefined cell, a hair less)
-    float band_search;  // the band of the list search (fp32 coordinates relative to the grid origin, image shifts added)
+    float quad_spread[3];   // how far four atoms searched together may lie apart
+    float band_rows;    // the band of the list search on float differences relative to a quad's first atom
 };
 
 struct Status {
     unsigned int need_stride;      // largest neighbour count seen (list rows that overflowed)
     unsigned int out_of_domain;    // atoms outside the mapped range or NaN
-    unsigned int rechecked;        // pair tests decided in fp64
+    unsigned int unused;
     unsigned int timeout;
     unsigned long long max_disp2;  // bits of the largest squared displacement (double, non-negative)
-    unsigned long long entries;    // directed list entries
-    unsigned long long interior;   // of which the partner is owned
     unsigned long long select_count;
     unsigned int dropped;          // owned atoms found outside the brick by a sort that removes them
     unsigned int constraint_failed;   // constraint clusters whose SHAKE / RATTLE sweeps did not converge
-    unsigned int boundary_atoms;      // owned atoms with a ghost partner in their list row (the boundary pass runs over them)
+    unsigned int boundary_pairs;      // pairs with a ghost partner in their list row (the boundary pass runs over them)
     unsigned int reserved;
 };
 

@@ -8,11 +8,9 @@
 //   type gid                               int32[capacity], two sets
 //   pq                                     int4[capacity]: fixed-point x, y, z and the type in w (what the kernels read)
 //   qf                                     float[capacity]: charge (read only with Coulomb on)
-//   xref yref zref                         double[capacity]: owned positions at the last build (displacement check)
+//   xref yref zref                         double[capacity]: positions at the last build (displacement check, list export)
 //   cell_start                             int32[2 * cells + 1]: first slot of every cell, owned cells then ghost cells
-//   nbr                                    uint32[ceil(n_owned / 32) * stride * 32]: 32-atom slices, entry k of the 32
-//                                          atoms of a slice is one 128-byte line; bit 31 = excluded pair
-//   deg, deg_int                           int32[n_owned]: entries per atom; of which the partner is owned (come first)
+//   quad, rows, row_end, row_int           the Verlet list: one row per pair of neighbouring owned atoms (dsmd_rows.cuh)
 //
 // No tensor cores: the path is a gather over a sparse geometric neighbourhood, not a dense contraction.
 
@@ -37,11 +35,11 @@ using dsmd::Status;
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kPairThreads = 128;
-constexpr int kBuildThreads = 64;   // k_build_list: 64, 128, 256 threads per block measured 2.62, 2.67, 2.86 ms (4 M atoms)
+constexpr int kDeviceSms = 148;                       // of a B200
+constexpr int64_t kPairLanesWanted = kDeviceSms * 1024;   // lanes that fill them
+constexpr int64_t kPairLanesWantedEwald = kDeviceSms * 768;   // two rounds of one block of 384 each
+constexpr int kLongRow = 240;                         // entries (with the row's spare room): about 150 partners per atom
 constexpr int kXRefine = 4;    // x cells per cell width of the y and z axes (tighter row windows in the list build)
-constexpr unsigned kExclBit = 0x80000000u;
-constexpr unsigned kIndexMask = 0x3FFFFFFFu;
 constexpr int kNumReal = 11;   // x y z vx vy vz fx fy fz mass charge
 constexpr double kCoulomb = 332.0636;
 
@@ -96,7 +94,7 @@ __global__ void k_cell_keys(Grid g, Brick brick, int first, int n_owned, int n_t
 __global__ void k_reorder(Grid g, int first, int n_owned, int n_total, const unsigned* __restrict__ key,
                           const int* __restrict__ val, RealArrays src, RealArrays dst, const int* __restrict__ type_src,
                           const int* __restrict__ gid_src, int* __restrict__ type_dst, int* __restrict__ gid_dst,
-                          int4* __restrict__ pq, float4* __restrict__ pf, float* __restrict__ qf, double* __restrict__ xref,
+                          int4* __restrict__ pq, float* __restrict__ qf, double* __restrict__ xref,
                           double* __restrict__ yref, double* __restrict__ zref, int* __restrict__ cell_start,
                           int* __restrict__ ghost_slot) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -118,19 +116,11 @@ __global__ void k_reorder(Grid g, int first, int n_owned, int n_total, const uns
     p.z = static_cast<int>(dsmd::to_fixed(r[2], 2, g, bad));
     p.w = ty;
     pq[s] = p;
-    // the list search's copy: single-precision offsets from the grid origin (the value of the fixed-point coordinate);
-    // the fourth word carries the global id, so that the exclusion test of a hit needs no second gather
-    pf[s] = make_float4(__uint2float_rn(static_cast<unsigned>(p.x)) * g.scale[0],
-                        __uint2float_rn(static_cast<unsigned>(p.y)) * g.scale[1],
-                        __uint2float_rn(static_cast<unsigned>(p.z)) * g.scale[2], __int_as_float(gid_src[from]));
     qf[s] = static_cast<float>(r[10]);
-    if (s < n_owned) {
-        xref[s] = r[0];
-        yref[s] = r[1];
-        zref[s] = r[2];
-    } else {
-        ghost_slot[from - n_owned] = s;
-    }
+    xref[s] = r[0];
+    yref[s] = r[1];
+    zref[s] = r[2];
+    if (s >= n_owned) ghost_slot[from - n_owned] = s;
     // Cell starts. Keys of the sorted range [first, n_total) are key[0 .. n_total - first). When only the owned atoms
     // are sorted (first == 0, n_total == n_owned) the ghost half of the table is filled by the later full build.
     const int k_here = static_cast<int>(key[t]);
@@ -147,7 +137,7 @@ __global__ void k_cell_tail(const unsigned* __restrict__ key, int n_sorted, int 
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
-// kernel: Verlet list build
+// kernels: support of the list build
 // ---------------------------------------------------------------------------------------------------------------------
 
 // A ghost-only sort gathers the ghosts into the other buffer set; this brings them back, so that the owned atoms
@@ -171,7 +161,7 @@ __global__ void k_layer_starts(const int* __restrict__ cell_start, int cells_per
 
 // Where the ghosts of a cell row sit: lo_end = one past the last x cell of the row's lower half that holds a ghost (0:
 // none), hi_begin = the first x cell of its upper half that holds one (nc[0]: none). One warp per (y, z) row.
-__global__ void k_ghost_row_extent(Grid g, const int* __restrict__ ghost_cell_start, int* __restrict__ lo_end,
+__global__ void k_ghost_row_specialtent(Grid g, const int* __restrict__ ghost_cell_start, int* __restrict__ lo_end,
                                    int* __restrict__ hi_begin) {
     const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -217,232 +207,6 @@ __global__ void k_ghost_rows_near(Grid g, const int* __restrict__ lo_end, const 
     near_hi[row] = hi;
 }
 
-struct ExclusionTable {
-    const int* offsets;    // [n_global + 1] by global id, or null
-    const int* partners;   // sorted per atom
-    int n_global;          // ids at or beyond this have no exclusions
-};
-
-__device__ __forceinline__ bool within_list_fp64(const Grid& g, const double* __restrict__ x,
-                                                 const double* __restrict__ y, const double* __restrict__ z, int i,
-                                                 int j) {
-    double dx = x[i] - x[j], dy = y[i] - y[j], dz = z[i] - z[j];
-    if (g.wrap[0]) dx -= g.box[0] * rint(dx / g.box[0]);
-    if (g.wrap[1]) dy -= g.box[1] * rint(dy / g.box[1]);
-    if (g.wrap[2]) dz -= g.box[2] * rint(dz / g.box[2]);
-    // No FMA contraction: the sum must round as the plain fp64 expression dx*dx + dy*dy + dz*dz does.
-    const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-    return r2 < g.r2_list_d;
-}
-
-// One thread per owned atom. The cell rows of the stencil are contiguous runs of slots (cells are sorted x fastest), so
-// a row costs two table reads and a linear scan. The candidate test runs in fp32 on `pf`, a copy of the positions as
-// single-precision offsets from the grid origin written at the sort; the periodic image of a cell row (or of the piece
-// of a row window that lies across the box boundary) is one shift of the CENTRE's coordinate per row, so a candidate
-// costs three subtractions, no integer arithmetic and no conversion. Results inside the rounding band around the list
-// radius are re-decided in fp64 on the caller's double positions, which makes list membership identical to an fp64
-// search. Owned partners are scanned first, then ghosts, so the first deg_int entries of a row are the interior part.
-// 16 resident blocks of 64 threads: the 64-register budget that gives is worth more than the registers (measured: 2.76 ms
-// against 4.24 ms per build at 4 M atoms with 110 registers and 8 blocks).
-// EXCL: launched for systems with an exclusion table; keeps the first four partners of an atom in registers. The other
-// instantiation is launched for systems without one and keeps the plain table walk (never taken there): written this way
-// because removing the exclusion code from it altogether made the compiler spill more in the search loop (2.76 ms
-// against 2.67 ms per build at 4 M atoms).
-template <bool EXCL>
-__global__ void __launch_bounds__(kBuildThreads, 16)
-k_build_list(Grid g, int n_owned, int n_total, const int4* __restrict__ pq, const float4* __restrict__ pf,
-             const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ z,
-             const int* __restrict__ gid, ExclusionTable excl, const int* __restrict__ cell_start,
-             const int* __restrict__ ghost_near_lo, const int* __restrict__ ghost_near_hi,
-             unsigned* __restrict__ nbr, int stride, int* __restrict__ deg, int* __restrict__ deg_int,
-             int* __restrict__ boundary_list, Status* st) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = i < n_owned;   // lanes past the end stay for the warp sums at the bottom
-    const int4 pi = active ? pq[i] : make_int4(0, 0, 0, 0);
-    const float4 fi = active ? pf[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const int cx = static_cast<int>(dsmd::cell_of(static_cast<unsigned>(pi.x), g.wrap[0], g.nc[0]));
-    const int cy = static_cast<int>(dsmd::cell_of(static_cast<unsigned>(pi.y), g.wrap[1], g.nc[1]));
-    const int cz = static_cast<int>(dsmd::cell_of(static_cast<unsigned>(pi.z), g.wrap[2], g.nc[2]));
-    const int S = g.stencil;
-    const size_t base = (static_cast<size_t>(i >> 5) * stride) * 32 + (i & 31);
-    int ex_begin = 0, ex_end = 0;
-    // the first four exclusion partners (rigid water has two) are kept in registers: a hit is compared with them without
-    // touching memory; atoms with more partners walk the rest of their table row
-    constexpr int kNoPartner = static_cast<int>(0x80000000u);   // no atom carries this id
-    int ex0 = kNoPartner, ex1 = kNoPartner, ex2 = kNoPartner, ex3 = kNoPartner;
-    if (active && excl.offsets) {
-        const int gi = gid[i];
-        if (gi >= 0 && gi < excl.n_global) {
-            ex_begin = excl.offsets[gi];
-            ex_end = excl.offsets[gi + 1];
-            if (EXCL) {
-                if (ex_end > ex_begin) ex0 = excl.partners[ex_begin];
-                if (ex_end > ex_begin + 1) ex1 = excl.partners[ex_begin + 1];
-                if (ex_end > ex_begin + 2) ex2 = excl.partners[ex_begin + 2];
-                if (ex_end > ex_begin + 3) ex3 = excl.partners[ex_begin + 3];
-            }
-        }
-    }
-    const float hi_band = g.r2_list + g.band_search;
-    const float in_band = g.r2_list - g.band_search;
-    // every hit of an atom with exclusions takes the slow path, which looks the partner up in the exclusion table
-    const float lo_band = ex_end > ex_begin ? -1.0f : in_band;
-    const float box_x = static_cast<float>(g.box[0]), box_y = static_cast<float>(g.box[1]), box_z = static_cast<float>(g.box[2]);
-    unsigned* dst = nbr + base;   // next entry of this atom's row (entries of a row are 32 words apart)
-    unsigned* const dst_end = dst + static_cast<size_t>(stride) * 32;
-    int interior = 0;
-    unsigned rechecked = 0;
-    // the ghost pass only for atoms whose x window reaches an x cell with ghosts in one of the rows they search (on an
-    // axis that wraps the window may come round the box: any ghost in those rows counts)
-    int n_seg = active ? 1 : 0;
-    if (active && n_total > n_owned) {
-        const int row_yz = cz * g.nc[1] + cy;
-        const int near_lo = ghost_near_lo[row_yz], near_hi = ghost_near_hi[row_yz];
-        const int reach_cells = static_cast<int>(g.x_reach / g.cellw[0]) + 2;
-        if (g.wrap[0] ? (near_lo > 0 || near_hi < g.nc[0]) : (cx - reach_cells < near_lo || cx + reach_cells >= near_hi))
-            n_seg = 2;
-    }
-    // The x window of a cell row is the chord of the list sphere at the row's distance from the atom in the y-z plane
-    // (dsmd::row_window spells the rule out): the distance has one term per axis, each a function of the cell offset and
-    // of the atom's place inside its home cell, so the z term is worked out per layer and the y term per row.
-    const unsigned ux = static_cast<unsigned>(pi.x), uy = static_cast<unsigned>(pi.y), uz = static_cast<unsigned>(pi.z);
-    const float ty = __uint2float_rn(g.wrap[1] ? uy : uy << 1) * (static_cast<float>(g.nc[1]) * 2.3283064e-10f);
-    const float tz = __uint2float_rn(g.wrap[2] ? uz : uz << 1) * (static_cast<float>(g.nc[2]) * 2.3283064e-10f);
-    const float in_y = fminf(fmaxf(ty - static_cast<float>(cy), 0.f), 1.f);   // place inside the home cell, 0 .. 1
-    const float in_z = fminf(fmaxf(tz - static_cast<float>(cz), 0.f), 1.f);
-    const float reach2 = g.r_pad * g.r_pad;
-    const float units_per_length = 1.0f / g.scale[0];
-    for (int seg = 0; seg < n_seg; ++seg) {
-        for (int dz = -S; dz <= S; ++dz) {
-            int zc = cz + dz;
-            float zi = fi.z;   // the centre as the atoms of this cell row see it
-            if (g.wrap[2]) { if (zc < 0) { zc += g.nc[2]; zi += box_z; } else if (zc >= g.nc[2]) { zc -= g.nc[2]; zi -= box_z; } }
-            else if (zc < 0 || zc >= g.nc[2]) continue;
-            float gz = dz > 0 ? (static_cast<float>(dz) - in_z) : (dz < 0 ? (in_z - static_cast<float>(dz + 1)) : 0.f);
-            gz = fmaxf(gz - 1e-4f, 0.f) * g.cellw[2];   // 1e-4 of a cell: rounding of the in-cell position
-            const float room2 = reach2 - gz * gz;
-            if (room2 <= 0.f) continue;
-            for (int dy = -S; dy <= S; ++dy) {
-                int yc = cy + dy;
-                float yi = fi.y;
-                if (g.wrap[1]) { if (yc < 0) { yc += g.nc[1]; yi += box_y; } else if (yc >= g.nc[1]) { yc -= g.nc[1]; yi -= box_y; } }
-                else if (yc < 0 || yc >= g.nc[1]) continue;
-                float gy = dy > 0 ? (static_cast<float>(dy) - in_y) : (dy < 0 ? (in_y - static_cast<float>(dy + 1)) : 0.f);
-                gy = fmaxf(gy - 1e-4f, 0.f) * g.cellw[1];
-                const float chord2 = room2 - gy * gy;
-                if (chord2 <= 0.f) continue;
-                // half window: the chord, never wider than the stencil, rounded outwards to whole x cells (r_pad carries
-                // 1e-4 of slack, far more than the approximate square root gives away)
-                const float hw = fminf(chord2 * rsqrtf(chord2), g.x_reach);
-                const unsigned hw_fixed = static_cast<unsigned>(hw * units_per_length) + 2u;
-                const int row = seg * g.ncells + (zc * g.nc[1] + yc) * g.nc[0];
-                dsmd::RowWindow win;
-                win.a1 = 0;
-                win.b1 = -1;
-                if (g.wrap[0]) {
-                    const int c_lo = static_cast<int>(dsmd::cell_of(ux - hw_fixed, 1, g.nc[0]));
-                    const int c_hi = static_cast<int>(dsmd::cell_of(ux + hw_fixed, 1, g.nc[0]));
-                    if (c_lo <= c_hi) { win.a0 = c_lo; win.b0 = c_hi; }
-                    else { win.a0 = 0; win.b0 = c_hi; win.a1 = c_lo; win.b1 = g.nc[0] - 1; }
-                } else {
-                    const long long lo = static_cast<long long>(ux) - hw_fixed, hi = static_cast<long long>(ux) + hw_fixed;
-                    win.a0 = static_cast<int>(dsmd::cell_of(static_cast<unsigned>(lo < 0 ? 0 : lo), 0, g.nc[0]));
-                    win.b0 = static_cast<int>(dsmd::cell_of(static_cast<unsigned>(hi > 2147483647ll ? 2147483647ll : hi), 0, g.nc[0]));
-                }
-                const bool two = win.b1 >= win.a1;   // the x window crosses the periodic boundary: [0, b0] and [a1, nc - 1]
-                for (int part = 0; part < 2; ++part) {
-                    const int a = part == 0 ? win.a0 : win.a1, b = part == 0 ? win.b0 : win.b1;
-                    if (b < a) continue;
-                    // the piece the centre's own cell is not in holds images one box length away
-                    float xi = fi.x;
-                    if (two) {
-                        const bool centre_low = cx <= win.b0;
-                        if (part == 0 && !centre_low) xi -= box_x;
-                        if (part == 1 && centre_low) xi += box_x;
-                    }
-                    const int s_begin = cell_start[row + a], s_end = cell_start[row + b + 1];
-                    for (int s = s_begin; s < s_end; ++s) {
-                        const float4 c = __ldg(&pf[s]);
-                        const float dx = c.x - xi, ddy = c.y - yi, ddz = c.z - zi;
-                        const float r2 = dx * dx + ddy * ddy + ddz * ddz;
-                        if (r2 < hi_band && s != i) {
-                            unsigned entry = static_cast<unsigned>(s);
-                            if (r2 >= lo_band) {   // inside the rounding band, or an atom with exclusions: the slow, exact way
-                                if (r2 >= in_band) {
-                                    ++rechecked;
-                                    if (!within_list_fp64(g, x, y, z, i, s)) continue;
-                                }
-                                if (ex_end > ex_begin) {
-                                    const int gj = __float_as_int(c.w);
-                                    if (EXCL && (gj == ex0 || gj == ex1 || gj == ex2 || gj == ex3)) entry |= kExclBit;   // an unused register never matches
-                                    for (int e = ex_begin + (EXCL ? 4 : 0); e < ex_end; ++e)
-                                        if (excl.partners[e] == gj) entry |= kExclBit;
-                                }
-                            }
-                            if (dst < dst_end) *dst = entry;
-                            dst += 32;
-                        }
-                    }
-                }
-            }
-        }
-        if (seg == 0) interior = static_cast<int>((dst - (nbr + base)) >> 5);
-    }
-    const int count = static_cast<int>((dst - (nbr + base)) >> 5);
-    if (active) {
-        deg[i] = min(count, stride);
-        deg_int[i] = min(interior, stride);
-        if (count > stride) atomicMax(&st->need_stride, static_cast<unsigned>(count));
-    }
-    // atoms with a ghost partner, collected for the boundary pass of the pair kernel (one atomic per warp; the order of
-    // the collection does not matter: every atom's sum is its own thread's)
-    {
-        const bool has_ghost_partner = active && count > interior;
-        const unsigned ballot = __ballot_sync(0xffffffffu, has_ghost_partner);
-        if (ballot) {
-            const int lane = threadIdx.x & 31;
-            unsigned first = 0;
-            if (lane == 0) first = atomicAdd(&st->boundary_atoms, static_cast<unsigned>(__popc(ballot)));
-            first = __shfl_sync(0xffffffffu, first, 0);
-            if (has_ghost_partner) boundary_list[first + __popc(ballot & ((1u << lane) - 1u))] = i;
-        }
-    }
-    // statistics: one atomic per warp
-    unsigned long long c64 = count, i64 = interior;
-    unsigned rc = rechecked;
-    for (int o = 16; o > 0; o >>= 1) {
-        c64 += __shfl_down_sync(0xffffffffu, c64, o);
-        i64 += __shfl_down_sync(0xffffffffu, i64, o);
-        rc += __shfl_down_sync(0xffffffffu, rc, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicAdd(&st->entries, c64);
-        atomicAdd(&st->interior, i64);
-        if (rc) atomicAdd(&st->rechecked, rc);
-    }
-}
-
-__global__ void k_list_export(int n_owned, const unsigned* __restrict__ nbr, int stride, const int* __restrict__ deg,
-                              const unsigned long long* __restrict__ offsets, int* out_i, int* out_j,
-                              unsigned char* out_flags, long long capacity) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_owned) return;
-    const size_t base = (static_cast<size_t>(i >> 5) * stride) * 32 + (i & 31);
-    unsigned long long o = offsets[i];
-    for (int k = 0; k < deg[i]; ++k, ++o) {
-        if (static_cast<long long>(o) >= capacity) return;
-        const unsigned e = nbr[base + static_cast<size_t>(k) * 32];
-        out_i[o] = i;
-        out_j[o] = static_cast<int>(e & kIndexMask);
-        if (out_flags) out_flags[o] = (e & kExclBit) ? 1 : 0;
-    }
-}
-
-__global__ void k_deg_to_u64(int n, const int* deg, unsigned long long* out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = static_cast<unsigned long long>(deg[i]);
-}
-
 // ---------------------------------------------------------------------------------------------------------------------
 // kernels: per-step pack, displacement, integration
 // ---------------------------------------------------------------------------------------------------------------------
@@ -470,11 +234,11 @@ __global__ void k_pack(Grid g, int first, int count, int n_owned, double* __rest
                        const double* __restrict__ fz, const double* __restrict__ mass, const int* __restrict__ type,
                        const double* __restrict__ xref, const double* __restrict__ yref,
                        const double* __restrict__ zref, int4* __restrict__ pq, double dt, double kick_c,
-                       Status* st) {
+                       const int* __restrict__ gid, const unsigned char* __restrict__ skip, Status* st) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int s = first + t;
     double d2 = 0.0;
-    if (t < count) {
+    if (t < count && !(skip && skip[gid[s]])) {   // skip: atoms of constraint clusters, by global id (k_constrained moves them)
         double px = x[s], py = y[s], pz = z[s];
         if (INTEGRATE) {
             const double a = kick_c / mass[s];
@@ -504,9 +268,10 @@ __global__ void k_pack(Grid g, int first, int count, int n_owned, double* __rest
 
 __global__ void k_vv2(int n, double half_dt_c, double* __restrict__ vx, double* __restrict__ vy,
                       double* __restrict__ vz, const double* __restrict__ fx, const double* __restrict__ fy,
-                      const double* __restrict__ fz, const double* __restrict__ mass) {
+                      const double* __restrict__ fz, const double* __restrict__ mass, const int* __restrict__ gid,
+                      const unsigned char* __restrict__ skip) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n) return;
+    if (s >= n || (skip && skip[gid[s]])) return;
     const double a = half_dt_c / mass[s];
     vx[s] += a * fx[s];
     vy[s] += a * fy[s];
@@ -524,10 +289,10 @@ __global__ void k_scale_velocities(int n, double factor, double* __restrict__ vx
     vz[s] *= factor;
 }
 
-// Deterministic two-level sums: per-block partials, then one block adds them in a fixed order.
+// Deterministic sums over a grid: every block leaves its partial sums, and the block that finishes last adds them up in a
+// fixed order (one launch instead of two). `ticket` counts finished blocks and is left at zero.
 template <int NV>
-__device__ __forceinline__ void block_sum_to_partials(double (&v)[NV], double* partials) {
-    __shared__ double sh[32][NV];
+__device__ __forceinline__ void block_sum(double (&v)[NV], double (&sh)[32][NV]) {   // thread 0 has the sums
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
     for (int k = 0; k < NV; ++k)
@@ -538,230 +303,53 @@ __device__ __forceinline__ void block_sum_to_partials(double (&v)[NV], double* p
     if (threadIdx.x == 0) {
         const int nw = blockDim.x >> 5;
         for (int k = 0; k < NV; ++k) {
-            double sum = 0.0;
-            for (int q = 0; q < nw; ++q) sum += sh[q][k];
-            partials[static_cast<size_t>(blockIdx.x) * NV + k] = sum;
+            v[k] = 0.0;
+            for (int q = 0; q < nw; ++q) v[k] += sh[q][k];
         }
     }
 }
 
 template <int NV>
-__global__ void k_reduce_partials(const double* __restrict__ partials, int n_blocks, double* __restrict__ out,
-                                  int accumulate) {
-    __shared__ double sh[kThreads];
-    for (int k = 0; k < NV; ++k) {
-        double sum = 0.0;
-        for (int b = threadIdx.x; b < n_blocks; b += blockDim.x) sum += partials[static_cast<size_t>(b) * NV + k];
-        sh[threadIdx.x] = sum;
-        __syncthreads();
-        for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-            if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) out[k] = accumulate ? out[k] + sh[0] : sh[0];
-        __syncthreads();
+__device__ __forceinline__ void sum_over_grid(double (&v)[NV], double* partials, unsigned* ticket, double* out, bool accumulate) {
+    __shared__ double sh[32][NV];
+    __shared__ bool last;
+    block_sum<NV>(v, sh);
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < NV; ++k) partials[static_cast<size_t>(blockIdx.x) * NV + k] = v[k];
+        __threadfence();
+        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int k = 0; k < NV; ++k) v[k] = 0.0;
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x)
+        for (int k = 0; k < NV; ++k) v[k] += __ldcg(&partials[static_cast<size_t>(b) * NV + k]);
+    block_sum<NV>(v, sh);
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < NV; ++k) out[k] = accumulate ? out[k] + v[k] : v[k];
+        *ticket = 0u;
     }
 }
 
 __global__ void k_kinetic(int n, const double* __restrict__ vx, const double* __restrict__ vy,
-                          const double* __restrict__ vz, const double* __restrict__ mass, double* partials) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+                          const double* __restrict__ vz, const double* __restrict__ mass, double* partials, unsigned* ticket,
+                          double* out) {
     double v[1] = {0.0};
-    if (s < n) v[0] = 0.5 * mass[s] * (vx[s] * vx[s] + vy[s] * vy[s] + vz[s] * vz[s]);
-    block_sum_to_partials<1>(v, partials);
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x)
+        v[0] += 0.5 * mass[s] * (vx[s] * vx[s] + vy[s] * vy[s] + vz[s] * vz[s]);
+    sum_over_grid<1>(v, partials, ticket, out, false);
 }
 
 }  // namespace
 
 #include "dsmd_constraints.cuh"
 #include "dsmd_bonded.cuh"
+#include "dsmd_f32x2.cuh"
+#include "dsmd_rows.cuh"
+#include "dsmd_pair.cuh"
 
 namespace {
-
-// ---------------------------------------------------------------------------------------------------------------------
-// kernel: LJ + real-space Ewald over the list
-// ---------------------------------------------------------------------------------------------------------------------
-
-struct PairParams {
-    float scale[3];
-    float rc2;
-    float rs2, inv_denom;        // CHARMM switch on r^2 (rs2 < 0: off)
-    float kq;                    // Coulomb constant
-    float alpha, two_alpha_sqrtpi;
-    int ntypes;
-    int ewald_intervals;
-    const float2* c6c12;         // [ntypes * ntypes]
-    const float4* ewald;         // [2 * intervals]: force cubic, energy cubic
-    const float* type_charge;    // [ntypes] when every atom's charge is that of its type (dsmd_set_type_charges), else null
-};
-
-// 1 / v: the hardware approximation (1 ulp) for the force-only kernels, one Newton step more (full single precision)
-// where energy and virial sums are taken.
-template <bool REFINE>
-__device__ __forceinline__ float fast_rcp(float v) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
-    return REFINE ? r * (2.0f - v * r) : r;
-}
-
-// One pair of the list, evaluated from atom i's side: adds to the force (and energy / virial) accumulators.
-template <bool COULOMB, bool ENERGY, bool MULTI, bool SWITCH>
-struct PairAccumulator {
-    float ax = 0.f, ay = 0.f, az = 0.f;
-    float e_sum = 0.f, w_sum = 0.f, wx = 0.f, wy = 0.f, wz = 0.f, n_in = 0.f;
-
-    __device__ __forceinline__ void add(const PairParams& p, const int4& pi, const int4& pj, float qi, float qj,
-                                        bool excluded, const float2* s_c6c12, const float4* s_ewald, float2 single,
-                                        int trow) {
-        const float dx = dsmd::fixed_delta(pi.x, pj.x, p.scale[0]);
-        const float dy = dsmd::fixed_delta(pi.y, pj.y, p.scale[1]);
-        const float dz = dsmd::fixed_delta(pi.z, pj.z, p.scale[2]);
-        const float r2 = dx * dx + dy * dy + dz * dz;
-        if (r2 < p.rc2 && r2 >= 1e-10f) {
-            float fmag = 0.f, epair = 0.f;
-            const float r2inv = fast_rcp<ENERGY>(r2);
-            if (!excluded) {
-                const float2 c = MULTI ? s_c6c12[trow + pj.w] : single;
-                const float r6 = r2inv * r2inv * r2inv;
-                const float t = c.y * r6;
-                float f = (r2inv * r6) * (12.f * t - 6.f * c.x);
-                float u = (ENERGY || SWITCH) ? r6 * (t - c.x) : 0.f;
-                if (SWITCH) {
-                    if (r2 > p.rs2) {
-                        const float a = p.rc2 - r2, b = p.rc2 + 2.f * r2 - 3.f * p.rs2;
-                        const float sw = a * a * b * p.inv_denom;
-                        f = sw * f + 12.f * u * a * (r2 - p.rs2) * p.inv_denom;
-                        u *= sw;
-                    }
-                }
-                fmag = f;
-                if (ENERGY) epair = u;
-            }
-            if (COULOMB) {
-                const float qq = qi * qj;
-                const unsigned shifted = __float_as_uint(r2) - dsmd::kEwaldBaseBits;
-                const unsigned idx = shifted >> dsmd::kEwaldIndexShift;
-                float ff, ef = 0.f;
-                if (idx < static_cast<unsigned>(p.ewald_intervals)) {
-                    const float t = __uint_as_float(0x3F800000u | ((shifted << dsmd::kEwaldBits) & 0x007FFFFFu)) - 1.0f;
-                    const float4 cf = s_ewald[2 * idx];
-                    ff = ((cf.w * t + cf.z) * t + cf.y) * t + cf.x;
-                    if (ENERGY) {
-                        const float4 ce = s_ewald[2 * idx + 1];
-                        ef = ((ce.w * t + ce.z) * t + ce.y) * t + ce.x;
-                    }
-                } else {   // below the table (r^2 < 0.5): analytic
-                    const float r = sqrtf(r2), ar = p.alpha * r;
-                    const float ec = erfcf(ar) / r;
-                    ff = (ec + p.two_alpha_sqrtpi * __expf(-ar * ar)) * r2inv;
-                    ef = ec;
-                }
-                if (excluded) {   // the pair's 1/r is not part of the Ewald sum: erfc -> -erf
-                    const float rinv = rsqrtf(r2);
-                    ff -= rinv * r2inv;
-                    ef -= rinv;
-                }
-                fmag += qq * ff;
-                if (ENERGY) epair += qq * ef;
-            }
-            ax += fmag * dx;
-            ay += fmag * dy;
-            az += fmag * dz;
-            if (ENERGY) {
-                e_sum += epair;
-                w_sum += fmag * r2;
-                wx += fmag * dx * dx;
-                wy += fmag * dy * dy;
-                wz += fmag * dz * dz;
-                n_in += 1.f;
-            }
-        }
-    }
-};
-
-// One thread per owned atom, 32 atoms of a slice per warp: entry k of the slice is one coalesced 128-byte read (streamed
-// past L2 with an evict-first hint, so that the positions stay resident there), the partner's int4 comes through the
-// read-only path. The loop runs four entries at a time with the next four entries and the current four positions in
-// flight before any arithmetic starts; rows are padded to the loop's stride with the atom's own index, which the
-// r^2 >= 1e-10 test discards. Every listed pair is evaluated from the side of each of its owned atoms (full list), so
-// forces need no scatter and no atomics, and the summation order is fixed (bitwise reproducible). Energy and virial
-// take half of every directed entry; an owned-ghost pair is then counted half on each rank, as the reference's list
-// kernel does (src/force_calculator_cuda.cu:1784-1789).
-template <bool COULOMB, bool ENERGY, bool MULTI, bool SWITCH, bool EXCL, bool QTYPE>
-__global__ void __launch_bounds__(kPairThreads)
-k_pair(PairParams p, int n_owned, const int4* __restrict__ pq, const float* __restrict__ qf,
-       const unsigned* __restrict__ nbr, int stride, const int* __restrict__ deg, const int* __restrict__ deg_int,
-       int phase, const int* __restrict__ atom_list, int first, int n_threads, double* __restrict__ fx,
-       double* __restrict__ fy, double* __restrict__ fz, double* __restrict__ partials) {
-    extern __shared__ float4 smem[];
-    float2* s_c6c12 = reinterpret_cast<float2*>(smem);
-    float4* s_ewald = smem + (MULTI ? (p.ntypes * p.ntypes + 1) / 2 : 0);
-    // charges by type: the partner's charge comes out of a small table in shared memory (its type arrives with its
-    // position) instead of a second gather from global memory
-    constexpr bool by_type = COULOMB && QTYPE;   // QTYPE: launched when dsmd_set_type_charges gave a table
-    float* s_type_charge = reinterpret_cast<float*>(s_ewald + (COULOMB ? 2 * p.ewald_intervals : 0));
-    if (MULTI)
-        for (int k = threadIdx.x; k < p.ntypes * p.ntypes; k += blockDim.x) s_c6c12[k] = p.c6c12[k];
-    if (COULOMB)
-        for (int k = threadIdx.x; k < 2 * p.ewald_intervals; k += blockDim.x) s_ewald[k] = p.ewald[k];
-    if (by_type)
-        for (int k = threadIdx.x; k < p.ntypes; k += blockDim.x) s_type_charge[k] = p.type_charge[k];
-    if (MULTI || COULOMB) __syncthreads();
-
-    // atom_list (boundary pass): the atoms that have a ghost partner, a small part of a brick; null: the owned atoms
-    // first .. first + n_threads
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = t < n_threads ? (atom_list ? atom_list[t] : first + t) : n_owned;
-    PairAccumulator<COULOMB, ENERGY, MULTI, SWITCH> acc;
-    if (i < n_owned) {
-        const int4 pi = pq[i];
-        const float qi = COULOMB ? p.kq * (by_type ? s_type_charge[pi.w] : qf[i]) : 0.f;
-        const float2 single = MULTI ? make_float2(0.f, 0.f) : p.c6c12[0];
-        const int trow = MULTI ? pi.w * p.ntypes : 0;
-        const int k_begin = phase == DSMD_PHASE_BOUNDARY ? deg_int[i] : 0;
-        const int k_end = phase == DSMD_PHASE_INTERIOR ? deg_int[i] : deg[i];
-        const unsigned* row = nbr + (static_cast<size_t>(i >> 5) * stride) * 32 + (i & 31);
-        const unsigned self = static_cast<unsigned>(i);
-        constexpr int U = 4;
-        unsigned e[U], e_next[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) e_next[u] = (k_begin + u < k_end) ? __ldcs(row + static_cast<size_t>(k_begin + u) * 32) : self;
-        for (int k = k_begin; k < k_end; k += U) {
-            int4 pj[U];
-            float qj[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                e[u] = e_next[u];
-                pj[u] = __ldg(&pq[EXCL ? (e[u] & kIndexMask) : e[u]]);
-                if (COULOMB && !by_type) qj[u] = __ldg(&qf[EXCL ? (e[u] & kIndexMask) : e[u]]);
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-                e_next[u] = (k + U + u < k_end) ? __ldcs(row + static_cast<size_t>(k + U + u) * 32) : self;
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-                acc.add(p, pi, pj[u], qi, COULOMB ? (by_type ? s_type_charge[pj[u].w] : qj[u]) : 0.f,
-                        EXCL && (e[u] & kExclBit) != 0u, s_c6c12, s_ewald, single, trow);
-        }
-        if (phase == DSMD_PHASE_BOUNDARY) {
-            if (k_end > k_begin) {   // most atoms of a brick have no ghost partner: leave their forces alone
-                fx[i] += static_cast<double>(acc.ax);
-                fy[i] += static_cast<double>(acc.ay);
-                fz[i] += static_cast<double>(acc.az);
-            }
-        } else {
-            fx[i] = static_cast<double>(acc.ax);
-            fy[i] = static_cast<double>(acc.ay);
-            fz[i] = static_cast<double>(acc.az);
-        }
-    }
-    if (ENERGY) {
-        double v[6] = {0.5 * static_cast<double>(acc.e_sum), 0.5 * static_cast<double>(acc.w_sum),
-                       0.5 * static_cast<double>(acc.wx),    0.5 * static_cast<double>(acc.wy),
-                       0.5 * static_cast<double>(acc.wz),    0.5 * static_cast<double>(acc.n_in)};
-        block_sum_to_partials<6>(v, partials);
-    }
-}
 
 // ---------------------------------------------------------------------------------------------------------------------
 // kernels: ghosts
@@ -905,7 +493,6 @@ struct dsmd_ctx {
     int* gid[2] = {};
     int cur = 0;
     int4* pq = nullptr;
-    float4* pf = nullptr;          // positions as fp32 offsets from the grid origin, as of the last sort (list search)
     float* qf = nullptr;
     double* ref[3] = {};
     unsigned* key[2] = {};
@@ -918,21 +505,28 @@ struct dsmd_ctx {
     int layer_capacity = 0;
     cudaStream_t copy_in = nullptr, copy_out = nullptr;
     cudaEvent_t piece_up[16] = {}, piece_done[16] = {}, pipe_begin = nullptr, pipe_end = nullptr;
-    int* boundary_list = nullptr;     // [capacity] owned atoms with a ghost partner, as the last list build found them
+    int* boundary_pairs = nullptr;    // pairs with a ghost partner, as the last list build found them
     int64_t n_boundary = 0;
     float* type_charge = nullptr;     // [ntypes] charges by type (dsmd_set_type_charges), or null: per-atom charges
     int* cell_start = nullptr;
     int64_t cell_capacity = 0;
     int* ghost_rows = nullptr;        // [4 * rows]: lo_end, hi_begin per (y, z) row, then the same over the rows searched
     int64_t ghost_rows_capacity = 0;
-    unsigned* nbr = nullptr;
-    size_t nbr_capacity = 0;   // entries
+    // list rows (dsmd_rows.cuh)
+    unsigned* quad = nullptr;
+    int* row_end = nullptr;
+    int* row_int = nullptr;
+    unsigned* row_special = nullptr;
+    int lane_shift = 0;
+    int64_t quad_capacity = 0;
+    int64_t n_quads = 0;
+    unsigned* rows = nullptr;
+    size_t rows_capacity = 0;  // entries
     int stride = 0;
-    int* deg = nullptr;
-    int* deg_int = nullptr;
+    unsigned long long* member_stats = nullptr;   // 3 words: k_list_members
     void* cub_temp = nullptr;
     size_t cub_temp_bytes = 0;
-    float2* c6c12 = nullptr;
+    float2* lj = nullptr;
     float4* ewald = nullptr;
     int* excl_off = nullptr;
     int* excl_partner = nullptr;
@@ -940,6 +534,7 @@ struct dsmd_ctx {
     double* partials = nullptr;
     int64_t partial_blocks = 0;
     double* scalars = nullptr;      // 6 force scalars + 1 kinetic
+    unsigned* tickets = nullptr;    // finished blocks of the sums: forces, kinetic energy, bonded terms, constraints
     Status* status = nullptr;
     Status* h_status = nullptr;     // pinned
     double* h_scalars = nullptr;    // pinned
@@ -971,18 +566,22 @@ struct dsmd_ctx {
     int n_clusters = 0;
     int64_t cons_n_global = 0;
     int* cl_gid = nullptr;
+    int* cl_slot = nullptr;           // [n_clusters * kClusterAtoms] as of the last sort
+    unsigned char* cl_member = nullptr;   // [cons_n_global] 1: the atom belongs to a cluster
+    bool cl_cover_all = false;        // every atom does
+    int cl_shape = 0;                 // 0: any, 1: triangles, 2: bonds
     unsigned char* cl_a = nullptr;
     unsigned char* cl_b = nullptr;
     double* cl_d2 = nullptr;
     int* slot_of_gid = nullptr;
     bool slot_map_valid = false;
-    double* pre[3] = {};
     double cons_tolerance = 1e-8;
     int cons_max_iterations = 500;
     bool owned_sorted_only = false;
     int64_t expect_dropped = 0;    // atoms the last owned-only sort was told to remove (checked with the build status)
-    int64_t stat_entries = 0, stat_interior = 0;
+    int64_t stat_entries = 0, stat_interior = 0;   // worked out when asked for (list_members)
     int stat_rechecked = 0;
+    long long stat_epoch = -1;     // list build they belong to
 };
 
 namespace {
@@ -1097,10 +696,12 @@ int make_grid(dsmd_ctx* c) {
         max_len = std::max(max_len, 1.0 / g.inv_len[a]);
     }
     g.r_pad = static_cast<float>(R * (1.0 + 1e-4) + 8.0 * max_len * 1.2e-7);
-    // Rounding band of the fp32 search: a coordinate is an offset of up to max_len from the grid origin, the centre's may
-    // carry one more box length (image shift), so each carries a few ulp of 2 max_len; the squares and sums add a few
-    // ulp of R^2; the fixed-point grid itself one unit per coordinate. Everything inside the band is re-decided in fp64.
-    g.band_search = static_cast<float>(1.1920929e-7 * (24.0 * R * max_len + 16.0 * R * R) + 8.0 * R * max_scale);
+    // Rounding band of the list search: coordinates are single-precision differences of up to three list radii (a candidate
+    // and an atom of a quad, both relative to the quad's first atom), each good to three roundings of 2^-24; squares and
+    // sums add a few more of R^2; the fixed-point grid one unit per coordinate. Everything inside the band is listed.
+    g.band_rows = static_cast<float>(5.9604645e-8 * 48.0 * R * R + 8.0 * R * max_scale);
+    for (int a = 0; a < 3; ++a)
+        g.quad_spread[a] = g.wrap[a] ? std::min(g.r_pad, static_cast<float>(0.49 * g.box[a]) - g.r_pad) : g.r_pad;
     c->grid_valid = true;
     return DSMD_OK;
 }
@@ -1116,21 +717,73 @@ int ensure_cells(dsmd_ctx* c) {
     return DSMD_OK;
 }
 
-int ensure_list(dsmd_ctx* c, int stride) {
-    const size_t slices = static_cast<size_t>((c->n_owned + 31) / 32);
-    const size_t need = slices * static_cast<size_t>(stride) * 32;
-    if (need > c->nbr_capacity) {
-        // with headroom: the owned count of a brick changes by a few atoms at every migration, and a reallocation of this
-        // (large) buffer synchronises the device
-        const size_t grown = need + need / 8 + 4096;
-        if (c->nbr) cudaFree(c->nbr);
-        c->nbr = nullptr;
-        c->nbr_capacity = 0;
-        DSMD_CUDA(c, cudaMalloc(&c->nbr, sizeof(unsigned) * grown));
-        c->nbr_capacity = grown;
+int ensure_rows(dsmd_ctx* c, int stride) {
+    if (c->n_quads > c->quad_capacity) {
+        // with headroom here and below: the owned count of a brick changes by a few atoms at every migration, and a
+        // reallocation synchronises the device
+        const int64_t grown = c->n_quads + c->n_quads / 8 + 64;
+        cudaFree(c->quad); cudaFree(c->row_end); cudaFree(c->row_int); cudaFree(c->row_special); cudaFree(c->boundary_pairs);
+        c->quad = nullptr;
+        c->row_end = c->row_int = c->boundary_pairs = nullptr;
+        c->row_special = nullptr;
+        c->quad_capacity = 0;
+        DSMD_CUDA(c, cudaMalloc(&c->quad, sizeof(unsigned) * grown));
+        DSMD_CUDA(c, cudaMalloc(&c->row_end, sizeof(int) * 2 * grown));
+        DSMD_CUDA(c, cudaMalloc(&c->row_int, sizeof(int) * 2 * grown));
+        DSMD_CUDA(c, cudaMalloc(&c->row_special, sizeof(unsigned) * 2 * grown));
+        DSMD_CUDA(c, cudaMalloc(&c->boundary_pairs, sizeof(int) * 2 * grown));
+        c->quad_capacity = grown;
     }
-    c->stride = stride;
+    const size_t slices = static_cast<size_t>((2 * c->n_quads + 31) / 32);
+    const size_t need = slices * static_cast<size_t>(stride) * 32;
+    if (need > c->rows_capacity) {
+        const size_t grown = need + need / 8 + 4096;
+        cudaFree(c->rows);
+        c->rows = nullptr;
+        c->rows_capacity = 0;
+        DSMD_CUDA(c, cudaMalloc(&c->rows, sizeof(unsigned) * grown));
+        c->rows_capacity = grown;
+    }
     return DSMD_OK;
+}
+
+int pair_lane_shift(const dsmd_ctx* c);
+
+// Copies of the Ewald table in the force kernel's shared memory: eight where rows are long enough to pay for them.
+int ewald_copies(const dsmd_ctx* c) { return !c->coulomb ? 0 : (c->stride >= kLongRow ? kEwaldCopiesMost : 1); }
+
+// Rows for `row_entries` entries each: lanes per row, stride, storage.
+int lay_out_rows(dsmd_ctx* c, int row_entries) {
+    const int64_t yz_rows = static_cast<int64_t>(c->grid.nc[1]) * c->grid.nc[2];
+    c->n_quads = quad_base(static_cast<int>(c->n_owned), static_cast<int>(yz_rows));
+    c->stride = (row_entries + 3) & ~3;
+    c->lane_shift = pair_lane_shift(c);
+    return ensure_rows(c, c->stride);
+}
+
+RowArrays rows_of(const dsmd_ctx* c) { return RowArrays{c->quad, c->rows, c->stride, c->row_end, c->row_int, c->row_special}; }
+
+// Lanes that share a pair's row in the force kernel: one where that fills the device, more for small systems, whose time
+// is the chain of dependent reads along a row. A function of the system alone, so that a pass over a part of the atoms
+// gives the same bits as a pass over all of them.
+int pair_lane_shift(const dsmd_ctx* c) {
+    const int64_t pairs = 2 * c->n_quads, wanted = ewald_copies(c) == kEwaldCopiesMost ? kPairLanesWantedEwald : kPairLanesWanted;
+    int shift = 0;
+    while (shift < 5 && (pairs << shift) < wanted && (8 << shift) <= c->stride) ++shift;
+    return shift;
+}
+
+// Blocks of the force kernel for that many rows: with Coulomb or energy sums no more than the device holds at a time (they
+// take further rows in turn).
+int64_t pair_blocks(const dsmd_ctx* c, int64_t pairs, bool energy) {
+    const int64_t lanes = pairs << c->lane_shift;
+    switch (ewald_copies(c)) {
+        case kEwaldCopiesMost: return std::min<int64_t>(blocks_for(lanes, kPairThreads<kEwaldCopiesMost, kOneType>), kDeviceSms);
+        case 1: return std::min<int64_t>(blocks_for(lanes, kPairThreads<1, kOneType>), kDeviceSms * kPairBlocks<1, kOneType, false>);
+        default: break;
+    }
+    const int threads = c->ntypes == 1 ? kPairThreads<0, kOneType> : kPairThreads<0, kFewTypes>;
+    return energy ? std::min<int64_t>(blocks_for(lanes, threads), kDeviceSms * (512 / threads)) : blocks_for(lanes, threads);
 }
 
 int ensure_partials(dsmd_ctx* c, int64_t blocks) {
@@ -1172,7 +825,7 @@ int sort_range(dsmd_ctx* c, int64_t first, cudaStream_t s, int64_t n_removed = 0
         k_reorder<<<blocks_for(n, kThreads), kThreads, 0, s>>>(
             c->grid, static_cast<int>(first), static_cast<int>(c->n_owned), static_cast<int>(c->n_total), c->key[1],
             c->val[1], arrays_of(c, from), arrays_of(c, to), c->type[from], c->gid[from], c->type[to], c->gid[to], c->pq,
-            c->pf, c->qf, c->ref[0], c->ref[1], c->ref[2], c->cell_start, c->ghost_slot);
+            c->qf, c->ref[0], c->ref[1], c->ref[2], c->cell_start, c->ghost_slot);
         DSMD_LAUNCHED(c);
         const int table = 2 * c->grid.ncells + 1;
         const int64_t kept = n - n_removed;
@@ -1205,30 +858,36 @@ int read_status(dsmd_ctx* c, cudaStream_t s) {
     return DSMD_OK;
 }
 
-template <bool COULOMB, bool ENERGY, bool MULTI>
-void launch_pair(dsmd_ctx* c, const PairParams& p, int phase, bool sw, cudaStream_t s, int first, int n_threads) {
-    const int* atom_list = phase == DSMD_PHASE_BOUNDARY ? c->boundary_list : nullptr;
-    const unsigned blocks = blocks_for(n_threads, kPairThreads);
-    size_t smem = 0;
-    if (MULTI) smem += sizeof(float4) * ((p.ntypes * p.ntypes + 1) / 2);
-    if (COULOMB) smem += sizeof(float4) * 2 * p.ewald_intervals;
-    if (COULOMB && p.type_charge) smem += sizeof(float4) * ((p.ntypes + 3) / 4);
-    double* fx = c->real[c->cur][DSMD_FX];
-    double* fy = c->real[c->cur][DSMD_FY];
-    double* fz = c->real[c->cur][DSMD_FZ];
-    const bool ex = c->excl_off != nullptr;
-#define DSMD_PAIR_LAUNCH(SW, EX, QT)                                                                                  \
-    k_pair<COULOMB, ENERGY, MULTI, SW, EX, QT><<<blocks, kPairThreads, smem, s>>>(                                      \
-        p, static_cast<int>(c->n_owned), c->pq, c->qf, c->nbr, c->stride, c->deg, c->deg_int, phase, atom_list, first,  \
-        n_threads, fx, fy, fz, c->partials)
-    if (COULOMB && p.type_charge) {   // charges by type: only the kernels with Coulomb have this form
-        if (sw) { if (ex) DSMD_PAIR_LAUNCH(true, true, COULOMB); else DSMD_PAIR_LAUNCH(true, false, COULOMB); }
-        else    { if (ex) DSMD_PAIR_LAUNCH(false, true, COULOMB); else DSMD_PAIR_LAUNCH(false, false, COULOMB); }
-    } else {
-        if (sw) { if (ex) DSMD_PAIR_LAUNCH(true, true, false); else DSMD_PAIR_LAUNCH(true, false, false); }
-        else    { if (ex) DSMD_PAIR_LAUNCH(false, true, false); else DSMD_PAIR_LAUNCH(false, false, false); }
+template <int COPIES, bool ENERGY, int TYPES, bool SWITCH, bool QTYPE>
+int launch_pair_kernel(dsmd_ctx* c, const PairParams& p, const ForceArgs& a, cudaStream_t s) {
+    const size_t smem = PairTables<COPIES, ENERGY, TYPES, QTYPE>::bytes(p.ntypes, p.ewald_intervals);
+    const auto kernel = k_pair<COPIES, ENERGY, TYPES, SWITCH, QTYPE>;
+    if (smem > 48 * 1024) DSMD_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    kernel<<<static_cast<unsigned>(pair_blocks(c, a.n_pairs, ENERGY)), kPairThreads<COPIES, TYPES>, smem, s>>>(p, a);
+    DSMD_LAUNCHED(c);
+    return DSMD_OK;
+}
+
+template <int COPIES, bool ENERGY, int TYPES>
+int launch_pair(dsmd_ctx* c, const PairParams& p, const ForceArgs& a, bool sw, cudaStream_t s) {
+    constexpr bool coulomb = COPIES > 0;
+    if (coulomb && p.type_charge)   // charges by type: only the kernels with Coulomb have this form
+        return sw ? launch_pair_kernel<COPIES, ENERGY, TYPES, true, coulomb>(c, p, a, s)
+                  : launch_pair_kernel<COPIES, ENERGY, TYPES, false, coulomb>(c, p, a, s);
+    return sw ? launch_pair_kernel<COPIES, ENERGY, TYPES, true, false>(c, p, a, s)
+              : launch_pair_kernel<COPIES, ENERGY, TYPES, false, false>(c, p, a, s);
+}
+
+template <int COPIES>
+int launch_pair_types(dsmd_ctx* c, const PairParams& p, const ForceArgs& a, bool energy, bool sw, cudaStream_t s) {
+    if (energy) {
+        if (p.ntypes == 1) return launch_pair<COPIES, true, kOneType>(c, p, a, sw, s);
+        if (p.ntypes <= kFewTypesMost) return launch_pair<COPIES, true, kFewTypes>(c, p, a, sw, s);
+        return launch_pair<COPIES, true, kManyTypes>(c, p, a, sw, s);
     }
-#undef DSMD_PAIR_LAUNCH
+    if (p.ntypes == 1) return launch_pair<COPIES, false, kOneType>(c, p, a, sw, s);
+    if (p.ntypes <= kFewTypesMost) return launch_pair<COPIES, false, kFewTypes>(c, p, a, sw, s);
+    return launch_pair<COPIES, false, kManyTypes>(c, p, a, sw, s);
 }
 
 }  // namespace
@@ -1259,17 +918,16 @@ int dsmd_create(int device, int64_t capacity, dsmd_ctx** out) {
         DSMD_CUDA(c, cudaMalloc(&c->val[set], sizeof(int) * capacity));
     }
     DSMD_CUDA(c, cudaMalloc(&c->pq, sizeof(int4) * capacity));
-    DSMD_CUDA(c, cudaMalloc(&c->pf, sizeof(float4) * capacity));
     DSMD_CUDA(c, cudaMalloc(&c->qf, sizeof(float) * capacity));
     for (int a = 0; a < 3; ++a) DSMD_CUDA(c, cudaMalloc(&c->ref[a], sizeof(double) * capacity));
     DSMD_CUDA(c, cudaMalloc(&c->ghost_slot, sizeof(int) * capacity));
-    DSMD_CUDA(c, cudaMalloc(&c->deg, sizeof(int) * capacity));
-    DSMD_CUDA(c, cudaMalloc(&c->deg_int, sizeof(int) * capacity));
-    DSMD_CUDA(c, cudaMalloc(&c->boundary_list, sizeof(int) * capacity));
+    DSMD_CUDA(c, cudaMalloc(&c->member_stats, sizeof(unsigned long long) * 3));
     DSMD_CUDA(c, cudaMalloc(&c->flag, capacity));
     DSMD_CUDA(c, cudaMalloc(&c->offsets64, sizeof(unsigned long long) * capacity));
     DSMD_CUDA(c, cudaMalloc(&c->scalars, sizeof(double) * 8));
     DSMD_CUDA(c, cudaMemset(c->scalars, 0, sizeof(double) * 8));
+    DSMD_CUDA(c, cudaMalloc(&c->tickets, sizeof(unsigned) * 4));
+    DSMD_CUDA(c, cudaMemset(c->tickets, 0, sizeof(unsigned) * 4));
     DSMD_CUDA(c, cudaMalloc(&c->status, sizeof(Status)));
     DSMD_CUDA(c, cudaMemset(c->status, 0, sizeof(Status)));
     DSMD_CUDA(c, cudaMallocHost(&c->h_status, sizeof(Status)));
@@ -1289,13 +947,15 @@ void dsmd_destroy(dsmd_ctx* c) {
         for (int f = 0; f < kNumReal; ++f) cudaFree(c->real[set][f]);
         cudaFree(c->type[set]); cudaFree(c->gid[set]); cudaFree(c->key[set]); cudaFree(c->val[set]);
     }
-    cudaFree(c->pq); cudaFree(c->pf); cudaFree(c->qf); cudaFree(c->type_charge);
+    cudaFree(c->pq); cudaFree(c->qf); cudaFree(c->type_charge);
     for (int a = 0; a < 3; ++a) cudaFree(c->ref[a]);
-    cudaFree(c->ghost_slot); cudaFree(c->cell_start); cudaFree(c->ghost_rows); cudaFree(c->nbr); cudaFree(c->deg); cudaFree(c->deg_int);
-    cudaFree(c->boundary_list);
-    cudaFree(c->cub_temp); cudaFree(c->c6c12); cudaFree(c->ewald); cudaFree(c->excl_off); cudaFree(c->excl_partner);
-    cudaFree(c->partials); cudaFree(c->scalars); cudaFree(c->status); cudaFree(c->flag); cudaFree(c->offsets64);
+    cudaFree(c->ghost_slot); cudaFree(c->cell_start); cudaFree(c->ghost_rows);
+    cudaFree(c->rows); cudaFree(c->quad); cudaFree(c->row_end); cudaFree(c->row_int); cudaFree(c->row_special); cudaFree(c->boundary_pairs);
+    cudaFree(c->member_stats);
+    cudaFree(c->cub_temp); cudaFree(c->lj); cudaFree(c->ewald); cudaFree(c->excl_off); cudaFree(c->excl_partner);
+    cudaFree(c->partials); cudaFree(c->scalars); cudaFree(c->tickets); cudaFree(c->status); cudaFree(c->flag); cudaFree(c->offsets64);
     cudaFree(c->cl_gid); cudaFree(c->cl_a); cudaFree(c->cl_b); cudaFree(c->cl_d2); cudaFree(c->slot_of_gid);
+    cudaFree(c->cl_slot); cudaFree(c->cl_member);
     free_bonded(c);
     cudaFree(c->d_layer_start);
     if (c->h_layer_start) cudaFreeHost(c->h_layer_start);
@@ -1307,7 +967,6 @@ void dsmd_destroy(dsmd_ctx* c) {
     }
     if (c->pipe_begin) cudaEventDestroy(c->pipe_begin);
     if (c->pipe_end) cudaEventDestroy(c->pipe_end);
-    for (int a = 0; a < 3; ++a) cudaFree(c->pre[a]);
     cudaFreeHost(c->h_status); cudaFreeHost(c->h_scalars);
     for (int k = 0; k < 2; ++k) {
         cudaFreeHost(c->h_disp[k]);
@@ -1347,12 +1006,12 @@ int dsmd_set_pair_params(dsmd_ctx* c, int ntypes, const double* eps, const doubl
     for (int k = 0; k < ntypes * ntypes; ++k) {
         const double s2 = sig[k] * sig[k], s6 = s2 * s2 * s2;
         const double c6 = 4.0 * eps[k] * s6;
-        table[k] = make_float2(static_cast<float>(c6), static_cast<float>(c6 * s6));
+        table[k] = make_float2(static_cast<float>(12.0 * c6 * s6), static_cast<float>(-6.0 * c6));
     }
-    if (c->c6c12) cudaFree(c->c6c12);
-    c->c6c12 = nullptr;
-    DSMD_CUDA(c, cudaMalloc(&c->c6c12, sizeof(float2) * table.size()));
-    DSMD_CUDA(c, cudaMemcpy(c->c6c12, table.data(), sizeof(float2) * table.size(), cudaMemcpyHostToDevice));
+    if (c->lj) cudaFree(c->lj);
+    c->lj = nullptr;
+    DSMD_CUDA(c, cudaMalloc(&c->lj, sizeof(float2) * table.size()));
+    DSMD_CUDA(c, cudaMemcpy(c->lj, table.data(), sizeof(float2) * table.size(), cudaMemcpyHostToDevice));
     c->ntypes = ntypes;
     c->cutoff = cutoff;
     c->skin = skin;
@@ -1369,7 +1028,6 @@ int dsmd_set_coulomb(dsmd_ctx* c, int enabled, double alpha) {
     c->coulomb = enabled != 0;
     if (!c->coulomb) return DSMD_OK;
     if (!c->params_set) return fail(c, DSMD_ERR_STATE, "set the pair parameters (cutoff) before Coulomb");
-    DSMD_CUDA(c, cudaSetDevice(c->device));
     c->alpha = alpha > 0.0 ? alpha : dsmd::ewald_alpha_for(c->cutoff);
     c->ewald_intervals = dsmd::ewald_intervals(c->cutoff * c->cutoff);
     const std::vector<float> coef = dsmd::ewald_build_table(c->alpha, c->ewald_intervals);
@@ -1560,13 +1218,16 @@ int dsmd_build_neighbor_list(dsmd_ctx* c, void* stream) {
     c->expect_dropped = 0;
     if (first == 0 || c->n_total > first) { const int rc = sort_range(c, first, s); if (rc) return rc; }
     // 2. list rows
+    int row_entries = c->stride;
     if (c->stride == 0) {
         double volume = 1.0;
         for (int a = 0; a < 3; ++a) volume *= 1.0 / c->grid.inv_len[a];
         const double R = c->cutoff + c->skin;
+        // partners of one atom, and how many more its pair-mate adds (the sphere that the pair's distance, about one atom
+        // spacing in a dense system, moves out of the first one)
         const double expect = static_cast<double>(c->n_total) / volume * 4.18879020479 * R * R * R;
-        c->stride = std::max(32, static_cast<int>(expect * 1.3) + 24);
-        c->stride = (c->stride + 3) & ~3;
+        const double apart = std::min(std::cbrt(volume / static_cast<double>(c->n_total)) / R, 1.0);
+        row_entries = std::max(32, static_cast<int>(expect * (1.0 + std::min(0.9 * apart, 1.0)) * 1.2) + 32);
     }
     const int64_t rows = static_cast<int64_t>(c->grid.nc[1]) * c->grid.nc[2];
     if (4 * rows > c->ghost_rows_capacity) {
@@ -1591,7 +1252,7 @@ int dsmd_build_neighbor_list(dsmd_ctx* c, void* stream) {
         DSMD_CUDA(c, cudaMemcpyAsync(c->h_layer_start, c->d_layer_start, sizeof(int) * (layers + 1), cudaMemcpyDeviceToHost, s));
     }
     if (c->n_total > c->n_owned) {
-        k_ghost_row_extent<<<blocks_for(rows * 32, kThreads), kThreads, 0, s>>>(c->grid, c->cell_start + c->grid.ncells,
+        k_ghost_row_specialtent<<<blocks_for(rows * 32, kThreads), kThreads, 0, s>>>(c->grid, c->cell_start + c->grid.ncells,
                                                                                c->ghost_rows, c->ghost_rows + rows);
         DSMD_LAUNCHED(c);
         k_ghost_rows_near<<<blocks_for(rows, kThreads), kThreads, 0, s>>>(c->grid, c->ghost_rows, c->ghost_rows + rows,
@@ -1599,18 +1260,24 @@ int dsmd_build_neighbor_list(dsmd_ctx* c, void* stream) {
         DSMD_LAUNCHED(c);
     }
     for (int attempt = 0; attempt < 4; ++attempt) {
-        { const int rc = ensure_list(c, c->stride); if (rc) return rc; }
-        ExclusionTable ex{c->excl_off, c->excl_partner, static_cast<int>(c->excl_n_global)};
+        { const int rc = lay_out_rows(c, row_entries); if (rc) return rc; }
+        const ExclusionTable ex{c->excl_off, c->excl_partner, static_cast<int>(c->excl_n_global)};
+        if (attempt == 0) {
+            k_quads<<<blocks_for(rows * 32, kThreads), kThreads, 0, s>>>(c->grid.nc[0], static_cast<int>(rows), static_cast<int>(c->n_owned),
+                                                                        c->cell_start, c->quad);
+            DSMD_LAUNCHED(c);
+        }
+        const unsigned blocks = blocks_for(c->n_quads * 32, kBuildThreads);
         if (ex.offsets)
-            k_build_list<true><<<blocks_for(c->n_owned, kBuildThreads), kBuildThreads, 0, s>>>(
-                c->grid, static_cast<int>(c->n_owned), static_cast<int>(c->n_total), c->pq, c->pf, c->real[c->cur][0],
-                c->real[c->cur][1], c->real[c->cur][2], c->gid[c->cur], ex, c->cell_start, c->ghost_rows + 2 * rows,
-                c->ghost_rows + 3 * rows, c->nbr, c->stride, c->deg, c->deg_int, c->boundary_list, c->status);
+            k_build_rows<true><<<blocks, kBuildThreads, 0, s>>>(c->grid, static_cast<int>(c->n_owned), static_cast<int>(c->n_total),
+                                                              static_cast<int>(c->n_quads), c->pq, c->gid[c->cur], ex, c->cell_start,
+                                                              c->ghost_rows + 2 * rows, c->ghost_rows + 3 * rows, rows_of(c),
+                                                              c->boundary_pairs, c->status);
         else
-            k_build_list<false><<<blocks_for(c->n_owned, kBuildThreads), kBuildThreads, 0, s>>>(
-                c->grid, static_cast<int>(c->n_owned), static_cast<int>(c->n_total), c->pq, c->pf, c->real[c->cur][0],
-                c->real[c->cur][1], c->real[c->cur][2], c->gid[c->cur], ex, c->cell_start, c->ghost_rows + 2 * rows,
-                c->ghost_rows + 3 * rows, c->nbr, c->stride, c->deg, c->deg_int, c->boundary_list, c->status);
+            k_build_rows<false><<<blocks, kBuildThreads, 0, s>>>(c->grid, static_cast<int>(c->n_owned), static_cast<int>(c->n_total),
+                                                               static_cast<int>(c->n_quads), c->pq, c->gid[c->cur], ex, c->cell_start,
+                                                               c->ghost_rows + 2 * rows, c->ghost_rows + 3 * rows, rows_of(c),
+                                                               c->boundary_pairs, c->status);
         DSMD_LAUNCHED(c);
         { const int rc = read_status(c, s); if (rc) return rc; }
         if (c->h_status->out_of_domain)
@@ -1619,14 +1286,11 @@ int dsmd_build_neighbor_list(dsmd_ctx* c, void* stream) {
             return fail(c, DSMD_ERR_STATE, "sort: the number of atoms outside the brick differs from the caller's count");
         if (c->h_status->need_stride <= static_cast<unsigned>(c->stride)) break;
         // a row overflowed: grow and build again
-        c->stride = (static_cast<int>(c->h_status->need_stride * 1.1) + 8 + 3) & ~3;
+        row_entries = static_cast<int>(c->h_status->need_stride * 1.1) + 8;
         DSMD_CUDA(c, cudaMemsetAsync(c->status, 0, sizeof(Status), s));
         if (attempt == 3) return fail(c, DSMD_ERR_CAPACITY, "neighbour rows kept overflowing");
     }
-    c->stat_entries = static_cast<int64_t>(c->h_status->entries);
-    c->stat_interior = static_cast<int64_t>(c->h_status->interior);
-    c->stat_rechecked = static_cast<int>(c->h_status->rechecked);
-    c->n_boundary = static_cast<int64_t>(c->h_status->boundary_atoms);
+    c->n_boundary = static_cast<int64_t>(c->h_status->boundary_pairs);
     ++c->build_epoch;
     DSMD_CUDA(c, cudaMemsetAsync(c->status, 0, sizeof(Status), s));   // displacement word restarts at zero
     c->list_valid = true;
@@ -1639,10 +1303,34 @@ int dsmd_ghost_slots(dsmd_ctx* c, const int32_t** out) {
     return DSMD_OK;
 }
 
+// The list proper (k_list_members): partners per atom into c->offsets64, sums into the context. Worked out when somebody
+// asks for it; forces need no membership finer than the rows'.
+static int list_members(dsmd_ctx* c, cudaStream_t s) {
+    const int n_pairs = static_cast<int>(2 * c->n_quads);
+    DSMD_CUDA(c, cudaSetDevice(c->device));
+    DSMD_CUDA(c, cudaMemsetAsync(c->member_stats, 0, sizeof(unsigned long long) * 3, s));
+    k_list_members<false><<<blocks_for(n_pairs, kThreads), kThreads, 0, s>>>(
+        c->grid, n_pairs, static_cast<int>(c->n_owned), rows_of(c), c->ref[0], c->ref[1], c->ref[2], c->offsets64, c->member_stats,
+        nullptr, nullptr, nullptr, 0);
+    DSMD_LAUNCHED(c);
+    unsigned long long sums[3] = {0, 0, 0};
+    DSMD_CUDA(c, cudaMemcpyAsync(sums, c->member_stats, sizeof(sums), cudaMemcpyDeviceToHost, s));
+    DSMD_CUDA(c, cudaStreamSynchronize(s));
+    c->stat_entries = static_cast<int64_t>(sums[0]);
+    c->stat_interior = static_cast<int64_t>(sums[1]);
+    c->stat_rechecked = static_cast<int>(sums[2]);
+    c->stat_epoch = c->build_epoch;
+    return DSMD_OK;
+}
+
 int dsmd_list_stats(dsmd_ctx* c, int64_t* directed_entries, int64_t* interior_entries, int32_t* row_stride,
                     int32_t* cells, int32_t* rechecked) {
     if (!c) return DSMD_ERR_INVALID;
     if (!c->list_valid) return fail(c, DSMD_ERR_STATE, "no neighbour list");
+    if ((directed_entries || interior_entries || rechecked) && c->stat_epoch != c->build_epoch) {
+        const int rc = list_members(c, nullptr);
+        if (rc) return rc;
+    }
     if (directed_entries) *directed_entries = c->stat_entries;
     if (interior_entries) *interior_entries = c->stat_interior;
     if (row_stride) *row_stride = c->stride;
@@ -1656,42 +1344,42 @@ int dsmd_list_export(dsmd_ctx* c, int32_t* d_i, int32_t* d_j, uint8_t* d_flags, 
     if (!c || !n_pairs) return DSMD_ERR_INVALID;
     if (!c->list_valid) return fail(c, DSMD_ERR_STATE, "no neighbour list");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int n = static_cast<int>(c->n_owned);
+    const bool size_query = !d_i || !d_j;
+    if (!size_query || c->stat_epoch != c->build_epoch) {
+        const int rc = list_members(c, s);
+        if (rc) return rc;
+    }
     *n_pairs = c->stat_entries;
-    if (!d_i || !d_j || capacity < c->stat_entries) return DSMD_OK;   // size query
-    unsigned long long* scratch = nullptr;
-    DSMD_CUDA(c, cudaMalloc(&scratch, sizeof(unsigned long long) * n));
-    k_deg_to_u64<<<blocks_for(n, kThreads), kThreads, 0, s>>>(n, c->deg, scratch);
-    DSMD_LAUNCHED(c);
+    if (size_query || capacity < c->stat_entries) return DSMD_OK;
+    const int n = static_cast<int>(c->n_owned), n_row_pairs = static_cast<int>(2 * c->n_quads);
     size_t need = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, need, scratch, c->offsets64, n, s);
+    cub::DeviceScan::ExclusiveSum(nullptr, need, c->offsets64, c->offsets64, n, s);
     void* temp = nullptr;
     DSMD_CUDA(c, cudaMalloc(&temp, need));
-    DSMD_CUDA(c, cub::DeviceScan::ExclusiveSum(temp, need, scratch, c->offsets64, n, s));
-    k_list_export<<<blocks_for(n, kThreads), kThreads, 0, s>>>(n, c->nbr, c->stride, c->deg, c->offsets64, d_i, d_j,
-                                                              d_flags, capacity);
+    DSMD_CUDA(c, cub::DeviceScan::ExclusiveSum(temp, need, c->offsets64, c->offsets64, n, s));
+    k_list_members<true><<<blocks_for(n_row_pairs, kThreads), kThreads, 0, s>>>(
+        c->grid, n_row_pairs, n, rows_of(c), c->ref[0], c->ref[1], c->ref[2], c->offsets64, nullptr, d_i, d_j, d_flags, capacity);
     DSMD_LAUNCHED(c);
     DSMD_CUDA(c, cudaStreamSynchronize(s));
     cudaFree(temp);
-    cudaFree(scratch);
     return DSMD_OK;
 }
 
 // kick: 0.5 for the first velocity-Verlet half, 1.0 for the merged second-and-first half.
 static int pack_impl(dsmd_ctx* c, int64_t first, int64_t count, bool integrate, double dt, double f2a, cudaStream_t s,
-                     double kick = 0.5) {
+                     double kick = 0.5, const unsigned char* skip = nullptr) {
     if (count <= 0) return DSMD_OK;
     double** r = c->real[c->cur];
     if (integrate)
         k_pack<true><<<blocks_for(count, kThreads), kThreads, 0, s>>>(
             c->grid, static_cast<int>(first), static_cast<int>(count), static_cast<int>(c->n_owned), r[0], r[1], r[2],
             r[3], r[4], r[5], r[6], r[7], r[8], r[9], c->type[c->cur], c->ref[0], c->ref[1], c->ref[2], c->pq, dt,
-            kick * dt * f2a, c->status);
+            kick * dt * f2a, c->gid[c->cur], skip, c->status);
     else
         k_pack<false><<<blocks_for(count, kThreads), kThreads, 0, s>>>(
             c->grid, static_cast<int>(first), static_cast<int>(count), static_cast<int>(c->n_owned), r[0], r[1], r[2],
             r[3], r[4], r[5], r[6], r[7], r[8], r[9], c->type[c->cur], c->ref[0], c->ref[1], c->ref[2], c->pq, 0.0, 0.0,
-            c->status);
+            c->gid[c->cur], nullptr, c->status);
     DSMD_LAUNCHED(c);
     return DSMD_OK;
 }
@@ -1737,14 +1425,14 @@ int dsmd_max_displacement_sq_lagged(dsmd_ctx* c, double* out, void* stream) {
     return DSMD_OK;
 }
 
-// The pair kernel over the owned atoms first .. first + count of a FULL or INTERIOR pass without energy (count < 0: all
-// of them, any phase), or over the atoms with a ghost partner (BOUNDARY).
+// The pair kernel over the pair rows first .. first + count of a FULL or INTERIOR pass without energy (count < 0: all of
+// them, any phase), or over the pairs with a ghost partner (BOUNDARY).
 static int compute_forces_impl(dsmd_ctx* c, int phase, int want_energy, int64_t first, int64_t count, void* stream) {
     if (!c || phase < DSMD_PHASE_FULL || phase > DSMD_PHASE_BOUNDARY) return DSMD_ERR_INVALID;
     if (!c->list_valid) return fail(c, DSMD_ERR_STATE, "build the neighbour list before computing forces");
     const bool ranged = count >= 0;
-    if (ranged && (phase == DSMD_PHASE_BOUNDARY || want_energy || first < 0 || first + count > c->n_owned))
-        return fail(c, DSMD_ERR_INVALID, "a range of atoms is for FULL or INTERIOR passes without energy, inside the owned atoms");
+    if (ranged && (phase == DSMD_PHASE_BOUNDARY || want_energy || first < 0 || first + count > 2 * c->n_quads))
+        return fail(c, DSMD_ERR_INVALID, "a range of pair rows is for FULL or INTERIOR passes without energy");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     PairParams p{};
     for (int a = 0; a < 3; ++a) p.scale[a] = c->grid.scale[a];
@@ -1760,32 +1448,25 @@ static int compute_forces_impl(dsmd_ctx* c, int phase, int want_energy, int64_t 
     p.kq = static_cast<float>(kCoulomb);
     p.alpha = static_cast<float>(c->alpha);
     p.two_alpha_sqrtpi = static_cast<float>(2.0 * c->alpha / std::sqrt(3.14159265358979323846));
-    p.ntypes = c->ntypes;
     p.ewald_intervals = c->ewald_intervals;
-    p.c6c12 = c->c6c12;
+    p.ewald_most = std::nextafter(std::ldexp(kEwaldFirst, c->ewald_intervals >> dsmd::kEwaldBits), 0.0f);
     p.ewald = c->ewald;
+    p.ntypes = c->ntypes;
+    p.lj = c->lj;
     p.type_charge = c->coulomb ? c->type_charge : nullptr;
-    const bool multi = c->ntypes > 1;
-    // the boundary pass runs over the atoms the list build found a ghost partner for (none: nothing to launch)
-    const int64_t pair_threads = phase == DSMD_PHASE_BOUNDARY ? c->n_boundary : (ranged ? count : c->n_owned);
-    const int f0 = static_cast<int>(ranged ? first : 0), nt = static_cast<int>(pair_threads);
-    const int64_t blocks = blocks_for(pair_threads, kPairThreads);
-    if (want_energy) { const int rc = ensure_partials(c, std::max<int64_t>(blocks, 1)); if (rc) return rc; }
+    // the boundary pass runs over the pairs the list build found a ghost partner for (none: nothing to launch)
+    const int64_t pairs = phase == DSMD_PHASE_BOUNDARY ? c->n_boundary : (ranged ? count : 2 * c->n_quads);
     const bool e = want_energy != 0;
-    if (pair_threads == 0) {
-        // nothing to add to the forces; the energy sums of a boundary pass stay as the interior pass left them
-    } else if (c->coulomb) {
-        if (e) { if (multi) launch_pair<true, true, true>(c, p, phase, sw, s, f0, nt); else launch_pair<true, true, false>(c, p, phase, sw, s, f0, nt); }
-        else   { if (multi) launch_pair<true, false, true>(c, p, phase, sw, s, f0, nt); else launch_pair<true, false, false>(c, p, phase, sw, s, f0, nt); }
-    } else {
-        if (e) { if (multi) launch_pair<false, true, true>(c, p, phase, sw, s, f0, nt); else launch_pair<false, true, false>(c, p, phase, sw, s, f0, nt); }
-        else   { if (multi) launch_pair<false, false, true>(c, p, phase, sw, s, f0, nt); else launch_pair<false, false, false>(c, p, phase, sw, s, f0, nt); }
-    }
-    if (pair_threads > 0) DSMD_LAUNCHED(c);
-    if (e && (pair_threads > 0 || phase != DSMD_PHASE_BOUNDARY)) {
-        k_reduce_partials<6><<<1, kThreads, 0, s>>>(c->partials, static_cast<int>(blocks), c->scalars,
-                                                   phase == DSMD_PHASE_BOUNDARY ? 1 : 0);
-        DSMD_LAUNCHED(c);
+    if (e) { const int rc = ensure_partials(c, std::max<int64_t>(pair_blocks(c, pairs, true), 1)); if (rc) return rc; }
+    double** r = c->real[c->cur];
+    const ForceArgs a{c->pq, c->qf, rows_of(c), phase, phase == DSMD_PHASE_BOUNDARY ? c->boundary_pairs : nullptr,
+                      static_cast<int>(ranged ? first : 0), static_cast<int>(pairs), c->lane_shift, r[DSMD_FX], r[DSMD_FY], r[DSMD_FZ], c->partials,
+                      c->tickets, c->scalars};
+    if (pairs > 0) {   // else nothing to add to the forces; the energy sums of a boundary pass stay as the interior pass left them
+        const int copies = ewald_copies(c);
+        const int rc = copies == 0 ? launch_pair_types<0>(c, p, a, e, sw, s)
+                                   : (copies == 1 ? launch_pair_types<1>(c, p, a, e, sw, s) : launch_pair_types<kEwaldCopiesMost>(c, p, a, e, sw, s));
+        if (rc) return rc;
     }
     return DSMD_OK;
 }
@@ -1808,11 +1489,10 @@ namespace {
 ClusterTable cluster_table(const dsmd_ctx* c) {
     ClusterTable t{};
     t.n_clusters = c->n_clusters;
-    t.atom_gid = c->cl_gid;
+    t.atom_slot = c->cl_slot;
     t.con_a = c->cl_a;
     t.con_b = c->cl_b;
     t.con_d2 = c->cl_d2;
-    t.slot_of_gid = c->slot_of_gid;
     for (int a = 0; a < 3; ++a) {
         t.box[a] = c->box[a];
         t.periodic[a] = c->periodic[a];
@@ -1820,44 +1500,56 @@ ClusterTable cluster_table(const dsmd_ctx* c) {
     return t;
 }
 
+// Where the clusters' atoms are since the last sort.
 int ensure_slot_map(dsmd_ctx* c, cudaStream_t s) {
     if (c->slot_map_valid) return DSMD_OK;
     k_slot_of_gid<<<blocks_for(c->n_owned, kThreads), kThreads, 0, s>>>(static_cast<int>(c->n_owned), c->gid[c->cur],
                                                                          static_cast<int>(c->cons_n_global), c->slot_of_gid);
     DSMD_LAUNCHED(c);
+    const int n = c->n_clusters * kClusterAtoms;
+    k_cluster_slots<<<blocks_for(n, kThreads), kThreads, 0, s>>>(n, c->cl_gid, c->slot_of_gid, c->cl_slot);
+    DSMD_LAUNCHED(c);
     c->slot_map_valid = true;
     return DSMD_OK;
 }
 
-// SHAKE after the drift of the first half step (positions before it are in c->pre), then the positions the kernels
-// read are converted again.
-int shake_impl(dsmd_ctx* c, double dt, cudaStream_t s) {
-    { const int rc = ensure_slot_map(c, s); if (rc) return rc; }
+int launch_constrained(dsmd_ctx* c, bool finish, bool start, double half_kick, double dt, double prefactor, double* d_virial3, cudaStream_t s) {
     double** r = c->real[c->cur];
-    k_shake<<<blocks_for(c->n_clusters, 128), 128, 0, s>>>(cluster_table(c), r[0], r[1], r[2], r[3], r[4], r[5], c->pre[0],
-                                                            c->pre[1], c->pre[2], r[9], 1.0 / dt, c->cons_tolerance,
-                                                            c->cons_max_iterations, &c->status->constraint_failed);
+    const AtomArrays at{r[0], r[1], r[2], r[3], r[4], r[5], r[6], r[7], r[8], r[9], c->type[c->cur], c->ref[0], c->ref[1], c->ref[2], c->pq};
+    const unsigned blocks = blocks_for(c->n_clusters, 128);
+    const auto launch = [&](auto shape) {
+        const auto kernel = finish && start ? k_constrained<decltype(shape), true, true>
+                                            : (finish ? k_constrained<decltype(shape), true, false> : k_constrained<decltype(shape), false, true>);
+        kernel<<<blocks, 128, 0, s>>>(cluster_table(c), c->grid, at, half_kick, dt, c->cons_tolerance, c->cons_max_iterations, prefactor,
+                                      c->partials, c->tickets + 3, d_virial3, c->status);
+    };
+    if (c->cl_shape == 1) launch(TriangleCluster());
+    else if (c->cl_shape == 2) launch(BondCluster());
+    else launch(AnyCluster());
+    DSMD_LAUNCHED(c);
+    return DSMD_OK;
+}
+
+// The velocity-Verlet halves of a system with constraints: the second half of a step with RATTLE (finish), the first half
+// with SHAKE (start), or both in one pass (a second half and the first half of the next step, the same forces).
+int constrained_halves(dsmd_ctx* c, bool finish, bool start, double dt, double f2a, cudaStream_t s) {
+    { const int rc = ensure_slot_map(c, s); if (rc) return rc; }
+    const double half_kick = 0.5 * dt * f2a;
+    const int rc = launch_constrained(c, finish, start, half_kick, dt, 0.0, nullptr, s);
+    if (rc || c->cl_cover_all) return rc;
+    // the free atoms
+    if (start) return pack_impl(c, 0, c->n_owned, true, dt, f2a, s, finish ? 1.0 : 0.5, c->cl_member);
+    double** r = c->real[c->cur];
+    k_vv2<<<blocks_for(c->n_owned, kThreads), kThreads, 0, s>>>(static_cast<int>(c->n_owned), half_kick, r[3], r[4], r[5], r[6], r[7], r[8],
+                                                               r[9], c->gid[c->cur], c->cl_member);
     DSMD_LAUNCHED(c);
     return DSMD_OK;
 }
 
 int rattle_impl(dsmd_ctx* c, double dt, double f2a, double* d_virial3, cudaStream_t s) {
     { const int rc = ensure_slot_map(c, s); if (rc) return rc; }
-    double** r = c->real[c->cur];
-    const unsigned blocks = blocks_for(c->n_clusters, 128);
-    double* partials = nullptr;
-    if (d_virial3) {
-        { const int rc = ensure_partials(c, blocks); if (rc) return rc; }
-        partials = c->partials;
-    }
-    k_rattle<<<blocks, 128, 0, s>>>(cluster_table(c), r[0], r[1], r[2], r[3], r[4], r[5], r[9], c->cons_tolerance,
-                                    c->cons_max_iterations, -2.0 / (f2a * dt), partials, &c->status->constraint_failed);
-    DSMD_LAUNCHED(c);
-    if (d_virial3) {
-        k_reduce_partials<3><<<1, kThreads, 0, s>>>(partials, static_cast<int>(blocks), d_virial3, 0);
-        DSMD_LAUNCHED(c);
-    }
-    return DSMD_OK;
+    if (d_virial3) { const int rc = ensure_partials(c, blocks_for(c->n_clusters, 128)); if (rc) return rc; }
+    return launch_constrained(c, true, false, 0.0, dt, -2.0 / (f2a * dt), d_virial3, s);
 }
 
 }  // namespace
@@ -1867,8 +1559,9 @@ int dsmd_set_constraints(dsmd_ctx* c, int64_t n_global, int64_t n_constraints, c
     if (!c || n_global < 0 || n_constraints < 0 || (n_constraints > 0 && (!a || !b || !distance))) return DSMD_ERR_INVALID;
     DSMD_CUDA(c, cudaSetDevice(c->device));
     cudaFree(c->cl_gid); cudaFree(c->cl_a); cudaFree(c->cl_b); cudaFree(c->cl_d2); cudaFree(c->slot_of_gid);
-    c->cl_gid = c->slot_of_gid = nullptr;
-    c->cl_a = c->cl_b = nullptr;
+    cudaFree(c->cl_slot); cudaFree(c->cl_member);
+    c->cl_gid = c->slot_of_gid = c->cl_slot = nullptr;
+    c->cl_a = c->cl_b = c->cl_member = nullptr;
     c->cl_d2 = nullptr;
     c->n_clusters = 0;
     c->slot_map_valid = false;
@@ -1934,8 +1627,23 @@ int dsmd_set_constraints(dsmd_ctx* c, int64_t n_global, int64_t n_constraints, c
     DSMD_CUDA(c, cudaMemcpy(c->cl_a, ca.data(), ca.size(), cudaMemcpyHostToDevice));
     DSMD_CUDA(c, cudaMemcpy(c->cl_b, cb.data(), cb.size(), cudaMemcpyHostToDevice));
     DSMD_CUDA(c, cudaMemcpy(c->cl_d2, d2.data(), sizeof(double) * d2.size(), cudaMemcpyHostToDevice));
-    for (int ax = 0; ax < 3; ++ax)
-        if (!c->pre[ax]) DSMD_CUDA(c, cudaMalloc(&c->pre[ax], sizeof(double) * c->capacity));
+    DSMD_CUDA(c, cudaMalloc(&c->cl_slot, sizeof(int) * gids.size()));
+    std::vector<unsigned char> member(static_cast<size_t>(n_global), 0);
+    for (int g : gids)
+        if (g >= 0) member[static_cast<size_t>(g)] = 1;
+    c->cl_cover_all = std::find(member.begin(), member.end(), 0) == member.end();
+    DSMD_CUDA(c, cudaMalloc(&c->cl_member, member.size()));
+    DSMD_CUDA(c, cudaMemcpy(c->cl_member, member.data(), member.size(), cudaMemcpyHostToDevice));
+    // one shape for all: compiled with the constraint order known
+    const auto all_are = [&](auto shape) {
+        for (size_t k = 0; k < ncl; ++k) {
+            if (n_atoms[k] != shape.atoms || n_cons[k] != shape.constraints) return false;
+            for (int j = 0; j < shape.constraints; ++j)
+                if (ca[k * kClusterCons + j] != shape.a(j) || cb[k * kClusterCons + j] != shape.b(j)) return false;
+        }
+        return true;
+    };
+    c->cl_shape = all_are(TriangleCluster()) ? 1 : (all_are(BondCluster()) ? 2 : 0);
     c->n_clusters = static_cast<int>(ncl);
     c->cons_n_global = n_global;
     return DSMD_OK;
@@ -1967,20 +1675,12 @@ int dsmd_integrate(dsmd_ctx* c, int half, double dt, double f2a, void* stream) {
         if (constrained) return fail(c, DSMD_ERR_STATE, "the merged half steps are not available with constraints");
         return pack_impl(c, 0, c->n_owned, true, dt, f2a, s, 1.0);
     }
-    if (half == 1) {
-        if (!constrained) return pack_impl(c, 0, c->n_owned, true, dt, f2a, s);
-        // constrained: keep the positions from before the drift, drift, SHAKE, then convert the corrected positions
-        for (int a = 0; a < 3; ++a)
-            DSMD_CUDA(c, cudaMemcpyAsync(c->pre[a], c->real[c->cur][a], sizeof(double) * c->n_owned, cudaMemcpyDeviceToDevice, s));
-        { const int rc = pack_impl(c, 0, c->n_owned, true, dt, f2a, s); if (rc) return rc; }
-        { const int rc = shake_impl(c, dt, s); if (rc) return rc; }
-        return pack_impl(c, 0, c->n_owned, false, 0.0, 0.0, s);
-    }
+    if (constrained) return constrained_halves(c, half == 2, half == 1, dt, f2a, s);
+    if (half == 1) return pack_impl(c, 0, c->n_owned, true, dt, f2a, s);
     double** r = c->real[c->cur];
     k_vv2<<<blocks_for(c->n_owned, kThreads), kThreads, 0, s>>>(static_cast<int>(c->n_owned), 0.5 * dt * f2a, r[3], r[4],
-                                                               r[5], r[6], r[7], r[8], r[9]);
+                                                               r[5], r[6], r[7], r[8], r[9], c->gid[c->cur], nullptr);
     DSMD_LAUNCHED(c);
-    if (constrained) return rattle_impl(c, dt, f2a, nullptr, s);
     return DSMD_OK;
 }
 
@@ -2122,13 +1822,12 @@ int dsmd_compute_bonded(dsmd_ctx* c, void* stream) {
     t.n_owned = static_cast<int>(c->n_owned);
     for (int a = 0; a < 3; ++a) { t.box[a] = c->box[a]; t.periodic[a] = c->periodic[a]; }
     double** r = c->real[c->cur];
-    k_bonded_terms<<<static_cast<unsigned>(b.blocks), kThreads, 0, s>>>(t, r[0], r[1], r[2], r[10], b.contrib, b.partials, b.missing);
+    k_bonded_terms<<<static_cast<unsigned>(b.blocks), kThreads, 0, s>>>(t, r[0], r[1], r[2], r[10], b.contrib, b.partials,
+                                                                        c->tickets + 2, b.scalars, b.missing);
     DSMD_LAUNCHED(c);
     k_bonded_gather<<<blocks_for(c->n_owned, kThreads), kThreads, 0, s>>>(static_cast<int>(c->n_owned), c->gid[c->cur],
                                                                          static_cast<int>(b.n_global), b.entries_of, b.entry,
                                                                          b.contrib, r[6], r[7], r[8]);
-    DSMD_LAUNCHED(c);
-    k_reduce_partials<5><<<1, kThreads, 0, s>>>(b.partials, static_cast<int>(b.blocks), b.scalars, 0);
     DSMD_LAUNCHED(c);
     return DSMD_OK;
 }
@@ -2154,13 +1853,11 @@ int dsmd_read_bonded_scalars(dsmd_ctx* c, double out[5], void* stream) {
 int dsmd_kinetic_energy(dsmd_ctx* c, double* out, void* stream) {
     if (!c || !out) return DSMD_ERR_INVALID;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int64_t blocks = blocks_for(c->n_owned, kThreads);
+    const int64_t blocks = std::min<int64_t>(blocks_for(c->n_owned, kThreads), kDeviceSms * 8);
     { const int rc = ensure_partials(c, blocks); if (rc) return rc; }
     double** r = c->real[c->cur];
     k_kinetic<<<static_cast<unsigned>(blocks), kThreads, 0, s>>>(static_cast<int>(c->n_owned), r[3], r[4], r[5], r[9],
-                                                                 c->partials);
-    DSMD_LAUNCHED(c);
-    k_reduce_partials<1><<<1, kThreads, 0, s>>>(c->partials, static_cast<int>(blocks), c->scalars + 6, 0);
+                                                                 c->partials, c->tickets + 1, c->scalars + 6);
     DSMD_LAUNCHED(c);
     DSMD_CUDA(c, cudaMemcpyAsync(c->h_scalars + 6, c->scalars + 6, sizeof(double), cudaMemcpyDeviceToHost, s));
     DSMD_CUDA(c, cudaStreamSynchronize(s));
@@ -2200,10 +1897,14 @@ int dsmd_run_nve(dsmd_ctx* c, int64_t n_steps, double dt, double f2a, double hi_
     int pending = -1;                      // read-back slot in flight
     auto bits_to_double = [](unsigned long long b) { double v; std::memcpy(&v, &b, sizeof(v)); return v; };
     // Between two steps of this loop nobody reads the velocities, so the second half of one step and the first half of the
-    // next (the same forces) are one pass over the atoms; with constraints RATTLE sits between them and they stay apart.
-    const bool merge = c->n_clusters == 0;
+    // next (the same forces) are one pass over the atoms, with RATTLE between them where there are constraints.
+    const bool constrained = c->n_clusters > 0;
     for (int64_t step = 0; step < n_steps; ++step) {
-        { const int rc = dsmd_integrate(c, merge && step > 0 ? 3 : 1, dt, f2a, s); if (rc) return rc; }   // with SHAKE when constraints are set
+        {
+            const int rc = constrained && step > 0 ? constrained_halves(c, true, true, dt, f2a, s)
+                                                   : dsmd_integrate(c, step > 0 ? 3 : 1, dt, f2a, s);
+            if (rc) return rc;
+        }
         ++since_build;
         bool rebuild = every > 0 && since_build >= every;
         if (!lagged) {
@@ -2240,7 +1941,7 @@ int dsmd_run_nve(dsmd_ctx* c, int64_t n_steps, double dt, double f2a, double hi_
         }
         { const int rc = dsmd_compute_forces(c, DSMD_PHASE_FULL, 0, s); if (rc) return rc; }
         { const int rc = dsmd_compute_bonded(c, s); if (rc) return rc; }
-        if (!merge || step + 1 == n_steps) { const int rc = dsmd_integrate(c, 2, dt, f2a, s); if (rc) return rc; }
+        if (step + 1 == n_steps) { const int rc = dsmd_integrate(c, 2, dt, f2a, s); if (rc) return rc; }
     }
     if (lagged && pending >= 0) {
         DSMD_CUDA(c, cudaEventSynchronize(c->disp_event[pending]));
@@ -2301,7 +2002,12 @@ static int forces_host_pipelined(dsmd_ctx* c, const double* x, const double* y, 
         const int64_t first = begin[k], count = begin[k + 1] - begin[k];
         const int needs[3] = {(k + pieces - 1) % pieces, k, (k + 1) % pieces};
         for (int q = 0; q < 3; ++q) DSMD_CUDA(c, cudaStreamWaitEvent(s, c->piece_up[needs[q]], 0));
-        if (count > 0) { const int rc = compute_forces_impl(c, DSMD_PHASE_FULL, 0, first, count, s); if (rc) return rc; }
+        // the pair rows of the slab: its first cell row's number fixes the first of them
+        const int row_lo = static_cast<int>(static_cast<int64_t>(layers) * k / pieces) * c->grid.nc[1];
+        const int row_hi = static_cast<int>(static_cast<int64_t>(layers) * (k + 1) / pieces) * c->grid.nc[1];
+        const int64_t pair_lo = k == 0 ? 0 : 2ll * quad_base(static_cast<int>(first), row_lo);
+        const int64_t pair_hi = 2ll * quad_base(static_cast<int>(first + count), row_hi);
+        if (count > 0) { const int rc = compute_forces_impl(c, DSMD_PHASE_FULL, 0, pair_lo, pair_hi - pair_lo, s); if (rc) return rc; }
         DSMD_CUDA(c, cudaEventRecord(c->piece_done[k], s));
         DSMD_CUDA(c, cudaStreamWaitEvent(c->copy_out, c->piece_done[k], 0));
         for (int a = 0; a < 3 && count > 0; ++a)

@@ -1,0 +1,443 @@
+// LJ + real-space Ewald over the pair rows of dsmd_rows.cuh. Included by dsmd_core.cu.
+#pragma once
+
+namespace {
+
+struct PairParams {
+    float scale[3];
+    float rc2;
+    float rs2, inv_denom;        // CHARMM switch on r^2 (rs2 < 0: off)
+    float kq;                    // Coulomb constant
+    float alpha, two_alpha_sqrtpi;
+    int ntypes;
+    int ewald_intervals;
+    float ewald_most;            // largest r^2 looked up: the last float inside the last interval
+    const float2* lj;            // [ntypes * ntypes] {12 c12, -6 c6}
+    const float4* ewald;         // [2 * intervals]: force cubic, energy cubic
+    const float* type_charge;    // [ntypes] when every atom's charge is that of its type (dsmd_set_type_charges), else null
+};
+
+// 1 / v: the hardware approximation (1 ulp) for the force-only kernels, one Newton step more (full single precision)
+// where energy and virial sums are taken.
+template <bool REFINE>
+__device__ __forceinline__ float reciprocal(float v) {
+    const float r = rcp_approx(v);
+    return REFINE ? fmaf(r, fmaf(-v, r, 1.0f), r) : r;
+}
+
+// Pair parameters by type. kOneType: constants. kFewTypes: a table over (type of the first atom, type of the second, type
+// of the partner) that holds what both atoms need side by side - up to 8 types, 16 KB. kManyTypes: a table over two types,
+// read once per atom.
+enum { kOneType = 0, kFewTypes = 1, kManyTypes = 2 };
+constexpr int kFewTypesMost = 8;
+
+// The real-space Ewald functions of r^2 as cubics on intervals of constant relative width (ewald_table.hpp). For rows of
+// hundreds of entries the table lies in shared memory eight times over, copy c in the 16-byte bank group c, and a lane reads
+// the copy of its place in its group of eight: a look-up by 32 lanes is 4 wavefronts whatever the intervals (8 to 11 with one
+// copy). For short rows, where laying the table out (36 KB at a cutoff of 10 A) would be most of the work, one copy.
+constexpr int kEwaldCopiesMost = 8;
+
+constexpr float kEwaldFirst = 0.5f;   // r^2 at which the table starts
+
+template <int COPIES>
+struct EwaldTable {
+    const float4* mine;   // this lane's copy of interval 0
+    int intervals;
+};
+
+__device__ __forceinline__ float ewald_cubic(const float4* at, float t) {
+    const float4 c = *at;   // coefficients of 32 t: powers of two, the same roundings
+    return ((c.w * t + c.z) * t + c.y) * t + c.x;
+}
+
+template <bool ENERGY, int COPIES>
+__device__ __forceinline__ void ewald_functions(const EwaldTable<COPIES>& table, float r2, float most, float& ff, float& ef) {
+    // the interval and the place in it (1 / 32 octave: the low 18 bits of the mantissa); beyond the cutoff the last one,
+    // below the table (the caller deals with that) the first one
+    const unsigned bits = __float_as_uint(fmaxf(fminf(r2, most), kEwaldFirst));
+    const unsigned idx = (bits - dsmd::kEwaldBaseBits) >> dsmd::kEwaldIndexShift;
+    const float t = __uint_as_float(0x3F800000u | (bits & ((1u << dsmd::kEwaldIndexShift) - 1u))) - 1.0f;
+    ff = ewald_cubic(table.mine + idx * COPIES, t);
+    if (ENERGY) ef = ewald_cubic(table.mine + (table.intervals + idx) * COPIES, t);
+}
+
+// What one evaluation needs to know of the two pairs.
+struct PairTerms {
+    F2 rep, att;   // 12 c12, -6 c6
+    F2 qq;         // Coulomb constant times the charges
+};
+
+// Sums of the two atoms of a pair row.
+//
+// What bounds the force kernel: the dispatch port, at which a packed instruction (two lanes: the two atoms) counts twice, and
+// beside it the L1 unit (13 wavefronts per gather of 32 partners). So what counts is the number of scalar operations: about
+// 55 per entry (two pairs) for Lennard-Jones, 75 with Ewald. The plain form below therefore leaves out what no pair of a sane
+// system needs and keeps the smallest r^2 for a look afterwards.
+template <int COPIES, bool ENERGY, bool SWITCH>
+struct PairAccumulator {
+    static constexpr bool COULOMB = COPIES > 0;
+    F2 ax{0}, ay{0}, az{0};
+    F2 e_sum{0}, w_sum{0}, wx{0}, wy{0}, wz{0};
+    float least = 3.0e38f;   // smallest r^2 seen
+    int n_in = 0;
+
+    // Forces of the two atoms out, and the sums back to zero.
+    __device__ __forceinline__ void take_forces(float (&a)[3], float (&b)[3]) {
+        parts(ax, a[0], b[0]);
+        parts(ay, a[1], b[1]);
+        parts(az, a[2], b[2]);
+        ax = ay = az = F2{0};
+    }
+
+    // Half of the energy sums (every pair is listed from both sides) added to v, and back to zero.
+    __device__ __forceinline__ void take_energies(bool both_lanes, double (&v)[6]) {
+        const F2 sums[5] = {e_sum, w_sum, wx, wy, wz};
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+            float a, b;
+            parts(sums[k], a, b);
+            v[k] += 0.5 * (static_cast<double>(a) + (both_lanes ? static_cast<double>(b) : 0.0));
+        }
+        v[5] += (both_lanes ? 0.5 : 0.25) * static_cast<double>(n_in);
+        e_sum = w_sum = wx = wy = wz = F2{0};
+        n_in = 0;
+    }
+
+    // Pair terms at the distances r2 of the two pairs: force over distance and energy. CAREFUL: Ewald functions below their
+    // table, excluded pairs (Lennard-Jones off; the pair's 1/r is not part of the Ewald sum: erfc -> -erf).
+    template <bool CAREFUL>
+    __device__ __forceinline__ void evaluate(const PairParams& p, const EwaldTable<COPIES>& table, const PairTerms& k, F2 r2, float ra, float rb,
+                                             bool ex_a, bool ex_b, F2& f, F2& u) {
+        const F2 r2inv = f2(reciprocal<ENERGY>(ra), reciprocal<ENERGY>(rb));
+        const F2 r6 = mul(mul(r2inv, r2inv), r2inv);
+        f = mul(mul(r2inv, r6), fma(k.rep, r6, k.att));
+        u = F2{0};
+        if (ENERGY || SWITCH) u = mul(r6, fma(mul(k.rep, both(1.0f / 12.0f)), r6, mul(k.att, both(1.0f / 6.0f))));
+        if (SWITCH) {
+            // smooth for r^2 > rs2: f -> sw f + 12 u a (r^2 - rs2) / denom, u -> sw u (a = rc2 - r^2)
+            const F2 a = fma(r2, both(-1.0f), both(p.rc2));
+            const F2 above = add(r2, both(-p.rs2));
+            const F2 aw = mul(a, both(p.inv_denom));
+            const F2 b = fma(r2, both(2.0f), both(p.rc2 - 3.0f * p.rs2));
+            float swa, swb, da, db;
+            parts(mul(mul(a, b), aw), swa, swb);
+            parts(mul(mul(mul(u, both(12.0f)), aw), above), da, db);
+            const bool s_a = ra > p.rs2, s_b = rb > p.rs2;
+            const F2 factor = f2(s_a ? swa : 1.0f, s_b ? swb : 1.0f);
+            f = fma(factor, f, f2(s_a ? da : 0.0f, s_b ? db : 0.0f));
+            u = mul(u, factor);
+        }
+        if (CAREFUL) {
+            float va, vb;
+            parts(f, va, vb);
+            f = f2(ex_a ? 0.0f : va, ex_b ? 0.0f : vb);
+            parts(u, va, vb);
+            u = f2(ex_a ? 0.0f : va, ex_b ? 0.0f : vb);
+        }
+        if (COULOMB) {
+            float ffa, ffb, efa = 0.0f, efb = 0.0f;
+            ewald_functions<ENERGY>(table, ra, p.ewald_most, ffa, efa);
+            ewald_functions<ENERGY>(table, rb, p.ewald_most, ffb, efb);
+            if (CAREFUL) {
+                const auto analytic = [&](float r2_, float& ff, float& ef) {
+                    const float r = sqrtf(r2_), ar = p.alpha * r, ec = erfcf(ar) / r;
+                    ff = (ec + p.two_alpha_sqrtpi * __expf(-ar * ar)) / r2_;
+                    ef = ec;
+                };
+                if (ra < kEwaldFirst) analytic(ra, ffa, efa);
+                if (rb < kEwaldFirst) analytic(rb, ffb, efb);
+                const float ia = rsqrtf(ra), ib = rsqrtf(rb);
+                if (ex_a) { ffa -= ia * ia * ia; efa -= ia; }
+                if (ex_b) { ffb -= ib * ib * ib; efb -= ib; }
+            }
+            f = fma(k.qq, f2(ffa, ffb), f);
+            if (ENERGY) u = fma(k.qq, f2(efa, efb), u);
+        }
+    }
+
+    __device__ __forceinline__ void sum(F2 dx, F2 dy, F2 dz, F2 r2, F2 f, F2 u, bool in_a, bool in_b) {
+        float va, vb;
+        parts(f, va, vb);
+        f = f2(in_a ? va : 0.0f, in_b ? vb : 0.0f);
+        ax = fma(f, dx, ax);
+        ay = fma(f, dy, ay);
+        az = fma(f, dz, az);
+        if (ENERGY) {
+            parts(u, va, vb);
+            e_sum = add(e_sum, f2(in_a ? va : 0.0f, in_b ? vb : 0.0f));
+            w_sum = fma(f, r2, w_sum);
+            wx = fma(mul(f, dx), dx, wx);
+            wy = fma(mul(f, dy), dy, wy);
+            wz = fma(mul(f, dz), dz, wz);
+            n_in += (in_a ? 1 : 0) + (in_b ? 1 : 0);
+        }
+    }
+
+    // One entry, seen from the two atoms at pa and pb (fixed-point positions: the 32-bit difference is the nearest image).
+    // The plain form takes every pair inside the cutoff; CAREFUL also tells pairs that coincide (r^2 < 1e-10: no force) and
+    // those named above.
+    template <bool CAREFUL>
+    __device__ __forceinline__ void add_partner(const PairParams& p, const EwaldTable<COPIES>& table, const int4& pa, const int4& pb,
+                                                const int4& pj, const PairTerms& k, unsigned entry) {
+        const F2 dx = mul(f2(static_cast<float>(pa.x - pj.x), static_cast<float>(pb.x - pj.x)), both(p.scale[0]));
+        const F2 dy = mul(f2(static_cast<float>(pa.y - pj.y), static_cast<float>(pb.y - pj.y)), both(p.scale[1]));
+        const F2 dz = mul(f2(static_cast<float>(pa.z - pj.z), static_cast<float>(pb.z - pj.z)), both(p.scale[2]));
+        const F2 r2 = fma(dz, dz, fma(dy, dy, mul(dx, dx)));
+        float ra, rb;
+        parts(r2, ra, rb);
+        F2 f, u;
+        evaluate<CAREFUL>(p, table, k, r2, ra, rb, CAREFUL && (entry & kExclFirst) != 0u, CAREFUL && (entry & kExclSecond) != 0u, f, u);
+        if (CAREFUL) {
+            sum(dx, dy, dz, r2, f, u, ra < p.rc2 && ra >= 1e-10f, rb < p.rc2 && rb >= 1e-10f);
+        } else {
+            asm("min.f32 %0, %0, %1, %2;" : "+f"(least) : "f"(ra), "f"(rb));
+            sum(dx, dy, dz, r2, f, u, ra < p.rc2, rb < p.rc2);
+        }
+    }
+};
+
+struct ForceArgs {
+    const int4* pq;
+    const float* qf;
+    RowArrays rows;
+    int phase;
+    const int* pair_list;    // the pairs to work on (boundary pass), or null: first_pair ...
+    int first_pair, n_pairs; // ... first_pair + n_pairs
+    int lane_shift;          // log2 of the lanes that share one row
+    double *fx, *fy, *fz;
+    double* partials;        // energy sums: per block, a count of finished blocks, and the total
+    unsigned* ticket;
+    double* scalars;
+};
+
+// Threads per block and blocks per SM, which fix the registers and with them how the compiler interleaves the partners of a
+// chunk; measured on a B200, the best of five to nine settings each. Long rows with Ewald: one block per SM, 118 registers
+// (1.08 to 1.12 ms per pass over 648,000 water atoms; 1.12 to 1.45 ms with two to six smaller blocks). One type: 64
+// registers, 0.427 ms at 4,000,000 Lennard-Jones atoms (0.44 to 0.56 ms at other settings; a row per atom took 0.498 ms).
+// Types by table: 80 registers, 0.177 ms for the 1,048,576-atom mixture (0.18 to 0.23 ms; a row per atom 0.213 ms).
+template <int COPIES, int TYPES>
+constexpr int kPairThreads = COPIES == kEwaldCopiesMost ? 384 : (COPIES == 0 && TYPES == kOneType ? 64 : 128);
+template <int COPIES, int TYPES, bool ENERGY>
+constexpr int kPairBlocks = ENERGY || COPIES == kEwaldCopiesMost ? 1 : (COPIES > 0 ? 5 : (TYPES == kOneType ? 16 : 6));
+
+// Tables in shared memory: Ewald cubics and pair parameters by type. Every thread of the block calls it once.
+template <int COPIES, bool ENERGY, int TYPES, bool QTYPE>
+struct PairTables {
+    static constexpr bool COULOMB = COPIES > 0;
+    static constexpr bool few = TYPES == kFewTypes, many = TYPES == kManyTypes, by_type = COULOMB && QTYPE;
+    static constexpr int functions = ENERGY ? 2 : 1;
+    EwaldTable<COPIES> ewald;
+    const ulonglong2* lj3;             // few: {rep, att} of both atoms by (type, type, partner's type)
+    const unsigned long long* qq3;     // few, by_type: charges likewise
+    const float2* lj2;                 // many
+    const float* charge;               // by_type && !few
+
+    __host__ __device__ static size_t bytes(int nt, int intervals) {
+        size_t n = COULOMB ? sizeof(float4) * COPIES * functions * intervals : 0;
+        if (few) n += static_cast<size_t>(nt) * nt * nt * (by_type ? 24 : 16);
+        if (many) n += static_cast<size_t>(nt) * nt * sizeof(float2);
+        if (by_type && !few) n += nt * sizeof(float);
+        return n;
+    }
+
+    __device__ __forceinline__ PairTables(const PairParams& p, float4* smem) {
+        const int nt = p.ntypes;
+        float4* s_ewald = smem;
+        ulonglong2* s_lj3 = reinterpret_cast<ulonglong2*>(s_ewald + (COULOMB ? functions * p.ewald_intervals * COPIES : 0));
+        unsigned long long* s_qq3 = reinterpret_cast<unsigned long long*>(s_lj3 + (few ? nt * nt * nt : 0));
+        float2* s_lj2 = reinterpret_cast<float2*>(s_qq3 + (few && by_type ? nt * nt * nt : 0));
+        float* s_charge = reinterpret_cast<float*>(s_lj2 + (many ? nt * nt : 0));
+        if (COULOMB)
+            for (int k = threadIdx.x; k < functions * p.ewald_intervals * COPIES; k += blockDim.x) {
+                const int entry = k / (COULOMB ? COPIES : 1);
+                const float4 v = p.ewald[entry < p.ewald_intervals ? 2 * entry : 2 * (entry - p.ewald_intervals) + 1];
+                s_ewald[k] = make_float4(v.x, v.y * 32.0f, v.z * 1024.0f, v.w * 32768.0f);
+            }
+        if (few)
+            for (int k = threadIdx.x; k < nt * nt * nt; k += blockDim.x) {
+                const int tj = k % nt, tb = (k / nt) % nt, ta = k / (nt * nt);
+                const float2 la = p.lj[ta * nt + tj], lb = p.lj[tb * nt + tj];
+                s_lj3[k] = make_ulonglong2(f2(la.x, lb.x).v, f2(la.y, lb.y).v);
+                if (by_type) {
+                    const float qj = p.type_charge[tj];
+                    s_qq3[k] = f2(p.kq * p.type_charge[ta] * qj, p.kq * p.type_charge[tb] * qj).v;
+                }
+            }
+        if (many)
+            for (int k = threadIdx.x; k < nt * nt; k += blockDim.x) s_lj2[k] = p.lj[k];
+        if (by_type && !few)
+            for (int k = threadIdx.x; k < nt; k += blockDim.x) s_charge[k] = p.type_charge[k];
+        if (COULOMB || TYPES != kOneType) __syncthreads();
+        ewald = EwaldTable<COPIES>{s_ewald + (threadIdx.x & (COPIES - 1)), p.ewald_intervals};
+        lj3 = s_lj3;
+        qq3 = s_qq3;
+        lj2 = s_lj2;
+        charge = s_charge;
+    }
+};
+
+// Forces on the atoms of one pair row, worked on by `lanes` lanes of a warp, which take the row's chunks of four entries in
+// turn; this lane's share of the sums. The next chunk of entries and the partners of the current one are in flight before
+// any arithmetic starts; the list is streamed with an evict-first hint so that the positions stay in L2.
+// Every listed pair is evaluated from the side of each of its owned atoms (a full list), so forces need no scatter and no
+// atomics and the order of the sums is fixed (bitwise reproducible). Energy and virial take half of every directed entry;
+// an owned-ghost pair is then counted half on each rank, as the reference's list kernel does
+// (src/force_calculator_cuda.cu:1784-1789).
+template <int COPIES, bool ENERGY, int TYPES, bool SWITCH, bool QTYPE>
+__device__ __forceinline__ void row_forces(const PairParams& p, const ForceArgs& a, const PairTables<COPIES, ENERGY, TYPES, QTYPE>& tables,
+                                           int pair, int sub, int lanes, int first, int atoms, float (&sum_a)[3], float (&sum_b)[3],
+                                           double (&v)[6]) {
+    constexpr bool COULOMB = COPIES > 0, few = TYPES == kFewTypes, many = TYPES == kManyTypes, by_type = COULOMB && QTYPE;
+    const int nt = p.ntypes;
+    const EwaldTable<COPIES>& table = tables.ewald;
+    PairAccumulator<COPIES, ENERGY, SWITCH> acc;
+    if (atoms > 0) {
+        const int4 pa = a.pq[first], pb = a.pq[first + atoms - 1];
+        const int mid = a.rows.row_int[pair], end = a.rows.row_end[pair];
+        const unsigned special = a.rows.row_special[pair];
+        const unsigned* words = a.rows.rows + row_base(static_cast<unsigned>(pair), a.rows.stride);
+        const uint4* row = reinterpret_cast<const uint4*>(words);
+        F2 q{0};
+        PairTerms one{};
+        const int row3 = (pa.w * nt + pb.w) * nt;
+        if (COULOMB && !(few && by_type))
+            q = mul(both(p.kq), by_type ? f2(tables.charge[pa.w], tables.charge[pb.w]) : f2(a.qf[first], a.qf[first + atoms - 1]));
+        if (TYPES == kOneType) {
+            const float2 lj = p.lj[0];
+            one.rep = both(lj.x);
+            one.att = both(lj.y);
+            if (by_type) one.qq = mul(q, both(tables.charge[0]));
+        }
+        const auto take = [&](unsigned e, int4& pos, float& charge) {
+            pos = __ldg(&a.pq[e]);
+            if (COULOMB && !by_type) charge = __ldg(&a.qf[e]);
+        };
+        const auto terms = [&](int type, float charge) {
+            PairTerms k = one;
+            if (few) {
+                const ulonglong2 lj = tables.lj3[row3 + type];
+                k.rep.v = lj.x;
+                k.att.v = lj.y;
+                if (by_type) k.qq.v = tables.qq3[row3 + type];
+            }
+            if (many) {
+                const float2 la = tables.lj2[pa.w * nt + type], lb = tables.lj2[pb.w * nt + type];
+                k.rep = f2(la.x, lb.x);
+                k.att = f2(la.y, lb.y);
+            }
+            if (COULOMB && by_type && many) k.qq = mul(q, both(tables.charge[type]));
+            if (COULOMB && !by_type) k.qq = mul(q, both(charge));
+            return k;
+        };
+        const int part_begin = a.phase == DSMD_PHASE_BOUNDARY ? 1 : 0;
+        const int part_end = a.phase == DSMD_PHASE_INTERIOR || end <= mid ? 1 : 2;
+        acc.least = (special & kRowCareful) ? 0.0f : 3.0e38f;
+        for (int part = part_begin; part < part_end && !(special & kRowCareful); ++part) {
+            int c = (part == 0 ? 0 : (mid + 3) >> 2) + sub;
+            const int c_end = ((part == 0 ? mid : end) + 3) >> 2;
+            const auto add = [&](const int4& pos, float charge) {
+                acc.template add_partner<false>(p, table, pa, pb, pos, terms(pos.w, charge), 0u);
+            };
+            if (c >= c_end) continue;
+            uint4 e = __ldcs(row + static_cast<size_t>(c) * 32);
+            if (TYPES == kOneType && !COULOMB && !ENERGY) {   // two partners are worked on while the next two are on their way
+                int4 p_x, p_y, p_z, p_w;
+                float none;
+                take(e.x, p_x, none);
+                take(e.y, p_y, none);
+                for (; c < c_end; c += lanes) {
+                    take(e.z, p_z, none);
+                    take(e.w, p_w, none);
+                    if (c + lanes < c_end) e = __ldcs(row + static_cast<size_t>(c + lanes) * 32);
+                    add(p_x, 0.f);
+                    add(p_y, 0.f);
+                    take(e.x, p_x, none);
+                    take(e.y, p_y, none);
+                    add(p_z, 0.f);
+                    add(p_w, 0.f);
+                }
+            } else {
+                for (; c < c_end; c += lanes) {
+                    int4 p_x, p_y, p_z, p_w;
+                    float q_x, q_y, q_z, q_w;
+                    take(e.x, p_x, q_x);
+                    take(e.y, p_y, q_y);
+                    take(e.z, p_z, q_z);
+                    take(e.w, p_w, q_w);
+                    if (c + lanes < c_end) e = __ldcs(row + static_cast<size_t>(c + lanes) * 32);
+                    add(p_x, q_x);
+                    add(p_y, q_y);
+                    add(p_z, q_z);
+                    add(p_w, q_w);
+                }
+            }
+        }
+        // What needs care, an entry per lane: the two atoms themselves (each is the other's partner), excluded partners, and
+        // all entries of a row with a pair closer than the plain form can tell (there is none in a sane system).
+        const unsigned row_lanes = (lanes == 32 ? 0xFFFFFFFFu : (1u << lanes) - 1u) << (threadIdx.x & 31 & -lanes);
+        const bool again = __any_sync(row_lanes, acc.least < (COULOMB ? kEwaldFirst : 1e-10f));
+        if (again) acc = PairAccumulator<COPIES, ENERGY, SWITCH>();
+        const int ex_own = special & kRowCountMask, ex_all = ex_own + static_cast<int>((special >> kRowCountBits) & kRowCountMask);
+        const int x0 = a.phase == DSMD_PHASE_BOUNDARY ? ex_own : 0, x1 = a.phase == DSMD_PHASE_INTERIOR ? ex_own : ex_all;
+        const int n_own = atoms > 1 && a.phase != DSMD_PHASE_BOUNDARY && !(special & kRowOwnExcluded) ? 2 : 0;
+        const int n_first = part_begin == 0 ? mid : 0, n_second = part_end == 2 ? end - ((mid + 3) & ~3) : 0;
+        const int n_care = n_own + (x1 - x0) + (again ? n_first + n_second : 0);
+#pragma unroll 1
+        for (int i = sub; i < n_care; i += lanes) {
+            const int x = i - n_own, k = x - (x1 - x0);
+            unsigned e = static_cast<unsigned>(first + i);
+            if (x >= 0) e = words[row_offset(k < 0 ? a.rows.stride - 1 - (x0 + x) : (k < n_first ? k : ((mid + 3) & ~3) + k - n_first))];
+            int4 pj;
+            float qj = 0.0f;
+            take(e & kIndexMask, pj, qj);
+            acc.template add_partner<true>(p, table, pa, pb, pj, terms(pj.w, qj), e);
+        }
+        if (ENERGY) acc.take_energies(atoms > 1, v);   // a lone atom's sums are in both lanes
+        acc.take_forces(sum_a, sum_b);
+    }
+}
+
+// QTYPE: charges by type (dsmd_set_type_charges): the partner's charge comes out of a table in shared memory, indexed by
+// the type that arrives with its position, instead of a second gather from global memory.
+// With Coulomb the blocks stay and take further rows in turn, so that the Ewald tables are laid out once per block; with
+// energy sums, so that the last block has few partial sums to add up.
+template <int COPIES, bool ENERGY, int TYPES, bool SWITCH, bool QTYPE>
+__global__ void __launch_bounds__((kPairThreads<COPIES, TYPES>), (kPairBlocks<COPIES, TYPES, ENERGY>)) k_pair(PairParams p, ForceArgs a) {
+    extern __shared__ float4 smem[];
+    const PairTables<COPIES, ENERGY, TYPES, QTYPE> tables(p, smem);
+    const int lanes = 1 << a.lane_shift;
+    double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};   // energy, virial and its diagonal, pairs
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; (t & ~31) >> a.lane_shift < a.n_pairs; t += gridDim.x * blockDim.x) {
+        const int slot = t >> a.lane_shift, sub = t & (lanes - 1);
+        const int pair = slot < a.n_pairs ? (a.pair_list ? a.pair_list[slot] : a.first_pair + slot) : -1;
+        int first = 0;
+        const int atoms = pair >= 0 ? pair_atoms(a.rows.quad, pair, first) : 0;
+        float sum_a[3] = {0.f, 0.f, 0.f}, sum_b[3] = {0.f, 0.f, 0.f};
+        row_forces<COPIES, ENERGY, TYPES, SWITCH, QTYPE>(p, a, tables, pair, sub, lanes, first, atoms, sum_a, sum_b, v);
+        for (int o = lanes >> 1; o > 0; o >>= 1) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                sum_a[k] += __shfl_xor_sync(0xFFFFFFFFu, sum_a[k], o);
+                sum_b[k] += __shfl_xor_sync(0xFFFFFFFFu, sum_b[k], o);
+            }
+        }
+        if (sub == 0 && atoms > 0) {
+            double* const out[3] = {a.fx, a.fy, a.fz};
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                double* f = out[k] + first;
+                if (a.phase == DSMD_PHASE_BOUNDARY) {
+                    f[0] += static_cast<double>(sum_a[k]);
+                    if (atoms > 1) f[1] += static_cast<double>(sum_b[k]);
+                } else {
+                    f[0] = static_cast<double>(sum_a[k]);
+                    if (atoms > 1) f[1] = static_cast<double>(sum_b[k]);
+                }
+            }
+        }
+        if (COPIES == 0 && !ENERGY) break;   // one row per lane group: the grid covers all
+    }
+    if (ENERGY) sum_over_grid<6>(v, a.partials, a.ticket, a.scalars, a.phase == DSMD_PHASE_BOUNDARY);
+}
+
+}  // namespace

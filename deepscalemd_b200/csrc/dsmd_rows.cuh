@@ -1,0 +1,474 @@
+// Verlet list rows for pairs of atoms: layout, builder, statistics and export. Included by dsmd_core.cu.
+//
+// Two neighbouring atoms share one row. Owned atoms are sorted by cell, x fastest, so consecutive slots of a cell row (a
+// run of x cells at one y, z) are neighbours in space (mean distance about one atom spacing); the union of their two
+// neighbourhoods is 1.3 times one of them for a Lennard-Jones liquid (cutoff + skin 2.8 sigma) and 1.2 times for water
+// (12 A). A row for two atoms therefore holds 0.65 entries per atom instead of one per partner: the force kernel gathers
+// 0.65 times the partner positions (its bound: the L1 unit, 13 wavefronts per 32 random 16-byte gathers) and the list
+// is 0.65 times as long. Entries that lie inside the list radius of one of the two atoms only are tested by both; the
+// cutoff test of the force kernel discards them.
+//
+// Units. Four consecutive atoms of one cell row form a quad (two pairs), the unit of the builder; quads never reach
+// across a cell row. Quad numbers follow from slots by arithmetic (quad_base), so no prefix sum is needed; a cell row
+// leaves at most one quad number unused (its word stays kNoQuad).
+//   quad[q]  = first slot * 4 + (atoms - 1); row of pair p = 2 q + h (h = 0, 1).
+//
+// Entries lie in chunks of four (one 16-byte word), 32 rows interleaved, so that a warp with a row per lane reads 512
+// consecutive bytes: entry k of row p at ((p >> 5) * stride + (k & ~3)) * 32 + (p & 31) * 4 + (k & 3) (row_base + row_offset).
+//   Owned partners come first, [0, row_int[p]); ghosts follow from the next multiple of four on and end at row_end[p];
+//   chunks are filled up with an atom that the search found outside the list radius of both atoms, so that the force kernel
+//   need not count (where the search met no such atom, the row is marked kRowCareful and is counted).
+//   The two atoms themselves are not listed. Partners that one of them excludes are kept apart, from the row's last place
+//   downwards, marked kExclFirst / kExclSecond: the main loop of the force kernel has no flags to look at.
+//   row_special[p] = owned excluded partners | ghosts << kRowCountBits | kRowCareful | kRowOwnExcluded (the two atoms exclude
+//   each other).
+#pragma once
+
+namespace {
+
+constexpr unsigned kExclFirst = 0x80000000u, kExclSecond = 0x40000000u;
+constexpr unsigned kIndexMask = 0x3FFFFFFFu;
+constexpr unsigned kNoQuad = 0xFFFFFFFFu;
+constexpr int kRowCountBits = 15, kRowCountMask = (1 << kRowCountBits) - 1;
+constexpr unsigned kRowCareful = 0x40000000u, kRowOwnExcluded = 0x80000000u;
+constexpr int kBuildThreads = 128;
+
+__host__ __device__ inline int quad_base(int first_slot, int row) { return (first_slot + 3 * row + 3) >> 2; }
+
+// Words of a row: where it starts, and entry k's place from there.
+__host__ __device__ inline size_t row_base(unsigned pair, int stride) {
+    return static_cast<size_t>(pair >> 5) * stride * 32 + (pair & 31u) * 4;
+}
+__host__ __device__ inline int row_offset(int k) { return k * 32 - (k & 3) * 31; }
+
+// First atom and number of atoms (0, 1, 2) of a pair.
+__device__ __forceinline__ int pair_atoms(const unsigned* __restrict__ quad, int pair, int& first) {
+    const unsigned w = quad[pair >> 1];
+    first = static_cast<int>(w >> 2) + 2 * (pair & 1);
+    return w == kNoQuad ? 0 : min(max(static_cast<int>(w & 3u) + 1 - 2 * (pair & 1), 0), 2);
+}
+
+// The quads of every cell row (one warp per row): the numbers between two rows' bases that no atoms fill are kNoQuad.
+__global__ void k_quads(int nx, int rows, int n_owned, const int* __restrict__ cell_start, unsigned* __restrict__ quad) {
+    const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (row >= rows) return;
+    const int begin = min(cell_start[static_cast<size_t>(row) * nx], n_owned);
+    const int end = row + 1 < rows ? min(cell_start[static_cast<size_t>(row + 1) * nx], n_owned) : n_owned;
+    const int q0 = row == 0 ? 0 : quad_base(begin, row), q1 = quad_base(end, row + 1);
+    const int q_first = quad_base(begin, row);
+    for (int q = q0 + lane; q < q1; q += 32) {
+        const int s = begin + 4 * (q - q_first);
+        quad[q] = (q >= q_first && s < end) ? static_cast<unsigned>(s) * 4u + static_cast<unsigned>(min(end - s, 4) - 1) : kNoQuad;
+    }
+}
+
+struct ExclusionTable {
+    const int* offsets;    // [n_global + 1] by global id, or null
+    const int* partners;   // sorted per atom
+    int n_global;          // ids at or beyond this have no exclusions
+};
+
+__device__ __forceinline__ bool within_list_fp64(const Grid& g, const double* __restrict__ x,
+                                                 const double* __restrict__ y, const double* __restrict__ z, int i,
+                                                 int j) {
+    double dx = x[i] - x[j], dy = y[i] - y[j], dz = z[i] - z[j];
+    if (g.wrap[0]) dx -= g.box[0] * rint(dx / g.box[0]);
+    if (g.wrap[1]) dy -= g.box[1] * rint(dy / g.box[1]);
+    if (g.wrap[2]) dz -= g.box[2] * rint(dz / g.box[2]);
+    // No FMA contraction: the sum must round as the plain fp64 expression dx*dx + dy*dy + dz*dz does.
+    const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+    return r2 < g.r2_list_d;
+}
+
+struct RowArrays {
+    const unsigned* quad;
+    unsigned* rows;
+    int stride;             // entries a row has room for, a multiple of four
+    int* row_end;
+    int* row_int;
+    unsigned* row_special;
+};
+
+// The search of one quad by one warp. Each lane takes one cell row of the stencil and works out the x window that the
+// four atoms' list spheres cut out of it (the union of their chords, rounded outwards to x cells). A scan over the lanes
+// numbers the candidates of all rows consecutively, the lanes write their rows' slots into shared memory under those
+// numbers, and the warp walks them 32 at a time: a position per lane, tested against the four atoms, hits of a pair
+// packed behind each other by ballot.
+// What bounds it: instruction issue; 8 to 9 rounds of 32 candidates per quad of a Lennard-Jones liquid (130 of the 250
+// candidates lie inside the list radius of one of the four atoms), about 60 for water. A thread-per-atom walk of the same
+// windows spent 340 warp instructions per atom at 20 of 32 active lanes.
+constexpr int kCandidates = 512;   // candidates numbered at a time (per warp, in shared memory)
+
+struct QuadSearch {
+    int x, y, z;            // the first atom (fixed-point)
+    F2 off[2][3];           // offsets of the four atoms from it, negated: {atom 0, atom 1}, {atom 2, atom 3}
+    float hi_band;
+    int first;              // first slot
+    unsigned *row0, *row1;  // rows of the two pairs
+    int stride;
+    int count0, count1;
+    unsigned special0, special1;   // row_special so far (owned excluded partners)
+    int far0, far1;                // a slot outside both atoms' list radius, or -1
+    int n_atoms;
+};
+
+// The ids an atom excludes lie in [lo, lo + span] (an id that no atom carries where it excludes none).
+struct ExcludedRange {
+    int lo[4];
+    unsigned span[4];
+};
+
+// NEAR: the quad is compact against the box, so that the image of a candidate nearest to the first atom is the nearest
+// to all four: one fixed-point difference and conversion per candidate, the other atoms by their float offsets from the
+// first. Otherwise every atom takes its own fixed-point difference (exact for any placement).
+template <bool NEAR, bool EXCL>
+__device__ __forceinline__ void test_candidates(const Grid& g, QuadSearch& q, int n, const int* __restrict__ s_slot,
+                                                const int4* __restrict__ pq, const int* __restrict__ gid, const ExclusionTable& excl,
+                                                const ExcludedRange& s_excluded) {
+    const int lane = threadIdx.x & 31;
+    const unsigned lt_mask = (1u << lane) - 1u;
+    for (int t = lane; t - lane < n; t += 32) {
+        const bool valid = t < n;
+        const int s = valid ? s_slot[t] : q.first;
+        const int4 c = __ldg(&pq[s]);
+        float r[4];
+        if (NEAR) {
+            const F2 rx = both(dsmd::fixed_delta(c.x, q.x, g.scale[0]));
+            const F2 ry = both(dsmd::fixed_delta(c.y, q.y, g.scale[1]));
+            const F2 rz = both(dsmd::fixed_delta(c.z, q.z, g.scale[2]));
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const F2 dx = add(rx, q.off[h][0]), dy = add(ry, q.off[h][1]), dz = add(rz, q.off[h][2]);
+                parts(fma(dz, dz, fma(dy, dy, mul(dx, dx))), r[2 * h], r[2 * h + 1]);
+            }
+        } else {
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                const int4 atom = __ldg(&pq[q.first + min(m, q.n_atoms - 1)]);
+                const float dx = dsmd::fixed_delta(c.x, atom.x, g.scale[0]);
+                const float dy = dsmd::fixed_delta(c.y, atom.y, g.scale[1]);
+                const float dz = dsmd::fixed_delta(c.z, atom.z, g.scale[2]);
+                r[m] = dx * dx + dy * dy + dz * dz;
+            }
+        }
+        const float limit = valid ? q.hi_band : -1.0f;
+        bool hit0 = fminf(r[0], r[1]) < limit, hit1 = fminf(r[2], r[3]) < limit;
+        if (q.far0 < 0 || q.far1 < 0) {   // as a rule found in the first round
+            const unsigned f0 = __ballot_sync(0xFFFFFFFFu, valid && !hit0), f1 = __ballot_sync(0xFFFFFFFFu, valid && !hit1);
+            if (f0) q.far0 = __shfl_sync(0xFFFFFFFFu, s, __ffs(f0) - 1);
+            if (f1) q.far1 = __shfl_sync(0xFFFFFFFFu, s, __ffs(f1) - 1);
+        }
+        // the two atoms of a pair are no partners of its row
+        const unsigned own = static_cast<unsigned>(s - q.first);
+        const bool own0 = own < static_cast<unsigned>(min(q.n_atoms, 2)), own1 = own - 2u < static_cast<unsigned>(max(q.n_atoms - 2, 0));
+        if (EXCL) {
+            // a candidate inside the range of ids that one of the four atoms excludes (molecules are numbered together: few
+            // are) is looked up in the atom's table row; the row's end holds those that are excluded for one of its atoms
+            const int gj = __ldg(&gid[s]);
+            const int4 lo = *reinterpret_cast<const int4*>(s_excluded.lo);
+            const uint4 span = *reinterpret_cast<const uint4*>(s_excluded.span);
+            const bool look = static_cast<unsigned>(gj - lo.x) <= span.x || static_cast<unsigned>(gj - lo.y) <= span.y ||
+                              static_cast<unsigned>(gj - lo.z) <= span.z || static_cast<unsigned>(gj - lo.w) <= span.w;
+            if (__any_sync(0xFFFFFFFFu, look && (hit0 || hit1))) {
+                unsigned flags0 = 0, flags1 = 0;
+#pragma unroll 1
+                for (int m = 0; m < q.n_atoms; ++m) {
+                    if (look && static_cast<unsigned>(gj - s_excluded.lo[m]) <= s_excluded.span[m]) {
+                        const int g_m = gid[q.first + m], end = excl.offsets[g_m + 1];
+                        for (int e = excl.offsets[g_m]; e < end; ++e)
+                            if (excl.partners[e] == gj) {
+                                if (m < 2) flags0 |= m == 0 ? kExclFirst : kExclSecond;
+                                else flags1 |= m == 2 ? kExclFirst : kExclSecond;
+                            }
+                    }
+                }
+                const unsigned x0 = __ballot_sync(0xFFFFFFFFu, hit0 && flags0), x1 = __ballot_sync(0xFFFFFFFFu, hit1 && flags1);
+                const int p0 = static_cast<int>((q.special0 & kRowCountMask) + __popc(x0 & lt_mask));
+                const int p1 = static_cast<int>((q.special1 & kRowCountMask) + __popc(x1 & lt_mask));
+                if (hit0 && flags0 && p0 < q.stride) q.row0[row_offset(q.stride - 1 - p0)] = static_cast<unsigned>(s) | flags0;
+                if (hit1 && flags1 && p1 < q.stride) q.row1[row_offset(q.stride - 1 - p1)] = static_cast<unsigned>(s) | flags1;
+                q.special0 += __popc(x0);
+                q.special1 += __popc(x1);
+                if (__any_sync(0xFFFFFFFFu, hit0 && flags0 && own0)) q.special0 |= kRowOwnExcluded;
+                if (__any_sync(0xFFFFFFFFu, hit1 && flags1 && own1)) q.special1 |= kRowOwnExcluded;
+                hit0 = hit0 && !flags0;
+                hit1 = hit1 && !flags1;
+            }
+        }
+        hit0 = hit0 && !own0;
+        hit1 = hit1 && !own1;
+        const unsigned m0 = __ballot_sync(0xFFFFFFFFu, hit0), m1 = __ballot_sync(0xFFFFFFFFu, hit1);
+        const int k0 = q.count0 + __popc(m0 & lt_mask), k1 = q.count1 + __popc(m1 & lt_mask);
+        if (hit0 && k0 < q.stride) q.row0[row_offset(k0)] = static_cast<unsigned>(s);
+        if (hit1 && k1 < q.stride) q.row1[row_offset(k1)] = static_cast<unsigned>(s);
+        q.count0 += __popc(m0);
+        q.count1 += __popc(m1);
+    }
+}
+
+template <bool EXCL>
+__global__ void __launch_bounds__(kBuildThreads, 8)
+k_build_rows(Grid g, int n_owned, int n_total, int n_quads, const int4* __restrict__ pq, const int* __restrict__ gid,
+             ExclusionTable excl, const int* __restrict__ cell_start, const int* __restrict__ ghost_near_lo,
+             const int* __restrict__ ghost_near_hi, RowArrays out, int* __restrict__ boundary_pairs, Status* st) {
+    __shared__ int s_slots[kBuildThreads / 32][kCandidates];
+    __shared__ __align__(16) ExcludedRange s_ranges[EXCL ? kBuildThreads / 32 : 1];
+    const int quad = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (quad >= n_quads) return;
+    int* slots = s_slots[threadIdx.x >> 5];
+    const unsigned word = out.quad[quad];
+    if (word == kNoQuad) {
+        if (lane < 2) out.row_end[2 * quad + lane] = out.row_int[2 * quad + lane] = 0;
+        if (lane < 2) out.row_special[2 * quad + lane] = 0u;
+        return;
+    }
+    QuadSearch q;
+    q.first = static_cast<int>(word >> 2);
+    const int n_atoms = static_cast<int>(word & 3u) + 1;
+    float off[4][3];
+    bool compact = true;
+    const int4 home = pq[q.first];
+    q.x = home.x;
+    q.y = home.y;
+    q.z = home.z;
+    int c_min = g.nc[0], c_max = -1;   // x cells of the atoms
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        const int4 atom = pq[q.first + min(m, n_atoms - 1)];   // a missing atom: a copy of the last one
+        off[m][0] = dsmd::fixed_delta(atom.x, home.x, g.scale[0]);
+        off[m][1] = dsmd::fixed_delta(atom.y, home.y, g.scale[1]);
+        off[m][2] = dsmd::fixed_delta(atom.z, home.z, g.scale[2]);
+        // how far the quad may spread for the nearest image of a candidate to be the same for all four atoms (wrapping
+        // axes), and for the rounding band to hold
+        compact = compact && fabsf(off[m][0]) <= g.quad_spread[0] && fabsf(off[m][1]) <= g.quad_spread[1] &&
+                  fabsf(off[m][2]) <= g.quad_spread[2];
+        const int cx = static_cast<int>(dsmd::cell_of(static_cast<unsigned>(atom.x), g.wrap[0], g.nc[0]));
+        c_min = min(c_min, cx);
+        c_max = max(c_max, cx);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) q.off[h][a] = f2(-off[2 * h][a], -off[2 * h + 1][a]);
+    // a pair inside the rounding band is listed whether or not it lies inside the list radius (the export decides in fp64)
+    q.hi_band = g.r2_list + g.band_rows;
+    q.stride = out.stride;
+    q.row0 = out.rows + row_base(2 * quad, out.stride);
+    q.row1 = q.row0 + 4;   // the rows of a quad are neighbours
+    q.count0 = q.count1 = 0;
+    q.special0 = q.special1 = 0u;
+    q.far0 = q.far1 = -1;
+    q.n_atoms = n_atoms;
+    ExcludedRange& s_excluded = s_ranges[EXCL ? threadIdx.x >> 5 : 0];
+    if (EXCL && lane < 4) {
+        int lo = static_cast<int>(0x80000000u);   // no atom carries this id
+        unsigned span = 0u;
+        const int g_m = gid[q.first + min(lane, n_atoms - 1)];
+        if (lane < n_atoms && g_m >= 0 && g_m < excl.n_global) {
+            const int b = excl.offsets[g_m], e = excl.offsets[g_m + 1];
+            if (e > b) {
+                lo = excl.partners[b];
+                span = static_cast<unsigned>(excl.partners[e - 1] - lo);
+            }
+        }
+        s_excluded.lo[lane] = lo;
+        s_excluded.span[lane] = span;
+    }
+
+    // this lane's cell row, (dy, dz) from the home row, and its x window in cells
+    const int S = g.stencil, side = 2 * S + 1;
+    const int lane_z = S == 2 ? (lane * 13) >> 6 : (lane * 11) >> 5;   // lane / 5, lane / 3
+    const int dz = lane_z - S, dy = lane - lane_z * side - S;
+    // places of the first atom on the three axes, in cells (float: good to 3e-4 of a cell)
+    const float at_x = __uint2float_rn(g.wrap[0] ? static_cast<unsigned>(home.x) : static_cast<unsigned>(home.x) << 1) *
+                       (static_cast<float>(g.nc[0]) * 2.3283064e-10f);
+    const float at_y = __uint2float_rn(g.wrap[1] ? static_cast<unsigned>(home.y) : static_cast<unsigned>(home.y) << 1) *
+                       (static_cast<float>(g.nc[1]) * 2.3283064e-10f);
+    const float at_z = __uint2float_rn(g.wrap[2] ? static_cast<unsigned>(home.z) : static_cast<unsigned>(home.z) << 1) *
+                       (static_cast<float>(g.nc[2]) * 2.3283064e-10f);
+    const int cy0 = static_cast<int>(dsmd::cell_of(static_cast<unsigned>(home.y), g.wrap[1], g.nc[1]));
+    const int cz0 = static_cast<int>(dsmd::cell_of(static_cast<unsigned>(home.z), g.wrap[2], g.nc[2]));
+    const float to_y = static_cast<float>(cy0 + dy) - at_y, to_z = static_cast<float>(cz0 + dz) - at_z;   // lower face of the row
+    int yc = cy0 + dy, zc = cz0 + dz;
+    bool open = lane < side * side;
+    if (g.wrap[1]) { if (yc < 0) yc += g.nc[1]; else if (yc >= g.nc[1]) yc -= g.nc[1]; }
+    else if (yc < 0 || yc >= g.nc[1]) open = false;
+    if (g.wrap[2]) { if (zc < 0) zc += g.nc[2]; else if (zc >= g.nc[2]) zc -= g.nc[2]; }
+    else if (zc < 0 || zc >= g.nc[2]) open = false;
+    // the chord of each atom's sphere at the row's distance from it (g.r_pad carries 1e-4 of slack, far more than the
+    // approximate square root gives away; 1e-3 of a cell covers the rounding of the places)
+    const float reach2 = g.r_pad * g.r_pad;
+    float lo = 3.0e38f, hi = -3.0e38f;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        const float y0 = to_y * g.cellw[1] - off[m][1], z0 = to_z * g.cellw[2] - off[m][2];   // from the atom to the lower face
+        const float gy = fmaxf(fmaxf(y0, -y0 - g.cellw[1]) - 1e-3f * g.cellw[1], 0.f);
+        const float gz = fmaxf(fmaxf(z0, -z0 - g.cellw[2]) - 1e-3f * g.cellw[2], 0.f);
+        const float chord2 = reach2 - gy * gy - gz * gz;
+        if (chord2 > 0.f) {
+            const float hw = fminf(chord2 * rsqrt_approx(chord2), g.x_reach);
+            lo = fminf(lo, off[m][0] - hw);
+            hi = fmaxf(hi, off[m][0] + hw);
+        }
+    }
+    open = open && lo <= hi;
+    int a0 = 0, b0 = -1, a1 = 0, b1 = -1;   // x cells [a0, b0] and, across the periodic boundary, [a1, b1]
+    if (open) {
+        const float per_cell = 1.0f / g.cellw[0];
+        const int c_lo = __float2int_rd(at_x + lo * per_cell - 2e-3f), c_hi = __float2int_rd(at_x + hi * per_cell + 2e-3f);
+        if (!g.wrap[0]) {
+            a0 = max(c_lo, 0);
+            b0 = min(c_hi, g.nc[0] - 1);
+        } else if (c_hi - c_lo >= g.nc[0] - 1) {
+            b0 = g.nc[0] - 1;   // the window is as long as the box
+        } else {
+            a0 = c_lo < 0 ? c_lo + g.nc[0] : (c_lo >= g.nc[0] ? c_lo - g.nc[0] : c_lo);
+            b0 = c_hi < 0 ? c_hi + g.nc[0] : (c_hi >= g.nc[0] ? c_hi - g.nc[0] : c_hi);
+            if (b0 < a0) {   // in ascending slots: the part at the lower end of the box first
+                a1 = a0;
+                b1 = g.nc[0] - 1;
+                a0 = 0;
+            }
+        }
+    }
+    // the ghost pass only for quads whose x windows reach an x cell with ghosts in one of the rows they search (on an
+    // axis that wraps the window may come round the box: any ghost in those rows counts)
+    int n_seg = 1;
+    if (n_total > n_owned) {
+        const int row_yz = cz0 * g.nc[1] + cy0;
+        const int near_lo = ghost_near_lo[row_yz], near_hi = ghost_near_hi[row_yz];
+        const int reach_cells = static_cast<int>(g.x_reach / g.cellw[0]) + 2;
+        if (g.wrap[0] ? (near_lo > 0 || near_hi < g.nc[0]) : (c_min - reach_cells < near_lo || c_max + reach_cells >= near_hi))
+            n_seg = 2;
+    }
+    int interior0 = 0, interior1 = 0;
+    unsigned interior_special0 = 0u, interior_special1 = 0u;
+    for (int seg = 0; seg < n_seg; ++seg) {
+        const int row = seg * g.ncells + (zc * g.nc[1] + yc) * g.nc[0];
+        int s0 = 0, len0 = 0, s1 = 0, len1 = 0;
+        if (b0 >= a0) { s0 = cell_start[row + a0]; len0 = cell_start[row + b0 + 1] - s0; }
+        if (b1 >= a1) { s1 = cell_start[row + a1]; len1 = cell_start[row + b1 + 1] - s1; }
+        const int len = len0 + len1;
+        int incl = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        const int total = __shfl_sync(0xFFFFFFFFu, incl, 31), begin = incl - len;
+        for (int base = 0; base < total; base += kCandidates) {
+            __syncwarp();
+            // this row's share of the numbers [base, base + kCandidates): the first run, then (rare) the second
+            int* to = slots + (begin - base);
+            const int k0 = max(base - begin, 0), k1 = min(base + kCandidates - begin, len);
+            const int first_end = min(k1, len0);
+            int k = k0;
+            for (; k + 3 < first_end; k += 4) {
+                to[k] = s0 + k;
+                to[k + 1] = s0 + k + 1;
+                to[k + 2] = s0 + k + 2;
+                to[k + 3] = s0 + k + 3;
+            }
+            if (k < first_end) to[k] = s0 + k;
+            if (k + 1 < first_end) to[k + 1] = s0 + k + 1;
+            if (k + 2 < first_end) to[k + 2] = s0 + k + 2;
+            if (len1 > 0)
+                for (k = max(k0, len0); k < k1; ++k) to[k] = s1 + (k - len0);
+            __syncwarp();
+            const int n = min(total - base, kCandidates);
+            if (compact) test_candidates<true, EXCL>(g, q, n, slots, pq, gid, excl, s_excluded);
+            else test_candidates<false, EXCL>(g, q, n, slots, pq, gid, excl, s_excluded);
+        }
+        if (n_atoms <= 2) { q.count1 = 0; q.special1 = 0u; }
+        if (seg == 0) { interior0 = q.count0; interior1 = q.count1; interior_special0 = q.special0; interior_special1 = q.special1; }
+        // fill up the last chunk
+        const int c = lane < 4 ? q.count0 : q.count1, far = lane < 4 ? q.far0 : q.far1;
+        const int k = (c & ~3) + (lane & 3);
+        if (lane < 8 && k >= c && (c & 3) && k < out.stride)
+            (lane < 4 ? q.row0 : q.row1)[row_offset(k)] = static_cast<unsigned>(far < 0 ? q.first : far);
+        if (seg == 0 && n_seg == 2) {
+            q.count0 = (q.count0 + 3) & ~3;
+            q.count1 = (q.count1 + 3) & ~3;
+        }
+    }
+    if (lane < 2) {
+        const int interior = lane ? interior1 : interior0, count = lane ? q.count1 : q.count0;
+        const unsigned special = lane ? q.special1 : q.special0, special_own = lane ? interior_special1 : interior_special0;
+        const unsigned n_special = special & kRowCountMask, n_own = special_own & kRowCountMask;
+        // a ghost pass without hits leaves the row as it was
+        const bool ghosts = n_seg == 2 && count > ((interior + 3) & ~3);
+        out.row_end[2 * quad + lane] = min(ghosts ? count : interior, out.stride);
+        out.row_int[2 * quad + lane] = min(interior, out.stride);
+        out.row_special[2 * quad + lane] = n_own | ((n_special - n_own) << kRowCountBits) | (special & kRowOwnExcluded) |
+                                           ((lane ? q.far1 : q.far0) < 0 ? kRowCareful : 0u);
+        const int need = ((count + 3) & ~3) + static_cast<int>(n_special);   // whole chunks, and the ones apart behind them
+        if (need > out.stride) atomicMax(&st->need_stride, static_cast<unsigned>(need));
+        // pairs with a ghost partner, collected for the boundary pass of the force kernel (the order of the collection
+        // does not matter: every pair's sums are its own threads')
+        if (ghosts || n_special > n_own) boundary_pairs[atomicAdd(&st->boundary_pairs, 1u)] = 2 * quad + lane;
+    }
+}
+
+// Members of the list proper, decided in fp64 on the reference positions of the last build (the builder lists every
+// candidate inside the rounding band and, for an atom, its pair-mate's partners): counts per atom, or (WRITE) the
+// directed pairs themselves, atom after atom in row order. stats: members, members with an owned partner, tests inside
+// the rounding band.
+template <bool WRITE>
+__global__ void k_list_members(Grid g, int n_pairs, int n_owned, RowArrays in, const double* __restrict__ x,
+                               const double* __restrict__ y, const double* __restrict__ z, unsigned long long* __restrict__ per_atom,
+                               unsigned long long* __restrict__ stats, int* __restrict__ out_i, int* __restrict__ out_j,
+                               unsigned char* __restrict__ out_flags, long long capacity) {
+    const int pair = blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned long long members = 0, interior = 0, banded = 0;
+    int first = 0;
+    const int atoms = pair < n_pairs ? pair_atoms(in.quad, pair, first) : 0;
+    for (int m = 0; m < atoms; ++m) {
+        const int i = first + m;
+        unsigned long long found = 0, at = WRITE ? per_atom[i] : 0ull;
+        const int mid = in.row_int[pair], end = in.row_end[pair];
+        const unsigned special = in.row_special[pair];
+        const int special_own = special & kRowCountMask, special_all = special_own + ((special >> kRowCountBits) & kRowCountMask);
+        const bool own_pair = atoms > 1 && !(special & kRowOwnExcluded);
+        const unsigned* row = in.rows + row_base(static_cast<unsigned>(pair), in.stride);
+        for (int k = 0; k < end + special_all + (own_pair ? 1 : 0); ++k) {
+            if (k >= mid && k < min((mid + 3) & ~3, end)) continue;
+            const int nth = k - end;   // then the ones at the row's end, then the pair's other atom
+            const bool owned = nth < 0 ? k < mid : (nth < special_own || nth >= special_all);
+            const unsigned e = nth < 0 ? row[row_offset(k)]
+                                       : (nth < special_all ? row[row_offset(in.stride - 1 - nth)] : static_cast<unsigned>(first + 1 - m));
+            const int j = static_cast<int>(e & kIndexMask);
+            if (j == i || !within_list_fp64(g, x, y, z, i, j)) continue;
+            if (WRITE) {
+                if (static_cast<long long>(at) < capacity) {
+                    out_i[at] = i;
+                    out_j[at] = j;
+                    if (out_flags) out_flags[at] = (e & (m == 0 ? kExclFirst : kExclSecond)) ? 1 : 0;
+                }
+                ++at;
+            } else {
+                ++found;
+                if (owned) ++interior;
+                double d[3] = {x[i] - x[j], y[i] - y[j], z[i] - z[j]};
+                for (int a = 0; a < 3; ++a)
+                    if (g.wrap[a]) d[a] -= g.box[a] * rint(d[a] / g.box[a]);
+                if (fabs(d[0] * d[0] + d[1] * d[1] + d[2] * d[2] - g.r2_list_d) < static_cast<double>(g.band_rows)) ++banded;
+            }
+        }
+        if (!WRITE) per_atom[i] = found;
+        members += found;
+    }
+    if (!WRITE) {
+        for (int o = 16; o > 0; o >>= 1) {
+            members += __shfl_down_sync(0xFFFFFFFFu, members, o);
+            interior += __shfl_down_sync(0xFFFFFFFFu, interior, o);
+            banded += __shfl_down_sync(0xFFFFFFFFu, banded, o);
+        }
+        if ((threadIdx.x & 31) == 0) {
+            atomicAdd(&stats[0], members);
+            atomicAdd(&stats[1], interior);
+            if (banded) atomicAdd(&stats[2], banded);
+        }
+    }
+}
+
+}  // namespace

@@ -168,7 +168,7 @@ struct AtomArrays {
 template <class Shape, bool FINISH, bool START>
 __global__ void __launch_bounds__(128) k_constrained(ClusterTable t, Grid g, AtomArrays at, double half_kick, double dt, double tolerance,
                                                      int max_iterations, double prefactor, double* __restrict__ partials, unsigned* __restrict__ ticket,
-                                                     double* __restrict__ virial, Status* st) {
+                                                     double* __restrict__ virial, DisplacementReport report) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     double wsum[3] = {0.0, 0.0, 0.0}, worst2 = 0.0;
     if (k < t.n_clusters) {
@@ -236,10 +236,10 @@ __global__ void __launch_bounds__(128) k_constrained(ClusterTable t, Grid g, Ato
                     worst2 = fmax(worst2, d2 == d2 ? d2 : __longlong_as_double(0x7FF0000000000000ll));
                 }
             }
-        if (bad) atomicAdd(&st->out_of_domain, 1u);
-        if (!good) atomicAdd(&st->constraint_failed, 1u);
+        if (bad) atomicAdd(&report.st->out_of_domain, 1u);
+        if (!good) atomicAdd(&report.st->constraint_failed, 1u);
     }
-    if (START) block_max_to_status(worst2, st);
+    if (START) report_displacement(worst2, report);
     if (virial) sum_over_grid<3>(wsum, partials, ticket, virial, false);
 }
 

@@ -18,6 +18,7 @@
 #include <thrust/iterator/counting_iterator.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -40,6 +41,7 @@ constexpr int64_t kPairLanesWanted = kDeviceSms * 1024;   // lanes that fill the
 constexpr int64_t kPairLanesWantedEwald = kDeviceSms * 768;   // two rounds of one block of 384 each
 constexpr int kLongRow = 240;                         // entries (with the row's spare room): about 150 partners per atom
 constexpr int kXRefine = 4;    // x cells per cell width of the y and z axes (tighter row windows in the list build)
+enum { kMailDisplacement = 0, kMailKinetic = 4, kMailScalars = 5, kMailSlots = 6 };   // report slots
 constexpr int kNumReal = 11;   // x y z vx vy vz fx fy fz mass charge
 constexpr double kCoulomb = 332.0636;
 
@@ -211,7 +213,31 @@ __global__ void k_ghost_rows_near(Grid g, const int* __restrict__ lo_end, const 
 // kernels: per-step pack, displacement, integration
 // ---------------------------------------------------------------------------------------------------------------------
 
-__device__ __forceinline__ void block_max_to_status(double v, Status* st) {
+// Values that the host waits for leave a kernel through pinned host memory: the block that finishes last writes them and
+// then the number of the launch, which the host polls (host/mail in dsmd_ctx). That saves the copy behind the kernel and
+// the wait for the copy: 3 us instead of 9 per value.
+struct Mail {
+    double value[7];
+    unsigned long long seq;
+};
+
+__device__ __forceinline__ void post(Mail* mail, const double* v, int n, unsigned long long seq) {   // one thread
+    volatile Mail* m = mail;
+    for (int k = 0; k < n; ++k) m->value[k] = v[k];
+    __threadfence_system();
+    m->seq = seq;
+}
+
+// Who writes where when a displacement check ends.
+struct DisplacementReport {
+    Status* st;
+    unsigned* ticket;      // blocks that have finished
+    Mail* mail;            // or null: no report
+    unsigned long long seq;
+};
+
+// The block's largest squared displacement goes into the status word; the last block of the grid reports the word.
+__device__ __forceinline__ void report_displacement(double v, const DisplacementReport& r) {
     for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
     __shared__ double warp_max[32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -220,7 +246,19 @@ __device__ __forceinline__ void block_max_to_status(double v, Status* st) {
     if (w == 0) {
         v = lane < (blockDim.x >> 5) ? warp_max[lane] : 0.0;
         for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
-        if (lane == 0 && v > 0.0) atomicMax(&st->max_disp2, static_cast<unsigned long long>(__double_as_longlong(v)));
+        if (lane == 0) {
+            if (v > 0.0) atomicMax(&r.st->max_disp2, static_cast<unsigned long long>(__double_as_longlong(v)));
+            if (r.mail) {
+                __threadfence();
+                if (atomicAdd(r.ticket, 1u) == gridDim.x - 1) {
+                    __threadfence();
+                    const double out[2] = {__longlong_as_double(static_cast<long long>(__ldcg(&r.st->max_disp2))),
+                                           static_cast<double>(__ldcg(&r.st->out_of_domain))};
+                    *r.ticket = 0u;
+                    post(r.mail, out, 2, r.seq);
+                }
+            }
+        }
     }
 }
 
@@ -234,7 +272,7 @@ __global__ void k_pack(Grid g, int first, int count, int n_owned, double* __rest
                        const double* __restrict__ fz, const double* __restrict__ mass, const int* __restrict__ type,
                        const double* __restrict__ xref, const double* __restrict__ yref,
                        const double* __restrict__ zref, int4* __restrict__ pq, double dt, double kick_c,
-                       const int* __restrict__ gid, const unsigned char* __restrict__ skip, Status* st) {
+                       const int* __restrict__ gid, const unsigned char* __restrict__ skip, DisplacementReport report) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int s = first + t;
     double d2 = 0.0;
@@ -254,7 +292,7 @@ __global__ void k_pack(Grid g, int first, int count, int n_owned, double* __rest
         p.z = static_cast<int>(dsmd::to_fixed(pz, 2, g, bad));
         p.w = type[s];
         pq[s] = p;
-        if (bad) atomicAdd(&st->out_of_domain, 1u);
+        if (bad) atomicAdd(&report.st->out_of_domain, 1u);
         if (s < n_owned) {
             const double ddx = px - xref[s], ddy = py - yref[s], ddz = pz - zref[s];
             d2 = ddx * ddx + ddy * ddy + ddz * ddz;
@@ -263,7 +301,7 @@ __global__ void k_pack(Grid g, int first, int count, int n_owned, double* __rest
             if (!(d2 == d2)) d2 = __longlong_as_double(0x7FF0000000000000ll);
         }
     }
-    block_max_to_status(d2, st);
+    report_displacement(d2, report);
 }
 
 __global__ void k_vv2(int n, double half_dt_c, double* __restrict__ vx, double* __restrict__ vy,
@@ -310,7 +348,8 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double (&sh)[32][NV])
 }
 
 template <int NV>
-__device__ __forceinline__ void sum_over_grid(double (&v)[NV], double* partials, unsigned* ticket, double* out, bool accumulate) {
+__device__ __forceinline__ void sum_over_grid(double (&v)[NV], double* partials, unsigned* ticket, double* out, bool accumulate,
+                                              Mail* mail = nullptr, unsigned long long seq = 0) {
     __shared__ double sh[32][NV];
     __shared__ bool last;
     block_sum<NV>(v, sh);
@@ -327,18 +366,19 @@ __device__ __forceinline__ void sum_over_grid(double (&v)[NV], double* partials,
         for (int k = 0; k < NV; ++k) v[k] += __ldcg(&partials[static_cast<size_t>(b) * NV + k]);
     block_sum<NV>(v, sh);
     if (threadIdx.x == 0) {
-        for (int k = 0; k < NV; ++k) out[k] = accumulate ? out[k] + v[k] : v[k];
+        for (int k = 0; k < NV; ++k) out[k] = v[k] = accumulate ? out[k] + v[k] : v[k];
         *ticket = 0u;
+        if (mail) post(mail, v, NV, seq);
     }
 }
 
 __global__ void k_kinetic(int n, const double* __restrict__ vx, const double* __restrict__ vy,
                           const double* __restrict__ vz, const double* __restrict__ mass, double* partials, unsigned* ticket,
-                          double* out) {
+                          double* out, Mail* mail, unsigned long long seq) {
     double v[1] = {0.0};
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x)
         v[0] += 0.5 * mass[s] * (vx[s] * vx[s] + vy[s] * vy[s] + vz[s] * vz[s]);
-    sum_over_grid<1>(v, partials, ticket, out, false);
+    sum_over_grid<1>(v, partials, ticket, out, false, mail, seq);
 }
 
 }  // namespace
@@ -492,7 +532,8 @@ struct dsmd_ctx {
     int* type[2] = {};
     int* gid[2] = {};
     int cur = 0;
-    int4* pq = nullptr;
+    int4* pq = nullptr;               // positions as the kernels read them; pq_next: where a fused step writes the next ones
+    int4* pq_next = nullptr;
     float* qf = nullptr;
     double* ref[3] = {};
     unsigned* key[2] = {};
@@ -534,7 +575,12 @@ struct dsmd_ctx {
     double* partials = nullptr;
     int64_t partial_blocks = 0;
     double* scalars = nullptr;      // 6 force scalars + 1 kinetic
-    unsigned* tickets = nullptr;    // finished blocks of the sums: forces, kinetic energy, bonded terms, constraints
+    unsigned* tickets = nullptr;    // finished blocks of the sums: forces, kinetic energy, bonded terms, constraints;
+                                    // from 4 on: displacement checks in turn
+    Mail* mail = nullptr;           // pinned: kMailDisplacement .. + 3 in turn, kMailKinetic, kMailScalars
+    bool captured = false;          // a call was captured into a graph: results are copied, not reported
+    unsigned long long seq = 0;     // launches that reported something so far
+    unsigned long long disp_seq = 0, scalars_seq = 0;   // the last displacement check / energy sum whose report still stands (0: none)
     Status* status = nullptr;
     Status* h_status = nullptr;     // pinned
     double* h_scalars = nullptr;    // pinned
@@ -852,6 +898,49 @@ int sort_range(dsmd_ctx* c, int64_t first, cudaStream_t s, int64_t n_removed = 0
     return DSMD_OK;
 }
 
+cudaError_t clear_status(dsmd_ctx* c, cudaStream_t s) {
+    c->disp_seq = 0;   // reports of displacement checks are void
+    return cudaMemsetAsync(c->status, 0, sizeof(Status), s);
+}
+
+// Waits for the report of a launch on `s`. The launch is in the stream; the loop ends with an error when the stream has run
+// dry (or failed) without it.
+int wait_mail(dsmd_ctx* c, int slot, unsigned long long seq, cudaStream_t s) {
+    const volatile Mail* m = c->mail + slot;
+    for (unsigned spins = 1;; ++spins) {
+        if (m->seq == seq) {
+            std::atomic_thread_fence(std::memory_order_acquire);
+            return DSMD_OK;
+        }
+        if ((spins & 0x3FFu) == 0) {
+            const cudaError_t q = cudaStreamQuery(s);
+            if (q == cudaErrorNotReady) continue;
+            // done or failed; the caller may have named another stream than the launch's
+            DSMD_CUDA(c, q);
+            DSMD_CUDA(c, cudaDeviceSynchronize());
+            if (m->seq == seq) continue;
+            return fail(c, DSMD_ERR_CUDA, "a kernel ended without its report");
+        }
+    }
+}
+
+// Reports carry the number of their launch, which a replayed graph would repeat: a context that was ever captured copies.
+bool reports_count(dsmd_ctx* c, cudaStream_t s) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &status) != cudaSuccess || status != cudaStreamCaptureStatusNone) c->captured = true;
+    return !c->captured;
+}
+
+// The report of a displacement check about to be launched: of all owned atoms, or none (a part says little, and parts may
+// run side by side on several streams). Slots and tickets in turn, so that the last three stay readable.
+DisplacementReport displacement_report(dsmd_ctx* c, bool all_atoms, cudaStream_t s) {
+    c->disp_seq = 0;
+    if (!all_atoms || !reports_count(c, s)) return DisplacementReport{c->status, nullptr, nullptr, 0};
+    c->disp_seq = ++c->seq;
+    const int slot = static_cast<int>(c->seq & 3);
+    return DisplacementReport{c->status, c->tickets + 4 + slot, c->mail + kMailDisplacement + slot, c->seq};
+}
+
 int read_status(dsmd_ctx* c, cudaStream_t s) {
     DSMD_CUDA(c, cudaMemcpyAsync(c->h_status, c->status, sizeof(Status), cudaMemcpyDeviceToHost, s));
     DSMD_CUDA(c, cudaStreamSynchronize(s));
@@ -918,6 +1007,7 @@ int dsmd_create(int device, int64_t capacity, dsmd_ctx** out) {
         DSMD_CUDA(c, cudaMalloc(&c->val[set], sizeof(int) * capacity));
     }
     DSMD_CUDA(c, cudaMalloc(&c->pq, sizeof(int4) * capacity));
+    DSMD_CUDA(c, cudaMalloc(&c->pq_next, sizeof(int4) * capacity));
     DSMD_CUDA(c, cudaMalloc(&c->qf, sizeof(float) * capacity));
     for (int a = 0; a < 3; ++a) DSMD_CUDA(c, cudaMalloc(&c->ref[a], sizeof(double) * capacity));
     DSMD_CUDA(c, cudaMalloc(&c->ghost_slot, sizeof(int) * capacity));
@@ -926,8 +1016,10 @@ int dsmd_create(int device, int64_t capacity, dsmd_ctx** out) {
     DSMD_CUDA(c, cudaMalloc(&c->offsets64, sizeof(unsigned long long) * capacity));
     DSMD_CUDA(c, cudaMalloc(&c->scalars, sizeof(double) * 8));
     DSMD_CUDA(c, cudaMemset(c->scalars, 0, sizeof(double) * 8));
-    DSMD_CUDA(c, cudaMalloc(&c->tickets, sizeof(unsigned) * 4));
-    DSMD_CUDA(c, cudaMemset(c->tickets, 0, sizeof(unsigned) * 4));
+    DSMD_CUDA(c, cudaMalloc(&c->tickets, sizeof(unsigned) * 8));
+    DSMD_CUDA(c, cudaMemset(c->tickets, 0, sizeof(unsigned) * 8));
+    DSMD_CUDA(c, cudaMallocHost(&c->mail, sizeof(Mail) * kMailSlots));
+    std::memset(c->mail, 0, sizeof(Mail) * kMailSlots);
     DSMD_CUDA(c, cudaMalloc(&c->status, sizeof(Status)));
     DSMD_CUDA(c, cudaMemset(c->status, 0, sizeof(Status)));
     DSMD_CUDA(c, cudaMallocHost(&c->h_status, sizeof(Status)));
@@ -947,7 +1039,7 @@ void dsmd_destroy(dsmd_ctx* c) {
         for (int f = 0; f < kNumReal; ++f) cudaFree(c->real[set][f]);
         cudaFree(c->type[set]); cudaFree(c->gid[set]); cudaFree(c->key[set]); cudaFree(c->val[set]);
     }
-    cudaFree(c->pq); cudaFree(c->qf); cudaFree(c->type_charge);
+    cudaFree(c->pq); cudaFree(c->pq_next); cudaFree(c->qf); cudaFree(c->type_charge);
     for (int a = 0; a < 3; ++a) cudaFree(c->ref[a]);
     cudaFree(c->ghost_slot); cudaFree(c->cell_start); cudaFree(c->ghost_rows);
     cudaFree(c->rows); cudaFree(c->quad); cudaFree(c->row_end); cudaFree(c->row_int); cudaFree(c->row_special); cudaFree(c->boundary_pairs);
@@ -967,7 +1059,7 @@ void dsmd_destroy(dsmd_ctx* c) {
     }
     if (c->pipe_begin) cudaEventDestroy(c->pipe_begin);
     if (c->pipe_end) cudaEventDestroy(c->pipe_end);
-    cudaFreeHost(c->h_status); cudaFreeHost(c->h_scalars);
+    cudaFreeHost(c->h_status); cudaFreeHost(c->h_scalars); cudaFreeHost(c->mail);
     for (int k = 0; k < 2; ++k) {
         cudaFreeHost(c->h_disp[k]);
         if (c->disp_event[k]) cudaEventDestroy(c->disp_event[k]);
@@ -993,6 +1085,7 @@ int dsmd_set_box(dsmd_ctx* c, const double box[3], const int periodic[3], const 
     c->box_set = true;
     c->grid_valid = false;
     c->list_valid = false;
+    c->disp_seq = 0;
     return DSMD_OK;
 }
 
@@ -1165,7 +1258,7 @@ static int sort_owned_impl(dsmd_ctx* c, const Brick* bounds, int64_t n_outside, 
     if (n_outside < 0 || n_outside >= c->n_owned) return fail(c, DSMD_ERR_INVALID, "sort: bad count of atoms to remove");
     if (!c->grid_valid) { const int rc = make_grid(c); if (rc) return rc; }
     { const int rc = ensure_cells(c); if (rc) return rc; }
-    DSMD_CUDA(c, cudaMemsetAsync(c->status, 0, sizeof(Status), s));
+    DSMD_CUDA(c, clear_status(c, s));
     const int64_t keep_total = c->n_total;
     c->n_total = c->n_owned;   // sort the owned segment alone
     const int rc = sort_range(c, 0, s, n_outside, bounds);
@@ -1213,7 +1306,7 @@ int dsmd_build_neighbor_list(dsmd_ctx* c, void* stream) {
     //    status words of that sort are then still unread and are kept)
     const int64_t first = c->owned_sorted_only ? c->n_owned : 0;
     const int64_t expect_dropped = c->owned_sorted_only ? c->expect_dropped : 0;
-    if (!c->owned_sorted_only) DSMD_CUDA(c, cudaMemsetAsync(c->status, 0, sizeof(Status), s));
+    if (!c->owned_sorted_only) DSMD_CUDA(c, clear_status(c, s));
     c->owned_sorted_only = false;
     c->expect_dropped = 0;
     if (first == 0 || c->n_total > first) { const int rc = sort_range(c, first, s); if (rc) return rc; }
@@ -1287,12 +1380,12 @@ int dsmd_build_neighbor_list(dsmd_ctx* c, void* stream) {
         if (c->h_status->need_stride <= static_cast<unsigned>(c->stride)) break;
         // a row overflowed: grow and build again
         row_entries = static_cast<int>(c->h_status->need_stride * 1.1) + 8;
-        DSMD_CUDA(c, cudaMemsetAsync(c->status, 0, sizeof(Status), s));
+        DSMD_CUDA(c, clear_status(c, s));
         if (attempt == 3) return fail(c, DSMD_ERR_CAPACITY, "neighbour rows kept overflowing");
     }
     c->n_boundary = static_cast<int64_t>(c->h_status->boundary_pairs);
     ++c->build_epoch;
-    DSMD_CUDA(c, cudaMemsetAsync(c->status, 0, sizeof(Status), s));   // displacement word restarts at zero
+    DSMD_CUDA(c, clear_status(c, s));   // displacement word restarts at zero
     c->list_valid = true;
     return DSMD_OK;
 }
@@ -1369,17 +1462,18 @@ int dsmd_list_export(dsmd_ctx* c, int32_t* d_i, int32_t* d_j, uint8_t* d_flags, 
 static int pack_impl(dsmd_ctx* c, int64_t first, int64_t count, bool integrate, double dt, double f2a, cudaStream_t s,
                      double kick = 0.5, const unsigned char* skip = nullptr) {
     if (count <= 0) return DSMD_OK;
+    const DisplacementReport report = displacement_report(c, first == 0 && count >= c->n_owned, s);
     double** r = c->real[c->cur];
     if (integrate)
         k_pack<true><<<blocks_for(count, kThreads), kThreads, 0, s>>>(
             c->grid, static_cast<int>(first), static_cast<int>(count), static_cast<int>(c->n_owned), r[0], r[1], r[2],
             r[3], r[4], r[5], r[6], r[7], r[8], r[9], c->type[c->cur], c->ref[0], c->ref[1], c->ref[2], c->pq, dt,
-            kick * dt * f2a, c->gid[c->cur], skip, c->status);
+            kick * dt * f2a, c->gid[c->cur], skip, report);
     else
         k_pack<false><<<blocks_for(count, kThreads), kThreads, 0, s>>>(
             c->grid, static_cast<int>(first), static_cast<int>(count), static_cast<int>(c->n_owned), r[0], r[1], r[2],
             r[3], r[4], r[5], r[6], r[7], r[8], r[9], c->type[c->cur], c->ref[0], c->ref[1], c->ref[2], c->pq, 0.0, 0.0,
-            c->gid[c->cur], nullptr, c->status);
+            c->gid[c->cur], nullptr, report);
     DSMD_LAUNCHED(c);
     return DSMD_OK;
 }
@@ -1393,13 +1487,19 @@ int dsmd_pack_positions(dsmd_ctx* c, int64_t first, int64_t count, void* stream)
 int dsmd_max_displacement_sq(dsmd_ctx* c, double* out, void* stream) {
     if (!c || !out) return DSMD_ERR_INVALID;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    { const int rc = read_status(c, s); if (rc) return rc; }
-    double v;
-    const unsigned long long bits = c->h_status->max_disp2;
-    std::memcpy(&v, &bits, sizeof(v));
-    *out = v;
-    if (c->h_status->out_of_domain)
-        return fail(c, DSMD_ERR_OUT_OF_DOMAIN, "an atom left the subdomain + halo, or has a NaN position");
+    bool outside;
+    if (c->disp_seq && !c->captured) {   // nothing has touched the status since the last displacement check: its report says it all
+        DSMD_CUDA(c, cudaStreamSynchronize(s));
+        const int slot = kMailDisplacement + static_cast<int>(c->disp_seq & 3);
+        { const int rc = wait_mail(c, slot, c->disp_seq, s); if (rc) return rc; }
+        *out = c->mail[slot].value[0];
+        outside = c->mail[slot].value[1] != 0.0;
+    } else {
+        { const int rc = read_status(c, s); if (rc) return rc; }
+        std::memcpy(out, &c->h_status->max_disp2, sizeof(*out));
+        outside = c->h_status->out_of_domain != 0;
+    }
+    if (outside) return fail(c, DSMD_ERR_OUT_OF_DOMAIN, "an atom left the subdomain + halo, or has a NaN position");
     return DSMD_OK;
 }
 
@@ -1425,20 +1525,11 @@ int dsmd_max_displacement_sq_lagged(dsmd_ctx* c, double* out, void* stream) {
     return DSMD_OK;
 }
 
-// The pair kernel over the pair rows first .. first + count of a FULL or INTERIOR pass without energy (count < 0: all of
-// them, any phase), or over the pairs with a ghost partner (BOUNDARY).
-static int compute_forces_impl(dsmd_ctx* c, int phase, int want_energy, int64_t first, int64_t count, void* stream) {
-    if (!c || phase < DSMD_PHASE_FULL || phase > DSMD_PHASE_BOUNDARY) return DSMD_ERR_INVALID;
-    if (!c->list_valid) return fail(c, DSMD_ERR_STATE, "build the neighbour list before computing forces");
-    const bool ranged = count >= 0;
-    if (ranged && (phase == DSMD_PHASE_BOUNDARY || want_energy || first < 0 || first + count > 2 * c->n_quads))
-        return fail(c, DSMD_ERR_INVALID, "a range of pair rows is for FULL or INTERIOR passes without energy");
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
+static PairParams pair_params(const dsmd_ctx* c) {
     PairParams p{};
     for (int a = 0; a < 3; ++a) p.scale[a] = c->grid.scale[a];
     p.rc2 = static_cast<float>(c->cutoff * c->cutoff);
-    const bool sw = c->switch_distance > 0.0;
-    if (sw) {
+    if (c->switch_distance > 0.0) {
         const double rs2 = c->switch_distance * c->switch_distance, d = c->cutoff * c->cutoff - rs2;
         p.rs2 = static_cast<float>(rs2);
         p.inv_denom = static_cast<float>(1.0 / (d * d * d));
@@ -1454,20 +1545,61 @@ static int compute_forces_impl(dsmd_ctx* c, int phase, int want_energy, int64_t 
     p.ntypes = c->ntypes;
     p.lj = c->lj;
     p.type_charge = c->coulomb ? c->type_charge : nullptr;
+    return p;
+}
+
+// The pair kernel over the pair rows first .. first + count of a FULL or INTERIOR pass without energy (count < 0: all of
+// them, any phase), or over the pairs with a ghost partner (BOUNDARY).
+static int compute_forces_impl(dsmd_ctx* c, int phase, int want_energy, int64_t first, int64_t count, void* stream) {
+    if (!c || phase < DSMD_PHASE_FULL || phase > DSMD_PHASE_BOUNDARY) return DSMD_ERR_INVALID;
+    if (!c->list_valid) return fail(c, DSMD_ERR_STATE, "build the neighbour list before computing forces");
+    const bool ranged = count >= 0;
+    if (ranged && (phase == DSMD_PHASE_BOUNDARY || want_energy || first < 0 || first + count > 2 * c->n_quads))
+        return fail(c, DSMD_ERR_INVALID, "a range of pair rows is for FULL or INTERIOR passes without energy");
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const bool sw = c->switch_distance > 0.0;
+    const PairParams p = pair_params(c);
     // the boundary pass runs over the pairs the list build found a ghost partner for (none: nothing to launch)
     const int64_t pairs = phase == DSMD_PHASE_BOUNDARY ? c->n_boundary : (ranged ? count : 2 * c->n_quads);
     const bool e = want_energy != 0;
     if (e) { const int rc = ensure_partials(c, std::max<int64_t>(pair_blocks(c, pairs, true), 1)); if (rc) return rc; }
+    const bool report = e && reports_count(c, s);
     double** r = c->real[c->cur];
     const ForceArgs a{c->pq, c->qf, rows_of(c), phase, phase == DSMD_PHASE_BOUNDARY ? c->boundary_pairs : nullptr,
                       static_cast<int>(ranged ? first : 0), static_cast<int>(pairs), c->lane_shift, r[DSMD_FX], r[DSMD_FY], r[DSMD_FZ], c->partials,
-                      c->tickets, c->scalars};
+                      c->tickets, c->scalars, report ? c->mail + kMailScalars : nullptr, report ? ++c->seq : 0};
+    if (e && pairs > 0) c->scalars_seq = a.seq;
     if (pairs > 0) {   // else nothing to add to the forces; the energy sums of a boundary pass stay as the interior pass left them
         const int copies = ewald_copies(c);
         const int rc = copies == 0 ? launch_pair_types<0>(c, p, a, e, sw, s)
                                    : (copies == 1 ? launch_pair_types<1>(c, p, a, e, sw, s) : launch_pair_types<kEwaldCopiesMost>(c, p, a, e, sw, s));
         if (rc) return rc;
     }
+    return DSMD_OK;
+}
+
+// Pair forces and, with them, the second half of this step and the first half of the next in one kernel (plain
+// Lennard-Jones systems of one rank). The atoms' forces stay inside the kernel.
+static int force_step(dsmd_ctx* c, double dt, double f2a, cudaStream_t s) {
+    const PairParams p = pair_params(c);
+    const int64_t pairs = 2 * c->n_quads;
+    double** r = c->real[c->cur];
+    const ForceArgs a{c->pq, c->qf, rows_of(c), DSMD_PHASE_FULL, nullptr, 0, static_cast<int>(pairs), c->lane_shift,
+                      nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0};
+    const StepArgs at{r[0], r[1], r[2], r[3], r[4], r[5], r[9], c->ref[0], c->ref[1], c->ref[2], c->pq_next, dt, dt * f2a};
+    const unsigned blocks = static_cast<unsigned>(pair_blocks(c, pairs, false));
+    const DisplacementReport report = displacement_report(c, true, s);
+    const auto launch = [&](auto types) {
+        constexpr int TYPES = decltype(types)::value;
+        const size_t smem = PairTables<0, false, TYPES, false>::bytes(p.ntypes, 0);
+        const auto kernel = c->switch_distance > 0.0 ? k_step<TYPES, true> : k_step<TYPES, false>;
+        kernel<<<blocks, kPairThreads<0, TYPES>, smem, s>>>(p, a, c->grid, at, report);
+    };
+    if (p.ntypes == 1) launch(std::integral_constant<int, kOneType>());
+    else if (p.ntypes <= kFewTypesMost) launch(std::integral_constant<int, kFewTypes>());
+    else launch(std::integral_constant<int, kManyTypes>());
+    DSMD_LAUNCHED(c);
+    std::swap(c->pq, c->pq_next);
     return DSMD_OK;
 }
 
@@ -1478,6 +1610,12 @@ int dsmd_compute_forces(dsmd_ctx* c, int phase, int want_energy, void* stream) {
 int dsmd_read_scalars(dsmd_ctx* c, double out[6], void* stream) {
     if (!c || !out) return DSMD_ERR_INVALID;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (c->scalars_seq && !c->captured) {
+        DSMD_CUDA(c, cudaStreamSynchronize(s));
+        { const int rc = wait_mail(c, kMailScalars, c->scalars_seq, s); if (rc) return rc; }
+        for (int k = 0; k < 6; ++k) out[k] = c->mail[kMailScalars].value[k];
+        return DSMD_OK;
+    }
     DSMD_CUDA(c, cudaMemcpyAsync(c->h_scalars, c->scalars, sizeof(double) * 6, cudaMemcpyDeviceToHost, s));
     DSMD_CUDA(c, cudaStreamSynchronize(s));
     for (int k = 0; k < 6; ++k) out[k] = c->h_scalars[k];
@@ -1517,11 +1655,12 @@ int launch_constrained(dsmd_ctx* c, bool finish, bool start, double half_kick, d
     double** r = c->real[c->cur];
     const AtomArrays at{r[0], r[1], r[2], r[3], r[4], r[5], r[6], r[7], r[8], r[9], c->type[c->cur], c->ref[0], c->ref[1], c->ref[2], c->pq};
     const unsigned blocks = blocks_for(c->n_clusters, 128);
+    const DisplacementReport report = start ? displacement_report(c, c->cl_cover_all, s) : DisplacementReport{c->status, nullptr, nullptr, 0};
     const auto launch = [&](auto shape) {
         const auto kernel = finish && start ? k_constrained<decltype(shape), true, true>
                                             : (finish ? k_constrained<decltype(shape), true, false> : k_constrained<decltype(shape), false, true>);
         kernel<<<blocks, 128, 0, s>>>(cluster_table(c), c->grid, at, half_kick, dt, c->cons_tolerance, c->cons_max_iterations, prefactor,
-                                      c->partials, c->tickets + 3, d_virial3, c->status);
+                                      c->partials, c->tickets + 3, d_virial3, report);
     };
     if (c->cl_shape == 1) launch(TriangleCluster());
     else if (c->cl_shape == 2) launch(BondCluster());
@@ -1857,11 +1996,11 @@ int dsmd_kinetic_energy(dsmd_ctx* c, double* out, void* stream) {
     { const int rc = ensure_partials(c, blocks); if (rc) return rc; }
     double** r = c->real[c->cur];
     k_kinetic<<<static_cast<unsigned>(blocks), kThreads, 0, s>>>(static_cast<int>(c->n_owned), r[3], r[4], r[5], r[9],
-                                                                 c->partials, c->tickets + 1, c->scalars + 6);
+                                                                 c->partials, c->tickets + 1, c->scalars + 6, c->mail + kMailKinetic, ++c->seq);
     DSMD_LAUNCHED(c);
-    DSMD_CUDA(c, cudaMemcpyAsync(c->h_scalars + 6, c->scalars + 6, sizeof(double), cudaMemcpyDeviceToHost, s));
     DSMD_CUDA(c, cudaStreamSynchronize(s));
-    *out = c->h_scalars[6];
+    { const int rc = wait_mail(c, kMailKinetic, c->seq, s); if (rc) return rc; }
+    *out = c->mail[kMailKinetic].value[0];
     return DSMD_OK;
 }
 
@@ -1893,41 +2032,57 @@ int dsmd_run_nve(dsmd_ctx* c, int64_t n_steps, double dt, double f2a, double hi_
     int64_t rebuilds = 0;
     double worst = 0.0;
     int since_build = 0;
-    double d_prev = 0.0, d_prev2 = 0.0;   // displacement (not squared) seen one and two steps ago (lagged mode)
-    int pending = -1;                      // read-back slot in flight
-    auto bits_to_double = [](unsigned long long b) { double v; std::memcpy(&v, &b, sizeof(v)); return v; };
+    double d_prev = 0.0, d_prev2 = 0.0;    // displacement (not squared) seen one and two steps ago (lagged mode)
+    unsigned long long pending = 0;        // the last displacement check whose report has not been looked at
+    // the loop reads the reports of its own launches only, whatever was captured before
+    struct Reporting {
+        dsmd_ctx* c;
+        bool captured;
+        ~Reporting() { c->captured |= captured; }
+    } reporting{c, c->captured};
+    c->captured = false;
+    const auto reported = [&](unsigned long long seq, double& d2) {
+        d2 = 0.0;
+        if (!seq) return static_cast<int>(DSMD_OK);   // no atoms, no check
+        const int slot = kMailDisplacement + static_cast<int>(seq & 3);
+        const int rc = wait_mail(c, slot, seq, s);
+        d2 = c->mail[slot].value[0];
+        if (!rc && !lagged && c->mail[slot].value[1] != 0.0)
+            return fail(c, DSMD_ERR_OUT_OF_DOMAIN, "an atom left the subdomain + halo, or has a NaN position");
+        return rc;
+    };
     // Between two steps of this loop nobody reads the velocities, so the second half of one step and the first half of the
-    // next (the same forces) are one pass over the atoms, with RATTLE between them where there are constraints.
-    const bool constrained = c->n_clusters > 0;
+    // next (the same forces) are one pass over the atoms, with RATTLE between them where there are constraints; and where
+    // the pair forces are all the forces there are, that pass is the end of the force kernel (k_step).
+    const bool constrained = c->n_clusters > 0, fused = !constrained && !c->coulomb && c->bonded.terms() == 0 && c->n_owned > 0;
     for (int64_t step = 0; step < n_steps; ++step) {
-        {
+        if (step == 0 || !fused) {
             const int rc = constrained && step > 0 ? constrained_halves(c, true, true, dt, f2a, s)
                                                    : dsmd_integrate(c, step > 0 ? 3 : 1, dt, f2a, s);
             if (rc) return rc;
         }
+        const unsigned long long check = c->disp_seq;   // the displacement check of the positions that are current now
         ++since_build;
         bool rebuild = every > 0 && since_build >= every;
         if (!lagged) {
             double d2 = 0.0;
-            const int rc = dsmd_max_displacement_sq(c, &d2, s);
+            const int rc = reported(check, d2);
             if (rc) return rc;
             if (d2 > limit2) rebuild = true;
             if (!rebuild) worst = std::max(worst, d2);
         } else {
-            // Read back what the previous step saw (its copy finished long ago), queue this step's copy, and decide on
-            // the linear extrapolation of the last two values, as the reference does on several ranks
-            // (src/md_simulation.cpp:1232-1245). The previous step's forces were evaluated under d_prev.
-            if (pending >= 0) {
-                DSMD_CUDA(c, cudaEventSynchronize(c->disp_event[pending]));
+            // Look at what the previous step saw (its report came long ago) and decide on the linear extrapolation of the
+            // last two values, as the reference does on several ranks (src/md_simulation.cpp:1232-1245). The previous
+            // step's forces were evaluated under d_prev.
+            if (pending) {
+                double d2 = 0.0;
+                const int rc = reported(pending, d2);
+                if (rc) return rc;
                 d_prev2 = d_prev;
-                d_prev = std::sqrt(bits_to_double(*c->h_disp[pending]));
+                d_prev = std::sqrt(d2);
                 worst = std::max(worst, d_prev * d_prev);
             }
-            const int slot = static_cast<int>(step & 1);
-            DSMD_CUDA(c, cudaMemcpyAsync(c->h_disp[slot], &c->status->max_disp2, sizeof(unsigned long long),
-                                         cudaMemcpyDeviceToHost, s));
-            DSMD_CUDA(c, cudaEventRecord(c->disp_event[slot], s));
-            pending = slot;
+            pending = check;
             const double predicted = d_prev + 1.5 * std::max(d_prev - d_prev2, 0.0);
             if (predicted * predicted > limit2) rebuild = true;
         }
@@ -1937,15 +2092,22 @@ int dsmd_run_nve(dsmd_ctx* c, int64_t n_steps, double dt, double f2a, double hi_
             ++rebuilds;
             since_build = 0;
             d_prev = d_prev2 = 0.0;
-            pending = -1;   // the copy queued above predates the new reference positions
+            pending = 0;   // that check was made against reference positions that are gone
+        }
+        if (fused && step + 1 < n_steps) {
+            const int rc = force_step(c, dt, f2a, s);
+            if (rc) return rc;
+            continue;
         }
         { const int rc = dsmd_compute_forces(c, DSMD_PHASE_FULL, 0, s); if (rc) return rc; }
         { const int rc = dsmd_compute_bonded(c, s); if (rc) return rc; }
         if (step + 1 == n_steps) { const int rc = dsmd_integrate(c, 2, dt, f2a, s); if (rc) return rc; }
     }
-    if (lagged && pending >= 0) {
-        DSMD_CUDA(c, cudaEventSynchronize(c->disp_event[pending]));
-        const double d = std::sqrt(bits_to_double(*c->h_disp[pending]));
+    if (lagged && pending) {
+        double d2 = 0.0;
+        const int rc = reported(pending, d2);
+        if (rc) return rc;
+        const double d = std::sqrt(d2);
         worst = std::max(worst, d * d);
     }
     DSMD_CUDA(c, cudaStreamSynchronize(s));
@@ -2085,6 +2247,7 @@ int dsmd_halo_unpack(dsmd_ctx* c, const double* d_in, int64_t first_ghost, int64
     if (!c->list_valid) return fail(c, DSMD_ERR_STATE, "halo unpack needs the ghost slots of a built list");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     double** r = c->real[c->cur];
+    c->disp_seq = 0;
     k_halo_unpack<<<blocks_for(count, kThreads), kThreads, 0, s>>>(c->grid, static_cast<int>(first_ghost),
                                                                   static_cast<int>(count), d_in, c->ghost_slot, r[0],
                                                                   r[1], r[2], c->type[c->cur], c->pq, c->status);

@@ -11,9 +11,11 @@
 //
 // A cluster's atoms meet nobody else between two force evaluations, so one thread takes them through the whole of it:
 // second half-kick and RATTLE, first half-kick, drift, SHAKE, conversion to fixed point and displacement check.
-// What bounds it: fp64 arithmetic of the sweeps (about 10 of them). The shapes that occur in numbers (three atoms with three
-// constraints, two atoms with one) are compiled with their constraint order known, which keeps the cluster in registers:
-// 648,000 water atoms, one step: 0.08 ms, against 0.78 ms for separate passes over clusters in local memory.
+// What bounds it: the chain of fp64 operations of the sweeps (some 20 of each kind). The shapes that occur in numbers (three
+// atoms with three constraints, two atoms with one) are compiled with their constraint order known, which keeps the cluster
+// in registers, and sweep over what the sweeps are about instead of over atoms (rattle_known, shake_known). Rigid water,
+// second half of a step and first half of the next: 0.098 ms at 648,000 atoms, 22 us at 3,993 (sweeps over the atoms'
+// positions and velocities: 0.277 ms and 60 us).
 //
 // Atoms are re-sorted by cell at every list build, so clusters name their atoms by global id; the slots are looked up
 // once per build. Clusters hold at most kClusterAtoms atoms and kClusterCons constraints.
@@ -123,32 +125,144 @@ struct Cluster {
         return false;
     }
 
+    // How the bond vector (or relative velocity) of constraint i changes per unit of a correction along constraint j, in
+    // which atom a(j) goes by -w and atom b(j) by +w.
+    __device__ __forceinline__ double coupling(int i, int j) const {
+        const int ai = Shape::a(i), bi = Shape::b(i), aj = Shape::a(j), bj = Shape::b(j);
+        double m = 0.0;
+        if (ai == aj) m -= w[aj];
+        if (ai == bj) m += w[bj];
+        if (bi == aj) m += w[aj];
+        if (bi == bj) m -= w[bj];
+        return m;
+    }
+
+    // The bond vectors of a known shape.
+    __device__ __forceinline__ void bonds(const ClusterTable& t, double (&d)[Shape::constraints][3]) const {
+#pragma unroll
+        for (int j = 0; j < Shape::constraints; ++j) {
+#pragma unroll
+            for (int x = 0; x < 3; ++x) d[j][x] = p[Shape::a(j)][x] - p[Shape::b(j)][x];
+            half_box_image(d[j], t);
+        }
+    }
+
+    // RATTLE of a known shape. A correction along one bond changes the relative velocity along the others by amounts that
+    // do not depend on the velocities, so the sweeps work on one number per constraint, d . (v_a - v_b): one dependent
+    // multiply-add per constraint instead of a pass through the atoms' velocities with a division. Atoms take the sum.
+    __device__ __forceinline__ bool rattle_known(const double (&d)[Shape::constraints][3], double tolerance, int max_iterations,
+                                                 double prefactor, double (&wsum)[3]) {
+        constexpr int N = Shape::constraints;
+        double along[N], inv[N], g[N][N], sum[N];
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            const int a = Shape::a(j), b = Shape::b(j);
+            const double r2 = d[j][0] * d[j][0] + d[j][1] * d[j][1] + d[j][2] * d[j][2];
+            along[j] = d[j][0] * (v[a][0] - v[b][0]) + d[j][1] * (v[a][1] - v[b][1]) + d[j][2] * (v[a][2] - v[b][2]);
+            inv[j] = r2 < 1e-20 ? 0.0 : 1.0 / ((w[a] + w[b]) * r2);   // no bond vector: nothing to correct
+            sum[j] = 0.0;
+        }
+#pragma unroll
+        for (int j = 0; j < N; ++j)
+#pragma unroll
+            for (int i = 0; i < N; ++i) g[i][j] = inv[j] * coupling(i, j) * (d[i][0] * d[j][0] + d[i][1] * d[j][1] + d[i][2] * d[j][2]);
+        bool done = false;
+        for (int sweep = 0; sweep < max_iterations && !done; ++sweep) {
+            done = true;
+#pragma unroll
+            for (int j = 0; j < N; ++j) {   // a constraint that holds is left alone (selected, not branched over)
+                const double now = along[j];
+                const bool holds = fabs(now) < tolerance || inv[j] == 0.0;
+                done &= holds;
+                sum[j] = holds ? sum[j] : fma(now, inv[j], sum[j]);
+#pragma unroll
+                for (int i = 0; i < N; ++i) along[i] = holds ? along[i] : fma(now, g[i][j], along[i]);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < N; ++j)
+#pragma unroll
+            for (int x = 0; x < 3; ++x) {
+                v[Shape::a(j)][x] -= sum[j] * w[Shape::a(j)] * d[j][x];
+                v[Shape::b(j)][x] += sum[j] * w[Shape::b(j)] * d[j][x];
+                wsum[x] += prefactor * sum[j] * d[j][x] * d[j][x];
+            }
+        return done;
+    }
+
+    // SHAKE of a known shape, o: the bond vectors before the drift. The sweeps work on the bond vectors and on their
+    // components along o (which change by amounts known in advance); atoms take the sum. Each component's reciprocal follows
+    // it from sweep to sweep by Newton's iteration, of third order, where it moved by less than 1 % (relative error below
+    // 1e-6 of a correction, gone with the next sweep; nothing is left of it when the sweeps end at 1e-8): half as long a
+    // chain of dependent operations as a division, and no branch.
+    __device__ __forceinline__ bool shake_known(const ClusterTable& t, int k, const double (&o)[Shape::constraints][3], double inv_dt,
+                                                double tolerance, int max_iterations) {
+        constexpr int N = Shape::constraints;
+        double d[N][3], target2[N], half_inv[N], sum[N], along[N], inv[N], move[N][N], change[N][N];
+        bonds(t, d);
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            target2[j] = t.con_d2[k * kClusterCons + j];
+            half_inv[j] = 0.5 / (w[Shape::a(j)] + w[Shape::b(j)]);
+            sum[j] = 0.0;
+            along[j] = o[j][0] * d[j][0] + o[j][1] * d[j][1] + o[j][2] * d[j][2];
+            inv[j] = fabs(along[j]) >= 1e-12 ? 1.0 / along[j] : 0.0;
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                move[i][j] = coupling(i, j);
+                change[i][j] = move[i][j] * (o[i][0] * o[j][0] + o[i][1] * o[j][1] + o[i][2] * o[j][2]);
+            }
+        }
+        bool done = false;
+        for (int sweep = 0; sweep < max_iterations && !done; ++sweep) {
+            done = true;
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                const double off = fma(-along[j], inv[j], 1.0);
+                double y = fma(inv[j], fma(off, off, off), inv[j]);
+                if (fabs(off) > 0.01) y = fabs(along[j]) >= 1e-12 ? 1.0 / along[j] : 0.0;   // 0, degenerate geometry: the next sweep tries again
+                inv[j] = y;
+                const double excess = fma(d[j][0], d[j][0], fma(d[j][1], d[j][1], fma(d[j][2], d[j][2], -target2[j])));
+                const bool holds = fabs(excess) < tolerance * target2[j];
+                done &= holds;
+                const double gm = holds ? 0.0 : excess * (half_inv[j] * y);
+                sum[j] += gm;
+#pragma unroll
+                for (int i = 0; i < N; ++i) {
+                    along[i] = fma(gm, change[i][j], along[i]);
+                    const double c = gm * move[i][j];
+#pragma unroll
+                    for (int x = 0; x < 3; ++x) d[i][x] = fma(c, o[j][x], d[i][x]);
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < N; ++j)
+#pragma unroll
+            for (int x = 0; x < 3; ++x) {
+                const int a = Shape::a(j), b = Shape::b(j);
+                const double corr = sum[j] * o[j][x];
+                p[a][x] -= corr * w[a];
+                p[b][x] += corr * w[b];
+                v[a][x] -= corr * w[a] * inv_dt;
+                v[b][x] += corr * w[b] * inv_dt;
+            }
+        return done;
+    }
+
+    // Any other shape: sweeps over the atoms.
     template <bool SHAKE>
     __device__ __forceinline__ bool solve(const ClusterTable& t, int k, const double (&q)[Shape::atoms][3], double inv_dt, double tolerance,
                                           int max_iterations, double prefactor, double (&wsum)[3]) {
-        if (Shape::known) {
-            double target2[Shape::constraints];
-#pragma unroll
-            for (int j = 0; j < Shape::constraints; ++j) target2[j] = t.con_d2[k * kClusterCons + j];
-            for (int sweep = 0; sweep < max_iterations; ++sweep) {
-                bool done = true;
-#pragma unroll
-                for (int j = 0; j < Shape::constraints; ++j)
-                    done &= SHAKE ? shake_one(t, q, Shape::a(j), Shape::b(j), target2[j], inv_dt, tolerance)
-                                  : rattle_one(t, Shape::a(j), Shape::b(j), tolerance, prefactor, wsum);
-                if (done) return true;
+        for (int sweep = 0; sweep < max_iterations; ++sweep) {
+            bool done = true;
+            for (int j = 0; j < Shape::constraints; ++j) {
+                const int a = t.con_a[k * kClusterCons + j], b = t.con_b[k * kClusterCons + j];
+                if (a == 255) break;
+                done &= SHAKE ? shake_one(t, q, a, b, t.con_d2[k * kClusterCons + j], inv_dt, tolerance)
+                              : rattle_one(t, a, b, tolerance, prefactor, wsum);
             }
-        } else {
-            for (int sweep = 0; sweep < max_iterations; ++sweep) {
-                bool done = true;
-                for (int j = 0; j < Shape::constraints; ++j) {
-                    const int a = t.con_a[k * kClusterCons + j], b = t.con_b[k * kClusterCons + j];
-                    if (a == 255) break;
-                    done &= SHAKE ? shake_one(t, q, a, b, t.con_d2[k * kClusterCons + j], inv_dt, tolerance)
-                                  : rattle_one(t, a, b, tolerance, prefactor, wsum);
-                }
-                if (done) return true;
-            }
+            if (done) return true;
         }
         return false;
     }
@@ -191,13 +305,16 @@ __global__ void __launch_bounds__(128) k_constrained(ClusterTable t, Grid g, Ato
                 a[m][0] = a[m][1] = a[m][2] = 0.0;
             }
         }
+        double o[Shape::constraints][3];   // bond vectors before the drift
+        if constexpr (Shape::known) c.bonds(t, o);
         bool good = true;
         if (FINISH) {
 #pragma unroll
             for (int m = 0; m < Shape::atoms; ++m)
                 if (Shape::known || m < c.n)
                     for (int x = 0; x < 3; ++x) c.v[m][x] += a[m][x];
-            good &= c.template solve<false>(t, k, c.p, 0.0, tolerance, max_iterations, prefactor, wsum);
+            if constexpr (Shape::known) good &= c.rattle_known(o, tolerance, max_iterations, prefactor, wsum);
+            else good &= c.template solve<false>(t, k, c.p, 0.0, tolerance, max_iterations, prefactor, wsum);
         }
         if (START) {
             double q[Shape::atoms][3];
@@ -215,7 +332,8 @@ __global__ void __launch_bounds__(128) k_constrained(ClusterTable t, Grid g, Ato
                     }
                     worst2 = fmax(worst2, d2 == d2 ? d2 : __longlong_as_double(0x7FF0000000000000ll));   // see k_pack
                 }
-            good &= c.template solve<true>(t, k, q, 1.0 / dt, tolerance, max_iterations, 0.0, wsum);
+            if constexpr (Shape::known) good &= c.shake_known(t, k, o, 1.0 / dt, tolerance, max_iterations);
+            else good &= c.template solve<true>(t, k, q, 1.0 / dt, tolerance, max_iterations, 0.0, wsum);
         }
         unsigned bad = 0;
 #pragma unroll

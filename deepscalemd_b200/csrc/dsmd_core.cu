@@ -262,48 +262,6 @@ __device__ __forceinline__ void report_displacement(double v, const Displacement
     }
 }
 
-// INTEGRATE: kick and drift before the pack (v += kick_c f / m, x += dt v): the first velocity-Verlet half with
-// kick_c = dt/2 (times the force-to-acceleration factor), or, with kick_c = dt, the second half of the previous step and
-// the first half of this one in one pass (both use the same forces).
-template <bool INTEGRATE>
-__global__ void k_pack(Grid g, int first, int count, int n_owned, double* __restrict__ x, double* __restrict__ y,
-                       double* __restrict__ z, double* __restrict__ vx, double* __restrict__ vy,
-                       double* __restrict__ vz, const double* __restrict__ fx, const double* __restrict__ fy,
-                       const double* __restrict__ fz, const double* __restrict__ mass, const int* __restrict__ type,
-                       const double* __restrict__ xref, const double* __restrict__ yref,
-                       const double* __restrict__ zref, int4* __restrict__ pq, double dt, double kick_c,
-                       const int* __restrict__ gid, const unsigned char* __restrict__ skip, DisplacementReport report) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int s = first + t;
-    double d2 = 0.0;
-    if (t < count && !(skip && skip[gid[s]])) {   // skip: atoms of constraint clusters, by global id (k_constrained moves them)
-        double px = x[s], py = y[s], pz = z[s];
-        if (INTEGRATE) {
-            const double a = kick_c / mass[s];
-            const double ux = vx[s] + a * fx[s], uy = vy[s] + a * fy[s], uz = vz[s] + a * fz[s];
-            vx[s] = ux; vy[s] = uy; vz[s] = uz;
-            px += dt * ux; py += dt * uy; pz += dt * uz;
-            x[s] = px; y[s] = py; z[s] = pz;
-        }
-        unsigned bad = 0;
-        int4 p;
-        p.x = static_cast<int>(dsmd::to_fixed(px, 0, g, bad));
-        p.y = static_cast<int>(dsmd::to_fixed(py, 1, g, bad));
-        p.z = static_cast<int>(dsmd::to_fixed(pz, 2, g, bad));
-        p.w = type[s];
-        pq[s] = p;
-        if (bad) atomicAdd(&report.st->out_of_domain, 1u);
-        if (s < n_owned) {
-            const double ddx = px - xref[s], ddy = py - yref[s], ddz = pz - zref[s];
-            d2 = ddx * ddx + ddy * ddy + ddz * ddz;
-            // a position that is no number must not vanish in the block maximum (fmax drops NaN): it forces a rebuild,
-            // and the rebuild reports the atom
-            if (!(d2 == d2)) d2 = __longlong_as_double(0x7FF0000000000000ll);
-        }
-    }
-    report_displacement(d2, report);
-}
-
 __global__ void k_vv2(int n, double half_dt_c, double* __restrict__ vx, double* __restrict__ vy,
                       double* __restrict__ vz, const double* __restrict__ fx, const double* __restrict__ fy,
                       const double* __restrict__ fz, const double* __restrict__ mass, const int* __restrict__ gid,
@@ -390,6 +348,51 @@ __global__ void k_kinetic(int n, const double* __restrict__ vx, const double* __
 #include "dsmd_pair.cuh"
 
 namespace {
+
+// INTEGRATE: kick and drift before the pack (v += kick_c f / m, x += dt v): the first velocity-Verlet half with
+// kick_c = dt/2 (times the force-to-acceleration factor), or, with kick_c = dt, the second half of the previous step and
+// the first half of this one in one pass (both use the same forces).
+// BONDED: the forces of the bonded terms are not in the force arrays yet.
+template <bool INTEGRATE, bool BONDED>
+__global__ void k_pack(Grid g, int first, int count, int n_owned, double* __restrict__ x, double* __restrict__ y,
+                       double* __restrict__ z, double* __restrict__ vx, double* __restrict__ vy,
+                       double* __restrict__ vz, const double* __restrict__ fx, const double* __restrict__ fy,
+                       const double* __restrict__ fz, const double* __restrict__ mass, const int* __restrict__ type,
+                       const double* __restrict__ xref, const double* __restrict__ yref,
+                       const double* __restrict__ zref, int4* __restrict__ pq, double dt, double kick_c,
+                       const int* __restrict__ gid, const unsigned char* __restrict__ skip, BondedForces bonded, DisplacementReport report) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int s = first + t;
+    double d2 = 0.0;
+    if (t < count && !(skip && skip[gid[s]])) {   // skip: atoms of constraint clusters, by global id (k_constrained moves them)
+        double px = x[s], py = y[s], pz = z[s];
+        if (INTEGRATE) {
+            const double a = kick_c / mass[s];
+            double f[3] = {0.0, 0.0, 0.0};
+            if (BONDED) bonded_force(bonded, s, f);
+            const double ux = vx[s] + a * (fx[s] + f[0]), uy = vy[s] + a * (fy[s] + f[1]), uz = vz[s] + a * (fz[s] + f[2]);
+            vx[s] = ux; vy[s] = uy; vz[s] = uz;
+            px += dt * ux; py += dt * uy; pz += dt * uz;
+            x[s] = px; y[s] = py; z[s] = pz;
+        }
+        unsigned bad = 0;
+        int4 p;
+        p.x = static_cast<int>(dsmd::to_fixed(px, 0, g, bad));
+        p.y = static_cast<int>(dsmd::to_fixed(py, 1, g, bad));
+        p.z = static_cast<int>(dsmd::to_fixed(pz, 2, g, bad));
+        p.w = type[s];
+        pq[s] = p;
+        if (bad) atomicAdd(&report.st->out_of_domain, 1u);
+        if (s < n_owned) {
+            const double ddx = px - xref[s], ddy = py - yref[s], ddz = pz - zref[s];
+            d2 = ddx * ddx + ddy * ddy + ddz * ddz;
+            // a position that is no number must not vanish in the block maximum (fmax drops NaN): it forces a rebuild,
+            // and the rebuild reports the atom
+            if (!(d2 == d2)) d2 = __longlong_as_double(0x7FF0000000000000ll);
+        }
+    }
+    report_displacement(d2, report);
+}
 
 // ---------------------------------------------------------------------------------------------------------------------
 // kernels: ghosts
@@ -600,8 +603,8 @@ struct dsmd_ctx {
         double *bond_par = nullptr, *angle_par = nullptr, *torsion_par = nullptr, *special_par = nullptr;
         int* slot_of_gid = nullptr;          // [n_global]
         long long* entries_of = nullptr;     // [n_global + 1]
-        int* entry = nullptr;                // [n_entries]
-        double* contrib = nullptr;           // [3 * n_entries]
+        int* place = nullptr;                // [n_entries]
+        double* contrib = nullptr;           // [3 * n_entries], by global id
         double* partials = nullptr;          // [5 * blocks]
         double* scalars = nullptr;           // device: PE, W, Wxx, Wyy, Wzz
         unsigned* missing = nullptr;         // device: terms with an owned atom and a partner that is not on this rank
@@ -655,7 +658,7 @@ void free_bonded(dsmd_ctx* c) {
     dsmd_ctx::Bonded& b = c->bonded;
     cudaFree(b.bond_atoms); cudaFree(b.angle_atoms); cudaFree(b.torsion_atoms); cudaFree(b.torsion_n); cudaFree(b.special_atoms);
     cudaFree(b.bond_par); cudaFree(b.angle_par); cudaFree(b.torsion_par); cudaFree(b.special_par);
-    cudaFree(b.slot_of_gid); cudaFree(b.entries_of); cudaFree(b.entry); cudaFree(b.contrib); cudaFree(b.partials);
+    cudaFree(b.slot_of_gid); cudaFree(b.entries_of); cudaFree(b.place); cudaFree(b.contrib); cudaFree(b.partials);
     cudaFree(b.scalars); cudaFree(b.missing);
     if (b.h_scalars) cudaFreeHost(b.h_scalars);
     b = dsmd_ctx::Bonded();
@@ -1460,20 +1463,15 @@ int dsmd_list_export(dsmd_ctx* c, int32_t* d_i, int32_t* d_j, uint8_t* d_flags, 
 
 // kick: 0.5 for the first velocity-Verlet half, 1.0 for the merged second-and-first half.
 static int pack_impl(dsmd_ctx* c, int64_t first, int64_t count, bool integrate, double dt, double f2a, cudaStream_t s,
-                     double kick = 0.5, const unsigned char* skip = nullptr) {
+                     double kick = 0.5, const unsigned char* skip = nullptr, const BondedForces* bonded = nullptr) {
     if (count <= 0) return DSMD_OK;
     const DisplacementReport report = displacement_report(c, first == 0 && count >= c->n_owned, s);
     double** r = c->real[c->cur];
-    if (integrate)
-        k_pack<true><<<blocks_for(count, kThreads), kThreads, 0, s>>>(
-            c->grid, static_cast<int>(first), static_cast<int>(count), static_cast<int>(c->n_owned), r[0], r[1], r[2],
-            r[3], r[4], r[5], r[6], r[7], r[8], r[9], c->type[c->cur], c->ref[0], c->ref[1], c->ref[2], c->pq, dt,
-            kick * dt * f2a, c->gid[c->cur], skip, report);
-    else
-        k_pack<false><<<blocks_for(count, kThreads), kThreads, 0, s>>>(
-            c->grid, static_cast<int>(first), static_cast<int>(count), static_cast<int>(c->n_owned), r[0], r[1], r[2],
-            r[3], r[4], r[5], r[6], r[7], r[8], r[9], c->type[c->cur], c->ref[0], c->ref[1], c->ref[2], c->pq, 0.0, 0.0,
-            c->gid[c->cur], nullptr, report);
+    const auto kernel = !integrate ? k_pack<false, false> : (bonded ? k_pack<true, true> : k_pack<true, false>);
+    kernel<<<blocks_for(count, kThreads), kThreads, 0, s>>>(
+        c->grid, static_cast<int>(first), static_cast<int>(count), static_cast<int>(c->n_owned), r[0], r[1], r[2], r[3], r[4], r[5],
+        r[6], r[7], r[8], r[9], c->type[c->cur], c->ref[0], c->ref[1], c->ref[2], c->pq, dt, kick * dt * f2a, c->gid[c->cur], skip,
+        bonded ? *bonded : BondedForces{}, report);
     DSMD_LAUNCHED(c);
     return DSMD_OK;
 }
@@ -1902,12 +1900,12 @@ int dsmd_set_bonded(dsmd_ctx* c, int64_t n_global, int64_t n_bonds, const int32_
             ++entries_of[static_cast<size_t>(g) + 1];
         }
     for (int64_t g = 0; g < n_global; ++g) entries_of[g + 1] += entries_of[g];
-    std::vector<int> entry(static_cast<size_t>(n_entries));
+    std::vector<int> place(static_cast<size_t>(n_entries));
     {
         std::vector<long long> next(entries_of.begin(), entries_of.end() - 1);
-        int place = 0;
+        size_t k = 0;
         for (const std::vector<int>* t : tables)
-            for (int g : *t) entry[static_cast<size_t>(next[g]++)] = place++;
+            for (int g : *t) place[k++] = static_cast<int>(next[g]++);
     }
     dsmd_ctx::Bonded& b = c->bonded;
     DSMD_TO_DEVICE(c, b.bond_atoms, ba);
@@ -1920,8 +1918,8 @@ int dsmd_set_bonded(dsmd_ctx* c, int64_t n_global, int64_t n_bonds, const int32_
     DSMD_TO_DEVICE(c, b.torsion_par, tp);
     DSMD_TO_DEVICE(c, b.special_par, sp);
     DSMD_TO_DEVICE(c, b.entries_of, entries_of);
-    DSMD_TO_DEVICE(c, b.entry, entry);
-    b.blocks = blocks_for(terms, kThreads);
+    DSMD_TO_DEVICE(c, b.place, place);
+    b.blocks = blocks_for(terms, kBondedThreads);
     DSMD_CUDA(c, cudaMalloc(&b.slot_of_gid, sizeof(int) * std::max<int64_t>(n_global, 1)));
     DSMD_CUDA(c, cudaMalloc(&b.contrib, sizeof(double) * 3 * n_entries));
     DSMD_CUDA(c, cudaMalloc(&b.partials, sizeof(double) * 5 * b.blocks));
@@ -1937,12 +1935,11 @@ int dsmd_set_bonded(dsmd_ctx* c, int64_t n_global, int64_t n_bonds, const int32_
     return DSMD_OK;
 }
 
-int dsmd_compute_bonded(dsmd_ctx* c, void* stream) {
-    if (!c) return DSMD_ERR_INVALID;
+// The terms' contributions into their scratch array.
+static int bonded_terms(dsmd_ctx* c, bool sums, cudaStream_t s) {
     dsmd_ctx::Bonded& b = c->bonded;
     if (b.terms() == 0) return DSMD_OK;
     if (!c->list_valid) return fail(c, DSMD_ERR_STATE, "no neighbour list built yet (bonded terms find their atoms through the sorted arrays)");
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (b.map_epoch != c->build_epoch) {   // the sort of a list build moved the atoms
         DSMD_CUDA(c, cudaMemsetAsync(b.slot_of_gid, 0x7F, sizeof(int) * b.n_global, s));   // 0x7F7F7F7F: beyond any slot
         k_bonded_slot_map<<<blocks_for(c->n_total, kThreads), kThreads, 0, s>>>(static_cast<int>(c->n_total), c->gid[c->cur],
@@ -1951,6 +1948,7 @@ int dsmd_compute_bonded(dsmd_ctx* c, void* stream) {
         b.map_epoch = c->build_epoch;
     }
     BondedTable t{};
+    t.place = b.place;
     t.n_bonds = static_cast<int>(b.n_bonds); t.n_angles = static_cast<int>(b.n_angles);
     t.n_torsions = static_cast<int>(b.n_torsions); t.n_specials = static_cast<int>(b.n_specials);
     t.bond_atoms = b.bond_atoms; t.bond_par = b.bond_par; t.angle_atoms = b.angle_atoms; t.angle_par = b.angle_par;
@@ -1961,12 +1959,24 @@ int dsmd_compute_bonded(dsmd_ctx* c, void* stream) {
     t.n_owned = static_cast<int>(c->n_owned);
     for (int a = 0; a < 3; ++a) { t.box[a] = c->box[a]; t.periodic[a] = c->periodic[a]; }
     double** r = c->real[c->cur];
-    k_bonded_terms<<<static_cast<unsigned>(b.blocks), kThreads, 0, s>>>(t, r[0], r[1], r[2], r[10], b.contrib, b.partials,
-                                                                        c->tickets + 2, b.scalars, b.missing);
+    const auto kernel = sums ? k_bonded_terms<true> : k_bonded_terms<false>;
+    kernel<<<static_cast<unsigned>(b.blocks), kBondedThreads, 0, s>>>(t, r[0], r[1], r[2], r[10], b.contrib, b.partials, c->tickets + 2,
+                                                                      b.scalars, b.missing);
     DSMD_LAUNCHED(c);
-    k_bonded_gather<<<blocks_for(c->n_owned, kThreads), kThreads, 0, s>>>(static_cast<int>(c->n_owned), c->gid[c->cur],
-                                                                         static_cast<int>(b.n_global), b.entries_of, b.entry,
-                                                                         b.contrib, r[6], r[7], r[8]);
+    return DSMD_OK;
+}
+
+static BondedForces bonded_forces(const dsmd_ctx* c) {
+    return BondedForces{c->gid[c->cur], static_cast<int>(c->bonded.n_global), c->bonded.entries_of, c->bonded.contrib};
+}
+
+int dsmd_compute_bonded(dsmd_ctx* c, void* stream) {
+    if (!c) return DSMD_ERR_INVALID;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (c->bonded.terms() == 0) return DSMD_OK;
+    { const int rc = bonded_terms(c, true, s); if (rc) return rc; }
+    double** r = c->real[c->cur];
+    k_bonded_gather<<<blocks_for(c->n_owned, kThreads), kThreads, 0, s>>>(static_cast<int>(c->n_owned), bonded_forces(c), r[6], r[7], r[8]);
     DSMD_LAUNCHED(c);
     return DSMD_OK;
 }
@@ -2054,10 +2064,13 @@ int dsmd_run_nve(dsmd_ctx* c, int64_t n_steps, double dt, double f2a, double hi_
     // Between two steps of this loop nobody reads the velocities, so the second half of one step and the first half of the
     // next (the same forces) are one pass over the atoms, with RATTLE between them where there are constraints; and where
     // the pair forces are all the forces there are, that pass is the end of the force kernel (k_step).
-    const bool constrained = c->n_clusters > 0, fused = !constrained && !c->coulomb && c->bonded.terms() == 0 && c->n_owned > 0;
+    const bool constrained = c->n_clusters > 0, bonded = !constrained && c->bonded.terms() > 0;
+    const bool fused = !constrained && !bonded && !c->coulomb && c->n_owned > 0;
     for (int64_t step = 0; step < n_steps; ++step) {
         if (step == 0 || !fused) {
+            const BondedForces terms = bonded_forces(c);
             const int rc = constrained && step > 0 ? constrained_halves(c, true, true, dt, f2a, s)
+                           : bonded && step > 0    ? pack_impl(c, 0, c->n_owned, true, dt, f2a, s, 1.0, nullptr, &terms)
                                                    : dsmd_integrate(c, step > 0 ? 3 : 1, dt, f2a, s);
             if (rc) return rc;
         }
@@ -2100,7 +2113,9 @@ int dsmd_run_nve(dsmd_ctx* c, int64_t n_steps, double dt, double f2a, double hi_
             continue;
         }
         { const int rc = dsmd_compute_forces(c, DSMD_PHASE_FULL, 0, s); if (rc) return rc; }
-        { const int rc = dsmd_compute_bonded(c, s); if (rc) return rc; }
+        // (between two steps the bonded contributions go straight into the pass over the atoms)
+        if (bonded && step + 1 < n_steps) { const int rc = bonded_terms(c, false, s); if (rc) return rc; }
+        else { const int rc = dsmd_compute_bonded(c, s); if (rc) return rc; }
         if (step + 1 == n_steps) { const int rc = dsmd_integrate(c, 2, dt, f2a, s); if (rc) return rc; }
     }
     if (lagged && pending) {

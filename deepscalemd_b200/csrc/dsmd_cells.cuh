@@ -1,0 +1,28 @@
+// Sort of atoms by cell, stable: atoms of a cell in the order of their index. A counting sort: atoms count themselves into
+// their cells (k_*_keys of the callers, arrival order), a scan over the cells gives the cell starts, k_cell_place lists the
+// atoms of each cell in arrival order, and whoever reads the list ranks an atom among the few of its cell (cell_slot).
+//
+// Against a radix sort of (cell, index) pairs: two light passes instead of a histogram and three heavy ones, and the cell
+// starts come with it. What bounds it: launches and atomics to L2 (small systems), scattered 4-byte writes (large ones).
+// The ranking is quadratic in the atoms of a cell, as the neighbour search behind it is.
+#pragma once
+
+#include <cuda_runtime.h>
+
+namespace dsmd {
+
+static __global__ void k_cell_place(int n, const unsigned* __restrict__ key, const int* __restrict__ arrival, const int* __restrict__ cell_start,
+                             int* __restrict__ list) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) list[cell_start[key[i]] + arrival[i]] = i;
+}
+
+// Final slot of the atom `a` of cell `cell`.
+__device__ __forceinline__ int cell_slot(int a, unsigned cell, const int* __restrict__ cell_start, const int* __restrict__ list) {
+    const int begin = cell_start[cell], end = cell_start[cell + 1];
+    int slot = begin;
+    for (int k = begin; k < end; ++k) slot += list[k] < a ? 1 : 0;
+    return slot;
+}
+
+}  // namespace dsmd

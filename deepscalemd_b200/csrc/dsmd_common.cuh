@@ -108,9 +108,10 @@ __device__ __forceinline__ bool row_window(const Grid& g, const int4& pi, int cy
     const float d2 = gy * gy + gz * gz;
     const float reach2 = g.r_pad * g.r_pad;
     if (d2 >= reach2) return false;
-    float hw = sqrtf(reach2 - d2);
+    // (approximations good to 1e-6: r_pad carries 1e-4)
+    float hw = (reach2 - d2) * rsqrtf(reach2 - d2);
     hw = fminf(hw, g.x_reach);
-    const unsigned hw_fixed = static_cast<unsigned>(hw / g.scale[0]) + 1u;
+    const unsigned hw_fixed = static_cast<unsigned>(hw * (1.0f / g.scale[0])) + 1u;
     w.a1 = 0;
     w.b1 = -1;
     if (g.wrap[0]) {

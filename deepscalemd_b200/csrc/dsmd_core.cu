@@ -28,10 +28,13 @@
 
 #include "../../include/dsmd_b200.h"
 #include "dsmd_common.cuh"
+#include "dsmd_report.cuh"
 #include "ewald_table.hpp"
 
 using dsmd::Grid;
+using dsmd::Mail;
 using dsmd::Status;
+using dsmd::post;
 
 namespace {
 
@@ -212,21 +215,6 @@ __global__ void k_ghost_rows_near(Grid g, const int* __restrict__ lo_end, const 
 // ---------------------------------------------------------------------------------------------------------------------
 // kernels: per-step pack, displacement, integration
 // ---------------------------------------------------------------------------------------------------------------------
-
-// Values that the host waits for leave a kernel through pinned host memory: the block that finishes last writes them and
-// then the number of the launch, which the host polls (host/mail in dsmd_ctx). That saves the copy behind the kernel and
-// the wait for the copy: 3 us instead of 9 per value.
-struct Mail {
-    double value[7];
-    unsigned long long seq;
-};
-
-__device__ __forceinline__ void post(Mail* mail, const double* v, int n, unsigned long long seq) {   // one thread
-    volatile Mail* m = mail;
-    for (int k = 0; k < n; ++k) m->value[k] = v[k];
-    __threadfence_system();
-    m->seq = seq;
-}
 
 // Who writes where when a displacement check ends.
 struct DisplacementReport {
@@ -906,25 +894,9 @@ cudaError_t clear_status(dsmd_ctx* c, cudaStream_t s) {
     return cudaMemsetAsync(c->status, 0, sizeof(Status), s);
 }
 
-// Waits for the report of a launch on `s`. The launch is in the stream; the loop ends with an error when the stream has run
-// dry (or failed) without it.
 int wait_mail(dsmd_ctx* c, int slot, unsigned long long seq, cudaStream_t s) {
-    const volatile Mail* m = c->mail + slot;
-    for (unsigned spins = 1;; ++spins) {
-        if (m->seq == seq) {
-            std::atomic_thread_fence(std::memory_order_acquire);
-            return DSMD_OK;
-        }
-        if ((spins & 0x3FFu) == 0) {
-            const cudaError_t q = cudaStreamQuery(s);
-            if (q == cudaErrorNotReady) continue;
-            // done or failed; the caller may have named another stream than the launch's
-            DSMD_CUDA(c, q);
-            DSMD_CUDA(c, cudaDeviceSynchronize());
-            if (m->seq == seq) continue;
-            return fail(c, DSMD_ERR_CUDA, "a kernel ended without its report");
-        }
-    }
+    const cudaError_t e = dsmd::wait_report(c->mail + slot, seq, s);
+    return e == cudaSuccess ? static_cast<int>(DSMD_OK) : fail(c, DSMD_ERR_CUDA, std::string("waiting for a kernel's report: ") + cudaGetErrorString(e));
 }
 
 // Reports carry the number of their launch, which a replayed graph would repeat: a context that was ever captured copies.

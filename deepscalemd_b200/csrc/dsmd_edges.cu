@@ -205,6 +205,7 @@ __device__ __forceinline__ void finish_search(const SearchArgs& a, int count) {
 }
 
 constexpr unsigned kUndecided = 0x80000000u;   // in a row: inside the rounding band
+constexpr int kAtATime = 3;                    // candidates in flight per thread (0.535 ms per graph of 1,000,000; 0.54 to 0.57 ms with 2, 4, 6)
 
 // One thread per sorted slot; hits go to the slot's column of its 32-atom slice: the neighbour's atom index, or, PERIODIC
 // (all axes wrap), its sorted slot (the expansion reads the neighbour's position by slot).
@@ -212,7 +213,7 @@ constexpr unsigned kUndecided = 0x80000000u;   // in a row: inside the rounding 
 // What bounds it: instruction issue. The loop over the candidates of a cell row does nothing but three subtractions, a sum
 // of squares and a comparison on float places: the image of a cell row is known (the row's window crosses the boundary or
 // not), so the atom's own place is shifted instead of taking nearest images of every candidate; hits inside the rounding
-// band are marked and decided in fp64 afterwards. 1,000,000 atoms, 100 candidates and 26 hits each: 0.33 ms (0.35 ms before).
+// band are marked and decided in fp64 afterwards. 1,000,000 atoms, 100 candidates and 26 hits each: 0.28 ms (0.35 ms before).
 template <bool PERIODIC>
 __global__ void __launch_bounds__(kSearchThreads) k_edge_search(Grid g, SearchArgs a) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -224,7 +225,7 @@ __global__ void __launch_bounds__(kSearchThreads) k_edge_search(Grid g, SearchAr
         const float fx = place_of(pi.x, g.scale[0]), fy = place_of(pi.y, g.scale[1]), fz = place_of(pi.z, g.scale[2]);
         const float len[3] = {static_cast<float>(g.box[0]), static_cast<float>(g.box[1]), static_cast<float>(g.box[2])};   // PERIODIC
         const float near2 = g.r2_list - a.band, far2 = g.r2_list + a.band;
-        bool undecided = false;
+        unsigned undecided = 0u;
         const int cx = static_cast<int>(dsmd::cell_of(static_cast<unsigned>(pi.x), g.wrap[0], g.nc[0]));
         const int cy = static_cast<int>(dsmd::cell_of(static_cast<unsigned>(pi.y), g.wrap[1], g.nc[1]));
         const int cz = static_cast<int>(dsmd::cell_of(static_cast<unsigned>(pi.z), g.wrap[2], g.nc[2]));
@@ -250,17 +251,20 @@ __global__ void __launch_bounds__(kSearchThreads) k_edge_search(Grid g, SearchAr
                 float sx = fx;
                 if (PERIODIC && win.b1 >= win.a1 && cx > win.b0) sx -= len[0];   // an atom near the upper face: the lower end first
                 for (;;) {
-#pragma unroll 4
-                    for (; s < end; ++s) {
-                        const float4 pj = __ldg(&a.pf[s]);
-                        const float dx = pj.x - sx, ey = pj.y - sy, ez = pj.z - sz;
-                        const float r2 = fmaf(dx, dx, fmaf(ey, ey, ez * ez));
-                        if (r2 < far2 && s != p && __float_as_int(pj.w) >= 0) {
-                            const bool open = r2 >= near2;
-                            undecided |= open;
-                            if (count < a.stride)
-                                row_of_p[count * 32] = static_cast<unsigned>(PERIODIC ? s : __float_as_int(pj.w)) | (open ? kUndecided : 0u);
-                            ++count;
+                    for (; s < end; s += kAtATime) {   // loads first, and no branch but the stores'
+                        float4 pj[kAtATime];
+#pragma unroll
+                        for (int u = 0; u < kAtATime; ++u) pj[u] = __ldg(&a.pf[min(s + u, end - 1)]);
+#pragma unroll
+                        for (int u = 0; u < kAtATime; ++u) {
+                            const float dx = pj[u].x - sx, ey = pj[u].y - sy, ez = pj[u].z - sz;
+                            const float r2 = fmaf(dx, dx, fmaf(ey, ey, ez * ez));
+                            const int w = __float_as_int(pj[u].w);
+                            const bool hit = r2 < far2 && s + u != p && s + u < end && (PERIODIC || w >= 0);
+                            const unsigned v = static_cast<unsigned>(PERIODIC ? s + u : w) | (r2 >= near2 ? kUndecided : 0u);
+                            if (hit && count < a.stride) row_of_p[count * 32] = v;
+                            undecided |= hit ? v : 0u;
+                            count += hit ? 1 : 0;
                         }
                     }
                     if (!PERIODIC || win.b1 < win.a1) break;
@@ -271,7 +275,7 @@ __global__ void __launch_bounds__(kSearchThreads) k_edge_search(Grid g, SearchAr
                 }
             }
         }
-        if (undecided && count <= a.stride) {
+        if ((undecided & kUndecided) && count <= a.stride) {
             int kept = 0;
             for (int k = 0; k < count; ++k) {
                 unsigned v = row_of_p[k * 32];
@@ -462,9 +466,10 @@ __global__ void __launch_bounds__(kFillThreads) k_edge_fill(int n, long long n_e
 // form. Rows hold neighbour slots, so positions and wrap counts are read where they lie whatever the caller's atom
 // numbering. Displacements come from the fixed-point coordinates (resolution box / 2^32); the lattice shift refers to the
 // caller's coordinates: x[dst] + shift * box - x[src] = vec. WRAPS: some atom lies outside the box.
-// What bounds it: writing 23 bytes per edge (0.6 GB for 26 million edges), then the gathers of the neighbours.
+// What bounds it: writing 23 bytes per edge (0.6 GB for 26 million edges: 0.09 ms at copy speed), then the gathers of the
+// neighbours; 0.19 ms (0.28 ms before). 14 blocks per SM: registers for 14 cost nothing and hide the start of a slice.
 template <bool WRAPS>
-__global__ void __launch_bounds__(kFillThreads) k_edge_fill_compact(
+__global__ void __launch_bounds__(kFillThreads, 14) k_edge_fill_compact(
     Grid g, int n, int stride, int group_shift, const int4* __restrict__ pq, const int* __restrict__ wraps,
     const unsigned* __restrict__ rows, const int* __restrict__ counts, const long long* __restrict__ group_start,
     int* __restrict__ src, int* __restrict__ dst, signed char* __restrict__ shift, float* __restrict__ vec) {
@@ -489,12 +494,26 @@ __global__ void __launch_bounds__(kFillThreads) k_edge_fill_compact(
     for (int from = 0; from < total; from += kFlat) {
         lay_flat(f, from, stride, rows);
         const int upto = min(total, from + kFlat);
-        for (int t0 = ((from + skip) & ~31) - skip + 32 * warp; t0 < upto; t0 += kFillThreads) {
+        int t0 = ((from + skip) & ~31) - skip + 32 * warp;
+        // the next tile's neighbours are on their way while this one is written
+        int4 pj_next{};
+        int wj_next = 0;
+        const auto fetch = [&](int t) {
+            if (t < from || t >= upto) return;
+            const int slot = f.entry[t - from];
+            pj_next = __ldg(&pq[slot]);
+            if (WRAPS) wj_next = __ldg(&wraps[slot]);
+        };
+        fetch(t0 + lane);
+        for (; t0 < upto; t0 += kFillThreads) {
             const int t = t0 + lane;
+            const int4 pj = pj_next;
+            const int wj = wj_next;
+            fetch(t + kFillThreads);
             if (t >= from && t < upto) {
-                const int slot = f.entry[t - from], c = f.atom[t - from];
-                const int4 pj = __ldg(&pq[slot]), pi = centres[c];
-                const int wj = WRAPS ? __ldg(&wraps[slot]) : 0, wi = WRAPS ? centre_wraps[c] : 0;
+                const int c = f.atom[t - from];
+                const int4 pi = centres[c];
+                const int wi = WRAPS ? centre_wraps[c] : 0;
                 const long long o = f.start + t;
                 const unsigned cj[3] = {static_cast<unsigned>(pj.x), static_cast<unsigned>(pj.y), static_cast<unsigned>(pj.z)};
                 const unsigned ci[3] = {static_cast<unsigned>(pi.x), static_cast<unsigned>(pi.y), static_cast<unsigned>(pi.z)};

@@ -11,10 +11,11 @@
 
 namespace dsmd {
 
-static __global__ void k_cell_place(int n, const unsigned* __restrict__ key, const int* __restrict__ arrival, const int* __restrict__ cell_start,
-                             int* __restrict__ list) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) list[cell_start[key[i]] + arrival[i]] = i;
+// Atoms [first, end); key, arrival by atom, list by slot.
+static __global__ void k_cell_place(int first, int end, const unsigned* __restrict__ key, const int* __restrict__ arrival,
+                                    const int* __restrict__ cell_start, int* __restrict__ list) {
+    const int i = first + blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < end) list[cell_start[key[i]] + arrival[i]] = i;
 }
 
 // Final slot of the atom `a` of cell `cell`.

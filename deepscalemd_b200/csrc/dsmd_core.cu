@@ -27,6 +27,7 @@
 #include <vector>
 
 #include "../../include/dsmd_b200.h"
+#include "dsmd_cells.cuh"
 #include "dsmd_common.cuh"
 #include "dsmd_report.cuh"
 #include "ewald_table.hpp"
@@ -44,7 +45,7 @@ constexpr int64_t kPairLanesWanted = kDeviceSms * 1024;   // lanes that fill the
 constexpr int64_t kPairLanesWantedEwald = kDeviceSms * 768;   // two rounds of one block of 384 each
 constexpr int kLongRow = 240;                         // entries (with the row's spare room): about 150 partners per atom
 constexpr int kXRefine = 4;    // x cells per cell width of the y and z axes (tighter row windows in the list build)
-enum { kMailDisplacement = 0, kMailKinetic = 4, kMailScalars = 5, kMailSlots = 6 };   // report slots
+enum { kMailDisplacement = 0, kMailKinetic = 4, kMailScalars = 5, kMailBuild = 6, kMailSlots = 7 };   // report slots
 constexpr int kNumReal = 11;   // x y z vx vy vz fx fy fz mass charge
 constexpr double kCoulomb = 332.0636;
 
@@ -65,9 +66,16 @@ struct Brick {
     int drop;
 };
 
+// Cells are numbered [0, ncells) for owned atoms, [ncells, 2 ncells) for ghosts; atoms to be removed (only in a sort without
+// ghosts) count as cell ncells, behind every other.
+__global__ void k_cell_begin(int cells, int* __restrict__ cell_count, Status* st) {   // st: to be cleared as well, or null
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < cells; k += gridDim.x * blockDim.x) cell_count[k] = 0;
+    if (st && blockIdx.x == 0 && threadIdx.x == 0) *st = Status{};
+}
+
 __global__ void k_cell_keys(Grid g, Brick brick, int first, int n_owned, int n_total, const double* __restrict__ x,
                             const double* __restrict__ y, const double* __restrict__ z, unsigned* __restrict__ key,
-                            int* __restrict__ val, Status* st) {
+                            int* __restrict__ arrival, int* __restrict__ cell_count, Status* st) {
     const int s = first + blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n_total) return;
     const double p[3] = {x[s], y[s], z[s]};
@@ -86,31 +94,33 @@ __global__ void k_cell_keys(Grid g, Brick brick, int first, int n_owned, int n_t
         for (int a = 0; a < 3; ++a)
             if (brick.split[a] && (p[a] < brick.lo[a] || p[a] >= brick.hi[a])) outside = true;
         if (outside) {
-            c = 2u * static_cast<unsigned>(g.ncells);
+            c = static_cast<unsigned>(g.ncells);
             atomicAdd(&st->dropped, 1u);
         }
     }
-    key[s - first] = c;
-    val[s - first] = s;
+    key[s] = c;
+    arrival[s] = atomicAdd(&cell_count[c], 1);
 }
 
-// Gathers every particle array into sorted order, writes the fixed-point layout, the displacement reference, the
-// ghost slot map and the cell start table (a thread whose key differs from its predecessor's owns the cells between).
+// Gathers every particle array into sorted order, writes the fixed-point layout, the displacement reference and the
+// ghost slot map. FORCES: the force arrays too (a loop that evaluates forces next does not need them).
+template <bool FORCES>
 __global__ void k_reorder(Grid g, int first, int n_owned, int n_total, const unsigned* __restrict__ key,
-                          const int* __restrict__ val, RealArrays src, RealArrays dst, const int* __restrict__ type_src,
+                          const int* __restrict__ list, const int* __restrict__ cell_start, RealArrays src, RealArrays dst, const int* __restrict__ type_src,
                           const int* __restrict__ gid_src, int* __restrict__ type_dst, int* __restrict__ gid_dst,
                           int4* __restrict__ pq, float* __restrict__ qf, double* __restrict__ xref,
-                          double* __restrict__ yref, double* __restrict__ zref, int* __restrict__ cell_start,
-                          int* __restrict__ ghost_slot) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int s = first + t;
-    if (s >= n_total) return;
-    const int from = val[t];
+                          double* __restrict__ yref, double* __restrict__ zref, int* __restrict__ ghost_slot) {
+    const int t = first + blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n_total) return;
+    const int from = list[t];
+    const int s = dsmd::cell_slot(from, key[from], cell_start, list);
     double r[kNumReal];
 #pragma unroll
-    for (int f = 0; f < kNumReal; ++f) r[f] = src.p[f][from];
+    for (int f = 0; f < kNumReal; ++f)
+        if (FORCES || f < DSMD_FX || f > DSMD_FZ) r[f] = src.p[f][from];
 #pragma unroll
-    for (int f = 0; f < kNumReal; ++f) dst.p[f][s] = r[f];
+    for (int f = 0; f < kNumReal; ++f)
+        if (FORCES || f < DSMD_FX || f > DSMD_FZ) dst.p[f][s] = r[f];
     const int ty = type_src[from];
     type_dst[s] = ty;
     gid_dst[s] = gid_src[from];
@@ -126,19 +136,6 @@ __global__ void k_reorder(Grid g, int first, int n_owned, int n_total, const uns
     yref[s] = r[1];
     zref[s] = r[2];
     if (s >= n_owned) ghost_slot[from - n_owned] = s;
-    // Cell starts. Keys of the sorted range [first, n_total) are key[0 .. n_total - first). When only the owned atoms
-    // are sorted (first == 0, n_total == n_owned) the ghost half of the table is filled by the later full build.
-    const int k_here = static_cast<int>(key[t]);
-    if (k_here >= 2 * g.ncells) return;   // an atom being removed: behind every cell
-    const int k_prev = t == 0 ? (first == 0 ? -1 : g.ncells - 1) : static_cast<int>(key[t - 1]);
-    for (int c = k_prev + 1; c <= k_here; ++c) cell_start[c] = s;
-}
-
-// Cells behind the last occupied one (and, when only owned atoms were sorted, the whole ghost half) start at the end.
-__global__ void k_cell_tail(const unsigned* __restrict__ key, int n_sorted, int n_total, int table_size,
-                            int* __restrict__ cell_start) {
-    const int c = static_cast<int>(key[n_sorted - 1]) + 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < table_size) cell_start[c] = n_total;
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -158,15 +155,18 @@ __global__ void k_copy_back(int first, int count, RealArrays from, RealArrays to
     gid_to[s] = gid_from[s];
 }
 
-// First slot of every z layer of (owned) cells, and the end: what lets a caller cut the sorted atoms into slabs.
-__global__ void k_layer_starts(const int* __restrict__ cell_start, int cells_per_layer, int layers, int* __restrict__ out) {
-    const int l = blockIdx.x * blockDim.x + threadIdx.x;
-    if (l <= layers) out[l] = cell_start[static_cast<size_t>(l) * cells_per_layer];
+// The end of a list build: its status goes to the host (out_of_domain, dropped, need_stride, boundary_pairs) and, unless the
+// host is going to report an error, starts again at zero, the displacement word with it.
+__global__ void k_build_done(Status* st, unsigned expect_dropped, Mail* mail, unsigned long long seq) {
+    const double out[4] = {static_cast<double>(st->out_of_domain), static_cast<double>(st->dropped), static_cast<double>(st->need_stride),
+                           static_cast<double>(st->boundary_pairs)};
+    if (st->out_of_domain == 0u && st->dropped == expect_dropped) *st = Status{};
+    post(mail, out, 4, seq);
 }
 
 // Where the ghosts of a cell row sit: lo_end = one past the last x cell of the row's lower half that holds a ghost (0:
 // none), hi_begin = the first x cell of its upper half that holds one (nc[0]: none). One warp per (y, z) row.
-__global__ void k_ghost_row_specialtent(Grid g, const int* __restrict__ ghost_cell_start, int* __restrict__ lo_end,
+__global__ void k_ghost_row_extent(Grid g, const int* __restrict__ ghost_cell_start, int* __restrict__ lo_end,
                                    int* __restrict__ hi_begin) {
     const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -527,12 +527,13 @@ struct dsmd_ctx {
     int4* pq_next = nullptr;
     float* qf = nullptr;
     double* ref[3] = {};
-    unsigned* key[2] = {};
-    int* val[2] = {};
+    unsigned* key = nullptr;       // cell of an atom, by the slot it came from
+    int* arrival = nullptr;        // its place among the atoms of the cell as they came
+    int* list = nullptr;           // the cells' atoms as they came
+    int* cell_count = nullptr;
     int* ghost_slot = nullptr;
     // the host-buffer force call as a pipeline (dsmd_forces_host): first slot of every z layer of cells as of the last
     // build, two copy streams, one event pair per piece
-    int* d_layer_start = nullptr;
     int* h_layer_start = nullptr;     // pinned, [nc_z + 1]
     int layer_capacity = 0;
     cudaStream_t copy_in = nullptr, copy_out = nullptr;
@@ -744,11 +745,13 @@ int make_grid(dsmd_ctx* c) {
 }
 
 int ensure_cells(dsmd_ctx* c) {
-    const int64_t need = 2ll * c->grid.ncells + 1;
+    const int64_t need = 2ll * c->grid.ncells + 2;
     if (need > c->cell_capacity) {
-        if (c->cell_start) cudaFree(c->cell_start);
-        c->cell_start = nullptr;
+        cudaFree(c->cell_start);
+        cudaFree(c->cell_count);
+        c->cell_start = c->cell_count = nullptr;
         DSMD_CUDA(c, cudaMalloc(&c->cell_start, sizeof(int) * need));
+        DSMD_CUDA(c, cudaMalloc(&c->cell_count, sizeof(int) * need));
         c->cell_capacity = need;
     }
     return DSMD_OK;
@@ -833,45 +836,44 @@ int ensure_partials(dsmd_ctx* c, int64_t blocks) {
     return DSMD_OK;
 }
 
-// Sorts slots [first, n_total) by cell and gathers everything into the other buffer set. n_removed > 0 (owned-only
-// sorts): that many atoms lie outside the brick; they sort behind every cell and fall off the end.
-int sort_range(dsmd_ctx* c, int64_t first, cudaStream_t s, int64_t n_removed = 0, const Brick* bounds = nullptr) {
+// Sorts slots [first, n_total) by cell and gathers everything into the other buffer set. bounds (owned-only sorts): atoms
+// outside the brick sort behind every cell and fall off the end.
+int sort_range(dsmd_ctx* c, int64_t first, cudaStream_t s, bool clear, const Brick* bounds = nullptr, bool forces = true) {
     const int64_t n = c->n_total - first;
     const int from = c->cur, to = 1 - c->cur;
+    if (clear) c->disp_seq = 0;   // reports of displacement checks are void
     if (n > 0) {
         Brick brick{};
-        if (bounds) brick = *bounds;
-        brick.drop = (bounds && n_removed > 0) ? 1 : 0;
-        k_cell_keys<<<blocks_for(n, kThreads), kThreads, 0, s>>>(
-            c->grid, brick, static_cast<int>(first), static_cast<int>(c->n_owned), static_cast<int>(c->n_total),
-            c->real[from][0], c->real[from][1], c->real[from][2], c->key[0], c->val[0], c->status);
+        if (bounds) { brick = *bounds; brick.drop = 1; }
+        const int in = static_cast<int>(c->n_total), i0 = static_cast<int>(first);
+        // cells this sort is about: the owned ones, the ghosts', or both; and one behind them
+        const int cell0 = first > 0 ? c->grid.ncells : 0, cells = (c->n_total > c->n_owned ? 2 : 1) * c->grid.ncells + 2 - cell0;
+        k_cell_begin<<<std::min<unsigned>(blocks_for(cells, kThreads), kDeviceSms * 8), kThreads, 0, s>>>(cells, c->cell_count + cell0,
+                                                                                                        clear ? c->status : nullptr);
         DSMD_LAUNCHED(c);
-        int bits = 1;
-        while ((1ll << bits) < 2ll * c->grid.ncells + 1) ++bits;
+        k_cell_keys<<<blocks_for(n, kThreads), kThreads, 0, s>>>(
+            c->grid, brick, i0, static_cast<int>(c->n_owned), in, c->real[from][0], c->real[from][1], c->real[from][2], c->key,
+            c->arrival, c->cell_count, c->status);
+        DSMD_LAUNCHED(c);
         size_t need = 0;
-        cub::DeviceRadixSort::SortPairs(nullptr, need, c->key[0], c->key[1], c->val[0], c->val[1], static_cast<int>(n), 0,
-                                        bits, s);
+        cub::DeviceScan::ExclusiveScan(nullptr, need, c->cell_count, c->cell_start, cuda::std::plus<int>(), i0, cells, s);
         if (need > c->cub_temp_bytes) {
             if (c->cub_temp) cudaFree(c->cub_temp);
             c->cub_temp = nullptr;
             DSMD_CUDA(c, cudaMalloc(&c->cub_temp, need + need / 4));
             c->cub_temp_bytes = need + need / 4;
         }
-        DSMD_CUDA(c, cub::DeviceRadixSort::SortPairs(c->cub_temp, need, c->key[0], c->key[1], c->val[0], c->val[1],
-                                                     static_cast<int>(n), 0, bits, s));
-        k_reorder<<<blocks_for(n, kThreads), kThreads, 0, s>>>(
-            c->grid, static_cast<int>(first), static_cast<int>(c->n_owned), static_cast<int>(c->n_total), c->key[1],
-            c->val[1], arrays_of(c, from), arrays_of(c, to), c->type[from], c->gid[from], c->type[to], c->gid[to], c->pq,
-            c->qf, c->ref[0], c->ref[1], c->ref[2], c->cell_start, c->ghost_slot);
+        DSMD_CUDA(c, cub::DeviceScan::ExclusiveScan(c->cub_temp, need, c->cell_count + cell0, c->cell_start + cell0,
+                                                    cuda::std::plus<int>(), i0, cells, s));
+        dsmd::k_cell_place<<<blocks_for(n, kThreads), kThreads, 0, s>>>(i0, in, c->key, c->arrival, c->cell_start, c->list);
         DSMD_LAUNCHED(c);
-        const int table = 2 * c->grid.ncells + 1;
-        const int64_t kept = n - n_removed;
-        if (kept > 0) {
-            k_cell_tail<<<blocks_for(table, kThreads), kThreads, 0, s>>>(c->key[1], static_cast<int>(kept),
-                                                                      static_cast<int>(c->n_total - n_removed), table,
-                                                                      c->cell_start);
-            DSMD_LAUNCHED(c);
-        }
+        const auto reorder = forces ? k_reorder<true> : k_reorder<false>;
+        reorder<<<blocks_for(n, kThreads), kThreads, 0, s>>>(
+            c->grid, i0, static_cast<int>(c->n_owned), in, c->key, c->list, c->cell_start, arrays_of(c, from), arrays_of(c, to),
+            c->type[from], c->gid[from], c->type[to], c->gid[to], c->pq, c->qf, c->ref[0], c->ref[1], c->ref[2], c->ghost_slot);
+        DSMD_LAUNCHED(c);
+    } else if (clear) {
+        DSMD_CUDA(c, cudaMemsetAsync(c->status, 0, sizeof(Status), s));
     }
     if (first > 0) {
         // a ghost-only sort: the owned atoms are in place in the current set, the sorted ghosts come back to it (far
@@ -887,11 +889,6 @@ int sort_range(dsmd_ctx* c, int64_t first, cudaStream_t s, int64_t n_removed = 0
     }
     c->slot_map_valid = false;
     return DSMD_OK;
-}
-
-cudaError_t clear_status(dsmd_ctx* c, cudaStream_t s) {
-    c->disp_seq = 0;   // reports of displacement checks are void
-    return cudaMemsetAsync(c->status, 0, sizeof(Status), s);
 }
 
 int wait_mail(dsmd_ctx* c, int slot, unsigned long long seq, cudaStream_t s) {
@@ -978,11 +975,12 @@ int dsmd_create(int device, int64_t capacity, dsmd_ctx** out) {
         }
         DSMD_CUDA(c, cudaMalloc(&c->type[set], sizeof(int) * capacity));
         DSMD_CUDA(c, cudaMalloc(&c->gid[set], sizeof(int) * capacity));
-        DSMD_CUDA(c, cudaMalloc(&c->key[set], sizeof(unsigned) * capacity));
-        DSMD_CUDA(c, cudaMalloc(&c->val[set], sizeof(int) * capacity));
     }
     DSMD_CUDA(c, cudaMalloc(&c->pq, sizeof(int4) * capacity));
     DSMD_CUDA(c, cudaMalloc(&c->pq_next, sizeof(int4) * capacity));
+    DSMD_CUDA(c, cudaMalloc(&c->key, sizeof(unsigned) * capacity));
+    DSMD_CUDA(c, cudaMalloc(&c->arrival, sizeof(int) * capacity));
+    DSMD_CUDA(c, cudaMalloc(&c->list, sizeof(int) * capacity));
     DSMD_CUDA(c, cudaMalloc(&c->qf, sizeof(float) * capacity));
     for (int a = 0; a < 3; ++a) DSMD_CUDA(c, cudaMalloc(&c->ref[a], sizeof(double) * capacity));
     DSMD_CUDA(c, cudaMalloc(&c->ghost_slot, sizeof(int) * capacity));
@@ -1012,9 +1010,9 @@ void dsmd_destroy(dsmd_ctx* c) {
     cudaSetDevice(c->device);
     for (int set = 0; set < 2; ++set) {
         for (int f = 0; f < kNumReal; ++f) cudaFree(c->real[set][f]);
-        cudaFree(c->type[set]); cudaFree(c->gid[set]); cudaFree(c->key[set]); cudaFree(c->val[set]);
+        cudaFree(c->type[set]); cudaFree(c->gid[set]); 
     }
-    cudaFree(c->pq); cudaFree(c->pq_next); cudaFree(c->qf); cudaFree(c->type_charge);
+    cudaFree(c->pq); cudaFree(c->pq_next); cudaFree(c->key); cudaFree(c->arrival); cudaFree(c->list); cudaFree(c->cell_count); cudaFree(c->qf); cudaFree(c->type_charge);
     for (int a = 0; a < 3; ++a) cudaFree(c->ref[a]);
     cudaFree(c->ghost_slot); cudaFree(c->cell_start); cudaFree(c->ghost_rows);
     cudaFree(c->rows); cudaFree(c->quad); cudaFree(c->row_end); cudaFree(c->row_int); cudaFree(c->row_special); cudaFree(c->boundary_pairs);
@@ -1024,7 +1022,6 @@ void dsmd_destroy(dsmd_ctx* c) {
     cudaFree(c->cl_gid); cudaFree(c->cl_a); cudaFree(c->cl_b); cudaFree(c->cl_d2); cudaFree(c->slot_of_gid);
     cudaFree(c->cl_slot); cudaFree(c->cl_member);
     free_bonded(c);
-    cudaFree(c->d_layer_start);
     if (c->h_layer_start) cudaFreeHost(c->h_layer_start);
     if (c->copy_in) cudaStreamDestroy(c->copy_in);
     if (c->copy_out) cudaStreamDestroy(c->copy_out);
@@ -1233,10 +1230,9 @@ static int sort_owned_impl(dsmd_ctx* c, const Brick* bounds, int64_t n_outside, 
     if (n_outside < 0 || n_outside >= c->n_owned) return fail(c, DSMD_ERR_INVALID, "sort: bad count of atoms to remove");
     if (!c->grid_valid) { const int rc = make_grid(c); if (rc) return rc; }
     { const int rc = ensure_cells(c); if (rc) return rc; }
-    DSMD_CUDA(c, clear_status(c, s));
     const int64_t keep_total = c->n_total;
     c->n_total = c->n_owned;   // sort the owned segment alone
-    const int rc = sort_range(c, 0, s, n_outside, bounds);
+    const int rc = sort_range(c, 0, s, true, n_outside > 0 ? bounds : nullptr);
     c->n_total = keep_total;
     if (rc) return rc;
     c->n_owned -= n_outside;
@@ -1270,9 +1266,8 @@ int dsmd_sort_owned_in_brick(dsmd_ctx* c, const double lo[3], const double hi[3]
     return sort_owned_impl(c, &bounds, n_outside, false, static_cast<cudaStream_t>(stream));
 }
 
-int dsmd_build_neighbor_list(dsmd_ctx* c, void* stream) {
-    if (!c) return DSMD_ERR_INVALID;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
+// forces: the force arrays move with the atoms.
+static int build_list(dsmd_ctx* c, bool forces, cudaStream_t s) {
     DSMD_CUDA(c, cudaSetDevice(c->device));
     if (c->n_owned <= 0) return fail(c, DSMD_ERR_STATE, "no atoms uploaded");
     if (!c->grid_valid) { const int rc = make_grid(c); if (rc) return rc; }
@@ -1281,10 +1276,10 @@ int dsmd_build_neighbor_list(dsmd_ctx* c, void* stream) {
     //    status words of that sort are then still unread and are kept)
     const int64_t first = c->owned_sorted_only ? c->n_owned : 0;
     const int64_t expect_dropped = c->owned_sorted_only ? c->expect_dropped : 0;
-    if (!c->owned_sorted_only) DSMD_CUDA(c, clear_status(c, s));
+    const bool clear = !c->owned_sorted_only;
     c->owned_sorted_only = false;
     c->expect_dropped = 0;
-    if (first == 0 || c->n_total > first) { const int rc = sort_range(c, first, s); if (rc) return rc; }
+    if (first == 0 || c->n_total > first) { const int rc = sort_range(c, first, s, clear, nullptr, forces); if (rc) return rc; }
     // 2. list rows
     int row_entries = c->stride;
     if (c->stride == 0) {
@@ -1304,23 +1299,17 @@ int dsmd_build_neighbor_list(dsmd_ctx* c, void* stream) {
         DSMD_CUDA(c, cudaMalloc(&c->ghost_rows, sizeof(int) * 4 * rows));
         c->ghost_rows_capacity = 4 * rows;
     }
-    {   // slab boundaries for the pipelined host-buffer call; they arrive with the status read-back below
+    {   // slab boundaries for the pipelined host-buffer call; k_quads writes them
         const int layers = c->grid.nc[2];
         if (layers + 1 > c->layer_capacity) {
-            cudaFree(c->d_layer_start);
             if (c->h_layer_start) cudaFreeHost(c->h_layer_start);
-            c->d_layer_start = c->h_layer_start = nullptr;
-            DSMD_CUDA(c, cudaMalloc(&c->d_layer_start, sizeof(int) * (layers + 1)));
+            c->h_layer_start = nullptr;
             DSMD_CUDA(c, cudaMallocHost(&c->h_layer_start, sizeof(int) * (layers + 1)));
             c->layer_capacity = layers + 1;
         }
-        k_layer_starts<<<blocks_for(layers + 1, kThreads), kThreads, 0, s>>>(c->cell_start, c->grid.nc[0] * c->grid.nc[1], layers,
-                                                                           c->d_layer_start);
-        DSMD_LAUNCHED(c);
-        DSMD_CUDA(c, cudaMemcpyAsync(c->h_layer_start, c->d_layer_start, sizeof(int) * (layers + 1), cudaMemcpyDeviceToHost, s));
     }
     if (c->n_total > c->n_owned) {
-        k_ghost_row_specialtent<<<blocks_for(rows * 32, kThreads), kThreads, 0, s>>>(c->grid, c->cell_start + c->grid.ncells,
+        k_ghost_row_extent<<<blocks_for(rows * 32, kThreads), kThreads, 0, s>>>(c->grid, c->cell_start + c->grid.ncells,
                                                                                c->ghost_rows, c->ghost_rows + rows);
         DSMD_LAUNCHED(c);
         k_ghost_rows_near<<<blocks_for(rows, kThreads), kThreads, 0, s>>>(c->grid, c->ghost_rows, c->ghost_rows + rows,
@@ -1331,8 +1320,8 @@ int dsmd_build_neighbor_list(dsmd_ctx* c, void* stream) {
         { const int rc = lay_out_rows(c, row_entries); if (rc) return rc; }
         const ExclusionTable ex{c->excl_off, c->excl_partner, static_cast<int>(c->excl_n_global)};
         if (attempt == 0) {
-            k_quads<<<blocks_for(rows * 32, kThreads), kThreads, 0, s>>>(c->grid.nc[0], static_cast<int>(rows), static_cast<int>(c->n_owned),
-                                                                        c->cell_start, c->quad);
+            k_quads<<<blocks_for(rows * 32, kThreads), kThreads, 0, s>>>(c->grid.nc[0], c->grid.nc[1], static_cast<int>(rows),
+                                                                        static_cast<int>(c->n_owned), c->cell_start, c->quad, c->h_layer_start);
             DSMD_LAUNCHED(c);
         }
         const unsigned blocks = blocks_for(c->n_quads * 32, kBuildThreads);
@@ -1347,22 +1336,28 @@ int dsmd_build_neighbor_list(dsmd_ctx* c, void* stream) {
                                                                c->ghost_rows + 2 * rows, c->ghost_rows + 3 * rows, rows_of(c),
                                                                c->boundary_pairs, c->status);
         DSMD_LAUNCHED(c);
-        { const int rc = read_status(c, s); if (rc) return rc; }
-        if (c->h_status->out_of_domain)
+        k_build_done<<<1, 1, 0, s>>>(c->status, attempt == 0 ? static_cast<unsigned>(expect_dropped) : 0u, c->mail + kMailBuild, ++c->seq);
+        DSMD_LAUNCHED(c);
+        { const int rc = wait_mail(c, kMailBuild, c->seq, s); if (rc) return rc; }
+        const double* const status = c->mail[kMailBuild].value;
+        c->disp_seq = 0;   // the displacement word starts again at zero
+        if (status[0] != 0.0)
             return fail(c, DSMD_ERR_OUT_OF_DOMAIN, "an atom lies outside the subdomain + halo, or has a NaN position");
-        if (attempt == 0 && c->h_status->dropped != static_cast<unsigned>(expect_dropped))
+        if (attempt == 0 && status[1] != static_cast<double>(expect_dropped))
             return fail(c, DSMD_ERR_STATE, "sort: the number of atoms outside the brick differs from the caller's count");
-        if (c->h_status->need_stride <= static_cast<unsigned>(c->stride)) break;
+        c->n_boundary = static_cast<int64_t>(status[3]);
+        if (status[2] <= c->stride) break;
         // a row overflowed: grow and build again
-        row_entries = static_cast<int>(c->h_status->need_stride * 1.1) + 8;
-        DSMD_CUDA(c, clear_status(c, s));
+        row_entries = static_cast<int>(status[2] * 1.1) + 8;
         if (attempt == 3) return fail(c, DSMD_ERR_CAPACITY, "neighbour rows kept overflowing");
     }
-    c->n_boundary = static_cast<int64_t>(c->h_status->boundary_pairs);
     ++c->build_epoch;
-    DSMD_CUDA(c, clear_status(c, s));   // displacement word restarts at zero
     c->list_valid = true;
     return DSMD_OK;
+}
+
+int dsmd_build_neighbor_list(dsmd_ctx* c, void* stream) {
+    return c ? build_list(c, true, static_cast<cudaStream_t>(stream)) : DSMD_ERR_INVALID;
 }
 
 int dsmd_ghost_slots(dsmd_ctx* c, const int32_t** out) {
@@ -2072,7 +2067,7 @@ int dsmd_run_nve(dsmd_ctx* c, int64_t n_steps, double dt, double f2a, double hi_
             if (predicted * predicted > limit2) rebuild = true;
         }
         if (rebuild) {
-            const int rc = dsmd_build_neighbor_list(c, s);
+            const int rc = build_list(c, false, s);   // forces are evaluated next
             if (rc) return rc;
             ++rebuilds;
             since_build = 0;
@@ -2255,7 +2250,7 @@ int dsmd_halo_select(dsmd_ctx* c, const double lo[3], const double hi[3], int32_
     DSMD_LAUNCHED(c);
     size_t need = 0;
     thrust::counting_iterator<int> iota(0);
-    int* d_selected = c->val[0];   // scratch of capacity entries
+    int* d_selected = c->list;   // scratch of capacity entries
     cub::DeviceSelect::Flagged(nullptr, need, iota, c->flag, d_selected, &c->status->select_count, n, s);
     if (need > c->cub_temp_bytes) {
         if (c->cub_temp) cudaFree(c->cub_temp);

@@ -978,7 +978,7 @@ int edge_search(dsmd_edges* e, const Grid& g, const double* d_x, const double* d
     EDGE_CUDA(e, cudaMemsetAsync(e->cell_count, 0, sizeof(int) * (table + kStatusWords), s));
     k_edge_keys<<<blocks_for(n, kThreads), kThreads, 0, s>>>(g, in, d_x, d_y, d_z, e->key, e->arrival, cell_count, st);
     EDGE_CUDA(e, cub::DeviceScan::ExclusiveSum(e->temp, scan_bytes, cell_count, e->cell_start, static_cast<int>(table), s));
-    dsmd::k_cell_place<<<blocks_for(n, kThreads), kThreads, 0, s>>>(in, e->key, e->arrival, e->cell_start, e->list);
+    dsmd::k_cell_place<<<blocks_for(n, kThreads), kThreads, 0, s>>>(0, in, e->key, e->arrival, e->cell_start, e->list);
     k_edge_gather<<<blocks_for(n, kThreads), kThreads, 0, s>>>(g, in, e->key, e->list, e->cell_start, d_x, d_y, d_z,
                                                               row == 1 ? d_ok : nullptr, d_owner, e->pq, e->pf,
                                                               PERIODIC ? e->wraps : nullptr, st);

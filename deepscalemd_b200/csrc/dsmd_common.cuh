@@ -48,7 +48,18 @@ struct Status {
     unsigned int constraint_failed;   // constraint clusters whose SHAKE / RATTLE sweeps did not converge
     unsigned int boundary_pairs;      // pairs with a ghost partner in their list row (the boundary pass runs over them)
     unsigned int reserved;
+    double gate;                   // largest squared displacement as of the last complete check (infinite: atoms outside)
 };
+
+// A loop that looks for the largest displacement before every force evaluation need not wait for it: the kernels behind the
+// check carry the limit, and do nothing when the check before them went beyond it (the host, which finds out later, then
+// rebuilds the list and launches them again). Read from a word that only the end of a check writes, so that all blocks of a
+// launch see the same.
+#ifdef __CUDACC__
+__device__ __forceinline__ bool gate_closed(const Status* st, double limit2) {
+    return limit2 < 1.0e300 && __ldcg(&st->gate) > limit2;
+}
+#endif
 
 __host__ __device__ inline unsigned int cell_of(unsigned int fixed, int wrap, int nc) {
 #ifdef __CUDA_ARCH__

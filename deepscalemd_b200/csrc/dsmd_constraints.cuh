@@ -283,6 +283,7 @@ template <class Shape, bool FINISH, bool START>
 __global__ void __launch_bounds__(128) k_constrained(ClusterTable t, Grid g, AtomArrays at, double half_kick, double dt, double tolerance,
                                                      int max_iterations, double prefactor, double* __restrict__ partials, unsigned* __restrict__ ticket,
                                                      double* __restrict__ virial, DisplacementReport report) {
+    if (START && dsmd::gate_closed(report.st, report.gate2)) return;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     double wsum[3] = {0.0, 0.0, 0.0}, worst2 = 0.0;
     if (k < t.n_clusters) {

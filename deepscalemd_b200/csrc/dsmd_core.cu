@@ -222,6 +222,7 @@ struct DisplacementReport {
     unsigned* ticket;      // blocks that have finished
     Mail* mail;            // or null: no report
     unsigned long long seq;
+    double gate2;          // see gate_closed
 };
 
 // The block's largest squared displacement goes into the status word; the last block of the grid reports the word.
@@ -243,6 +244,7 @@ __device__ __forceinline__ void report_displacement(double v, const Displacement
                     const double out[2] = {__longlong_as_double(static_cast<long long>(__ldcg(&r.st->max_disp2))),
                                            static_cast<double>(__ldcg(&r.st->out_of_domain))};
                     *r.ticket = 0u;
+                    r.st->gate = out[1] != 0.0 ? __longlong_as_double(0x7FF0000000000000ll) : out[0];
                     post(r.mail, out, 2, r.seq);
                 }
             }
@@ -349,6 +351,7 @@ __global__ void k_pack(Grid g, int first, int count, int n_owned, double* __rest
                        const double* __restrict__ xref, const double* __restrict__ yref,
                        const double* __restrict__ zref, int4* __restrict__ pq, double dt, double kick_c,
                        const int* __restrict__ gid, const unsigned char* __restrict__ skip, BondedForces bonded, DisplacementReport report) {
+    if (dsmd::gate_closed(report.st, report.gate2)) return;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int s = first + t;
     double d2 = 0.0;
@@ -570,6 +573,7 @@ struct dsmd_ctx {
     unsigned* tickets = nullptr;    // finished blocks of the sums: forces, kinetic energy, bonded terms, constraints;
                                     // from 4 on: displacement checks in turn
     Mail* mail = nullptr;           // pinned: kMailDisplacement .. + 3 in turn, kMailKinetic, kMailScalars
+    double gate2 = HUGE_VAL;        // limit that the launches of the MD loop carry (gate_closed)
     bool captured = false;          // a call was captured into a graph: results are copied, not reported
     unsigned long long seq = 0;     // launches that reported something so far
     unsigned long long disp_seq = 0, scalars_seq = 0;   // the last displacement check / energy sum whose report still stands (0: none)
@@ -891,8 +895,8 @@ int sort_range(dsmd_ctx* c, int64_t first, cudaStream_t s, bool clear, const Bri
     return DSMD_OK;
 }
 
-int wait_mail(dsmd_ctx* c, int slot, unsigned long long seq, cudaStream_t s) {
-    const cudaError_t e = dsmd::wait_report(c->mail + slot, seq, s);
+int wait_mail(dsmd_ctx* c, int slot, int n, unsigned long long seq, cudaStream_t s) {
+    const cudaError_t e = dsmd::wait_report(c->mail + slot, n, seq, s);
     return e == cudaSuccess ? static_cast<int>(DSMD_OK) : fail(c, DSMD_ERR_CUDA, std::string("waiting for a kernel's report: ") + cudaGetErrorString(e));
 }
 
@@ -907,10 +911,10 @@ bool reports_count(dsmd_ctx* c, cudaStream_t s) {
 // run side by side on several streams). Slots and tickets in turn, so that the last three stay readable.
 DisplacementReport displacement_report(dsmd_ctx* c, bool all_atoms, cudaStream_t s) {
     c->disp_seq = 0;
-    if (!all_atoms || !reports_count(c, s)) return DisplacementReport{c->status, nullptr, nullptr, 0};
+    if (!all_atoms || !reports_count(c, s)) return DisplacementReport{c->status, nullptr, nullptr, 0, c->gate2};
     c->disp_seq = ++c->seq;
     const int slot = static_cast<int>(c->seq & 3);
-    return DisplacementReport{c->status, c->tickets + 4 + slot, c->mail + kMailDisplacement + slot, c->seq};
+    return DisplacementReport{c->status, c->tickets + 4 + slot, c->mail + kMailDisplacement + slot, c->seq, c->gate2};
 }
 
 int read_status(dsmd_ctx* c, cudaStream_t s) {
@@ -1338,17 +1342,17 @@ static int build_list(dsmd_ctx* c, bool forces, cudaStream_t s) {
         DSMD_LAUNCHED(c);
         k_build_done<<<1, 1, 0, s>>>(c->status, attempt == 0 ? static_cast<unsigned>(expect_dropped) : 0u, c->mail + kMailBuild, ++c->seq);
         DSMD_LAUNCHED(c);
-        { const int rc = wait_mail(c, kMailBuild, c->seq, s); if (rc) return rc; }
-        const double* const status = c->mail[kMailBuild].value;
+        { const int rc = wait_mail(c, kMailBuild, 4, c->seq, s); if (rc) return rc; }
+        const Mail& report = c->mail[kMailBuild];
         c->disp_seq = 0;   // the displacement word starts again at zero
-        if (status[0] != 0.0)
+        if (report.value(0) != 0.0)
             return fail(c, DSMD_ERR_OUT_OF_DOMAIN, "an atom lies outside the subdomain + halo, or has a NaN position");
-        if (attempt == 0 && status[1] != static_cast<double>(expect_dropped))
+        if (attempt == 0 && report.value(1) != static_cast<double>(expect_dropped))
             return fail(c, DSMD_ERR_STATE, "sort: the number of atoms outside the brick differs from the caller's count");
-        c->n_boundary = static_cast<int64_t>(status[3]);
-        if (status[2] <= c->stride) break;
+        c->n_boundary = static_cast<int64_t>(report.value(3));
+        if (report.value(2) <= c->stride) break;
         // a row overflowed: grow and build again
-        row_entries = static_cast<int>(status[2] * 1.1) + 8;
+        row_entries = static_cast<int>(report.value(2) * 1.1) + 8;
         if (attempt == 3) return fail(c, DSMD_ERR_CAPACITY, "neighbour rows kept overflowing");
     }
     ++c->build_epoch;
@@ -1456,9 +1460,9 @@ int dsmd_max_displacement_sq(dsmd_ctx* c, double* out, void* stream) {
     if (c->disp_seq && !c->captured) {   // nothing has touched the status since the last displacement check: its report says it all
         DSMD_CUDA(c, cudaStreamSynchronize(s));
         const int slot = kMailDisplacement + static_cast<int>(c->disp_seq & 3);
-        { const int rc = wait_mail(c, slot, c->disp_seq, s); if (rc) return rc; }
-        *out = c->mail[slot].value[0];
-        outside = c->mail[slot].value[1] != 0.0;
+        { const int rc = wait_mail(c, slot, 2, c->disp_seq, s); if (rc) return rc; }
+        *out = c->mail[slot].value(0);
+        outside = c->mail[slot].value(1) != 0.0;
     } else {
         { const int rc = read_status(c, s); if (rc) return rc; }
         std::memcpy(out, &c->h_status->max_disp2, sizeof(*out));
@@ -1532,7 +1536,7 @@ static int compute_forces_impl(dsmd_ctx* c, int phase, int want_energy, int64_t 
     double** r = c->real[c->cur];
     const ForceArgs a{c->pq, c->qf, rows_of(c), phase, phase == DSMD_PHASE_BOUNDARY ? c->boundary_pairs : nullptr,
                       static_cast<int>(ranged ? first : 0), static_cast<int>(pairs), c->lane_shift, r[DSMD_FX], r[DSMD_FY], r[DSMD_FZ], c->partials,
-                      c->tickets, c->scalars, report ? c->mail + kMailScalars : nullptr, report ? ++c->seq : 0};
+                      c->tickets, c->scalars, report ? c->mail + kMailScalars : nullptr, report ? ++c->seq : 0, c->status, c->gate2};
     if (e && pairs > 0) c->scalars_seq = a.seq;
     if (pairs > 0) {   // else nothing to add to the forces; the energy sums of a boundary pass stay as the interior pass left them
         const int copies = ewald_copies(c);
@@ -1550,7 +1554,7 @@ static int force_step(dsmd_ctx* c, double dt, double f2a, cudaStream_t s) {
     const int64_t pairs = 2 * c->n_quads;
     double** r = c->real[c->cur];
     const ForceArgs a{c->pq, c->qf, rows_of(c), DSMD_PHASE_FULL, nullptr, 0, static_cast<int>(pairs), c->lane_shift,
-                      nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0};
+                      nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, c->status, c->gate2};
     const StepArgs at{r[0], r[1], r[2], r[3], r[4], r[5], r[9], c->ref[0], c->ref[1], c->ref[2], c->pq_next, dt, dt * f2a};
     const unsigned blocks = static_cast<unsigned>(pair_blocks(c, pairs, false));
     const DisplacementReport report = displacement_report(c, true, s);
@@ -1577,8 +1581,8 @@ int dsmd_read_scalars(dsmd_ctx* c, double out[6], void* stream) {
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (c->scalars_seq && !c->captured) {
         DSMD_CUDA(c, cudaStreamSynchronize(s));
-        { const int rc = wait_mail(c, kMailScalars, c->scalars_seq, s); if (rc) return rc; }
-        for (int k = 0; k < 6; ++k) out[k] = c->mail[kMailScalars].value[k];
+        { const int rc = wait_mail(c, kMailScalars, 6, c->scalars_seq, s); if (rc) return rc; }
+        for (int k = 0; k < 6; ++k) out[k] = c->mail[kMailScalars].value(k);
         return DSMD_OK;
     }
     DSMD_CUDA(c, cudaMemcpyAsync(c->h_scalars, c->scalars, sizeof(double) * 6, cudaMemcpyDeviceToHost, s));
@@ -1620,7 +1624,7 @@ int launch_constrained(dsmd_ctx* c, bool finish, bool start, double half_kick, d
     double** r = c->real[c->cur];
     const AtomArrays at{r[0], r[1], r[2], r[3], r[4], r[5], r[6], r[7], r[8], r[9], c->type[c->cur], c->ref[0], c->ref[1], c->ref[2], c->pq};
     const unsigned blocks = blocks_for(c->n_clusters, 128);
-    const DisplacementReport report = start ? displacement_report(c, c->cl_cover_all, s) : DisplacementReport{c->status, nullptr, nullptr, 0};
+    const DisplacementReport report = start ? displacement_report(c, c->cl_cover_all, s) : DisplacementReport{c->status, nullptr, nullptr, 0, HUGE_VAL};
     const auto launch = [&](auto shape) {
         const auto kernel = finish && start ? k_constrained<decltype(shape), true, true>
                                             : (finish ? k_constrained<decltype(shape), true, false> : k_constrained<decltype(shape), false, true>);
@@ -1976,8 +1980,8 @@ int dsmd_kinetic_energy(dsmd_ctx* c, double* out, void* stream) {
                                                                  c->partials, c->tickets + 1, c->scalars + 6, c->mail + kMailKinetic, ++c->seq);
     DSMD_LAUNCHED(c);
     DSMD_CUDA(c, cudaStreamSynchronize(s));
-    { const int rc = wait_mail(c, kMailKinetic, c->seq, s); if (rc) return rc; }
-    *out = c->mail[kMailKinetic].value[0];
+    { const int rc = wait_mail(c, kMailKinetic, 1, c->seq, s); if (rc) return rc; }
+    *out = c->mail[kMailKinetic].value(0);
     return DSMD_OK;
 }
 
@@ -2022,9 +2026,9 @@ int dsmd_run_nve(dsmd_ctx* c, int64_t n_steps, double dt, double f2a, double hi_
         d2 = 0.0;
         if (!seq) return static_cast<int>(DSMD_OK);   // no atoms, no check
         const int slot = kMailDisplacement + static_cast<int>(seq & 3);
-        const int rc = wait_mail(c, slot, seq, s);
-        d2 = c->mail[slot].value[0];
-        if (!rc && !lagged && c->mail[slot].value[1] != 0.0)
+        const int rc = wait_mail(c, slot, 2, seq, s);
+        d2 = c->mail[slot].value(0);
+        if (!rc && !lagged && c->mail[slot].value(1) != 0.0)
             return fail(c, DSMD_ERR_OUT_OF_DOMAIN, "an atom left the subdomain + halo, or has a NaN position");
         return rc;
     };
@@ -2033,18 +2037,42 @@ int dsmd_run_nve(dsmd_ctx* c, int64_t n_steps, double dt, double f2a, double hi_
     // the pair forces are all the forces there are, that pass is the end of the force kernel (k_step).
     const bool constrained = c->n_clusters > 0, bonded = !constrained && c->bonded.terms() > 0;
     const bool fused = !constrained && !bonded && !c->coulomb && c->n_owned > 0;
-    for (int64_t step = 0; step < n_steps; ++step) {
-        if (step == 0 || !fused) {
-            const BondedForces terms = bonded_forces(c);
-            const int rc = constrained && step > 0 ? constrained_halves(c, true, true, dt, f2a, s)
-                           : bonded && step > 0    ? pack_impl(c, 0, c->n_owned, true, dt, f2a, s, 1.0, nullptr, &terms)
-                                                   : dsmd_integrate(c, step > 0 ? 3 : 1, dt, f2a, s);
-            if (rc) return rc;
+    // Forces at the current positions and on to the next ones, up to their displacement check; nothing happens on the device
+    // when the check of the current ones went beyond `gate2`.
+    const auto advance = [&](double gate2) {
+        c->gate2 = gate2;
+        int rc = DSMD_OK;
+        if (fused) {
+            rc = force_step(c, dt, f2a, s);
+        } else {
+            rc = dsmd_compute_forces(c, DSMD_PHASE_FULL, 0, s);
+            if (bonded) {   // the bonded contributions go straight into the pass over the atoms
+                if (!rc) rc = bonded_terms(c, false, s);
+                const BondedForces terms = bonded_forces(c);
+                if (!rc) rc = pack_impl(c, 0, c->n_owned, true, dt, f2a, s, 1.0, nullptr, &terms);
+            } else {
+                if (!rc) rc = dsmd_compute_bonded(c, s);
+                if (!rc) rc = constrained ? constrained_halves(c, true, true, dt, f2a, s) : dsmd_integrate(c, 3, dt, f2a, s);
+            }
         }
+        c->gate2 = HUGE_VAL;
+        return rc;
+    };
+    // With constraints and bonded terms at once the forces are added to in place: not a thing to do twice.
+    const bool ahead_of_check = !lagged && !(constrained && c->bonded.terms() > 0);
+    if (n_steps > 0) { const int rc = dsmd_integrate(c, 1, dt, f2a, s); if (rc) return rc; }
+    for (int64_t step = 0; step < n_steps; ++step) {
         const unsigned long long check = c->disp_seq;   // the displacement check of the positions that are current now
+        const bool last = step + 1 == n_steps;
         ++since_build;
-        bool rebuild = every > 0 && since_build >= every;
+        bool rebuild = every > 0 && since_build >= every, advanced = false;
         if (!lagged) {
+            // unless a rebuild is due or this is the end, the next kernels are queued before the host looks at the check
+            if (ahead_of_check && !rebuild && !last) {
+                const int rc = advance(limit2);
+                if (rc) return rc;
+                advanced = true;
+            }
             double d2 = 0.0;
             const int rc = reported(check, d2);
             if (rc) return rc;
@@ -2074,16 +2102,14 @@ int dsmd_run_nve(dsmd_ctx* c, int64_t n_steps, double dt, double f2a, double hi_
             d_prev = d_prev2 = 0.0;
             pending = 0;   // that check was made against reference positions that are gone
         }
-        if (fused && step + 1 < n_steps) {
-            const int rc = force_step(c, dt, f2a, s);
+        if (last) {
+            { const int rc = dsmd_compute_forces(c, DSMD_PHASE_FULL, 0, s); if (rc) return rc; }
+            { const int rc = dsmd_compute_bonded(c, s); if (rc) return rc; }
+            { const int rc = dsmd_integrate(c, 2, dt, f2a, s); if (rc) return rc; }
+        } else if (!advanced || rebuild) {
+            const int rc = advance(HUGE_VAL);
             if (rc) return rc;
-            continue;
         }
-        { const int rc = dsmd_compute_forces(c, DSMD_PHASE_FULL, 0, s); if (rc) return rc; }
-        // (between two steps the bonded contributions go straight into the pass over the atoms)
-        if (bonded && step + 1 < n_steps) { const int rc = bonded_terms(c, false, s); if (rc) return rc; }
-        else { const int rc = dsmd_compute_bonded(c, s); if (rc) return rc; }
-        if (step + 1 == n_steps) { const int rc = dsmd_integrate(c, 2, dt, f2a, s); if (rc) return rc; }
     }
     if (lagged && pending) {
         double d2 = 0.0;

@@ -997,13 +997,13 @@ int edge_search(dsmd_edges* e, const Grid& g, const double* d_x, const double* d
         ++e->launches;
         EDGE_CUDA(e, cudaGetLastError());
         // the one wait of a build that does not overflow: edge count, bounds flag, row overflow
-        EDGE_CUDA(e, dsmd::wait_report(e->mail, e->seq, s));
-        if (e->mail->value[1] != 0.0)
+        EDGE_CUDA(e, dsmd::wait_report(e->mail, 4, e->seq, s));
+        if (e->mail->value(1) != 0.0)
             return efail(e, DSMD_ERR_OUT_OF_DOMAIN, "an atom lies outside the given box (or has a NaN position)");
-        const int need = static_cast<int>(e->mail->value[2]);
+        const int need = static_cast<int>(e->mail->value(2));
         if (need <= e->stride) {
-            *n_edges = static_cast<int64_t>(e->mail->value[0]);
-            e->outside_box = e->mail->value[3] != 0.0;
+            *n_edges = static_cast<int64_t>(e->mail->value(0));
+            e->outside_box = e->mail->value(3) != 0.0;
             return DSMD_OK;
         }
         e->stride = (static_cast<int>(need * 1.2) + 8 + 3) & ~3;
@@ -1075,8 +1075,8 @@ int dsmd_edges_build(dsmd_edges* e, const double* d_x, const double* d_y, const 
             static_cast<int>(n), d_x, d_y, d_z, e->partials, e->ticket, e->mail, ++e->seq);
         ++e->launches;
         EDGE_CUDA(e, cudaGetLastError());
-        EDGE_CUDA(e, dsmd::wait_report(e->mail, e->seq, s));
-        for (int a = 0; a < 3; ++a) { box_lo[a] = e->mail->value[a]; box_hi[a] = e->mail->value[3 + a]; }
+        EDGE_CUDA(e, dsmd::wait_report(e->mail, 6, e->seq, s));
+        for (int a = 0; a < 3; ++a) { box_lo[a] = e->mail->value(a); box_hi[a] = e->mail->value(3 + a); }
     }
     for (int a = 0; a < 3; ++a)
         if (!(box_lo[a] <= box_hi[a]) || !std::isfinite(box_lo[a]) || !std::isfinite(box_hi[a]))
@@ -1224,8 +1224,8 @@ int dsmd_virial_from_forces(dsmd_edges* e, const double* d_x, const double* d_y,
     k_virial<<<blocks, kThreads, 0, s>>>(n, d_x, d_y, d_z, d_fx, d_fy, d_fz, e->partials, e->ticket, e->mail, ++e->seq);
     ++e->launches;
     EDGE_CUDA(e, cudaGetLastError());
-    EDGE_CUDA(e, dsmd::wait_report(e->mail, e->seq, s));
-    for (int k = 0; k < 4; ++k) out[k] = e->mail->value[k];
+    EDGE_CUDA(e, dsmd::wait_report(e->mail, 4, e->seq, s));
+    for (int k = 0; k < 4; ++k) out[k] = e->mail->value(k);
     return DSMD_OK;
 }
 

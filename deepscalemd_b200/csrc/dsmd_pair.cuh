@@ -210,6 +210,8 @@ struct ForceArgs {
     double* scalars;
     Mail* mail;              // where the total is reported to the host
     unsigned long long seq;
+    const Status* st;
+    double gate2;            // see gate_closed
 };
 
 // Threads per block and blocks per SM, which fix the registers and with them how the compiler interleaves the partners of a
@@ -406,6 +408,7 @@ __device__ __forceinline__ void row_forces(const PairParams& p, const ForceArgs&
 template <int COPIES, bool ENERGY, int TYPES, bool SWITCH, bool QTYPE>
 __global__ void __launch_bounds__((kPairThreads<COPIES, TYPES>), (kPairBlocks<COPIES, TYPES, ENERGY>)) k_pair(PairParams p, ForceArgs a) {
     extern __shared__ float4 smem[];
+    if (!ENERGY && dsmd::gate_closed(a.st, a.gate2)) return;
     const PairTables<COPIES, ENERGY, TYPES, QTYPE> tables(p, smem);
     const int lanes = 1 << a.lane_shift;
     double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};   // energy, virial and its diagonal, pairs
@@ -458,6 +461,7 @@ template <int TYPES, bool SWITCH>
 __global__ void __launch_bounds__((kPairThreads<0, TYPES>), (kPairBlocks<0, TYPES, false>))
 k_step(PairParams p, ForceArgs a, Grid g, StepArgs at, DisplacementReport report) {
     extern __shared__ float4 smem[];
+    if (dsmd::gate_closed(report.st, report.gate2)) return;
     const PairTables<0, false, TYPES, false> tables(p, smem);
     const int lanes = 1 << a.lane_shift, t = blockIdx.x * blockDim.x + threadIdx.x;
     const int pair = t >> a.lane_shift, sub = t & (lanes - 1);

@@ -23,7 +23,7 @@ FIELD_ID = {name: k for k, name in enumerate(FIELDS)}
 SYMBOLS = [
     "dsmd_create", "dsmd_destroy", "dsmd_last_error", "dsmd_set_box", "dsmd_set_pair_params", "dsmd_set_coulomb",
     "dsmd_get_ewald_alpha", "dsmd_set_exclusions", "dsmd_set_constraints", "dsmd_constraint_failures", "dsmd_rattle",
-    "dsmd_set_bonded", "dsmd_compute_bonded", "dsmd_read_bonded_scalars", "dsmd_set_type_charges", "dsmd_upload", "dsmd_upload_positions", "dsmd_download",
+    "dsmd_set_bonded", "dsmd_compute_bonded", "dsmd_read_bonded_scalars", "dsmd_set_type_charges", "dsmd_upload", "dsmd_upload_rows", "dsmd_upload_positions", "dsmd_download",
     "dsmd_device_pointer", "dsmd_counts", "dsmd_set_counts", "dsmd_build_neighbor_list", "dsmd_sort_owned", "dsmd_sort_owned_in_brick",
     "dsmd_ghost_slots", "dsmd_list_stats", "dsmd_list_export", "dsmd_pack_positions", "dsmd_max_displacement_sq", "dsmd_max_displacement_sq_lagged",
     "dsmd_displacement_word", "dsmd_compute_forces", "dsmd_read_scalars", "dsmd_integrate", "dsmd_kinetic_energy", "dsmd_scale_velocities",
@@ -208,16 +208,14 @@ class Context:
 
     # -- particles ----------------------------------------------------------------------------------------------------
     def upload(self, pos, n_owned=None, vel=None, mass=None, charge=None, types=None, gid=None, stream=None):
-        pos = np.asarray(pos, dtype=np.float64)
+        pos = np.ascontiguousarray(np.asarray(pos)[:, :3], dtype=np.float64)
         n = len(pos)
         n_owned = n if n_owned is None else n_owned
-        cols = [_arr(pos[:, k], np.float64) for k in range(3)]
-        vcols = [None] * 3 if vel is None else [_arr(np.asarray(vel)[:, k], np.float64) for k in range(3)]
+        vel = None if vel is None else np.ascontiguousarray(np.asarray(vel)[:, :3], dtype=np.float64)
         m, q = _arr(mass, np.float64), _arr(charge, np.float64)
         t, g = _arr(types, np.int32), _arr(gid, np.int32)
-        self._check(self.lib.dsmd_upload(self.h, c_int64(n_owned), c_int64(n), _p(cols[0]), _p(cols[1]), _p(cols[2]),
-                                         _p(vcols[0]), _p(vcols[1]), _p(vcols[2]), _p(m), _p(q), _p(t), _p(g),
-                                         _stream_handle(stream)))
+        self._check(self.lib.dsmd_upload_rows(self.h, c_int64(n_owned), c_int64(n), _p(pos), _p(vel), _p(m), _p(q), _p(t),
+                                              _p(g), _stream_handle(stream)))
         import torch
         torch.cuda.synchronize()
 

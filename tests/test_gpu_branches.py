@@ -1,0 +1,190 @@
+"""GPU tests of the branches that a size, a type or the layout of the input picks, at the sizes where they can go wrong,
+against the CPU oracle."""
+import numpy as np
+import pytest
+
+from deepscalemd_b200 import capi
+from oracle import cpu_oracle as co
+
+pytestmark = pytest.mark.gpu
+
+
+# atoms, box, cutoff, skin, types, Coulomb, exclusions: lone atoms and two; rows of one to four atoms; one, few and more than
+# eight types; Ewald tables in one copy (short rows) and in eight (rows of 240 and more); atoms that coincide with their row
+ROWS = [
+    (1, 20.0, 4.0, 0.5, 1, False, False), (2, 20.0, 4.0, 0.5, 1, True, False), (37, 20.0, 4.0, 0.5, 3, False, False),
+    (333, 20.0, 4.0, 0.5, 8, True, True), (334, 20.0, 4.0, 0.5, 9, True, True), (600, 16.0, 3.0, 0.3, 9, False, True),
+    (2500, 25.0, 6.0, 0.5, 2, True, True), (2500, 25.0, 6.0, 0.5, 1, False, False),
+]
+
+
+@pytest.mark.parametrize("n,L,rc,skin,nt,coulomb,excl", ROWS)
+@pytest.mark.parametrize("switched", [False, True])
+def test_forces_of_every_row_form(cuda_device, n, L, rc, skin, nt, coulomb, excl, switched):
+    rng = np.random.default_rng(n + nt)
+    side = int(np.ceil(n ** (1 / 3)))
+    sites = np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij"), -1).reshape(-1, 3)[rng.permutation(side ** 3)[:n]]
+    pos = ((sites + 0.5 + rng.uniform(-0.2, 0.2, (n, 3))) * (L / side)) % L
+    box = np.full(3, L)
+    types = rng.integers(0, nt, n).astype(np.int32)
+    sig = 0.5 * (rng.uniform(0.8, 1.2, nt)[:, None] + rng.uniform(0.8, 1.2, nt)[None])
+    sig, eps = 0.5 * (sig + sig.T), np.full((nt, nt), 0.3)
+    charge = rng.uniform(-0.5, 0.5, n) if coulomb else np.zeros(n)
+    pairs = co.pairs(*pos.T, n, box, search=rc + skin)
+    exclusions = pairs[:: 5] if excl else None
+    switch = 0.8 * rc if switched else -1.0
+    ctx = capi.Context(n)
+    ctx.set_box(box)
+    ctx.set_pair_params(eps, sig, rc, skin, switch)
+    if coulomb:
+        ctx.set_coulomb(True)
+    if excl:
+        ctx.set_exclusions(n, exclusions)
+    ctx.upload(pos, types=types, charge=charge)
+    ctx.build_neighbor_list()
+    alpha = co.ewald_alpha(rc) if coulomb else 0.0
+    c6, c12 = co.lj_tables(eps, sig)
+    want, scalars = co.forces(*pos.T, n, box, pairs, c6, c12, rc, charge=charge, types=types, switch=switch, do_coulomb=coulomb,
+                              alpha=alpha, exclusions=exclusions)
+    scale = max(np.abs(want).max(), 1e-12)
+    for energy in (False, True):
+        ctx.compute_forces(capi.PHASE_FULL, want_energy=energy)
+        assert np.abs(ctx.forces_by_gid(n) - want).max() <= 2e-5 * scale
+    got = ctx.read_scalars()
+    assert abs(got["pe"] - scalars["pe"]) <= 1e-5 * max(abs(scalars["pe"]), 1.0)
+    assert got["pairs_in_cutoff"] == scalars["pairs_in_cutoff"]
+    ctx.close()
+
+
+@pytest.mark.parametrize("free", [False, True])
+@pytest.mark.parametrize("shape", ["bond", "triangle", "chain"])
+def test_constraint_shapes(cuda_device, shape, free):
+    """Groups that are compiled for (two atoms, three atoms in a ring) and any other, with and without atoms outside every
+    group: positions after the drift and velocities after the second half equal the oracle's."""
+    ring = {"bond": [(0, 1)], "triangle": [(0, 1), (0, 2), (1, 2)], "chain": [(0, 1), (1, 2), (2, 3)]}[shape]
+    size, groups, L, dt = {"bond": 2, "triangle": 3, "chain": 4}[shape], 65, 30.0, 1.0
+    rng = np.random.default_rng(size)
+    shapes = np.array([[0.0, 0.0, 0.0], [1.0, 0.1, 0.0], [0.3, 0.9, 0.0], [0.4, 1.0, 1.0]])[:size]
+    centres = np.stack(np.meshgrid(*[np.arange(5)] * 3, indexing="ij"), -1).reshape(-1, 3)[:groups] * 6.0
+    pos = (centres[:, None] + shapes[None]).reshape(-1, 3)
+    constraints = np.array([(g * size + a, g * size + b, np.linalg.norm(shapes[a] - shapes[b])) for g in range(groups) for a, b in ring])
+    if free:
+        pos = np.concatenate([pos, rng.uniform(0, L, (7, 3))])
+    n, box = len(pos), np.full(3, L)
+    pos = pos % L
+    mass = rng.uniform(1.0, 16.0, n)
+    vel = rng.normal(scale=0.02, size=(n, 3))
+    ctx = capi.Context(n)
+    ctx.set_box(box)
+    ctx.set_pair_params([[0.0]], [[1.0]], 3.0, 0.5)
+    ctx.set_constraints(n, constraints)
+    ctx.upload(pos, vel=vel, mass=mass)
+    ctx.build_neighbor_list()
+    gid = ctx.download("global_id", n)
+
+    def fields(names):
+        out = np.empty((n, 3))
+        out[gid] = np.stack([ctx.download(k, n) for k in names], axis=1)
+        return out
+
+    pre = [np.ascontiguousarray(c) for c in pos.T]
+    p = [np.ascontiguousarray(c) for c in (pos + dt * vel).T]
+    v = [np.ascontiguousarray(c) for c in vel.T]
+    ctx.integrate(1, dt)
+    assert co.shake(constraints, p, v, mass, pre, box, dt)
+    assert np.abs(fields("xyz") - np.stack(p, 1)).max() <= 1e-9
+    assert np.abs(fields(("vx", "vy", "vz")) - np.stack(v, 1)).max() <= 1e-9
+    ctx.integrate(2, dt)
+    assert co.rattle(constraints, p, v, mass, box, dt, 1.0)[0]
+    assert np.abs(fields(("vx", "vy", "vz")) - np.stack(v, 1)).max() <= 1e-9
+    assert ctx.constraint_failures() == 0
+    ctx.close()
+
+
+# a warp per atom up to 32,768 atoms, a thread per atom beyond; slices of 32; rows of more than 1,024 edges per slice (the flat
+# order in pieces); atoms outside the box
+@pytest.mark.parametrize("n,density,outside", [(2, 0.05, False), (33, 0.05, True), (2000, 0.05, True), (1000, 0.6, False),
+                                               (32768, 0.02, False), (32769, 0.02, True)])
+def test_graphs_of_every_search_and_slice_form(cuda_device, n, density, outside):
+    import torch
+    rng = np.random.default_rng(n)
+    cutoff = 4.0
+    L = max((n / density) ** (1 / 3), 3.2 * cutoff)
+    pos = rng.uniform(0, L, (n, 3))
+    x, y, z = (torch.tensor(np.ascontiguousarray(c), device="cuda") for c in pos.T)
+    eb = capi.EdgeBuilder()
+    want, _ = co.edges(*pos.T, cutoff)
+    got = eb.build(x, y, z, cutoff)[0].cpu().numpy()
+    assert np.array_equal(got[:, np.lexsort(got[::-1])], want[:, np.lexsort(want[::-1])])
+    moved = pos + (rng.integers(-1, 2, (n, 3)) * L if outside else 0.0)
+    src, dst, shift, vec = (t.cpu().numpy() for t in eb.build_periodic(*[torch.tensor(np.ascontiguousarray(c), device="cuda") for c in moved.T],
+                                                                       np.full(3, L), cutoff))
+    half = co.pairs(*pos.T, n, np.full(3, L), search=cutoff)
+    both = np.concatenate([half, half[:, ::-1]])
+    order, order_want = np.lexsort((dst, src)), np.lexsort((both[:, 1], both[:, 0]))
+    assert np.array_equal(np.stack([src, dst], 1)[order], both[order_want])
+    assert np.abs(moved[dst] + shift * L - moved[src] - vec).max(initial=0.0) <= 1e-5
+    eb.close()
+
+
+@pytest.mark.parametrize("n,cells", [(500, 5), (256000, 40)])
+def test_host_buffers_pinned_and_not(cuda_device, n, cells):
+    """The host-buffer call by kernels that read the host's memory (few atoms), by slabs (many), and with memory that kernels
+    cannot read: the same forces, bit for bit."""
+    import torch
+    from deepscalemd_b200 import synthetic as syn
+    s = syn.fcc_lj(cells)
+    assert s.n == n
+    ctx = capi.Context(n)
+    ctx.set_box(s.box)
+    ctx.set_pair_params(s.eps, s.sig, s.cutoff, s.skin)
+    ctx.upload(s.pos)
+    ctx.build_neighbor_list()
+    order = ctx.download("global_id")
+    moved = s.pos[order] + np.random.default_rng(5).uniform(-0.08, 0.08, s.pos.shape)
+    plain = [np.ascontiguousarray(c) for c in moved.T]
+    ctx.upload_positions_ptr(*[c.ctypes.data for c in plain])
+    ctx.pack_positions(0, None)
+    ctx.compute_forces()
+    want = [ctx.download(k) for k in ("fx", "fy", "fz")]
+    pinned = [torch.from_numpy(c).pin_memory() for c in plain]
+    out_pinned, out_plain = [torch.zeros(n, dtype=torch.float64).pin_memory() for _ in range(3)], [np.zeros(n) for _ in range(3)]
+    ctx.forces_host(*[t.data_ptr() for t in pinned], *[t.data_ptr() for t in out_pinned])
+    ctx.forces_host(*[c.ctypes.data for c in plain], *[c.ctypes.data for c in out_plain])
+    for k in range(3):
+        assert np.array_equal(out_pinned[k].numpy(), want[k]) and np.array_equal(out_plain[k], want[k])
+    ctx.close()
+
+
+@pytest.mark.parametrize("lagged", [False, True])
+@pytest.mark.parametrize("n_cells,nt", [(5, 1), (8, 2), (8, 9)])
+def test_loop_equals_step_by_step(cuda_device, n_cells, nt, lagged):
+    """The MD loop (forces, both velocity halves and the drift in one kernel, the next step queued before the check is read)
+    against the same steps through the single entry points."""
+    from deepscalemd_b200 import synthetic as syn
+    s = syn.fcc_lj(n_cells)
+    types = np.arange(s.n, dtype=np.int32) % nt
+    eps, sig = np.full((nt, nt), 1.0), np.full((nt, nt), 1.0)
+    ends = []
+    for loop in (True, False):
+        ctx = capi.Context(s.n)
+        ctx.set_box(s.box)
+        ctx.set_pair_params(eps, sig, s.cutoff, s.skin)
+        ctx.upload(s.pos, vel=s.vel, types=types)
+        ctx.build_neighbor_list()
+        ctx.compute_forces()
+        if loop:
+            ctx.run_nve(25, 0.004, lagged=lagged)
+        else:
+            for _ in range(25):
+                ctx.integrate(1, 0.004)
+                if ctx.max_displacement_sq() > (0.5 * s.skin) ** 2:
+                    ctx.build_neighbor_list()
+                ctx.compute_forces()
+                ctx.integrate(2, 0.004)
+        gid = ctx.download("global_id", s.n)
+        out = np.empty((s.n, 6))
+        out[gid] = np.stack([ctx.download(k, s.n) for k in ("x", "y", "z", "vx", "vy", "vz")], axis=1)
+        ends.append(out)
+        ctx.close()
+    assert np.abs(ends[0] - ends[1]).max() <= 1e-4

@@ -471,7 +471,7 @@ def single_gpu(args):
         "algorithmic_bytes_per_launch": pair_bytes, "algorithmic_flops_per_launch": pair_flops,
         "hbm": {"achieved": pk["gbs"], "peak": hbm_peak, "unit": "GB/s", "frac": pk["frac_hbm"],
                 "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)"},
-        "list_build": {"kernel": "bin + sort + reorder + k_build_list", "bound": "hbm", "ms": t_build,
+        "list_build": {"kernel": "bin + sort + reorder + k_build_rows", "bound": "hbm", "ms": t_build,
                        "achieved": kernels["list_build_total"]["gbs"], "peak": hbm_peak, "unit": "GB/s",
                        "frac": kernels["list_build_total"]["frac_hbm"], "algorithmic_bytes_per_launch": build_bytes},
     }

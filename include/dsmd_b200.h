@@ -126,7 +126,7 @@ int dsmd_set_counts(dsmd_ctx* ctx, int64_t n_owned, int64_t n_total);
 /* ForceCalculatorCUDA::build_neighbor_list_on_device (src/force_calculator_cuda.cu:4604) = launch_cuda_tile_list_build
  * (src/neighbor_list_kernels.cu:554) + build_tile_lists_on_device (:4817): bins the atoms into cells, sorts them by
  * cell (owned and ghost segments separately), reorders every particle array, converts positions to the fixed-point
- * layout and builds the per-atom Verlet list with skin. Takes the current positions as the displacement reference
+ * layout and builds the Verlet list with skin (one row for two neighbouring atoms). Takes the current positions as the displacement reference
  * (update_reference_positions_on_device). Synchronises `stream` once to read the build status. */
 int dsmd_build_neighbor_list(dsmd_ctx* ctx, void* stream);
 
@@ -252,9 +252,10 @@ int dsmd_run_nve(dsmd_ctx* ctx, int64_t n_steps, double dt, double force_to_acce
 
 /* One force evaluation with host buffers, as a force-provider plugin is called: uploads positions (context order),
  * packs, evaluates, downloads forces (and the six scalars of dsmd_read_scalars when out6 != NULL). Rebuilds the list first when rebuild != 0.
- * Without rebuild and without out6, on a single-rank system tall enough to cut into at least four slabs of cell layers,
- * the call runs as a pipeline over two internal copy streams: slabs of the sorted atoms are uploaded, evaluated and
- * downloaded side by side (the same forces, bit for bit); pinned host buffers are what makes the copies overlap.
+ * Without rebuild and without out6, on a large single-rank system tall enough to cut into at least four slabs of cell
+ * layers, the call runs as a pipeline over two internal copy streams: slabs of the sorted atoms are uploaded, evaluated and
+ * downloaded side by side (the same forces, bit for bit); pinned host buffers are what makes the copies overlap. Of a small
+ * system kernels read and write pinned (or registered) host buffers themselves.
  * Synchronises. */
 int dsmd_forces_host(dsmd_ctx* ctx, const double* x, const double* y, const double* z, int rebuild, double* fx,
                      double* fy, double* fz, double* out6, void* stream);

@@ -34,6 +34,8 @@ struct Grid {
     float r_pad;        // list radius plus a rounding margin: the reach used to prune cell rows
     float x_reach;      // widest half window along x (stencil * width of an unrefined cell, a hair less)
     float quad_spread[3];   // how far four atoms searched together may lie apart
+    float cells_per_unit[3];  // cells per fixed-point unit
+    float cells_per_length;   // x cells per length
     float band_rows;    // the band of the list search on float differences relative to a quad's first atom
 };
 

@@ -789,8 +789,11 @@ int make_grid(dsmd_ctx* c) {
     // and an atom of a quad, both relative to the quad's first atom), each good to three roundings of 2^-24; squares and
     // sums add a few more of R^2; the fixed-point grid one unit per coordinate. Everything inside the band is listed.
     g.band_rows = static_cast<float>(5.9604645e-8 * 48.0 * R * R + 8.0 * R * max_scale);
-    for (int a = 0; a < 3; ++a)
+    for (int a = 0; a < 3; ++a) {
+        g.cells_per_unit[a] = static_cast<float>(g.nc[a] / (g.wrap[a] ? 4294967296.0 : 2147483648.0));
         g.quad_spread[a] = g.wrap[a] ? std::min(g.r_pad, static_cast<float>(0.49 * g.box[a]) - g.r_pad) : g.r_pad;
+    }
+    g.cells_per_length = 1.0f / g.cellw[0];
     c->grid_valid = true;
     return DSMD_OK;
 }

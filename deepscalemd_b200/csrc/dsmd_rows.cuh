@@ -101,7 +101,8 @@ struct RowArrays {
 // packed behind each other by ballot.
 // What bounds it: instruction issue; 8 to 9 rounds of 32 candidates per quad of a Lennard-Jones liquid (130 of the 250
 // candidates lie inside the list radius of one of the four atoms), about 60 for water. A thread-per-atom walk of the same
-// windows spent 340 warp instructions per atom at 20 of 32 active lanes.
+// windows spent 340 warp instructions per atom at 20 of 32 active lanes. Rebuild of 4,000,000 Lennard-Jones atoms 1.79 ms, of
+// 1,048,575 of the mixture 0.59, of 648,000 of water 1.87 (thread per atom: 2.58, 1.02, 5.97 ms).
 constexpr int kCandidates = 512;   // candidates numbered at a time (per warp, in shared memory)
 
 struct QuadSearch {
@@ -132,10 +133,13 @@ __device__ __forceinline__ void test_candidates(const Grid& g, QuadSearch& q, in
                                                 const ExcludedRange& s_excluded) {
     const int lane = threadIdx.x & 31;
     const unsigned lt_mask = (1u << lane) - 1u;
+    const unsigned own_first = static_cast<unsigned>(min(q.n_atoms, 2)), own_second = static_cast<unsigned>(max(q.n_atoms - 2, 0));
+    int s_next = lane < n ? s_slot[lane] : q.first;   // a round ahead
     for (int t = lane; t - lane < n; t += 32) {
         const bool valid = t < n;
-        const int s = valid ? s_slot[t] : q.first;
+        const int s = s_next;
         const int4 c = __ldg(&pq[s]);
+        s_next = t + 32 < n ? s_slot[t + 32] : q.first;
         float r[4];
         if (NEAR) {
             const F2 rx = both(dsmd::fixed_delta(c.x, q.x, g.scale[0]));
@@ -165,7 +169,7 @@ __device__ __forceinline__ void test_candidates(const Grid& g, QuadSearch& q, in
         }
         // the two atoms of a pair are no partners of its row
         const unsigned own = static_cast<unsigned>(s - q.first);
-        const bool own0 = own < static_cast<unsigned>(min(q.n_atoms, 2)), own1 = own - 2u < static_cast<unsigned>(max(q.n_atoms - 2, 0));
+        const bool own0 = own < own_first, own1 = own - 2u < own_second;
         if (EXCL) {
             // a candidate inside the range of ids that one of the four atoms excludes (molecules are numbered together: few
             // are) is looked up in the atom's table row; the row's end holds those that are excluded for one of its atoms
@@ -236,7 +240,6 @@ k_build_rows(Grid g, int n_owned, int n_total, int n_quads, const int4* __restri
     q.x = home.x;
     q.y = home.y;
     q.z = home.z;
-    int c_min = g.nc[0], c_max = -1;   // x cells of the atoms
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
         const int4 atom = pq[q.first + min(m, n_atoms - 1)];   // a missing atom: a copy of the last one
@@ -247,9 +250,6 @@ k_build_rows(Grid g, int n_owned, int n_total, int n_quads, const int4* __restri
         // axes), and for the rounding band to hold
         compact = compact && fabsf(off[m][0]) <= g.quad_spread[0] && fabsf(off[m][1]) <= g.quad_spread[1] &&
                   fabsf(off[m][2]) <= g.quad_spread[2];
-        const int cx = static_cast<int>(dsmd::cell_of(static_cast<unsigned>(atom.x), g.wrap[0], g.nc[0]));
-        c_min = min(c_min, cx);
-        c_max = max(c_max, cx);
     }
 #pragma unroll
     for (int h = 0; h < 2; ++h)
@@ -285,12 +285,9 @@ k_build_rows(Grid g, int n_owned, int n_total, int n_quads, const int4* __restri
     const int lane_z = S == 2 ? (lane * 13) >> 6 : (lane * 11) >> 5;   // lane / 5, lane / 3
     const int dz = lane_z - S, dy = lane - lane_z * side - S;
     // places of the first atom on the three axes, in cells (float: good to 3e-4 of a cell)
-    const float at_x = __uint2float_rn(g.wrap[0] ? static_cast<unsigned>(home.x) : static_cast<unsigned>(home.x) << 1) *
-                       (static_cast<float>(g.nc[0]) * 2.3283064e-10f);
-    const float at_y = __uint2float_rn(g.wrap[1] ? static_cast<unsigned>(home.y) : static_cast<unsigned>(home.y) << 1) *
-                       (static_cast<float>(g.nc[1]) * 2.3283064e-10f);
-    const float at_z = __uint2float_rn(g.wrap[2] ? static_cast<unsigned>(home.z) : static_cast<unsigned>(home.z) << 1) *
-                       (static_cast<float>(g.nc[2]) * 2.3283064e-10f);
+    const float at_x = __uint2float_rn(static_cast<unsigned>(home.x)) * g.cells_per_unit[0];
+    const float at_y = __uint2float_rn(static_cast<unsigned>(home.y)) * g.cells_per_unit[1];
+    const float at_z = __uint2float_rn(static_cast<unsigned>(home.z)) * g.cells_per_unit[2];
     const int cy0 = static_cast<int>(dsmd::cell_of(static_cast<unsigned>(home.y), g.wrap[1], g.nc[1]));
     const int cz0 = static_cast<int>(dsmd::cell_of(static_cast<unsigned>(home.z), g.wrap[2], g.nc[2]));
     const float to_y = static_cast<float>(cy0 + dy) - at_y, to_z = static_cast<float>(cz0 + dz) - at_z;   // lower face of the row
@@ -319,8 +316,7 @@ k_build_rows(Grid g, int n_owned, int n_total, int n_quads, const int4* __restri
     open = open && lo <= hi;
     int a0 = 0, b0 = -1, a1 = 0, b1 = -1;   // x cells [a0, b0] and, across the periodic boundary, [a1, b1]
     if (open) {
-        const float per_cell = 1.0f / g.cellw[0];
-        const int c_lo = __float2int_rd(at_x + lo * per_cell - 2e-3f), c_hi = __float2int_rd(at_x + hi * per_cell + 2e-3f);
+        const int c_lo = __float2int_rd(at_x + lo * g.cells_per_length - 2e-3f), c_hi = __float2int_rd(at_x + hi * g.cells_per_length + 2e-3f);
         if (!g.wrap[0]) {
             a0 = max(c_lo, 0);
             b0 = min(c_hi, g.nc[0] - 1);
@@ -343,6 +339,12 @@ k_build_rows(Grid g, int n_owned, int n_total, int n_quads, const int4* __restri
         const int row_yz = cz0 * g.nc[1] + cy0;
         const int near_lo = ghost_near_lo[row_yz], near_hi = ghost_near_hi[row_yz];
         const int reach_cells = static_cast<int>(g.x_reach / g.cellw[0]) + 2;
+        int c_min = g.nc[0], c_max = -1;   // x cells of the atoms
+        for (int m = 0; m < n_atoms; ++m) {
+            const int cx = static_cast<int>(dsmd::cell_of(static_cast<unsigned>(pq[q.first + m].x), g.wrap[0], g.nc[0]));
+            c_min = min(c_min, cx);
+            c_max = max(c_max, cx);
+        }
         if (g.wrap[0] ? (near_lo > 0 || near_hi < g.nc[0]) : (c_min - reach_cells < near_lo || c_max + reach_cells >= near_hi))
             n_seg = 2;
     }

@@ -659,6 +659,13 @@ __global__ void k_image_masks(ImageLattice L, int n, const double* __restrict__ 
     counts[i] = static_cast<long long>(__popc(mx)) * __popc(my) * __popc(mz) - (self ? 1 : 0);
 }
 
+// Images of the whole system, reported to the host.
+__global__ void k_image_total(int n, const long long* __restrict__ counts, const long long* __restrict__ first_image, dsmd::Mail* mail,
+                              unsigned long long seq) {
+    const double total[1] = {static_cast<double>(first_image[n - 1] + counts[n - 1])};
+    dsmd::post(mail, total, 1, seq);
+}
+
 // One thread per output slot: slots [0, n) are the wrapped atoms, slot n + m is image number m of the whole system, which
 // belongs to the last atom whose first image number is <= m.
 __global__ void k_image_fill(ImageLattice L, int n, long long n_images, const double* __restrict__ x,
@@ -1177,11 +1184,10 @@ int dsmd_images_build(dsmd_edges* e, const double* d_x, const double* d_y, const
                                                               e->img_counts);
     EDGE_CUDA(e, cub::DeviceScan::ExclusiveSum(e->temp, scan_bytes, e->img_counts, e->img_offsets, static_cast<int>(n), s));
     // the image count comes to the host: the one synchronisation (MLIPStep::prepare does the same, src/MLIPStep.cu:254-255)
-    long long last[2] = {0, 0};
-    EDGE_CUDA(e, cudaMemcpyAsync(&last[0], e->img_offsets + (n - 1), sizeof(long long), cudaMemcpyDeviceToHost, s));
-    EDGE_CUDA(e, cudaMemcpyAsync(&last[1], e->img_counts + (n - 1), sizeof(long long), cudaMemcpyDeviceToHost, s));
-    EDGE_CUDA(e, cudaStreamSynchronize(s));
-    const int64_t n_images = last[0] + last[1];
+    k_image_total<<<1, 1, 0, s>>>(static_cast<int>(n), e->img_counts, e->img_offsets, e->mail, ++e->seq);
+    EDGE_CUDA(e, cudaGetLastError());
+    EDGE_CUDA(e, dsmd::wait_report(e->mail, 1, e->seq, s));
+    const int64_t n_images = static_cast<int64_t>(e->mail->value(0));
     const int64_t total = n + n_images;
     if (total >= std::numeric_limits<int32_t>::max() / 2) return efail(e, DSMD_ERR_CAPACITY, "too many image atoms");
     for (int k = 0; k < 6; ++k) EDGE_ALLOC(e, grow(e->ext[k], e->cap_ext[k], static_cast<size_t>(total)));
@@ -1190,7 +1196,7 @@ int dsmd_images_build(dsmd_edges* e, const double* d_x, const double* d_y, const
     k_image_fill<<<blocks_for(total, kThreads), kThreads, 0, s>>>(lattice, static_cast<int>(n), n_images, d_x, d_y, d_z, d_type,
                                                                  e->img_masks, e->img_offsets, e->ext[0], e->ext[1], e->ext[2],
                                                                  e->ext_type, e->ext_owner, e->ext[3], e->ext[4], e->ext[5]);
-    e->launches += 2;
+    e->launches += 3;
     EDGE_CUDA(e, cudaGetLastError());
     e->n_ext = total;
     e->n_img_src = n;

@@ -41,10 +41,5 @@ __device__ __forceinline__ float rsqrt_approx(float v) {
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
     return r;
 }
-__device__ __forceinline__ float exp2_approx(float v) {
-    float r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
-    return r;
-}
 
 }  // namespace

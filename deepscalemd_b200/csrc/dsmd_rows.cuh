@@ -17,7 +17,7 @@
 // consecutive bytes: entry k of row p at ((p >> 5) * stride + (k & ~3)) * 32 + (p & 31) * 4 + (k & 3) (row_base + row_offset).
 //   Owned partners come first, [0, row_int[p]); ghosts follow from the next multiple of four on and end at row_end[p];
 //   chunks are filled up with an atom that the search found outside the list radius of both atoms, so that the force kernel
-//   need not count (where the search met no such atom, the row is marked kRowCareful and is counted).
+//   need not count (where the search had met no such atom by then, the row is marked kRowCareful and is counted).
 //   The two atoms themselves are not listed. Partners that one of them excludes are kept apart, from the row's last place
 //   downwards, marked kExclFirst / kExclSecond: the main loop of the force kernel has no flags to look at.
 //   row_special[p] = owned excluded partners | ghosts << kRowCountBits | kRowCareful | kRowOwnExcluded (the two atoms exclude
@@ -350,6 +350,7 @@ k_build_rows(Grid g, int n_owned, int n_total, int n_quads, const int4* __restri
     }
     int interior0 = 0, interior1 = 0;
     unsigned interior_special0 = 0u, interior_special1 = 0u;
+    unsigned counted = 0u;   // bit h: row h has a chunk that no atom could fill up
     for (int seg = 0; seg < n_seg; ++seg) {
         const int row = seg * g.ncells + (zc * g.nc[1] + yc) * g.nc[0];
         int s0 = 0, len0 = 0, s1 = 0, len1 = 0;
@@ -393,6 +394,8 @@ k_build_rows(Grid g, int n_owned, int n_total, int n_quads, const int4* __restri
         const int k = (c & ~3) + (lane & 3);
         if (lane < 8 && k >= c && (c & 3) && k < out.stride)
             (lane < 4 ? q.row0 : q.row1)[row_offset(k)] = static_cast<unsigned>(far < 0 ? q.first : far);
+        // decided here and not at the end: the ghosts may still bring an atom that the owned chunk had to do without
+        counted |= (q.far0 < 0 && (q.count0 & 3) ? 1u : 0u) | (q.far1 < 0 && (q.count1 & 3) ? 2u : 0u);
         if (seg == 0 && n_seg == 2) {
             q.count0 = (q.count0 + 3) & ~3;
             q.count1 = (q.count1 + 3) & ~3;
@@ -407,7 +410,7 @@ k_build_rows(Grid g, int n_owned, int n_total, int n_quads, const int4* __restri
         out.row_end[2 * quad + lane] = min(ghosts ? count : interior, out.stride);
         out.row_int[2 * quad + lane] = min(interior, out.stride);
         out.row_special[2 * quad + lane] = n_own | ((n_special - n_own) << kRowCountBits) | (special & kRowOwnExcluded) |
-                                           ((lane ? q.far1 : q.far0) < 0 ? kRowCareful : 0u);
+                                           (counted >> lane & 1u ? kRowCareful : 0u);
         const int need = ((count + 3) & ~3) + static_cast<int>(n_special);   // whole chunks, and the ones apart behind them
         if (need > out.stride) atomicMax(&st->need_stride, static_cast<unsigned>(need));
         // pairs with a ghost partner, collected for the boundary pass of the force kernel (the order of the collection

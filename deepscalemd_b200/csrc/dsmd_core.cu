@@ -277,12 +277,23 @@ __global__ void k_push(int first, int count, const double* __restrict__ fx, cons
     }
 }
 
+// Atoms that k_constrained takes through the step, by global id; ids the constraints do not reach up to are free.
+struct ClusterMembers {
+    const unsigned char* member;   // [n_global], or null: no atom
+    int n_global;
+    const int* gid;
+    __device__ __forceinline__ bool has(int s) const {
+        if (!member) return false;
+        const int g = gid[s];
+        return g >= 0 && g < n_global && member[g];
+    }
+};
+
 __global__ void k_vv2(int n, double half_dt_c, double* __restrict__ vx, double* __restrict__ vy,
                       double* __restrict__ vz, const double* __restrict__ fx, const double* __restrict__ fy,
-                      const double* __restrict__ fz, const double* __restrict__ mass, const int* __restrict__ gid,
-                      const unsigned char* __restrict__ skip) {
+                      const double* __restrict__ fz, const double* __restrict__ mass, ClusterMembers skip) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n || (skip && skip[gid[s]])) return;
+    if (s >= n || skip.has(s)) return;
     const double a = half_dt_c / mass[s];
     vx[s] += a * fx[s];
     vy[s] += a * fy[s];
@@ -395,12 +406,12 @@ __global__ void k_pack(Grid g, int first, int count, int n_owned, double* __rest
                        const double* __restrict__ fz, const double* __restrict__ mass, const int* __restrict__ type,
                        const double* __restrict__ xref, const double* __restrict__ yref,
                        const double* __restrict__ zref, int4* __restrict__ pq, double dt, double kick_c,
-                       const int* __restrict__ gid, const unsigned char* __restrict__ skip, BondedForces bonded, DisplacementReport report) {
+                       ClusterMembers skip, BondedForces bonded, DisplacementReport report) {
     if (dsmd::gate_closed(report.st, report.gate2)) return;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int s = first + t;
     double d2 = 0.0;
-    if (t < count && !(skip && skip[gid[s]])) {   // skip: atoms of constraint clusters, by global id (k_constrained moves them)
+    if (t < count && !skip.has(s)) {
         double px = x[s], py = y[s], pz = z[s];
         if (INTEGRATE) {
             const double a = kick_c / mass[s];
@@ -657,7 +668,7 @@ struct dsmd_ctx {
     int* cl_gid = nullptr;
     int* cl_slot = nullptr;           // [n_clusters * kClusterAtoms] as of the last sort
     unsigned char* cl_member = nullptr;   // [cons_n_global] 1: the atom belongs to a cluster
-    bool cl_cover_all = false;        // every atom does
+    int64_t cl_atoms = 0;             // that do
     int cl_shape = 0;                 // 0: any, 1: triangles, 2: bonds
     unsigned char* cl_a = nullptr;
     unsigned char* cl_b = nullptr;
@@ -1513,14 +1524,14 @@ int dsmd_list_export(dsmd_ctx* c, int32_t* d_i, int32_t* d_j, uint8_t* d_flags, 
 
 // kick: 0.5 for the first velocity-Verlet half, 1.0 for the merged second-and-first half.
 static int pack_impl(dsmd_ctx* c, int64_t first, int64_t count, bool integrate, double dt, double f2a, cudaStream_t s,
-                     double kick = 0.5, const unsigned char* skip = nullptr, const BondedForces* bonded = nullptr) {
+                     double kick = 0.5, const ClusterMembers& skip = {}, const BondedForces* bonded = nullptr) {
     if (count <= 0) return DSMD_OK;
     const DisplacementReport report = displacement_report(c, first == 0 && count >= c->n_owned, s);
     double** r = c->real[c->cur];
     const auto kernel = !integrate ? k_pack<false, false> : (bonded ? k_pack<true, true> : k_pack<true, false>);
     kernel<<<blocks_for(count, kThreads), kThreads, 0, s>>>(
         c->grid, static_cast<int>(first), static_cast<int>(count), static_cast<int>(c->n_owned), r[0], r[1], r[2], r[3], r[4], r[5],
-        r[6], r[7], r[8], r[9], c->type[c->cur], c->ref[0], c->ref[1], c->ref[2], c->pq, dt, kick * dt * f2a, c->gid[c->cur], skip,
+        r[6], r[7], r[8], r[9], c->type[c->cur], c->ref[0], c->ref[1], c->ref[2], c->pq, dt, kick * dt * f2a, skip,
         bonded ? *bonded : BondedForces{}, report);
     DSMD_LAUNCHED(c);
     return DSMD_OK;
@@ -1703,7 +1714,7 @@ int launch_constrained(dsmd_ctx* c, bool finish, bool start, double half_kick, d
     double** r = c->real[c->cur];
     const AtomArrays at{r[0], r[1], r[2], r[3], r[4], r[5], r[6], r[7], r[8], r[9], c->type[c->cur], c->ref[0], c->ref[1], c->ref[2], c->pq};
     const unsigned blocks = blocks_for(c->n_clusters, 128);
-    const DisplacementReport report = start ? displacement_report(c, c->cl_cover_all, s) : DisplacementReport{c->status, nullptr, nullptr, 0, HUGE_VAL};
+    const DisplacementReport report = start ? displacement_report(c, c->cl_atoms == c->n_owned, s) : DisplacementReport{c->status, nullptr, nullptr, 0, HUGE_VAL};
     const auto launch = [&](auto shape) {
         const auto kernel = finish && start ? k_constrained<decltype(shape), true, true>
                                             : (finish ? k_constrained<decltype(shape), true, false> : k_constrained<decltype(shape), false, true>);
@@ -1723,12 +1734,13 @@ int constrained_halves(dsmd_ctx* c, bool finish, bool start, double dt, double f
     { const int rc = ensure_slot_map(c, s); if (rc) return rc; }
     const double half_kick = 0.5 * dt * f2a;
     const int rc = launch_constrained(c, finish, start, half_kick, dt, 0.0, nullptr, s);
-    if (rc || c->cl_cover_all) return rc;
+    if (rc || c->cl_atoms == c->n_owned) return rc;
     // the free atoms
-    if (start) return pack_impl(c, 0, c->n_owned, true, dt, f2a, s, finish ? 1.0 : 0.5, c->cl_member);
+    const ClusterMembers members{c->cl_member, static_cast<int>(c->cons_n_global), c->gid[c->cur]};
+    if (start) return pack_impl(c, 0, c->n_owned, true, dt, f2a, s, finish ? 1.0 : 0.5, members);
     double** r = c->real[c->cur];
     k_vv2<<<blocks_for(c->n_owned, kThreads), kThreads, 0, s>>>(static_cast<int>(c->n_owned), half_kick, r[3], r[4], r[5], r[6], r[7], r[8],
-                                                               r[9], c->gid[c->cur], c->cl_member);
+                                                               r[9], members);
     DSMD_LAUNCHED(c);
     return DSMD_OK;
 }
@@ -1818,7 +1830,7 @@ int dsmd_set_constraints(dsmd_ctx* c, int64_t n_global, int64_t n_constraints, c
     std::vector<unsigned char> member(static_cast<size_t>(n_global), 0);
     for (int g : gids)
         if (g >= 0) member[static_cast<size_t>(g)] = 1;
-    c->cl_cover_all = std::find(member.begin(), member.end(), 0) == member.end();
+    c->cl_atoms = std::count(member.begin(), member.end(), 1);
     DSMD_CUDA(c, cudaMalloc(&c->cl_member, member.size()));
     DSMD_CUDA(c, cudaMemcpy(c->cl_member, member.data(), member.size(), cudaMemcpyHostToDevice));
     // one shape for all: compiled with the constraint order known
@@ -1866,7 +1878,7 @@ int dsmd_integrate(dsmd_ctx* c, int half, double dt, double f2a, void* stream) {
     if (half == 1) return pack_impl(c, 0, c->n_owned, true, dt, f2a, s);
     double** r = c->real[c->cur];
     k_vv2<<<blocks_for(c->n_owned, kThreads), kThreads, 0, s>>>(static_cast<int>(c->n_owned), 0.5 * dt * f2a, r[3], r[4],
-                                                               r[5], r[6], r[7], r[8], r[9], c->gid[c->cur], nullptr);
+                                                               r[5], r[6], r[7], r[8], r[9], ClusterMembers{});
     DSMD_LAUNCHED(c);
     return DSMD_OK;
 }
@@ -2128,7 +2140,7 @@ int dsmd_run_nve(dsmd_ctx* c, int64_t n_steps, double dt, double f2a, double hi_
             if (bonded) {   // the bonded contributions go straight into the pass over the atoms
                 if (!rc) rc = bonded_terms(c, false, s);
                 const BondedForces terms = bonded_forces(c);
-                if (!rc) rc = pack_impl(c, 0, c->n_owned, true, dt, f2a, s, 1.0, nullptr, &terms);
+                if (!rc) rc = pack_impl(c, 0, c->n_owned, true, dt, f2a, s, 1.0, {}, &terms);
             } else {
                 if (!rc) rc = dsmd_compute_bonded(c, s);
                 if (!rc) rc = constrained ? constrained_halves(c, true, true, dt, f2a, s) : dsmd_integrate(c, 3, dt, f2a, s);

@@ -48,3 +48,36 @@ def _owned_share(pairs, pos, box, rc, n):
     d[:, 1:] -= box[1:] * np.rint(d[:, 1:] / box[1:])
     inside = (d * d).sum(1) < rc * rc
     return 0.5 * (2 * inside.sum() - (inside & (pairs.max(1) >= n)).sum())
+
+
+@pytest.mark.parametrize("free_below", [False, True])
+def test_constraints_on_fewer_ids_than_atoms(cuda_device, free_below):
+    """Molecules numbered first, other atoms behind them, and constraints set for the molecules' ids only: the others move as
+    free atoms do, in the single halves and in the loop. free_below: an unconstrained id among the molecules' ids as well."""
+    rng = np.random.default_rng(1)
+    shape, groups, L, dt = np.array([[0.0, 0.0, 0.0], [1.0, 0.1, 0.0], [0.3, 0.9, 0.0]]), 40, 30.0, 0.5
+    sites = np.stack(np.meshgrid(*[np.arange(5)] * 3, indexing="ij"), -1).reshape(-1, 3) * 6.0 + 0.5
+    bound = (sites[:groups, None] + shape).reshape(-1, 3)
+    pos = np.concatenate([bound, sites[groups:groups + 50]])
+    n, box, n_ids = len(pos), np.full(3, L), len(bound) + (1 if free_below else 0)
+    rows = np.array([(3 * g + a, 3 * g + b, np.linalg.norm(shape[a] - shape[b])) for g in range(groups) for a, b in ((0, 1), (0, 2), (1, 2))])
+    vel = np.concatenate([np.repeat(rng.normal(scale=0.01, size=(groups, 3)), 3, axis=0), rng.normal(scale=0.01, size=(50, 3))])
+    for loop in (False, True):
+        ctx = capi.Context(n)
+        ctx.set_box(box)
+        ctx.set_pair_params([[0.0]], [[1.0]], 3.0, 0.5)
+        ctx.set_constraints(n_ids, rows)
+        ctx.upload(pos, vel=vel, mass=rng.uniform(1.0, 16.0, n))
+        ctx.build_neighbor_list()
+        ctx.compute_forces()
+        if loop:
+            ctx.run_nve(4, dt)
+        else:
+            for _ in range(4):
+                ctx.integrate(1, dt)
+                ctx.compute_forces()
+                ctx.integrate(2, dt)
+        assert np.abs(ctx.field_by_gid("xyz", n) - (pos + 4 * dt * vel)).max() <= 1e-9   # no forces: all drift, molecules as a whole
+        if not loop:
+            assert abs(ctx.max_displacement_sq() - ((4 * dt * vel) ** 2).sum(1).max()) <= 1e-9
+        ctx.close()

@@ -77,6 +77,14 @@ def _arr(a, dtype):
     return None if a is None else np.ascontiguousarray(a, dtype=dtype)
 
 
+def _rows_of_three(a):
+    """The first three columns as contiguous rows: what the library reads is three values per row, so fewer are refused."""
+    a = np.asarray(a)
+    if a.ndim < 2 or a.shape[1] < 3:
+        raise IndexError(f"three values per atom wanted, got an array of shape {a.shape}")
+    return np.ascontiguousarray(a[:, :3], dtype=np.float64)
+
+
 def _p(a):
     return None if a is None else a.ctypes.data_as(c_void_p)
 
@@ -208,10 +216,10 @@ class Context:
 
     # -- particles ----------------------------------------------------------------------------------------------------
     def upload(self, pos, n_owned=None, vel=None, mass=None, charge=None, types=None, gid=None, stream=None):
-        pos = np.ascontiguousarray(np.asarray(pos)[:, :3], dtype=np.float64)
+        pos = _rows_of_three(pos)
         n = len(pos)
         n_owned = n if n_owned is None else n_owned
-        vel = None if vel is None else np.ascontiguousarray(np.asarray(vel)[:, :3], dtype=np.float64)
+        vel = None if vel is None else _rows_of_three(vel)
         m, q = _arr(mass, np.float64), _arr(charge, np.float64)
         t, g = _arr(types, np.int32), _arr(gid, np.int32)
         self._check(self.lib.dsmd_upload_rows(self.h, c_int64(n_owned), c_int64(n), _p(pos), _p(vel), _p(m), _p(q), _p(t),

@@ -631,6 +631,7 @@ struct dsmd_ctx {
     Mail* mail = nullptr;           // pinned: kMailDisplacement .. + 3 in turn, kMailKinetic, kMailScalars
     double gate2 = HUGE_VAL;        // limit that the launches of the MD loop carry (gate_closed)
     bool captured = false;          // a call was captured into a graph: results are copied, not reported
+    bool word_shared = false;       // the caller has the displacement word's address and may write there
     unsigned long long seq = 0;     // launches that reported something so far
     unsigned long long disp_seq = 0, scalars_seq = 0;   // the last displacement check / energy sum whose report still stands (0: none)
     Status* status = nullptr;
@@ -1547,7 +1548,7 @@ int dsmd_max_displacement_sq(dsmd_ctx* c, double* out, void* stream) {
     if (!c || !out) return DSMD_ERR_INVALID;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     bool outside;
-    if (c->disp_seq && !c->captured) {   // nothing has touched the status since the last displacement check: its report says it all
+    if (c->disp_seq && !c->captured && !c->word_shared) {   // nothing has touched the status since the last displacement check: its report says it all
         DSMD_CUDA(c, cudaStreamSynchronize(s));
         const int slot = kMailDisplacement + static_cast<int>(c->disp_seq & 3);
         { const int rc = wait_mail(c, slot, 2, c->disp_seq, s); if (rc) return rc; }
@@ -2389,6 +2390,7 @@ int dsmd_halo_pack(dsmd_ctx* c, const int32_t* d_index, const int8_t* d_image, i
 int dsmd_displacement_word(dsmd_ctx* c, void** device_word) {
     if (!c || !device_word) return DSMD_ERR_INVALID;
     *device_word = &c->status->max_disp2;
+    c->word_shared = true;
     return DSMD_OK;
 }
 

@@ -81,3 +81,21 @@ def test_constraints_on_fewer_ids_than_atoms(cuda_device, free_below):
         if not loop:
             assert abs(ctx.max_displacement_sq() - ((4 * dt * vel) ** 2).sum(1).max()) <= 1e-9
         ctx.close()
+
+
+def test_displacement_word_written_by_the_caller(cuda_device):
+    """Ranks reduce over the displacement word in place: the query answers with what stands there."""
+    import torch
+    pos = np.array([[1.0, 1.0, 1.0], [5.0, 5.0, 5.0], [9.0, 3.0, 2.0]])
+    ctx = capi.Context(3)
+    ctx.set_box(np.full(3, 12.0))
+    ctx.set_pair_params([[1.0]], [[1.0]], 2.5, 0.3)
+    ctx.upload(pos)
+    ctx.build_neighbor_list()
+    word = ctx.displacement_word()
+    ctx.pack_positions()
+    assert ctx.max_displacement_sq() == 0.0
+    word.copy_(torch.tensor([4.0], dtype=torch.float64).view(torch.int64))
+    torch.cuda.synchronize()
+    assert ctx.max_displacement_sq() == 4.0
+    ctx.close()

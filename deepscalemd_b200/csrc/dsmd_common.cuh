@@ -57,9 +57,10 @@ struct Status {
 // check carry the limit, and do nothing when the check before them went beyond it (the host, which finds out later, then
 // rebuilds the list and launches them again). Read from a word that only the end of a check writes, so that all blocks of a
 // launch see the same.
+constexpr double kGateOpen = 1.0e300;   // a limit from here on: no gate
 #ifdef __CUDACC__
 __device__ __forceinline__ bool gate_closed(const Status* st, double limit2) {
-    return limit2 < 1.0e300 && __ldcg(&st->gate) > limit2;
+    return limit2 < kGateOpen && __ldcg(&st->gate) > limit2;
 }
 #endif
 

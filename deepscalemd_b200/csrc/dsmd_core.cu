@@ -2167,7 +2167,11 @@ int dsmd_run_nve(dsmd_ctx* c, int64_t n_steps, double dt, double f2a, double hi_
             }
             double d2 = 0.0;
             const int rc = reported(check, d2);
-            if (rc) return rc;
+            if (rc) {
+                // an atom outside closed the gate: the kernel queued above left its buffer of positions unwritten
+                if (advanced && fused && limit2 < dsmd::kGateOpen) std::swap(c->pq, c->pq_next);
+                return rc;
+            }
             if (d2 > limit2) rebuild = true;
             if (!rebuild) worst = std::max(worst, d2);
         } else {

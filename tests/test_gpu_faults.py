@@ -99,3 +99,27 @@ def test_displacement_word_written_by_the_caller(cuda_device):
     torch.cuda.synchronize()
     assert ctx.max_displacement_sq() == 4.0
     ctx.close()
+
+
+def test_loop_that_ends_with_an_atom_outside(cuda_device):
+    """The MD loop queues the next step before it looks at the check of the current one. When that check ends the loop with an
+    error, forces are those of the positions the context holds."""
+    box = np.array([12.0, 12.0, 12.0])
+    pos = np.array([[2.0, 2.0, 2.0], [3.15, 2.0, 2.0], [11.5, 8.0, 8.0]])
+    vel = np.array([[0.3, 0.0, 0.0], [-0.2, 0.0, 0.0], [4.0, 0.0, 0.0]])
+    for steps in (40, 41):
+        ctx = capi.Context(3)
+        ctx.set_box(box, (0, 1, 1))
+        ctx.set_pair_params([[1.0]], [[1.0]], 2.5, 0.3)
+        ctx.upload(pos, vel=vel)
+        ctx.build_neighbor_list()
+        ctx.compute_forces()
+        with pytest.raises(RuntimeError):
+            ctx.run_nve(steps, 0.01, lagged=False)
+        ctx.compute_forces()
+        got = ctx.forces_by_gid(3)
+        ctx.pack_positions()
+        ctx.compute_forces()
+        want = ctx.forces_by_gid(3)
+        assert np.abs(want[:2]).max() > 0.1 and np.array_equal(got, want)
+        ctx.close()

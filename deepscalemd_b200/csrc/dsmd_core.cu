@@ -1623,7 +1623,7 @@ static int compute_forces_impl(dsmd_ctx* c, int phase, int want_energy, int64_t 
     const int64_t pairs = phase == DSMD_PHASE_BOUNDARY ? c->n_boundary : (ranged ? count : 2 * c->n_quads);
     const bool e = want_energy != 0;
     if (e) { const int rc = ensure_partials(c, std::max<int64_t>(pair_blocks(c, pairs, true), 1)); if (rc) return rc; }
-    const bool report = e && reports_count(c, s);
+    const bool report = reports_count(c, s) && e;
     double** r = c->real[c->cur];
     const ForceArgs a{c->pq, c->qf, rows_of(c), phase, phase == DSMD_PHASE_BOUNDARY ? c->boundary_pairs : nullptr,
                       static_cast<int>(ranged ? first : 0), static_cast<int>(pairs), c->lane_shift, r[DSMD_FX], r[DSMD_FY], r[DSMD_FZ], c->partials,
@@ -2128,7 +2128,9 @@ int dsmd_run_nve(dsmd_ctx* c, int64_t n_steps, double dt, double f2a, double hi_
     // next (the same forces) are one pass over the atoms, with RATTLE between them where there are constraints; and where
     // the pair forces are all the forces there are, that pass is the end of the force kernel (k_step).
     const bool constrained = c->n_clusters > 0, bonded = !constrained && c->bonded.terms() > 0;
-    const bool fused = !constrained && !bonded && !c->coulomb && c->n_owned > 0;
+    // (Not for a context that was ever captured: the loop of such steps swaps the two buffers of positions that kernels read,
+    // and a graph holds the address of one of them.)
+    const bool fused = !constrained && !bonded && !c->coulomb && c->n_owned > 0 && !reporting.captured;
     // Forces at the current positions and on to the next ones, up to their displacement check; nothing happens on the device
     // when the check of the current ones went beyond `gate2`.
     const auto advance = [&](double gate2) {

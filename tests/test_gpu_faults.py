@@ -123,3 +123,35 @@ def test_loop_that_ends_with_an_atom_outside(cuda_device):
         want = ctx.forces_by_gid(3)
         assert np.abs(want[:2]).max() > 0.1 and np.array_equal(got, want)
         ctx.close()
+
+
+@pytest.mark.parametrize("steps", [2, 3])
+def test_captured_forces_after_the_loop(cuda_device, steps):
+    """A force evaluation with energy sums captured into a graph, then a loop without a rebuild: a replay evaluates the positions
+    the loop left, and the sums are read from the device."""
+    import torch
+    rng = np.random.default_rng(3)
+    side = 8
+    sites = np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    pos, n, box = (sites + rng.uniform(0.4, 0.6, sites.shape)) * 1.1, side ** 3, np.full(3, side * 1.1)
+    ctx = capi.Context(n)
+    ctx.set_box(box)
+    ctx.set_pair_params([[1.0]], [[1.0]], 2.5, 0.35)
+    ctx.upload(pos, vel=rng.normal(size=(n, 3)))
+    ctx.build_neighbor_list()
+    ctx.compute_forces(want_energy=True)
+    before = ctx.read_scalars()["pe"]
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        ctx.compute_forces(want_energy=True, stream=stream)
+    assert ctx.run_nve(steps, 0.005, hi_frac=1.0, lagged=False)["rebuilds"] == 0
+    graph.replay()
+    torch.cuda.synchronize()
+    got, pe = ctx.forces_by_gid(n), ctx.read_scalars()["pe"]
+    ctx.pack_positions()
+    ctx.compute_forces(want_energy=True)
+    want = ctx.forces_by_gid(n)
+    assert np.array_equal(got, want) and pe == ctx.read_scalars()["pe"] and pe != before
+    del graph
+    ctx.close()

@@ -593,7 +593,8 @@ struct dsmd_ctx {
     int* ghost_slot = nullptr;
     // the host-buffer force call as a pipeline (dsmd_forces_host): first slot of every z layer of cells as of the last
     // build, two copy streams, one event pair per piece
-    int* h_layer_start = nullptr;     // pinned, [nc_z + 1]
+    unsigned long long* h_layer_start = nullptr;   // pinned, [nc_z + 1]: slot, and in the upper half the build's layer_tag
+    unsigned layer_tag = 0;
     int layer_capacity = 0;
     cudaStream_t copy_in = nullptr, copy_out = nullptr;
     cudaEvent_t piece_up[16] = {}, piece_done[16] = {}, pipe_begin = nullptr, pipe_end = nullptr;
@@ -1399,7 +1400,8 @@ static int build_list(dsmd_ctx* c, bool forces, cudaStream_t s) {
         if (layers + 1 > c->layer_capacity) {
             if (c->h_layer_start) cudaFreeHost(c->h_layer_start);
             c->h_layer_start = nullptr;
-            DSMD_CUDA(c, cudaMallocHost(&c->h_layer_start, sizeof(int) * (layers + 1)));
+            DSMD_CUDA(c, cudaMallocHost(&c->h_layer_start, sizeof(unsigned long long) * (layers + 1)));
+            std::memset(c->h_layer_start, 0, sizeof(unsigned long long) * (layers + 1));
             c->layer_capacity = layers + 1;
         }
     }
@@ -1415,8 +1417,9 @@ static int build_list(dsmd_ctx* c, bool forces, cudaStream_t s) {
         { const int rc = lay_out_rows(c, row_entries); if (rc) return rc; }
         const ExclusionTable ex{c->excl_off, c->excl_partner, static_cast<int>(c->excl_n_global)};
         if (attempt == 0) {
+            c->layer_tag = static_cast<unsigned>(++c->seq);
             k_quads<<<blocks_for(rows * 32, kThreads), kThreads, 0, s>>>(c->grid.nc[0], c->grid.nc[1], static_cast<int>(rows),
-                                                                        static_cast<int>(c->n_owned), c->cell_start, c->quad, c->h_layer_start);
+                                                                        static_cast<int>(c->n_owned), c->cell_start, c->quad, c->h_layer_start, c->layer_tag);
             DSMD_LAUNCHED(c);
         }
         const unsigned blocks = blocks_for(c->n_quads * 32, kBuildThreads);
@@ -2272,6 +2275,13 @@ static int forces_host_pipelined(dsmd_ctx* c, const double* x, const double* y, 
     const int layers = c->grid.nc[2], S = c->grid.stencil;
     const int pieces = std::min(std::max(4, std::min(kSlabs, static_cast<int>(c->n_owned / kSlabAtoms))), layers / (2 * S));
     if (pieces < 4 || !c->h_layer_start || c->n_total != c->n_owned) return DSMD_ERR_STATE;
+    // the build's own report says nothing about words that an earlier kernel wrote to the host: each one says it for itself
+    const volatile unsigned long long* layer_start = c->h_layer_start;
+    for (int l = 0; l <= layers; ++l)
+        if (static_cast<unsigned>(layer_start[l] >> 32) != c->layer_tag) {
+            DSMD_CUDA(c, cudaDeviceSynchronize());
+            break;
+        }
     if (!c->copy_in) {
         DSMD_CUDA(c, cudaStreamCreateWithFlags(&c->copy_in, cudaStreamNonBlocking));
         DSMD_CUDA(c, cudaStreamCreateWithFlags(&c->copy_out, cudaStreamNonBlocking));
@@ -2283,7 +2293,7 @@ static int forces_host_pipelined(dsmd_ctx* c, const double* x, const double* y, 
         DSMD_CUDA(c, cudaEventCreateWithFlags(&c->pipe_end, cudaEventDisableTiming));
     }
     const auto layer_of = [&](int k) { return static_cast<int>(static_cast<int64_t>(layers) * k / pieces); };
-    const auto slot_of = [&](int layer) { return layer == 0 ? 0 : (layer == layers ? c->n_owned : static_cast<int64_t>(c->h_layer_start[layer])); };
+    const auto slot_of = [&](int layer) { return layer == 0 ? 0 : (layer == layers ? c->n_owned : static_cast<int64_t>(layer_start[layer] & 0xFFFFFFFFull)); };
     // everything queued on the caller's stream so far comes first
     DSMD_CUDA(c, cudaEventRecord(c->pipe_begin, s));
     DSMD_CUDA(c, cudaStreamWaitEvent(c->copy_in, c->pipe_begin, 0));

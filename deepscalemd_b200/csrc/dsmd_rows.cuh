@@ -50,17 +50,18 @@ __device__ __forceinline__ int pair_atoms(const unsigned* __restrict__ quad, int
 
 // The quads of every cell row (one warp per row): the numbers between two rows' bases that no atoms fill are kNoQuad.
 // layer_start (pinned host memory): first slot of every z layer of cells, and the end, by which a caller cuts the sorted
-// atoms into slabs.
+// atoms into slabs; with `tag` in the same word, so that the host sees of each whether it has arrived.
 __global__ void k_quads(int nx, int ny, int rows, int n_owned, const int* __restrict__ cell_start, unsigned* __restrict__ quad,
-                        int* __restrict__ layer_start) {
+                        volatile unsigned long long* layer_start, unsigned tag) {
     const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (row >= rows) return;
     const int begin = min(cell_start[static_cast<size_t>(row) * nx], n_owned);
     const int end = row + 1 < rows ? min(cell_start[static_cast<size_t>(row + 1) * nx], n_owned) : n_owned;
     const int q0 = row == 0 ? 0 : quad_base(begin, row), q1 = quad_base(end, row + 1);
     const int q_first = quad_base(begin, row);
-    if (lane == 0 && row % ny == 0) layer_start[row / ny] = begin;
-    if (lane == 0 && row + 1 == rows) layer_start[rows / ny] = end;
+    const unsigned long long tagged = static_cast<unsigned long long>(tag) << 32;
+    if (lane == 0 && row % ny == 0) layer_start[row / ny] = tagged | static_cast<unsigned>(begin);
+    if (lane == 0 && row + 1 == rows) layer_start[rows / ny] = tagged | static_cast<unsigned>(end);
     for (int q = q0 + lane; q < q1; q += 32) {
         const int s = begin + 4 * (q - q_first);
         quad[q] = (q >= q_first && s < end) ? static_cast<unsigned>(s) * 4u + static_cast<unsigned>(min(end - s, 4) - 1) : kNoQuad;

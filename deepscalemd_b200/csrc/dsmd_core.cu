@@ -111,9 +111,10 @@ __global__ void k_cell_keys(Grid g, Brick brick, int first, int n_owned, int n_t
 }
 
 // Gathers every particle array into sorted order, writes the fixed-point layout, the displacement reference and the
-// ghost slot map. FORCES: the force arrays too (a loop that evaluates forces next does not need them).
+// ghost slot map. FORCES: the force arrays too (a loop that evaluates forces next does not need them). unranked: the cell of
+// atoms that are about to be removed, any number of them in any order, or a number that no cell has.
 template <bool FORCES>
-__global__ void k_reorder(Grid g, int first, int n_owned, int n_total, const unsigned* __restrict__ key,
+__global__ void k_reorder(Grid g, int first, int n_owned, int n_total, unsigned unranked, const unsigned* __restrict__ key,
                           const int* __restrict__ list, const int* __restrict__ cell_start, RealArrays src, RealArrays dst, const int* __restrict__ type_src,
                           const int* __restrict__ gid_src, int* __restrict__ type_dst, int* __restrict__ gid_dst,
                           int4* __restrict__ pq, float* __restrict__ qf, double* __restrict__ xref,
@@ -121,7 +122,7 @@ __global__ void k_reorder(Grid g, int first, int n_owned, int n_total, const uns
     const int t = first + blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n_total) return;
     const int from = list[t];
-    const int s = dsmd::cell_slot(from, key[from], cell_start, list);
+    const int s = key[from] == unranked ? t : dsmd::cell_slot(from, key[from], cell_start, list);
     double r[kNumReal];
 #pragma unroll
     for (int f = 0; f < kNumReal; ++f)
@@ -936,7 +937,7 @@ int sort_range(dsmd_ctx* c, int64_t first, cudaStream_t s, bool clear, const Bri
         DSMD_LAUNCHED(c);
         const auto reorder = forces ? k_reorder<true> : k_reorder<false>;
         reorder<<<blocks_for(n, kThreads), kThreads, 0, s>>>(
-            c->grid, i0, static_cast<int>(c->n_owned), in, c->key, c->list, c->cell_start, arrays_of(c, from), arrays_of(c, to),
+            c->grid, i0, static_cast<int>(c->n_owned), in, brick.drop ? static_cast<unsigned>(c->grid.ncells) : 0xFFFFFFFFu, c->key, c->list, c->cell_start, arrays_of(c, from), arrays_of(c, to),
             c->type[from], c->gid[from], c->type[to], c->gid[to], c->pq, c->qf, c->ref[0], c->ref[1], c->ref[2], c->ghost_slot);
         DSMD_LAUNCHED(c);
     } else if (clear) {

@@ -46,6 +46,7 @@ constexpr int kDeviceSms = 148;                       // of a B200
 constexpr int64_t kPairLanesWanted = kDeviceSms * 512;
 constexpr int64_t kPairLanesWantedEwald = kDeviceSms * 768;   // two rounds of one block of 384 each
 constexpr int kLongRow = 240;                         // entries (with the row's spare room): about 150 partners per atom
+constexpr int64_t kRowsAlways = 4096;                 // cell rows that any system may have: 2 MB of list rows
 constexpr int kXRefine = 4;    // x cells per cell width of the y and z axes (tighter row windows in the list build)
 enum { kMailDisplacement = 0, kMailKinetic = 4, kMailScalars = 5, kMailBuild = 6, kMailSlots = 7 };   // report slots
 constexpr int kStageAtoms = 16384;
@@ -777,6 +778,19 @@ int make_grid(dsmd_ctx* c) {
         }
         stencil = 1;
     }
+    // A cell row costs the list most of a quad's number and storage whether atoms are in it or not (quad_base): no more rows
+    // than half the atoms there is room for. Emptier boxes get wider y and z cells.
+    const int64_t rows_most = std::max<int64_t>(kRowsAlways, c->capacity / 2);
+    for (bool narrower = true; narrower && static_cast<int64_t>(g.nc[1]) * g.nc[2] > rows_most;) {
+        const double share = std::sqrt(static_cast<double>(rows_most) / (static_cast<double>(g.nc[1]) * g.nc[2]));
+        narrower = false;
+        for (int a = 1; a < 3; ++a) {
+            const int fewer = std::max(g.wrap[a] ? 2 * g.stencil + 1 : 1, static_cast<int>(g.nc[a] * share));
+            if (fewer >= g.nc[a]) continue;
+            g.nc[a] = fewer;
+            narrower = true;
+        }
+    }
     // Rows of cells along x are contiguous runs of slots, searched through a window that is rounded outwards to whole
     // cells: finer x cells (kXRefine per unrefined cell) make the windows tighter at no cost per row.
     g.x_reach = static_cast<float>(g.stencil * (1.0 / (g.inv_len[0] * g.nc[0])) * 0.9999999);
@@ -875,7 +889,8 @@ RowArrays rows_of(const dsmd_ctx* c) { return RowArrays{c->quad, c->rows, c->str
 // is the chain of dependent reads along a row. A function of the system alone, so that a pass over a part of the atoms
 // gives the same bits as a pass over all of them.
 int pair_lane_shift(const dsmd_ctx* c) {
-    const int64_t pairs = 2 * c->n_quads, wanted = ewald_copies(c) == kEwaldCopiesMost ? kPairLanesWantedEwald : kPairLanesWanted;
+    const int64_t pairs = std::min(2 * c->n_quads, c->n_owned);   // as many rows at most have atoms
+    const int64_t wanted = ewald_copies(c) == kEwaldCopiesMost ? kPairLanesWantedEwald : kPairLanesWanted;
     int shift = 0;
     while (shift < 5 && (pairs << shift) < wanted && (8 << shift) <= c->stride) ++shift;
     return shift;

@@ -185,3 +185,32 @@ def test_sort_that_removes_most_atoms(cuda_device):
         assert np.array_equal(ctx.download("global_id"), kept[name])   # a sort of sorted atoms changes nothing
     assert seconds["most"] <= 5.0 * seconds["few"]
     ctx.close()
+
+
+@pytest.mark.parametrize("n,L,periodic", [(2000, 360.0, 1), (2000, 360.0, 0), (9000, 300.0, 1)])
+def test_mostly_empty_box(cuda_device, n, L, periodic):
+    """A droplet in a box many times its size: memory goes with the atoms and not with the cross-section of the box (it was
+    324 MB for the first case), and list and forces are the oracle's."""
+    import torch
+    rng = np.random.default_rng(n)
+    side = int(np.ceil(n ** (1 / 3)))
+    sites = np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij"), -1).reshape(-1, 3)[:n]
+    pos = (sites + rng.uniform(-0.05, 0.05, (n, 3))) * 1.1 + 0.5 * L
+    pos[:20] = rng.uniform(0.05 * L, 0.4 * L, (20, 3))
+    box, rc, skin = np.full(3, L), 2.5, 0.3
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    ctx = capi.Context(n)
+    ctx.set_box(box, (periodic, periodic, periodic))
+    ctx.set_pair_params([[1.0]], [[1.0]], rc, skin)
+    ctx.upload(pos)
+    ctx.build_neighbor_list()
+    ctx.compute_forces()
+    assert free - torch.cuda.mem_get_info()[0] <= 160 << 20
+    pairs = co.pairs(*pos.T, n, box, periodic=(periodic,) * 3, search=rc + skin)
+    want, _ = co.forces(*pos.T, n, box, pairs, *co.lj_tables([[1.0]], [[1.0]]), rc, periodic=(periodic,) * 3)
+    assert np.abs(ctx.forces_by_gid(n) - want).max() <= 2e-5 * np.abs(want).max()
+    gid = ctx.download("global_id")
+    i, j, _ = ctx.list_pairs()
+    assert np.array_equal(co.canonical_pairs(np.stack([gid[i], gid[j]], 1)[gid[i] < gid[j]]), co.canonical_pairs(pairs))
+    ctx.close()

@@ -61,6 +61,13 @@ __device__ __forceinline__ void ewald_functions(const EwaldTable<COPIES>& table,
     if (ENERGY) ef = ewald_cubic(table.mine + (table.intervals + idx) * COPIES, t);
 }
 
+// The same in closed form, for r^2 below the table.
+__device__ __forceinline__ void ewald_functions_analytic(const PairParams& p, float r2, float& ff, float& ef) {
+    const float r = sqrtf(r2), ar = p.alpha * r, ec = erfcf(ar) / r;
+    ff = (ec + p.two_alpha_sqrtpi * __expf(-ar * ar)) / r2;
+    ef = ec;
+}
+
 // What one evaluation needs to know of the two pairs.
 struct PairTerms {
     F2 rep, att;   // 12 c12, -6 c6
@@ -139,13 +146,8 @@ struct PairAccumulator {
             ewald_functions<ENERGY>(table, ra, p.ewald_most, ffa, efa);
             ewald_functions<ENERGY>(table, rb, p.ewald_most, ffb, efb);
             if (CAREFUL) {
-                const auto analytic = [&](float r2_, float& ff, float& ef) {
-                    const float r = sqrtf(r2_), ar = p.alpha * r, ec = erfcf(ar) / r;
-                    ff = (ec + p.two_alpha_sqrtpi * __expf(-ar * ar)) / r2_;
-                    ef = ec;
-                };
-                if (ra < kEwaldFirst) analytic(ra, ffa, efa);
-                if (rb < kEwaldFirst) analytic(rb, ffb, efb);
+                if (ra < kEwaldFirst) ewald_functions_analytic(p, ra, ffa, efa);
+                if (rb < kEwaldFirst) ewald_functions_analytic(p, rb, ffb, efb);
                 const float ia = rsqrtf(ra), ib = rsqrtf(rb);
                 if (ex_a) { ffa -= ia * ia * ia; efa -= ia; }
                 if (ex_b) { ffb -= ib * ib * ib; efb -= ib; }
@@ -173,16 +175,60 @@ struct PairAccumulator {
         }
     }
 
+    // What the plain form, which takes the table's first value for any distance below the table, left out of one entry's Ewald
+    // terms. qq: Coulomb constant times the charges of the two pairs.
+    __device__ __forceinline__ void add_close_rest(const PairParams& p, const EwaldTable<COPIES>& table, const int4& pa, const int4& pb,
+                                                   const int4& pj, F2 qq) {
+        F2 dx, dy, dz;
+        const F2 r2 = distance(p, pa, pb, pj, dx, dy, dz);
+        float ra, rb;
+        parts(r2, ra, rb);
+        if (fminf(ra, rb) >= kEwaldFirst) return;
+        float ffa, ffb, efa = 0.0f, efb = 0.0f, tfa, tfb, tea = 0.0f, teb = 0.0f;
+        ewald_functions_analytic(p, ra, ffa, efa);
+        ewald_functions_analytic(p, rb, ffb, efb);
+        ewald_functions<ENERGY>(table, ra, p.ewald_most, tfa, tea);
+        ewald_functions<ENERGY>(table, rb, p.ewald_most, tfb, teb);
+        sum(dx, dy, dz, r2, mul(qq, f2(ffa - tfa, ffb - tfb)), mul(qq, f2(efa - tea, efb - teb)), ra < kEwaldFirst && ra < p.rc2,
+            rb < kEwaldFirst && rb < p.rc2);
+        n_in = 0;   // counted already
+    }
+
+    // Sums of all lanes of a warp, in every lane.
+    __device__ __forceinline__ void over_warp() {
+        F2* const sums[8] = {&ax, &ay, &az, &e_sum, &w_sum, &wx, &wy, &wz};
+#pragma unroll
+        for (int k = 0; k < (ENERGY ? 8 : 3); ++k)
+            for (int o = 16; o > 0; o >>= 1) *sums[k] = add(*sums[k], F2{__shfl_xor_sync(0xFFFFFFFFu, sums[k]->v, o)});
+    }
+    __device__ __forceinline__ void add_sums(const PairAccumulator& other) {
+        ax = add(ax, other.ax);
+        ay = add(ay, other.ay);
+        az = add(az, other.az);
+        if (ENERGY) {
+            e_sum = add(e_sum, other.e_sum);
+            w_sum = add(w_sum, other.w_sum);
+            wx = add(wx, other.wx);
+            wy = add(wy, other.wy);
+            wz = add(wz, other.wz);
+        }
+    }
+
+    static __device__ __forceinline__ F2 distance(const PairParams& p, const int4& pa, const int4& pb, const int4& pj, F2& dx, F2& dy, F2& dz) {
+        dx = mul(f2(static_cast<float>(pa.x - pj.x), static_cast<float>(pb.x - pj.x)), both(p.scale[0]));
+        dy = mul(f2(static_cast<float>(pa.y - pj.y), static_cast<float>(pb.y - pj.y)), both(p.scale[1]));
+        dz = mul(f2(static_cast<float>(pa.z - pj.z), static_cast<float>(pb.z - pj.z)), both(p.scale[2]));
+        return fma(dz, dz, fma(dx, dx, mul(dy, dy)));   // (in this order: it decides which pairs lie inside a plain cutoff)
+    }
+
     // One entry, seen from the two atoms at pa and pb (fixed-point positions: the 32-bit difference is the nearest image).
     // The plain form takes every pair inside the cutoff; CAREFUL also tells pairs that coincide (r^2 < 1e-10: no force) and
     // those named above.
     template <bool CAREFUL>
     __device__ __forceinline__ void add_partner(const PairParams& p, const EwaldTable<COPIES>& table, const int4& pa, const int4& pb,
                                                 const int4& pj, const PairTerms& k, unsigned entry) {
-        const F2 dx = mul(f2(static_cast<float>(pa.x - pj.x), static_cast<float>(pb.x - pj.x)), both(p.scale[0]));
-        const F2 dy = mul(f2(static_cast<float>(pa.y - pj.y), static_cast<float>(pb.y - pj.y)), both(p.scale[1]));
-        const F2 dz = mul(f2(static_cast<float>(pa.z - pj.z), static_cast<float>(pb.z - pj.z)), both(p.scale[2]));
-        const F2 r2 = fma(dz, dz, fma(dx, dx, mul(dy, dy)));   // (in this order: it decides which pairs lie inside a plain cutoff)
+        F2 dx, dy, dz;
+        const F2 r2 = distance(p, pa, pb, pj, dx, dy, dz);
         float ra, rb;
         parts(r2, ra, rb);
         F2 f, u;
@@ -280,6 +326,29 @@ struct PairTables {
     }
 };
 
+// What the plain form left out of a row's entries (add_close_rest), by all lanes of a warp.
+template <int COPIES, bool ENERGY, bool SWITCH, bool BY_TYPE>
+__device__ __forceinline__ PairAccumulator<COPIES, ENERGY, SWITCH> close_rest(const PairParams& p, const ForceArgs& a,
+                                                                              const EwaldTable<COPIES>& table, int pair) {
+    PairAccumulator<COPIES, ENERGY, SWITCH> rest;
+    int first;
+    const int atoms = pair_atoms(a.rows.quad, pair, first), last = first + atoms - 1;
+    const int4 pa = a.pq[first], pb = a.pq[last];
+    const F2 q = mul(both(p.kq), BY_TYPE ? f2(p.type_charge[pa.w], p.type_charge[pb.w]) : f2(a.qf[first], a.qf[last]));
+    const int mid = a.rows.row_int[pair], end = a.rows.row_end[pair], ghosts = (mid + 3) & ~3;
+    const int k0 = a.phase == DSMD_PHASE_BOUNDARY ? ghosts : 0, k1 = a.phase == DSMD_PHASE_INTERIOR ? mid : end;
+    const unsigned* words = a.rows.rows + row_base(static_cast<unsigned>(pair), a.rows.stride);
+#pragma unroll 1
+    for (int k = k0 + (threadIdx.x & 31); k < k1; k += 32) {
+        if (k >= mid && k < ghosts) continue;
+        const unsigned e = words[row_offset(k)];
+        const int4 pj = __ldg(&a.pq[e]);
+        rest.add_close_rest(p, table, pa, pb, pj, mul(q, both(BY_TYPE ? p.type_charge[pj.w] : __ldg(&a.qf[e]))));
+    }
+    rest.over_warp();
+    return rest;
+}
+
 // Forces on the atoms of one pair row, worked on by `lanes` lanes of a warp, which take the row's chunks of four entries in
 // turn; this lane's share of the sums. The next chunk of entries and the partners of the current one are in flight before
 // any arithmetic starts; the list is streamed with an evict-first hint so that the positions stay in L2.
@@ -295,6 +364,7 @@ __device__ __forceinline__ void row_forces(const PairParams& p, const ForceArgs&
     const int nt = p.ntypes;
     const EwaldTable<COPIES>& table = tables.ewald;
     PairAccumulator<COPIES, ENERGY, SWITCH> acc;
+    bool close = false;   // the row has a pair below the Ewald table
     if (atoms > 0) {
         const int4 pa = a.pq[first], pb = a.pq[first + atoms - 1];
         const int mid = a.rows.row_int[pair], end = a.rows.row_end[pair];
@@ -377,9 +447,10 @@ __device__ __forceinline__ void row_forces(const PairParams& p, const ForceArgs&
             }
         }
         // What needs care, an entry per lane: the two atoms themselves (each is the other's partner), excluded partners, and
-        // all entries of a row with a pair closer than the plain form can tell (there is none in a sane system).
+        // all entries of a row with a pair that coincides (there is none in a sane system).
         const unsigned row_lanes = (lanes == 32 ? 0xFFFFFFFFu : (1u << lanes) - 1u) << (threadIdx.x & 31 & -lanes);
-        const bool again = __any_sync(row_lanes, acc.least < (COULOMB ? kEwaldFirst : 1e-10f));
+        const bool again = __any_sync(row_lanes, acc.least < 1e-10f);
+        if (COULOMB) close = !again && __any_sync(row_lanes, acc.least < kEwaldFirst);
         if (again) acc = PairAccumulator<COPIES, ENERGY, SWITCH>();
         const int ex_own = special & kRowCountMask, ex_all = ex_own + static_cast<int>((special >> kRowCountBits) & kRowCountMask);
         const int x0 = a.phase == DSMD_PHASE_BOUNDARY ? ex_own : 0, x1 = a.phase == DSMD_PHASE_INTERIOR ? ex_own : ex_all;
@@ -396,6 +467,18 @@ __device__ __forceinline__ void row_forces(const PairParams& p, const ForceArgs&
             take(e & kIndexMask, pj, qj);
             acc.template add_partner<true>(p, table, pa, pb, pj, terms(pj.w, qj), e);
         }
+    }
+    // Rows with a pair below the Ewald table, one after the other by the whole warp, an entry per lane. A warp has such a row now
+    // and then (a box of 648,000 water atoms, started from jittered places, has 15 such pairs), and one lane on its own would keep
+    // the others, and in a grid of one round the device, waiting for hundreds of entries: 1.56 ms for that box with the row done
+    // again by its lane, 1.14 this way, 1.53 with a row per atom and a branch per pair.
+    if (COULOMB)
+        for (unsigned todo = __ballot_sync(0xFFFFFFFFu, close && sub == 0); todo; todo &= todo - 1) {
+            const int leader = __ffs(todo) - 1;
+            const auto rest = close_rest<COPIES, ENERGY, SWITCH, by_type>(p, a, table, __shfl_sync(0xFFFFFFFFu, pair, leader));
+            if ((threadIdx.x & 31) == leader) acc.add_sums(rest);
+        }
+    if (atoms > 0) {
         if (ENERGY) acc.take_energies(atoms > 1, v);   // a lone atom's sums are in both lanes
         acc.take_forces(sum_a, sum_b);
     }

@@ -1,4 +1,6 @@
 """GPU tests of single faults that were found by reading: each one fails with the fault it names."""
+import math
+
 import numpy as np
 import pytest
 
@@ -214,3 +216,100 @@ def test_mostly_empty_box(cuda_device, n, L, periodic):
     i, j, _ = ctx.list_pairs()
     assert np.array_equal(co.canonical_pairs(np.stack([gid[i], gid[j]], 1)[gid[i] < gid[j]]), co.canonical_pairs(pairs))
     ctx.close()
+
+
+# rows of few and of many entries (one copy of the Ewald table and eight), shared by several lanes and not (the last), charges
+# by type and by atom, one, few and many types
+@pytest.mark.parametrize("n,L,rc,nt,by_type", [(400, 20.0, 5.0, 1, True), (400, 20.0, 5.0, 3, False), (3000, 31.0, 9.0, 2, True),
+                                               (3000, 31.0, 9.0, 9, True), (3000, 31.0, 9.0, 2, False), (90000, 90.0, 4.0, 2, True)])
+def test_pairs_below_the_ewald_table(cuda_device, n, L, rc, nt, by_type):
+    """Pairs closer than the table reaches (r^2 < 0.5), across cell rows and within one: forces and energy of the oracle, and
+    the same bits from a second evaluation."""
+    rng = np.random.default_rng(n + nt)
+    side = int(np.ceil(n ** (1 / 3)))
+    sites = np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij"), -1).reshape(-1, 3)[rng.permutation(side ** 3)[:n]]
+    pos = ((sites + 0.5 + rng.uniform(-0.1, 0.1, (n, 3))) * (L / side)) % L
+    apart = rng.permutation(np.concatenate([[0.05, 0.3, 0.69, 0.7071, 0.7072, 0.72], rng.uniform(0.2, 0.75, 24)]))
+    way = rng.normal(size=(30, 3))
+    way[:10, :2] *= 0.05   # along z: as a rule another cell row
+    way[10:20, 1:] *= 0.05
+    pos[30:60] = (pos[:30] + way * (apart / np.linalg.norm(way, axis=1))[:, None]) % L
+    box, types = np.full(3, L), rng.integers(0, nt, n).astype(np.int32)
+    of_type = rng.uniform(-0.6, 0.6, nt)
+    charge = of_type[types] if by_type else rng.uniform(-0.6, 0.6, n)
+    eps, sig = np.zeros((nt, nt)), np.ones((nt, nt))
+    ctx = capi.Context(n)
+    ctx.set_box(box)
+    ctx.set_pair_params(eps, sig, rc, 0.5)
+    ctx.set_coulomb(True)
+    ctx.upload(pos, types=types, charge=charge)
+    if by_type:
+        ctx.set_type_charges(of_type)
+    ctx.build_neighbor_list()
+    pairs = co.pairs(*pos.T, n, box, search=rc + 0.5)
+    c6, c12 = co.lj_tables(eps, sig)
+    want, scalars = co.forces(*pos.T, n, box, pairs, c6, c12, rc, charge=charge, types=types, do_coulomb=True, alpha=co.ewald_alpha(rc))
+    size = np.linalg.norm(want, axis=1)
+    # single-precision r^2 (16 roundings of 2^-24) may put a pair on the other side of the cutoff: its atoms may differ by the
+    # force there, Coulomb constant times the largest charges times (erfc(a r) / r + 2 a / sqrt(pi) exp(-(a r)^2)) / r
+    d = pos[pairs[:, 0]] - pos[pairs[:, 1]]
+    d -= L * np.rint(d / L)
+    edge = np.abs((d * d).sum(1) - rc * rc) <= 2.0 ** -20 * rc * rc
+    a = co.ewald_alpha(rc)
+    jump = np.bincount(pairs[edge].ravel(), minlength=n) * 332.0636 * 0.36 * (math.erfc(a * rc) / rc + 2.0 * a / math.pi ** 0.5 * math.exp(-(a * rc) ** 2)) / rc
+    for energy in (False, True):
+        got = []
+        for _ in range(2):
+            ctx.compute_forces(capi.PHASE_FULL, want_energy=energy)
+            got.append(ctx.forces_by_gid(n))
+        assert np.array_equal(*got)
+        # the table is good to 1e-5 of a pair's force; single-precision sums of some hundred pairs of the median size
+        assert (np.linalg.norm(got[0] - want, axis=1) <= 2e-5 * size + 5e-5 * np.median(size) + jump).all()
+    sums = ctx.read_scalars()
+    assert abs(sums["pe"] - scalars["pe"]) <= 2e-6 * np.abs(scalars["pe"]) + 1e-5 * n ** 0.5
+    assert abs(sums["pairs_in_cutoff"] - scalars["pairs_in_cutoff"]) <= edge.sum()
+    assert abs(sums["virial"] - scalars["virial"]) <= 2e-6 * np.abs(scalars["virial"]) + 1e-5 * n ** 0.5
+    ctx.close()
+
+
+def test_few_pairs_below_the_ewald_table_cost_little(cuda_device):
+    """A box of water with some ten such pairs takes as long as the same box with the molecules pushed apart (1.6 times as long
+    when a row with such a pair was done again by its one lane)."""
+    import torch
+    from scipy.spatial import cKDTree
+    from deepscalemd_b200 import synthetic as syn
+    s = syn.water_box(50, seed=3)
+    least = {}
+    for form in ("as made", "apart"):
+        pos = s.pos % s.box
+        for _ in range(8):
+            i, j = cKDTree(pos, boxsize=s.box).query_pairs(0.75, output_type="ndarray").T
+            if form == "as made":
+                break
+            d = pos[j] - pos[i]
+            d -= s.box * np.rint(d / s.box)
+            for k in range(len(i)):
+                pos[3 * (j[k] // 3): 3 * (j[k] // 3) + 3] += 0.3 * d[k] / np.linalg.norm(d[k])
+            pos %= s.box
+        assert (len(i) == 0) == (form == "apart")
+        ctx = capi.Context(s.n)
+        ctx.set_box(s.box)
+        ctx.set_pair_params(s.eps, s.sig, s.cutoff, s.skin)
+        ctx.set_coulomb(True)
+        ctx.set_exclusions(s.n, s.exclusions)
+        ctx.upload(pos, types=s.types, charge=s.charge)
+        of_type = np.zeros(len(s.eps))
+        of_type[s.types] = s.charge
+        ctx.set_type_charges(of_type)
+        ctx.build_neighbor_list()
+        times = []
+        for _ in range(15):
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            begin.record()
+            ctx.compute_forces()
+            end.record()
+            end.synchronize()
+            times.append(begin.elapsed_time(end))
+        least[form] = min(times)
+        ctx.close()
+    assert least["as made"] <= 1.12 * least["apart"], least

@@ -28,7 +28,7 @@ struct Grid {
     int ncells;
     int stencil;        // cells searched in each direction (1 or 2)
     float r2_list;      // (cutoff + skin)^2
-    float band;         // |r2 - r2_list| below this is decided in fp64
+    float band;         // of the edge searches: |r2 - r2_list| below this is decided in fp64
     double r2_list_d;
     float cellw[3];     // cell width per axis (length units); the x cells are finer than the y and z cells
     float r_pad;        // list radius plus a rounding margin: the reach used to prune cell rows

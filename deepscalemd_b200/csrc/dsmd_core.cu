@@ -806,7 +806,6 @@ int make_grid(dsmd_ctx* c) {
     g.ncells = static_cast<int>(ncells);
     g.r2_list = static_cast<float>(R * R);
     g.r2_list_d = R * R;
-    g.band = static_cast<float>(8.0 * R * max_scale + 16.0 * R * R * 5.9604645e-8);
     double max_len = 0.0;
     for (int a = 0; a < 3; ++a) {
         g.cellw[a] = static_cast<float>(1.0 / (g.inv_len[a] * g.nc[a]));

@@ -26,7 +26,7 @@ __device__ __forceinline__ float reciprocal(float v) {
 }
 
 // Pair parameters by type. kOneType: constants. kFewTypes: a table over (type of the first atom, type of the second, type
-// of the partner) that holds what both atoms need side by side - up to 8 types, 16 KB. kManyTypes: a table over two types,
+// of the partner) that holds what both atoms need side by side - up to 8 types, 8 KB (12 KB with charges by type). kManyTypes: a table over two types,
 // read once per atom.
 enum { kOneType = 0, kFewTypes = 1, kManyTypes = 2 };
 constexpr int kFewTypesMost = 8;
@@ -214,10 +214,14 @@ struct PairAccumulator {
         }
     }
 
+    // (unsigned: the difference of two places half a box apart and more wraps, which signed arithmetic must not)
+    static __device__ __forceinline__ float offset(int a, int b) {
+        return static_cast<float>(static_cast<int>(static_cast<unsigned>(a) - static_cast<unsigned>(b)));
+    }
     static __device__ __forceinline__ F2 distance(const PairParams& p, const int4& pa, const int4& pb, const int4& pj, F2& dx, F2& dy, F2& dz) {
-        dx = mul(f2(static_cast<float>(pa.x - pj.x), static_cast<float>(pb.x - pj.x)), both(p.scale[0]));
-        dy = mul(f2(static_cast<float>(pa.y - pj.y), static_cast<float>(pb.y - pj.y)), both(p.scale[1]));
-        dz = mul(f2(static_cast<float>(pa.z - pj.z), static_cast<float>(pb.z - pj.z)), both(p.scale[2]));
+        dx = mul(f2(offset(pa.x, pj.x), offset(pb.x, pj.x)), both(p.scale[0]));
+        dy = mul(f2(offset(pa.y, pj.y), offset(pb.y, pj.y)), both(p.scale[1]));
+        dz = mul(f2(offset(pa.z, pj.z), offset(pb.z, pj.z)), both(p.scale[2]));
         return fma(dz, dz, fma(dx, dx, mul(dy, dy)));   // (in this order: it decides which pairs lie inside a plain cutoff)
     }
 
@@ -318,7 +322,7 @@ struct PairTables {
         if (by_type && !few)
             for (int k = threadIdx.x; k < nt; k += blockDim.x) s_charge[k] = p.type_charge[k];
         if (COULOMB || TYPES != kOneType) __syncthreads();
-        ewald = EwaldTable<COPIES>{s_ewald + (threadIdx.x & (COPIES - 1)), p.ewald_intervals};
+        ewald = EwaldTable<COPIES>{s_ewald + (threadIdx.x & (COPIES > 0 ? COPIES - 1u : 0u)), p.ewald_intervals};
         lj3 = s_lj3;
         qq3 = s_qq3;
         lj2 = s_lj2;

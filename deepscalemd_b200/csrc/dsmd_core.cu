@@ -908,6 +908,17 @@ int64_t pair_blocks(const dsmd_ctx* c, int64_t pairs, bool energy) {
     return energy ? std::min<int64_t>(blocks_for(lanes, threads), kDeviceSms * (512 / threads)) : blocks_for(lanes, threads);
 }
 
+int ensure_cub_temp(dsmd_ctx* c, size_t need) {
+    if (need > c->cub_temp_bytes) {
+        cudaFree(c->cub_temp);
+        c->cub_temp = nullptr;
+        c->cub_temp_bytes = 0;
+        DSMD_CUDA(c, cudaMalloc(&c->cub_temp, need + need / 4));
+        c->cub_temp_bytes = need + need / 4;
+    }
+    return DSMD_OK;
+}
+
 int ensure_partials(dsmd_ctx* c, int64_t blocks) {
     if (blocks > c->partial_blocks) {
         if (c->partials) cudaFree(c->partials);
@@ -939,12 +950,7 @@ int sort_range(dsmd_ctx* c, int64_t first, cudaStream_t s, bool clear, const Bri
         DSMD_LAUNCHED(c);
         size_t need = 0;
         cub::DeviceScan::ExclusiveScan(nullptr, need, c->cell_count, c->cell_start, cuda::std::plus<int>(), i0, cells, s);
-        if (need > c->cub_temp_bytes) {
-            if (c->cub_temp) cudaFree(c->cub_temp);
-            c->cub_temp = nullptr;
-            DSMD_CUDA(c, cudaMalloc(&c->cub_temp, need + need / 4));
-            c->cub_temp_bytes = need + need / 4;
-        }
+        { const int rc = ensure_cub_temp(c, need); if (rc) return rc; }
         DSMD_CUDA(c, cub::DeviceScan::ExclusiveScan(c->cub_temp, need, c->cell_count + cell0, c->cell_start + cell0,
                                                     cuda::std::plus<int>(), i0, cells, s));
         dsmd::k_cell_place<<<blocks_for(n, kThreads), kThreads, 0, s>>>(i0, in, c->key, c->arrival, c->cell_start, c->list);
@@ -1479,16 +1485,24 @@ int dsmd_ghost_slots(dsmd_ctx* c, const int32_t** out) {
     return DSMD_OK;
 }
 
-// The list proper (k_list_members): partners per atom into c->offsets64, sums into the context. Worked out when somebody
-// asks for it; forces need no membership finer than the rows'.
+// The list proper (k_list_members): where each atom's partners start (c->offsets64), sums into the context. Worked out once
+// per list build, when somebody asks for it; forces need no membership finer than the rows'.
+static unsigned member_blocks(const dsmd_ctx* c) {
+    return std::min<unsigned>(blocks_for(2 * c->n_quads * 32, kMemberThreads), kDeviceSms * 8);
+}
+
 static int list_members(dsmd_ctx* c, cudaStream_t s) {
-    const int n_pairs = static_cast<int>(2 * c->n_quads);
+    if (c->stat_epoch == c->build_epoch) return DSMD_OK;
+    const int n = static_cast<int>(c->n_owned);
     DSMD_CUDA(c, cudaSetDevice(c->device));
     DSMD_CUDA(c, cudaMemsetAsync(c->member_stats, 0, sizeof(unsigned long long) * 3, s));
-    k_list_members<false><<<blocks_for(n_pairs, kThreads), kThreads, 0, s>>>(
-        c->grid, n_pairs, static_cast<int>(c->n_owned), rows_of(c), c->ref[0], c->ref[1], c->ref[2], c->offsets64, c->member_stats,
-        nullptr, nullptr, nullptr, 0);
+    k_list_members<false><<<member_blocks(c), kMemberThreads, 0, s>>>(c->grid, static_cast<int>(2 * c->n_quads), rows_of(c), c->ref[0], c->ref[1],
+                                                                   c->ref[2], c->offsets64, c->member_stats, nullptr, nullptr, nullptr);
     DSMD_LAUNCHED(c);
+    size_t need = 0;
+    cub::DeviceScan::ExclusiveSum(nullptr, need, c->offsets64, c->offsets64, n, s);
+    { const int rc = ensure_cub_temp(c, need); if (rc) return rc; }
+    DSMD_CUDA(c, cub::DeviceScan::ExclusiveSum(c->cub_temp, need, c->offsets64, c->offsets64, n, s));
     unsigned long long sums[3] = {0, 0, 0};
     DSMD_CUDA(c, cudaMemcpyAsync(sums, c->member_stats, sizeof(sums), cudaMemcpyDeviceToHost, s));
     DSMD_CUDA(c, cudaStreamSynchronize(s));
@@ -1503,7 +1517,7 @@ int dsmd_list_stats(dsmd_ctx* c, int64_t* directed_entries, int64_t* interior_en
                     int32_t* cells, int32_t* rechecked) {
     if (!c) return DSMD_ERR_INVALID;
     if (!c->list_valid) return fail(c, DSMD_ERR_STATE, "no neighbour list");
-    if ((directed_entries || interior_entries || rechecked) && c->stat_epoch != c->build_epoch) {
+    if (directed_entries || interior_entries || rechecked) {
         const int rc = list_members(c, nullptr);
         if (rc) return rc;
     }
@@ -1520,24 +1534,13 @@ int dsmd_list_export(dsmd_ctx* c, int32_t* d_i, int32_t* d_j, uint8_t* d_flags, 
     if (!c || !n_pairs) return DSMD_ERR_INVALID;
     if (!c->list_valid) return fail(c, DSMD_ERR_STATE, "no neighbour list");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const bool size_query = !d_i || !d_j;
-    if (!size_query || c->stat_epoch != c->build_epoch) {
-        const int rc = list_members(c, s);
-        if (rc) return rc;
-    }
+    { const int rc = list_members(c, s); if (rc) return rc; }
     *n_pairs = c->stat_entries;
-    if (size_query || capacity < c->stat_entries) return DSMD_OK;
-    const int n = static_cast<int>(c->n_owned), n_row_pairs = static_cast<int>(2 * c->n_quads);
-    size_t need = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, need, c->offsets64, c->offsets64, n, s);
-    void* temp = nullptr;
-    DSMD_CUDA(c, cudaMalloc(&temp, need));
-    DSMD_CUDA(c, cub::DeviceScan::ExclusiveSum(temp, need, c->offsets64, c->offsets64, n, s));
-    k_list_members<true><<<blocks_for(n_row_pairs, kThreads), kThreads, 0, s>>>(
-        c->grid, n_row_pairs, n, rows_of(c), c->ref[0], c->ref[1], c->ref[2], c->offsets64, nullptr, d_i, d_j, d_flags, capacity);
+    if (!d_i || !d_j || capacity < c->stat_entries) return DSMD_OK;   // size query
+    k_list_members<true><<<member_blocks(c), kMemberThreads, 0, s>>>(c->grid, static_cast<int>(2 * c->n_quads), rows_of(c), c->ref[0], c->ref[1],
+                                                                  c->ref[2], c->offsets64, nullptr, d_i, d_j, d_flags);
     DSMD_LAUNCHED(c);
     DSMD_CUDA(c, cudaStreamSynchronize(s));
-    cudaFree(temp);
     return DSMD_OK;
 }
 

@@ -146,7 +146,8 @@ int dsmd_sort_owned_in_brick(dsmd_ctx* ctx, const double lo[3], const double hi[
  * array of n_total - n_owned entries). The halo refresh unpacks through it. */
 int dsmd_ghost_slots(dsmd_ctx* ctx, const int32_t** device_ghost_slot);
 
-/* List statistics of the last build. pairs_listed counts directed entries (each owned-owned pair twice). */
+/* List statistics of the last build. directed_entries counts each owned-owned pair twice. The entries are counted by a kernel
+ * when they are first asked for after a build (row_stride and cells alone need none); that call synchronises. */
 int dsmd_list_stats(dsmd_ctx* ctx, int64_t* directed_entries, int64_t* interior_entries, int32_t* row_stride,
                     int32_t* cells, int32_t* rechecked_fp64);
 

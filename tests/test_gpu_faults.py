@@ -313,3 +313,30 @@ def test_few_pairs_below_the_ewald_table_cost_little(cuda_device):
         least[form] = min(times)
         ctx.close()
     assert least["as made"] <= 1.12 * least["apart"], least
+
+
+def test_list_queries_count_once(cuda_device):
+    """Members of the list are counted once per build whoever asks first, by all lanes of a warp (a thread per row took 16 times
+    as long as the build of this system)."""
+    import time
+    import torch
+    from deepscalemd_b200 import synthetic as syn
+    s = syn.water_box(11, seed=3)
+    ctx = capi.Context(s.n)
+    ctx.set_box(s.box)
+    ctx.set_pair_params(s.eps, s.sig, s.cutoff, s.skin)
+    ctx.upload(s.pos, types=s.types)
+    least = {}
+    for _ in range(8):
+        for name, call in (("build", ctx.build_neighbor_list), ("stats", ctx.list_stats), ("pairs", ctx.list_pairs_device)):
+            torch.cuda.synchronize()
+            launches, begin = ctx.launch_count(), time.perf_counter()
+            call()
+            torch.cuda.synchronize()
+            least[name] = min(least.get(name, 1.0), time.perf_counter() - begin)
+            assert name == "build" or ctx.launch_count() - launches == 1
+        launches = ctx.launch_count()
+        ctx.list_stats()
+        assert ctx.launch_count() == launches
+    assert least["stats"] <= 4.0 * least["build"] and least["pairs"] <= 4.0 * least["build"], least
+    ctx.close()

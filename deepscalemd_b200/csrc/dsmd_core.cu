@@ -1183,6 +1183,7 @@ int dsmd_set_coulomb(dsmd_ctx* c, int enabled, double alpha) {
     c->coulomb = enabled != 0;
     if (!c->coulomb) return DSMD_OK;
     if (!c->params_set) return fail(c, DSMD_ERR_STATE, "set the pair parameters (cutoff) before Coulomb");
+    DSMD_CUDA(c, cudaSetDevice(c->device));
     c->alpha = alpha > 0.0 ? alpha : dsmd::ewald_alpha_for(c->cutoff);
     c->ewald_intervals = dsmd::ewald_intervals(c->cutoff * c->cutoff);
     const std::vector<float> coef = dsmd::ewald_build_table(c->alpha, c->ewald_intervals);

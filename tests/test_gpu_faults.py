@@ -340,3 +340,20 @@ def test_list_queries_count_once(cuda_device):
         assert ctx.launch_count() == launches
     assert least["stats"] <= 4.0 * least["build"] and least["pairs"] <= 4.0 * least["build"], least
     ctx.close()
+
+
+def test_set_up_calls_work_on_the_context_s_device(cuda_device):
+    """Calls that allocate do so on the context's device, whichever one the caller's thread has current."""
+    import torch
+    if torch.cuda.device_count() < 2:
+        pytest.skip("needs two GPUs")
+    ctx = capi.Context(64, device=1)
+    calls = [lambda: ctx.set_box(np.full(3, 20.0)), lambda: ctx.set_pair_params([[1.0]], [[1.0]], 2.5, 0.3), lambda: ctx.set_coulomb(True),
+             lambda: ctx.set_exclusions(2, [[0, 1]]), lambda: ctx.set_constraints(2, [[0, 1, 1.0]]), lambda: ctx.set_type_charges([0.1])]
+    for call in calls[1:]:
+        torch.cuda.set_device(0)
+        calls[0]()
+        call()
+        assert torch.cuda.current_device() == 1
+    torch.cuda.set_device(0)
+    ctx.close()

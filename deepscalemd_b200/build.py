@@ -11,14 +11,15 @@ import subprocess
 import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-SOURCES = ["csrc/dsmd_core.cu", "csrc/dsmd_edges.cu", "csrc/dsmd_domain.cu", "csrc/dsmd_noalloc.cu"]
+SOURCES = ["csrc/dsmd_core.cu", "csrc/dsmd_pair_lj.cu", "csrc/dsmd_pair_lj_sums.cu", "csrc/dsmd_pair_ewald.cu", "csrc/dsmd_pair_ewald_sums.cu",
+           "csrc/dsmd_pair_ewald_long.cu", "csrc/dsmd_pair_ewald_long_sums.cu", "csrc/dsmd_edges.cu", "csrc/dsmd_domain.cu", "csrc/dsmd_noalloc.cu"]
 LIBRARY = os.path.join(HERE, "libdsmd_b200.so")
 # host-side input layer (run description, coordinate / topology / restart files): plain C++, no CUDA
 HOST_SOURCES = ["csrc/host/run_config.cpp", "csrc/host/system_input.cpp", "csrc/host/restart_file.cpp",
                 "csrc/host/dynamics.cpp", "csrc/host/dsmd_input_capi.cpp"]
 HOST_LIBRARY = os.path.join(HERE, "libdsmd_input.so")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17", "--use_fast_math=false",
-         "-Xcompiler", "-fPIC", "-shared"]
+         "-Xcompiler", "-fPIC", "-shared", "--threads", "0"]
 
 
 def nvcc_path() -> str:

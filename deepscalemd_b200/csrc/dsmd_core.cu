@@ -29,12 +29,23 @@
 #include "../../include/dsmd_b200.h"
 #include "dsmd_cells.cuh"
 #include "dsmd_common.cuh"
+#include "dsmd_force.cuh"
 #include "dsmd_report.cuh"
+#include "dsmd_sums.cuh"
 #include "ewald_table.hpp"
 
+using dsmd::ForceArgs;
 using dsmd::Grid;
 using dsmd::Mail;
+using dsmd::PairParams;
 using dsmd::Status;
+using dsmd::StepArgs;
+using dsmd::kEwaldCopiesMost;
+using dsmd::kEwaldFirst;
+using dsmd::kFewTypes;
+using dsmd::kOneType;
+using dsmd::kPairBlocks;
+using dsmd::kPairThreads;
 using dsmd::post;
 
 namespace {
@@ -226,42 +237,6 @@ __global__ void k_ghost_rows_near(Grid g, const int* __restrict__ lo_end, const 
 // kernels: per-step pack, displacement, integration
 // ---------------------------------------------------------------------------------------------------------------------
 
-// Who writes where when a displacement check ends.
-struct DisplacementReport {
-    Status* st;
-    unsigned* ticket;      // blocks that have finished
-    Mail* mail;            // or null: no report
-    unsigned long long seq;
-    double gate2;          // see gate_closed
-};
-
-// The block's largest squared displacement goes into the status word; the last block of the grid reports the word.
-__device__ __forceinline__ void report_displacement(double v, const DisplacementReport& r) {
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
-    __shared__ double warp_max[32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (lane == 0) warp_max[w] = v;
-    __syncthreads();
-    if (w == 0) {
-        v = lane < (blockDim.x >> 5) ? warp_max[lane] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
-        if (lane == 0) {
-            if (v > 0.0) atomicMax(&r.st->max_disp2, static_cast<unsigned long long>(__double_as_longlong(v)));
-            if (r.mail) {
-                __threadfence();
-                if (atomicAdd(r.ticket, 1u) == gridDim.x - 1) {
-                    __threadfence();
-                    const double out[2] = {__longlong_as_double(static_cast<long long>(__ldcg(&r.st->max_disp2))),
-                                           static_cast<double>(__ldcg(&r.st->out_of_domain))};
-                    *r.ticket = 0u;
-                    r.st->gate = out[1] != 0.0 ? __longlong_as_double(0x7FF0000000000000ll) : out[0];
-                    post(r.mail, out, 2, r.seq);
-                }
-            }
-        }
-    }
-}
-
 // Positions out of pinned host memory into the context, and forces back: a kernel that reads or writes the host's memory moves
 // three arrays at once and needs no copy engine: 3 us instead of three copies of 8 us each, 41 GB/s instead of 52.
 __global__ void k_pull(int first, int count, const double* __restrict__ hx, const double* __restrict__ hy, const double* __restrict__ hz,
@@ -333,51 +308,6 @@ __global__ void k_scale_velocities(int n, double factor, double* __restrict__ vx
     vz[s] *= factor;
 }
 
-// Deterministic sums over a grid: every block leaves its partial sums, and the block that finishes last adds them up in a
-// fixed order (one launch instead of two). `ticket` counts finished blocks and is left at zero.
-template <int NV>
-__device__ __forceinline__ void block_sum(double (&v)[NV], double (&sh)[32][NV]) {   // thread 0 has the sums
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int k = 0; k < NV; ++k)
-        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-    if (lane == 0)
-        for (int k = 0; k < NV; ++k) sh[w][k] = v[k];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const int nw = blockDim.x >> 5;
-        for (int k = 0; k < NV; ++k) {
-            v[k] = 0.0;
-            for (int q = 0; q < nw; ++q) v[k] += sh[q][k];
-        }
-    }
-}
-
-template <int NV>
-__device__ __forceinline__ void sum_over_grid(double (&v)[NV], double* partials, unsigned* ticket, double* out, bool accumulate,
-                                              Mail* mail = nullptr, unsigned long long seq = 0) {
-    __shared__ double sh[32][NV];
-    __shared__ bool last;
-    block_sum<NV>(v, sh);
-    if (threadIdx.x == 0) {
-        for (int k = 0; k < NV; ++k) partials[static_cast<size_t>(blockIdx.x) * NV + k] = v[k];
-        __threadfence();
-        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    for (int k = 0; k < NV; ++k) v[k] = 0.0;
-    for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x)
-        for (int k = 0; k < NV; ++k) v[k] += __ldcg(&partials[static_cast<size_t>(b) * NV + k]);
-    block_sum<NV>(v, sh);
-    if (threadIdx.x == 0) {
-        for (int k = 0; k < NV; ++k) out[k] = v[k] = accumulate ? out[k] + v[k] : v[k];
-        *ticket = 0u;
-        if (mail) post(mail, v, NV, seq);
-    }
-}
-
 __global__ void k_kinetic(int n, const double* __restrict__ vx, const double* __restrict__ vy,
                           const double* __restrict__ vz, const double* __restrict__ mass, double* partials, unsigned* ticket,
                           double* out, Mail* mail, unsigned long long seq) {
@@ -393,7 +323,6 @@ __global__ void k_kinetic(int n, const double* __restrict__ vx, const double* __
 #include "dsmd_bonded.cuh"
 #include "dsmd_f32x2.cuh"
 #include "dsmd_rows.cuh"
-#include "dsmd_pair.cuh"
 
 namespace {
 
@@ -1005,38 +934,6 @@ int read_status(dsmd_ctx* c, cudaStream_t s) {
     DSMD_CUDA(c, cudaMemcpyAsync(c->h_status, c->status, sizeof(Status), cudaMemcpyDeviceToHost, s));
     DSMD_CUDA(c, cudaStreamSynchronize(s));
     return DSMD_OK;
-}
-
-template <int COPIES, bool ENERGY, int TYPES, bool SWITCH, bool QTYPE>
-int launch_pair_kernel(dsmd_ctx* c, const PairParams& p, const ForceArgs& a, cudaStream_t s) {
-    const size_t smem = PairTables<COPIES, ENERGY, TYPES, QTYPE>::bytes(p.ntypes, p.ewald_intervals);
-    const auto kernel = k_pair<COPIES, ENERGY, TYPES, SWITCH, QTYPE>;
-    if (smem > 48 * 1024) DSMD_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    kernel<<<static_cast<unsigned>(pair_blocks(c, a.n_pairs, ENERGY)), kPairThreads<COPIES, TYPES>, smem, s>>>(p, a);
-    DSMD_LAUNCHED(c);
-    return DSMD_OK;
-}
-
-template <int COPIES, bool ENERGY, int TYPES>
-int launch_pair(dsmd_ctx* c, const PairParams& p, const ForceArgs& a, bool sw, cudaStream_t s) {
-    constexpr bool coulomb = COPIES > 0;
-    if (coulomb && p.type_charge)   // charges by type: only the kernels with Coulomb have this form
-        return sw ? launch_pair_kernel<COPIES, ENERGY, TYPES, true, coulomb>(c, p, a, s)
-                  : launch_pair_kernel<COPIES, ENERGY, TYPES, false, coulomb>(c, p, a, s);
-    return sw ? launch_pair_kernel<COPIES, ENERGY, TYPES, true, false>(c, p, a, s)
-              : launch_pair_kernel<COPIES, ENERGY, TYPES, false, false>(c, p, a, s);
-}
-
-template <int COPIES>
-int launch_pair_types(dsmd_ctx* c, const PairParams& p, const ForceArgs& a, bool energy, bool sw, cudaStream_t s) {
-    if (energy) {
-        if (p.ntypes == 1) return launch_pair<COPIES, true, kOneType>(c, p, a, sw, s);
-        if (p.ntypes <= kFewTypesMost) return launch_pair<COPIES, true, kFewTypes>(c, p, a, sw, s);
-        return launch_pair<COPIES, true, kManyTypes>(c, p, a, sw, s);
-    }
-    if (p.ntypes == 1) return launch_pair<COPIES, false, kOneType>(c, p, a, sw, s);
-    if (p.ntypes <= kFewTypesMost) return launch_pair<COPIES, false, kFewTypes>(c, p, a, sw, s);
-    return launch_pair<COPIES, false, kManyTypes>(c, p, a, sw, s);
 }
 
 }  // namespace
@@ -1652,10 +1549,13 @@ static int compute_forces_impl(dsmd_ctx* c, int phase, int want_energy, int64_t 
                       c->tickets, c->scalars, report ? c->mail + kMailScalars : nullptr, report ? ++c->seq : 0, c->status, c->gate2};
     if (e && pairs > 0) c->scalars_seq = a.seq;
     if (pairs > 0) {   // else nothing to add to the forces; the energy sums of a boundary pass stay as the interior pass left them
+        const unsigned blocks = static_cast<unsigned>(pair_blocks(c, pairs, e));
         const int copies = ewald_copies(c);
-        const int rc = copies == 0 ? launch_pair_types<0>(c, p, a, e, sw, s)
-                                   : (copies == 1 ? launch_pair_types<1>(c, p, a, e, sw, s) : launch_pair_types<kEwaldCopiesMost>(c, p, a, e, sw, s));
-        if (rc) return rc;
+        const auto launch = copies == 0 ? (e ? dsmd::launch_pair<0, true> : dsmd::launch_pair<0, false>)
+                            : copies == 1 ? (e ? dsmd::launch_pair<1, true> : dsmd::launch_pair<1, false>)
+                                          : (e ? dsmd::launch_pair<kEwaldCopiesMost, true> : dsmd::launch_pair<kEwaldCopiesMost, false>);
+        DSMD_CUDA(c, launch(p, a, sw, blocks, s));
+        ++c->launches;
     }
     return DSMD_OK;
 }
@@ -1671,16 +1571,8 @@ static int force_step(dsmd_ctx* c, double dt, double f2a, cudaStream_t s) {
     const StepArgs at{r[0], r[1], r[2], r[3], r[4], r[5], r[9], c->ref[0], c->ref[1], c->ref[2], c->pq_next, dt, dt * f2a};
     const unsigned blocks = static_cast<unsigned>(pair_blocks(c, pairs, false));
     const DisplacementReport report = displacement_report(c, true, s);
-    const auto launch = [&](auto types) {
-        constexpr int TYPES = decltype(types)::value;
-        const size_t smem = PairTables<0, false, TYPES, false>::bytes(p.ntypes, 0);
-        const auto kernel = c->switch_distance > 0.0 ? k_step<TYPES, true> : k_step<TYPES, false>;
-        kernel<<<blocks, kPairThreads<0, TYPES>, smem, s>>>(p, a, c->grid, at, report);
-    };
-    if (p.ntypes == 1) launch(std::integral_constant<int, kOneType>());
-    else if (p.ntypes <= kFewTypesMost) launch(std::integral_constant<int, kFewTypes>());
-    else launch(std::integral_constant<int, kManyTypes>());
-    DSMD_LAUNCHED(c);
+    DSMD_CUDA(c, dsmd::launch_step(p, a, c->grid, at, report, c->switch_distance > 0.0, blocks, s));
+    ++c->launches;
     std::swap(c->pq, c->pq_next);
     return DSMD_OK;
 }

@@ -1,21 +1,18 @@
-// LJ + real-space Ewald over the pair rows of dsmd_rows.cuh. Included by dsmd_core.cu.
+// LJ + real-space Ewald over the pair rows of dsmd_row_layout.cuh. Included by dsmd_pair_*.cu, each of which compiles some of the forms.
 #pragma once
+
+#include <type_traits>
+
+#include "../../include/dsmd_b200.h"
+#include "dsmd_f32x2.cuh"
+#include "dsmd_force.cuh"
+#include "dsmd_row_layout.cuh"
+#include "dsmd_sums.cuh"
+#include "ewald_table.hpp"
 
 namespace {
 
-struct PairParams {
-    float scale[3];
-    float rc2;
-    float rs2, inv_denom;        // CHARMM switch on r^2 (rs2 < 0: off)
-    float kq;                    // Coulomb constant
-    float alpha, two_alpha_sqrtpi;
-    int ntypes;
-    int ewald_intervals;
-    float ewald_most;            // largest r^2 looked up: the last float inside the last interval
-    const float2* lj;            // [ntypes * ntypes] {12 c12, -6 c6}
-    const float4* ewald;         // [2 * intervals]: force cubic, energy cubic
-    const float* type_charge;    // [ntypes] when every atom's charge is that of its type (dsmd_set_type_charges), else null
-};
+using namespace dsmd;
 
 // 1 / v: the hardware approximation (1 ulp) for the force-only kernels, one Newton step more (full single precision)
 // where energy and virial sums are taken.
@@ -25,19 +22,10 @@ __device__ __forceinline__ float reciprocal(float v) {
     return REFINE ? fmaf(r, fmaf(-v, r, 1.0f), r) : r;
 }
 
-// Pair parameters by type. kOneType: constants. kFewTypes: a table over (type of the first atom, type of the second, type
-// of the partner) that holds what both atoms need side by side - up to 8 types, 8 KB (12 KB with charges by type). kManyTypes: a table over two types,
-// read once per atom.
-enum { kOneType = 0, kFewTypes = 1, kManyTypes = 2 };
-constexpr int kFewTypesMost = 8;
-
 // The real-space Ewald functions of r^2 as cubics on intervals of constant relative width (ewald_table.hpp). For rows of
 // hundreds of entries the table lies in shared memory eight times over, copy c in the 16-byte bank group c, and a lane reads
 // the copy of its place in its group of eight: a look-up by 32 lanes is 4 wavefronts whatever the intervals (8 to 11 with one
 // copy). For short rows, where laying the table out (36 KB at a cutoff of 10 A) would be most of the work, one copy.
-constexpr int kEwaldCopiesMost = 8;
-
-constexpr float kEwaldFirst = 0.5f;   // r^2 at which the table starts
 
 template <int COPIES>
 struct EwaldTable {
@@ -245,34 +233,6 @@ struct PairAccumulator {
         }
     }
 };
-
-struct ForceArgs {
-    const int4* pq;
-    const float* qf;
-    RowArrays rows;
-    int phase;
-    const int* pair_list;    // the pairs to work on (boundary pass), or null: first_pair ...
-    int first_pair, n_pairs; // ... first_pair + n_pairs
-    int lane_shift;          // log2 of the lanes that share one row
-    double *fx, *fy, *fz;
-    double* partials;        // energy sums: per block, a count of finished blocks, and the total
-    unsigned* ticket;
-    double* scalars;
-    Mail* mail;              // where the total is reported to the host
-    unsigned long long seq;
-    const Status* st;
-    double gate2;            // see gate_closed
-};
-
-// Threads per block and blocks per SM, which fix the registers and with them how the compiler interleaves the partners of a
-// chunk; measured on a B200, the best of five to nine settings each. Long rows with Ewald: one block per SM, 118 registers
-// (1.08 to 1.12 ms per pass over 648,000 water atoms; 1.12 to 1.45 ms with two to six smaller blocks). One type: 64
-// registers, 0.427 ms at 4,000,000 Lennard-Jones atoms (0.44 to 0.56 ms at other settings; a row per atom took 0.498 ms).
-// Types by table: 80 registers, 0.177 ms for the 1,048,576-atom mixture (0.18 to 0.23 ms; a row per atom 0.213 ms).
-template <int COPIES, int TYPES>
-constexpr int kPairThreads = COPIES == kEwaldCopiesMost ? 384 : (COPIES == 0 && TYPES == kOneType ? 64 : 128);
-template <int COPIES, int TYPES, bool ENERGY>
-constexpr int kPairBlocks = ENERGY || COPIES == kEwaldCopiesMost ? 1 : (COPIES > 0 ? 5 : (TYPES == kOneType ? 16 : 6));
 
 // Tables in shared memory: Ewald cubics and pair parameters by type. Every thread of the block calls it once.
 template <int COPIES, bool ENERGY, int TYPES, bool QTYPE>
@@ -532,13 +492,6 @@ __global__ void __launch_bounds__((kPairThreads<COPIES, TYPES>), (kPairBlocks<CO
     if (ENERGY) sum_over_grid<6>(v, a.partials, a.ticket, a.scalars, a.phase == DSMD_PHASE_BOUNDARY, a.mail, a.seq);
 }
 
-struct StepArgs {
-    double *x, *y, *z, *vx, *vy, *vz;
-    const double *mass, *xref, *yref, *zref;
-    int4* pq_next;
-    double dt, kick;    // kick = dt times the force-to-acceleration factor: half of it ends this step, half begins the next
-};
-
 // The force pass of a step and what follows it up to the next force pass, for loops in which nobody reads forces or
 // velocities in between: v += kick f / m, x += dt v, fixed-point positions of the next step (into the other buffer: rows
 // still read this one's), displacement check. A separate pass would read and write the forces and read everything else again
@@ -607,3 +560,31 @@ k_step(PairParams p, ForceArgs a, Grid g, StepArgs at, DisplacementReport report
 }
 
 }  // namespace
+
+namespace dsmd {
+
+template <int COPIES, bool ENERGY>
+cudaError_t launch_pair(const PairParams& p, const ForceArgs& a, bool sw, unsigned blocks, cudaStream_t s) {
+    const auto launch = [&](auto types, auto switched, auto qtype) {
+        constexpr int TYPES = decltype(types)::value;
+        constexpr bool SWITCH = decltype(switched)::value, QTYPE = decltype(qtype)::value;
+        const size_t smem = PairTables<COPIES, ENERGY, TYPES, QTYPE>::bytes(p.ntypes, p.ewald_intervals);
+        const auto kernel = k_pair<COPIES, ENERGY, TYPES, SWITCH, QTYPE>;
+        if (smem > 48 * 1024) {
+            const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+            if (e != cudaSuccess) return e;
+        }
+        kernel<<<blocks, kPairThreads<COPIES, TYPES>, smem, s>>>(p, a);
+        return cudaGetLastError();
+    };
+    const auto by_charge = [&](auto types, auto switched) {   // charges by type: only the kernels with Coulomb have this form
+        if (COPIES > 0 && p.type_charge) return launch(types, switched, std::integral_constant<bool, (COPIES > 0)>());
+        return launch(types, switched, std::false_type());
+    };
+    const auto by_switch = [&](auto types) { return sw ? by_charge(types, std::true_type()) : by_charge(types, std::false_type()); };
+    if (p.ntypes == 1) return by_switch(std::integral_constant<int, kOneType>());
+    if (p.ntypes <= kFewTypesMost) return by_switch(std::integral_constant<int, kFewTypes>());
+    return by_switch(std::integral_constant<int, kManyTypes>());
+}
+
+}  // namespace dsmd

@@ -1,52 +1,11 @@
-// Verlet list rows for pairs of atoms: layout, builder, statistics and export. Included by dsmd_core.cu.
-//
-// Two neighbouring atoms share one row. Owned atoms are sorted by cell, x fastest, so consecutive slots of a cell row (a
-// run of x cells at one y, z) are neighbours in space (mean distance about one atom spacing); the union of their two
-// neighbourhoods is 1.3 times one of them for a Lennard-Jones liquid (cutoff + skin 2.8 sigma) and 1.2 times for water
-// (12 A). A row for two atoms therefore holds 0.65 entries per atom instead of one per partner: the force kernel gathers
-// 0.65 times the partner positions (its bound: the L1 unit, 13 wavefronts per 32 random 16-byte gathers) and the list
-// is 0.65 times as long. Entries that lie inside the list radius of one of the two atoms only are tested by both; the
-// cutoff test of the force kernel discards them.
-//
-// Units. Four consecutive atoms of one cell row form a quad (two pairs), the unit of the builder; quads never reach
-// across a cell row. Quad numbers follow from slots by arithmetic (quad_base), so no prefix sum is needed; a cell row
-// leaves at most one quad number unused (its word stays kNoQuad).
-//   quad[q]  = first slot * 4 + (atoms - 1); row of pair p = 2 q + h (h = 0, 1).
-//
-// Entries lie in chunks of four (one 16-byte word), 32 rows interleaved, so that a warp with a row per lane reads 512
-// consecutive bytes: entry k of row p at ((p >> 5) * stride + (k & ~3)) * 32 + (p & 31) * 4 + (k & 3) (row_base + row_offset).
-//   Owned partners come first, [0, row_int[p]); ghosts follow from the next multiple of four on and end at row_end[p];
-//   chunks are filled up with an atom that the search found outside the list radius of both atoms, so that the force kernel
-//   need not count (where the search had met no such atom by then, the row is marked kRowCareful and is counted).
-//   The two atoms themselves are not listed. Partners that one of them excludes are kept apart, from the row's last place
-//   downwards, marked kExclFirst / kExclSecond: the main loop of the force kernel has no flags to look at.
-//   row_special[p] = owned excluded partners | ghosts << kRowCountBits | kRowCareful | kRowOwnExcluded (the two atoms exclude
-//   each other).
+// Verlet list rows (dsmd_row_layout.cuh): builder, statistics and export. Included by dsmd_core.cu.
 #pragma once
+
+#include "dsmd_row_layout.cuh"
 
 namespace {
 
-constexpr unsigned kExclFirst = 0x80000000u, kExclSecond = 0x40000000u;
-constexpr unsigned kIndexMask = 0x3FFFFFFFu;
-constexpr unsigned kNoQuad = 0xFFFFFFFFu;
-constexpr int kRowCountBits = 15, kRowCountMask = (1 << kRowCountBits) - 1;
-constexpr unsigned kRowCareful = 0x40000000u, kRowOwnExcluded = 0x80000000u;
 constexpr int kBuildThreads = 128;
-
-__host__ __device__ inline int quad_base(int first_slot, int row) { return (first_slot + 3 * row + 3) >> 2; }
-
-// Words of a row: where it starts, and entry k's place from there.
-__host__ __device__ inline size_t row_base(unsigned pair, int stride) {
-    return static_cast<size_t>(pair >> 5) * stride * 32 + (pair & 31u) * 4;
-}
-__host__ __device__ inline int row_offset(int k) { return k * 32 - (k & 3) * 31; }
-
-// First atom and number of atoms (0, 1, 2) of a pair.
-__device__ __forceinline__ int pair_atoms(const unsigned* __restrict__ quad, int pair, int& first) {
-    const unsigned w = quad[pair >> 1];
-    first = static_cast<int>(w >> 2) + 2 * (pair & 1);
-    return w == kNoQuad ? 0 : min(max(static_cast<int>(w & 3u) + 1 - 2 * (pair & 1), 0), 2);
-}
 
 // The quads of every cell row (one warp per row): the numbers between two rows' bases that no atoms fill are kNoQuad.
 // layer_start (pinned host memory): first slot of every z layer of cells, and the end, by which a caller cuts the sorted
@@ -86,15 +45,6 @@ __device__ __forceinline__ double list_distance2(const Grid& g, const double (&p
     }
     return __dadd_rn(__dadd_rn(__dmul_rn(d[0], d[0]), __dmul_rn(d[1], d[1])), __dmul_rn(d[2], d[2]));
 }
-
-struct RowArrays {
-    const unsigned* quad;
-    unsigned* rows;
-    int stride;             // entries a row has room for, a multiple of four
-    int* row_end;
-    int* row_int;
-    unsigned* row_special;
-};
 
 // The search of one quad by one warp. Each lane takes one cell row of the stencil and works out the x window that the
 // four atoms' list spheres cut out of it (the union of their chords, rounded outwards to x cells). A scan over the lanes

@@ -921,7 +921,8 @@ bool reports_count(dsmd_ctx* c, cudaStream_t s) {
 }
 
 // The report of a displacement check about to be launched: of all owned atoms, or none (a part says little, and parts may
-// run side by side on several streams). Slots and tickets in turn, so that the last three stay readable.
+// run side by side on several streams). Slot and ticket follow from the launch's number: the MD loop has a check unread while
+// the next one is under way, and their numbers differ by one (only a list build takes numbers in between, and it voids the check).
 DisplacementReport displacement_report(dsmd_ctx* c, bool all_atoms, cudaStream_t s) {
     c->disp_seq = 0;
     if (!all_atoms || !reports_count(c, s)) return DisplacementReport{c->status, nullptr, nullptr, 0, c->gate2};

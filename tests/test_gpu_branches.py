@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 
 # atoms, box, cutoff, skin, types, Coulomb, exclusions: lone atoms and two; rows of one to four atoms; one, few and more than
-# eight types; Ewald tables in one copy (short rows) and in eight (rows of 240 and more); atoms that coincide with their row
+# eight types; Ewald tables in one copy (short rows) and in eight (rows of 240 and more)
 ROWS = [
     (1, 20.0, 4.0, 0.5, 1, False, False), (2, 20.0, 4.0, 0.5, 1, True, False), (37, 20.0, 4.0, 0.5, 3, False, False),
     (333, 20.0, 4.0, 0.5, 8, True, True), (334, 20.0, 4.0, 0.5, 9, True, True), (600, 16.0, 3.0, 0.3, 9, False, True),
@@ -50,6 +50,40 @@ def test_forces_of_every_row_form(cuda_device, n, L, rc, skin, nt, coulomb, excl
     for energy in (False, True):
         ctx.compute_forces(capi.PHASE_FULL, want_energy=energy)
         assert np.abs(ctx.forces_by_gid(n) - want).max() <= 2e-5 * scale
+    got = ctx.read_scalars()
+    assert abs(got["pe"] - scalars["pe"]) <= 1e-5 * max(abs(scalars["pe"]), 1.0)
+    assert got["pairs_in_cutoff"] == scalars["pairs_in_cutoff"]
+    ctx.close()
+
+
+@pytest.mark.parametrize("n,L,rc,nt,coulomb", [(300, 20.0, 4.0, 1, False), (300, 20.0, 4.0, 3, True), (2500, 25.0, 6.0, 2, True)])
+def test_atoms_that_coincide(cuda_device, n, L, rc, nt, coulomb):
+    """Pairs at r^2 < 1e-10 exert nothing on each other, and the rest of their rows is as it would be without them."""
+    rng = np.random.default_rng(n)
+    side = int(np.ceil(n ** (1 / 3)))
+    sites = np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij"), -1).reshape(-1, 3)[rng.permutation(side ** 3)[:n]]
+    pos = ((sites + 0.5 + rng.uniform(-0.2, 0.2, (n, 3))) * (L / side)) % L
+    pos[10:20] = pos[:10]
+    pos[30:40] = pos[20:30] + [4e-6, 0.0, 0.0]
+    pos[50:60] = pos[40:50]   # three at a place, and rows that hold them from elsewhere
+    pos[60:70] = pos[40:50]
+    box, types = np.full(3, L), rng.integers(0, nt, n).astype(np.int32)
+    charge = rng.uniform(-0.5, 0.5, n) if coulomb else np.zeros(n)
+    eps, sig = np.full((nt, nt), 0.3), np.ones((nt, nt))
+    ctx = capi.Context(n)
+    ctx.set_box(box)
+    ctx.set_pair_params(eps, sig, rc, 0.5)
+    if coulomb:
+        ctx.set_coulomb(True)
+    ctx.upload(pos, types=types, charge=charge)
+    ctx.build_neighbor_list()
+    pairs = co.pairs(*pos.T, n, box, search=rc + 0.5)
+    c6, c12 = co.lj_tables(eps, sig)
+    want, scalars = co.forces(*pos.T, n, box, pairs, c6, c12, rc, charge=charge, types=types, do_coulomb=coulomb,
+                              alpha=co.ewald_alpha(rc) if coulomb else 0.0)
+    for energy in (False, True):
+        ctx.compute_forces(capi.PHASE_FULL, want_energy=energy)
+        assert np.abs(ctx.forces_by_gid(n) - want).max() <= 2e-5 * np.abs(want).max()
     got = ctx.read_scalars()
     assert abs(got["pe"] - scalars["pe"]) <= 1e-5 * max(abs(scalars["pe"]), 1.0)
     assert got["pairs_in_cutoff"] == scalars["pairs_in_cutoff"]

@@ -17,7 +17,8 @@
 // consecutive bytes: entry k of row p at ((p >> 5) * stride + (k & ~3)) * 32 + (p & 31) * 4 + (k & 3) (row_base + row_offset).
 //   Owned partners come first, [0, row_int[p]); ghosts follow from the next multiple of four on and end at row_end[p];
 //   chunks are filled up with an atom that the search found outside the list radius of both atoms, so that the force kernel
-//   need not count (where the search had met no such atom by then, the row is marked kRowCareful and is counted).
+//   need not count, or, where the search had met none by then, with the row's own first atom, whose r^2 = 0 makes the force
+//   kernel count after all (a row for which no such atom turned up is marked kRowCareful and is counted from the start).
 //   The two atoms themselves are not listed. Partners that one of them excludes are kept apart, from the row's last place
 //   downwards, marked kExclFirst / kExclSecond: the main loop of the force kernel has no flags to look at.
 //   row_special[p] = owned excluded partners | ghosts << kRowCountBits | kRowCareful | kRowOwnExcluded (the two atoms exclude

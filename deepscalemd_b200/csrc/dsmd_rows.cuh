@@ -302,7 +302,6 @@ k_build_rows(Grid g, int n_owned, int n_total, int n_quads, const int4* __restri
     }
     int interior0 = 0, interior1 = 0;
     unsigned interior_special0 = 0u, interior_special1 = 0u;
-    unsigned counted = 0u;   // bit h: row h has a chunk that no atom could fill up
     for (int seg = 0; seg < n_seg; ++seg) {
         const int row = seg * g.ncells + (zc * g.nc[1] + yc) * g.nc[0];
         int s0 = 0, len0 = 0, s1 = 0, len1 = 0;
@@ -341,13 +340,12 @@ k_build_rows(Grid g, int n_owned, int n_total, int n_quads, const int4* __restri
         }
         if (n_atoms <= 2) { q.count1 = 0; q.special1 = 0u; }
         if (seg == 0) { interior0 = q.count0; interior1 = q.count1; interior_special0 = q.special0; interior_special1 = q.special1; }
-        // fill up the last chunk
+        // Fill up the last chunk. Where the search has met no atom to fill it with, the row's own first atom does: the force kernel
+        // sees r^2 = 0 and counts the row's entries (as it does from the start if no such atom turns up at all: kRowCareful).
         const int c = lane < 4 ? q.count0 : q.count1, far = lane < 4 ? q.far0 : q.far1;
         const int k = (c & ~3) + (lane & 3);
         if (lane < 8 && k >= c && (c & 3) && k < out.stride)
-            (lane < 4 ? q.row0 : q.row1)[row_offset(k)] = static_cast<unsigned>(far < 0 ? q.first : far);
-        // decided here and not at the end: the ghosts may still bring an atom that the owned chunk had to do without
-        counted |= (q.far0 < 0 && (q.count0 & 3) ? 1u : 0u) | (q.far1 < 0 && (q.count1 & 3) ? 2u : 0u);
+            (lane < 4 ? q.row0 : q.row1)[row_offset(k)] = static_cast<unsigned>(far < 0 ? q.first + (lane < 4 ? 0 : 2) : far);
         if (seg == 0 && n_seg == 2) {
             q.count0 = (q.count0 + 3) & ~3;
             q.count1 = (q.count1 + 3) & ~3;
@@ -362,7 +360,7 @@ k_build_rows(Grid g, int n_owned, int n_total, int n_quads, const int4* __restri
         out.row_end[2 * quad + lane] = min(ghosts ? count : interior, out.stride);
         out.row_int[2 * quad + lane] = min(interior, out.stride);
         out.row_special[2 * quad + lane] = n_own | ((n_special - n_own) << kRowCountBits) | (special & kRowOwnExcluded) |
-                                           (counted >> lane & 1u ? kRowCareful : 0u);
+                                           ((lane ? q.far1 : q.far0) < 0 ? kRowCareful : 0u);
         const int need = ((count + 3) & ~3) + static_cast<int>(n_special);   // whole chunks, and the ones apart behind them
         if (need > out.stride) atomicMax(&st->need_stride, static_cast<unsigned>(need));
         // pairs with a ghost partner, collected for the boundary pass of the force kernel (the order of the collection

@@ -78,8 +78,8 @@ struct StepArgs {
 };
 
 // Threads per block and blocks per SM, which fix the registers and with them how the compiler interleaves the partners of a
-// chunk; measured on a B200, the best of five to nine settings each. Long rows with Ewald: one block per SM, 118 registers
-// (1.08 to 1.12 ms per pass over 648,000 water atoms; 1.12 to 1.45 ms with two to six smaller blocks). One type: 64
+// chunk; measured on a B200, the best of five to nine settings each. Long rows with Ewald: one block per SM, 120 registers
+// (1.08 to 1.13 ms per pass over 648,000 water atoms; 1.12 to 1.45 ms with two to six smaller blocks). One type: 64
 // registers, 0.427 ms at 4,000,000 Lennard-Jones atoms (0.44 to 0.56 ms at other settings; a row per atom took 0.498 ms).
 // Types by table: 80 registers, 0.177 ms for the 1,048,576-atom mixture (0.18 to 0.23 ms; a row per atom 0.213 ms).
 template <int COPIES, int TYPES>

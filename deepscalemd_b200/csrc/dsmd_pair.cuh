@@ -413,8 +413,12 @@ __device__ __forceinline__ void row_forces(const PairParams& p, const ForceArgs&
         // What needs care, an entry per lane: the two atoms themselves (each is the other's partner), excluded partners, and
         // all entries of a row with a pair that coincides (there is none in a sane system).
         const unsigned row_lanes = (lanes == 32 ? 0xFFFFFFFFu : (1u << lanes) - 1u) << (threadIdx.x & 31 & -lanes);
-        const bool again = __any_sync(row_lanes, acc.least < 1e-10f);
-        if (COULOMB) close = !again && __any_sync(row_lanes, acc.least < kEwaldFirst);
+        // (one vote per row as a rule)
+        bool again = __any_sync(row_lanes, acc.least < (COULOMB ? kEwaldFirst : 1e-10f));
+        if (COULOMB && again) {
+            again = __any_sync(row_lanes, acc.least < 1e-10f);
+            close = !again;
+        }
         if (again) acc = PairAccumulator<COPIES, ENERGY, SWITCH>();
         const int ex_own = special & kRowCountMask, ex_all = ex_own + static_cast<int>((special >> kRowCountBits) & kRowCountMask);
         const int x0 = a.phase == DSMD_PHASE_BOUNDARY ? ex_own : 0, x1 = a.phase == DSMD_PHASE_INTERIOR ? ex_own : ex_all;
@@ -436,7 +440,8 @@ __device__ __forceinline__ void row_forces(const PairParams& p, const ForceArgs&
     // and then (a box of 648,000 water atoms, started from jittered places, has 15 such pairs), and one lane on its own would keep
     // the others, and in a grid of one round the device, waiting for hundreds of entries: 1.56 ms for that box with the row done
     // again by its lane, 1.14 this way, 1.53 with a row per atom and a branch per pair. A box without such pairs
-    // takes 1.13 ms (1.11 with the row done again: another schedule of the loop; with per-atom charges it is 1.12 against 1.13).
+    // takes 1.12 ms (1.11 with the row done again: another schedule of the loop; with per-atom charges it is 1.11 against 1.13,
+    // with energy sums 1.49 against 1.51).
     // Noting the rows and going over them every 32 rows, or a function that is not inlined: 1.12 to 1.16 and 1.10 to 1.14 ms, and the
     // parameters by address cost the plain Lennard-Jones form 7 %.
     if (COULOMB)

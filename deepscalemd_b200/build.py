@@ -11,7 +11,8 @@ import subprocess
 import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-SOURCES = ["csrc/dsmd_core.cu", "csrc/dsmd_pair_lj.cu", "csrc/dsmd_pair_lj_sums.cu", "csrc/dsmd_pair_ewald.cu", "csrc/dsmd_pair_ewald_sums.cu",
+SOURCES = ["csrc/dsmd_core.cu", "csrc/dsmd_pair_lj.cu", "csrc/dsmd_pair_lj_sums.cu", "csrc/dsmd_pair_lj_long.cu",
+           "csrc/dsmd_pair_lj_long_sums.cu", "csrc/dsmd_pair_ewald.cu", "csrc/dsmd_pair_ewald_sums.cu",
            "csrc/dsmd_pair_ewald_long.cu", "csrc/dsmd_pair_ewald_long_sums.cu", "csrc/dsmd_edges.cu", "csrc/dsmd_domain.cu", "csrc/dsmd_noalloc.cu"]
 LIBRARY = os.path.join(HERE, "libdsmd_b200.so")
 # host-side input layer (run description, coordinate / topology / restart files): plain C++, no CUDA

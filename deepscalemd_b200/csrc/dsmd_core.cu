@@ -55,7 +55,7 @@ constexpr int kDeviceSms = 148;                       // of a B200
 // Lanes that keep them busy. Steps of 12,000, 32,000, 64,000 and 130,000 Lennard-Jones atoms: 12.9, 16.1, 18.5 and 28.2 us;
 // with twice as many 17.4, 20.7, 27.2 and 33.4 us, with half as many 12.0, 14.1, 19.2 and 33.3 us.
 constexpr int64_t kPairLanesWanted = kDeviceSms * 512;
-constexpr int64_t kPairLanesWantedEwald = kDeviceSms * 768;   // two rounds of one block of 384 each
+constexpr int64_t kPairLanesWantedEwald = kDeviceSms * 768;   // one and a half rounds of one block of 512 each
 constexpr int kLongRow = 240;                         // entries (with the row's spare room): about 150 partners per atom
 constexpr int64_t kRowsAlways = 4096;                 // cell rows that any system may have: 2 MB of list rows
 constexpr int kXRefine = 4;    // x cells per cell width of the y and z axes (tighter row windows in the list build)
@@ -799,27 +799,30 @@ int ensure_rows(dsmd_ctx* c, int stride) {
 
 int pair_lane_shift(const dsmd_ctx* c);
 
-// Copies of the Ewald table in the force kernel's shared memory: eight where rows are long enough to pay for them.
-int ewald_copies(const dsmd_ctx* c) { return !c->coulomb ? 0 : (c->stride >= kLongRow ? kEwaldCopiesMost : 1); }
+// Long rows have their entries in another order (dsmd_row_layout.cuh), and with Ewald several copies of the table in the force
+// kernel's shared memory.
+bool long_rows(const dsmd_ctx* c) { return c->stride >= kLongRow; }
+int ewald_copies(const dsmd_ctx* c) { return !c->coulomb ? 0 : (long_rows(c) ? kEwaldCopiesMost : 1); }
 
 // Rows for `row_entries` entries each: lanes per row, stride, storage.
 int lay_out_rows(dsmd_ctx* c, int row_entries) {
     const int64_t yz_rows = static_cast<int64_t>(c->grid.nc[1]) * c->grid.nc[2];
     c->n_quads = quad_base(static_cast<int>(c->n_owned), static_cast<int>(yz_rows));
-    c->stride = (row_entries + 3) & ~3;
+    c->stride = whole_groups<0>(row_entries);
+    if (long_rows(c)) c->stride = whole_groups<kLongOrder>(row_entries);
     c->lane_shift = pair_lane_shift(c);
     return ensure_rows(c, c->stride);
 }
 
 RowArrays rows_of(const dsmd_ctx* c) { return RowArrays{c->quad, c->rows, c->stride, c->row_end, c->row_int, c->row_special}; }
 
-// Lanes that share a pair's row in the force kernel: one where that fills the device, more for small systems, whose time
+// Lanes that share a pair's row in the force kernel: one (four if rows are long) where that fills the device, more for small systems, whose time
 // is the chain of dependent reads along a row. A function of the system alone, so that a pass over a part of the atoms
 // gives the same bits as a pass over all of them.
 int pair_lane_shift(const dsmd_ctx* c) {
     const int64_t pairs = std::min(2 * c->n_quads, c->n_owned);   // as many rows at most have atoms
     const int64_t wanted = ewald_copies(c) == kEwaldCopiesMost ? kPairLanesWantedEwald : kPairLanesWanted;
-    int shift = 0;
+    int shift = long_rows(c) ? kLongOrder : 0;
     while (shift < 5 && (pairs << shift) < wanted && (8 << shift) <= c->stride) ++shift;
     return shift;
 }
@@ -1343,16 +1346,11 @@ static int build_list(dsmd_ctx* c, bool forces, cudaStream_t s) {
             DSMD_LAUNCHED(c);
         }
         const unsigned blocks = blocks_for(c->n_quads * 32, kBuildThreads);
-        if (ex.offsets)
-            k_build_rows<true><<<blocks, kBuildThreads, 0, s>>>(c->grid, static_cast<int>(c->n_owned), static_cast<int>(c->n_total),
-                                                              static_cast<int>(c->n_quads), c->pq, c->gid[c->cur], ex, c->cell_start,
-                                                              c->ghost_rows + 2 * rows, c->ghost_rows + 3 * rows, rows_of(c),
-                                                              c->boundary_pairs, c->status);
-        else
-            k_build_rows<false><<<blocks, kBuildThreads, 0, s>>>(c->grid, static_cast<int>(c->n_owned), static_cast<int>(c->n_total),
-                                                               static_cast<int>(c->n_quads), c->pq, c->gid[c->cur], ex, c->cell_start,
-                                                               c->ghost_rows + 2 * rows, c->ghost_rows + 3 * rows, rows_of(c),
-                                                               c->boundary_pairs, c->status);
+        const auto build = ex.offsets ? (long_rows(c) ? k_build_rows<true, kLongOrder> : k_build_rows<true, 0>)
+                                      : (long_rows(c) ? k_build_rows<false, kLongOrder> : k_build_rows<false, 0>);
+        build<<<blocks, kBuildThreads, 0, s>>>(c->grid, static_cast<int>(c->n_owned), static_cast<int>(c->n_total), static_cast<int>(c->n_quads),
+                                               c->pq, c->gid[c->cur], ex, c->cell_start, c->ghost_rows + 2 * rows, c->ghost_rows + 3 * rows,
+                                               rows_of(c), c->boundary_pairs, c->status);
         DSMD_LAUNCHED(c);
         k_build_done<<<1, 1, 0, s>>>(c->status, attempt == 0 ? static_cast<unsigned>(expect_dropped) : 0u, c->mail + kMailBuild, ++c->seq);
         DSMD_LAUNCHED(c);
@@ -1395,7 +1393,8 @@ static int list_members(dsmd_ctx* c, cudaStream_t s) {
     const int n = static_cast<int>(c->n_owned);
     DSMD_CUDA(c, cudaSetDevice(c->device));
     DSMD_CUDA(c, cudaMemsetAsync(c->member_stats, 0, sizeof(unsigned long long) * 3, s));
-    k_list_members<false><<<member_blocks(c), kMemberThreads, 0, s>>>(c->grid, static_cast<int>(2 * c->n_quads), rows_of(c), c->ref[0], c->ref[1],
+    const auto count = long_rows(c) ? k_list_members<false, kLongOrder> : k_list_members<false, 0>;
+    count<<<member_blocks(c), kMemberThreads, 0, s>>>(c->grid, static_cast<int>(2 * c->n_quads), rows_of(c), c->ref[0], c->ref[1],
                                                                    c->ref[2], c->offsets64, c->member_stats, nullptr, nullptr, nullptr);
     DSMD_LAUNCHED(c);
     size_t need = 0;
@@ -1436,7 +1435,8 @@ int dsmd_list_export(dsmd_ctx* c, int32_t* d_i, int32_t* d_j, uint8_t* d_flags, 
     { const int rc = list_members(c, s); if (rc) return rc; }
     *n_pairs = c->stat_entries;
     if (!d_i || !d_j || capacity < c->stat_entries) return DSMD_OK;   // size query
-    k_list_members<true><<<member_blocks(c), kMemberThreads, 0, s>>>(c->grid, static_cast<int>(2 * c->n_quads), rows_of(c), c->ref[0], c->ref[1],
+    const auto write = long_rows(c) ? k_list_members<true, kLongOrder> : k_list_members<true, 0>;
+    write<<<member_blocks(c), kMemberThreads, 0, s>>>(c->grid, static_cast<int>(2 * c->n_quads), rows_of(c), c->ref[0], c->ref[1],
                                                                   c->ref[2], c->offsets64, nullptr, d_i, d_j, d_flags);
     DSMD_LAUNCHED(c);
     DSMD_CUDA(c, cudaStreamSynchronize(s));
@@ -1552,9 +1552,10 @@ static int compute_forces_impl(dsmd_ctx* c, int phase, int want_energy, int64_t 
     if (pairs > 0) {   // else nothing to add to the forces; the energy sums of a boundary pass stay as the interior pass left them
         const unsigned blocks = static_cast<unsigned>(pair_blocks(c, pairs, e));
         const int copies = ewald_copies(c);
-        const auto launch = copies == 0 ? (e ? dsmd::launch_pair<0, true> : dsmd::launch_pair<0, false>)
-                            : copies == 1 ? (e ? dsmd::launch_pair<1, true> : dsmd::launch_pair<1, false>)
-                                          : (e ? dsmd::launch_pair<kEwaldCopiesMost, true> : dsmd::launch_pair<kEwaldCopiesMost, false>);
+        const auto launch = copies == 0 ? (long_rows(c) ? (e ? dsmd::launch_pair<0, true, kLongOrder> : dsmd::launch_pair<0, false, kLongOrder>)
+                                                       : (e ? dsmd::launch_pair<0, true, 0> : dsmd::launch_pair<0, false, 0>))
+                            : copies == 1 ? (e ? dsmd::launch_pair<1, true, 0> : dsmd::launch_pair<1, false, 0>)
+                                          : (e ? dsmd::launch_pair<kEwaldCopiesMost, true, kLongOrder> : dsmd::launch_pair<kEwaldCopiesMost, false, kLongOrder>);
         DSMD_CUDA(c, launch(p, a, sw, blocks, s));
         ++c->launches;
     }
@@ -1572,7 +1573,8 @@ static int force_step(dsmd_ctx* c, double dt, double f2a, cudaStream_t s) {
     const StepArgs at{r[0], r[1], r[2], r[3], r[4], r[5], r[9], c->ref[0], c->ref[1], c->ref[2], c->pq_next, dt, dt * f2a};
     const unsigned blocks = static_cast<unsigned>(pair_blocks(c, pairs, false));
     const DisplacementReport report = displacement_report(c, true, s);
-    DSMD_CUDA(c, dsmd::launch_step(p, a, c->grid, at, report, c->switch_distance > 0.0, blocks, s));
+    const auto launch = long_rows(c) ? dsmd::launch_step<kLongOrder> : dsmd::launch_step<0>;
+    DSMD_CUDA(c, launch(p, a, c->grid, at, report, c->switch_distance > 0.0, blocks, s));
     ++c->launches;
     std::swap(c->pq, c->pq_next);
     return DSMD_OK;

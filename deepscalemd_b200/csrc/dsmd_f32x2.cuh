@@ -29,6 +29,13 @@ __device__ __forceinline__ F2 fma(F2 a, F2 b, F2 c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
     return r;
 }
+// The first lane of a, the second of b.
+__device__ __forceinline__ F2 first_second(F2 a, F2 b) {
+    float ax, ay, bx, by;
+    parts(a, ax, ay);
+    parts(b, bx, by);
+    return f2(ax, by);
+}
 __device__ __forceinline__ F2 both(float a) { return f2(a, a); }
 
 __device__ __forceinline__ float rcp_approx(float v) {

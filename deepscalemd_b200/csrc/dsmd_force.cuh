@@ -14,7 +14,7 @@ namespace dsmd {
 struct RowArrays {
     const unsigned* quad;
     unsigned* rows;
-    int stride;             // entries a row has room for, a multiple of four
+    int stride;             // entries a row has room for, whole groups
     int* row_end;
     int* row_int;
     unsigned* row_special;
@@ -43,10 +43,10 @@ struct PairParams {
     const float* type_charge;    // [ntypes] when every atom's charge is that of its type (dsmd_set_type_charges), else null
 };
 
-// Pair parameters by type. kOneType: constants. kFewTypes: a table over (type of the first atom, type of the second, type
+// Pair parameters by type. kOneType: constants. kTwoTypes (without Ewald): both in registers, the partner's type picks. kFewTypes: a table over (type of the first atom, type of the second, type
 // of the partner) that holds what both atoms need side by side - up to 8 types, 8 KB (12 KB with charges by type). kManyTypes: a table over two types,
 // read once per atom.
-enum { kOneType = 0, kFewTypes = 1, kManyTypes = 2 };
+enum { kOneType = 0, kFewTypes = 1, kManyTypes = 2, kTwoTypes = 3 };
 constexpr int kFewTypesMost = 8;
 
 constexpr int kEwaldCopiesMost = 8;   // see EwaldTable
@@ -78,18 +78,21 @@ struct StepArgs {
 };
 
 // Threads per block and blocks per SM, which fix the registers and with them how the compiler interleaves the partners of a
-// chunk; measured on a B200, the best of five to nine settings each. Long rows with Ewald: one block per SM, 120 registers
-// (1.08 to 1.13 ms per pass over 648,000 water atoms; 1.12 to 1.45 ms with two to six smaller blocks). One type: 64
-// registers, 0.427 ms at 4,000,000 Lennard-Jones atoms (0.44 to 0.56 ms at other settings; a row per atom took 0.498 ms).
-// Types by table: 80 registers, 0.177 ms for the 1,048,576-atom mixture (0.18 to 0.23 ms; a row per atom 0.213 ms).
+// chunk; measured on a B200, the best of five to nine settings each. Long rows with Ewald: one block of 512 per SM, 128 registers
+// (0.97 ms per pass over 648,000 water atoms; 0.97 to 1.16 ms with one of 384 to 768 or two to four smaller ones; 1.12 ms with a row per
+// lane). One type: 64 registers, 0.356 ms at 4,000,000 Lennard-Jones atoms (0.37 to 0.41 ms at 14 to 20 blocks; 0.418 ms while what the
+// end of a row needs was kept in registers through its loop). Two types: 80 registers, 0.164 ms for the 1,048,576-atom mixture
+// (0.17 to 0.19 ms at other settings, 0.174 with the pair table in shared memory, 0.185 before).
 template <int COPIES, int TYPES>
-constexpr int kPairThreads = COPIES == kEwaldCopiesMost ? 384 : (COPIES == 0 && TYPES == kOneType ? 64 : 128);
+constexpr int kPairThreads = COPIES == kEwaldCopiesMost ? 512 : (COPIES == 0 && TYPES == kOneType ? 64 : 128);
 template <int COPIES, int TYPES, bool ENERGY>
 constexpr int kPairBlocks = ENERGY || COPIES == kEwaldCopiesMost ? 1 : (COPIES > 0 ? 5 : (TYPES == kOneType ? 16 : 6));
 
-// Both return what the launch returned. sw: with the switching function. ENERGY: with energy sums.
-template <int COPIES, bool ENERGY>
+// Both return what the launch returned. sw: with the switching function. ENERGY: with energy sums. ORDER: of the rows' entries
+// (dsmd_row_layout.cuh).
+template <int COPIES, bool ENERGY, int ORDER>
 cudaError_t launch_pair(const PairParams& p, const ForceArgs& a, bool sw, unsigned blocks, cudaStream_t s);
+template <int ORDER>
 cudaError_t launch_step(const PairParams& p, const ForceArgs& a, const Grid& g, const StepArgs& at, const DisplacementReport& report,
                         bool sw, unsigned blocks, cudaStream_t s);
 

@@ -64,16 +64,18 @@ struct PairTerms {
 
 // Sums of the two atoms of a pair row.
 //
-// What bounds the force kernel: the dispatch port, at which a packed instruction (two lanes: the two atoms) counts twice, and
-// beside it the L1 unit (13 wavefronts per gather of 32 partners). So what counts is the number of scalar operations: about
-// 55 per entry (two pairs) for Lennard-Jones, 75 with Ewald. The plain form below therefore leaves out what no pair of a sane
-// system needs and keeps the smallest r^2 for a look afterwards.
+// What bounds the force kernel: the multiply-add and the integer / select pipes, each busy half of the time and often at once (a packed
+// instruction, two lanes: the two atoms, counts twice; about 55 scalar operations per entry (two pairs) for Lennard-Jones, 75 with Ewald),
+// and beside them the L1 unit (13 wavefronts per gather of 32 random partners, half of that where four lanes gather neighbours).
+// So what counts is the number of operations and that the compiler has registers to interleave four partners with. The plain form
+// therefore leaves out what no pair of a sane system needs: with Ewald or energies it keeps the smallest r^2 for a look
+// afterwards, without them a pair that coincides leaves sums that are not finite.
 template <int COPIES, bool ENERGY, bool SWITCH>
 struct PairAccumulator {
     static constexpr bool COULOMB = COPIES > 0;
     F2 ax{0}, ay{0}, az{0};
     F2 e_sum{0}, w_sum{0}, wx{0}, wy{0}, wz{0};
-    float least = 3.0e38f;   // smallest r^2 seen
+    float least = 3.0e38f;   // smallest r^2 seen (Ewald or energies)
     int n_in = 0;
 
     // Forces of the two atoms out, and the sums back to zero.
@@ -163,12 +165,9 @@ struct PairAccumulator {
         }
     }
 
-    // What the plain form, which takes the table's first value for any distance below the table, left out of one entry's Ewald
-    // terms. qq: Coulomb constant times the charges of the two pairs.
-    __device__ __forceinline__ void add_close_rest(const PairParams& p, const EwaldTable<COPIES>& table, const int4& pa, const int4& pb,
-                                                   const int4& pj, F2 qq) {
-        F2 dx, dy, dz;
-        const F2 r2 = distance(p, pa, pb, pj, dx, dy, dz);
+    // What the plain form, which takes the table's first value for any distance below the table, left out of the Ewald terms of
+    // two pairs at those distances. qq: Coulomb constant times the charges of the two pairs.
+    __device__ __forceinline__ void add_close_rest(const PairParams& p, const EwaldTable<COPIES>& table, F2 dx, F2 dy, F2 dz, F2 r2, F2 qq) {
         float ra, rb;
         parts(r2, ra, rb);
         if (fminf(ra, rb) >= kEwaldFirst) return;
@@ -213,6 +212,29 @@ struct PairAccumulator {
         return fma(dz, dz, fma(dx, dx, mul(dy, dy)));   // (in this order: it decides which pairs lie inside a plain cutoff)
     }
 
+    // The distance of the row's own two atoms, from each of them.
+    static __device__ __forceinline__ F2 own_distance(const PairParams& p, const int4& pa, const int4& pb, F2& dx, F2& dy, F2& dz) {
+        dx = mul(f2(offset(pa.x, pb.x), offset(pb.x, pa.x)), both(p.scale[0]));
+        dy = mul(f2(offset(pa.y, pb.y), offset(pb.y, pa.y)), both(p.scale[1]));
+        dz = mul(f2(offset(pa.z, pb.z), offset(pb.z, pa.z)), both(p.scale[2]));
+        return fma(dz, dz, fma(dx, dx, mul(dy, dy)));
+    }
+
+    // The row's own two atoms, each the other's partner, in the plain form. k_a: terms of the second as the first sees it, k_b: of
+    // the first as the second does. there: the pair counts.
+    __device__ __forceinline__ void add_own(const PairParams& p, const EwaldTable<COPIES>& table, const int4& pa, const int4& pb,
+                                            const PairTerms& k_a, const PairTerms& k_b, bool there) {
+        F2 dx, dy, dz;
+        const F2 r2 = own_distance(p, pa, pb, dx, dy, dz);
+        float ra, rb;
+        parts(r2, ra, rb);
+        const PairTerms k{first_second(k_a.rep, k_b.rep), first_second(k_a.att, k_b.att), first_second(k_a.qq, k_b.qq)};
+        F2 f, u;
+        evaluate<false>(p, table, k, r2, ra, rb, false, false, f, u);
+        if (there) least = fminf(least, fminf(ra, rb));
+        sum(dx, dy, dz, r2, f, u, there && ra < p.rc2, there && rb < p.rc2);
+    }
+
     // One entry, seen from the two atoms at pa and pb (fixed-point positions: the 32-bit difference is the nearest image).
     // The plain form takes every pair inside the cutoff; CAREFUL also tells pairs that coincide (r^2 < 1e-10: no force) and
     // those named above.
@@ -228,7 +250,7 @@ struct PairAccumulator {
         if (CAREFUL) {
             sum(dx, dy, dz, r2, f, u, ra < p.rc2 && ra >= 1e-10f, rb < p.rc2 && rb >= 1e-10f);
         } else {
-            asm("min.f32 %0, %0, %1, %2;" : "+f"(least) : "f"(ra), "f"(rb));
+            if (COULOMB || ENERGY) asm("min.f32 %0, %0, %1, %2;" : "+f"(least) : "f"(ra), "f"(rb));
             sum(dx, dy, dz, r2, f, u, ra < p.rc2, rb < p.rc2);
         }
     }
@@ -281,7 +303,7 @@ struct PairTables {
             for (int k = threadIdx.x; k < nt * nt; k += blockDim.x) s_lj2[k] = p.lj[k];
         if (by_type && !few)
             for (int k = threadIdx.x; k < nt; k += blockDim.x) s_charge[k] = p.type_charge[k];
-        if (COULOMB || TYPES != kOneType) __syncthreads();
+        if (COULOMB || few || many) __syncthreads();
         ewald = EwaldTable<COPIES>{s_ewald + (threadIdx.x & (COPIES > 0 ? COPIES - 1u : 0u)), p.ewald_intervals};
         lj3 = s_lj3;
         qq3 = s_qq3;
@@ -291,50 +313,72 @@ struct PairTables {
 };
 
 // What the plain form left out of a row's entries (add_close_rest), by all lanes of a warp.
-template <int COPIES, bool ENERGY, bool SWITCH, bool BY_TYPE>
+template <int COPIES, bool ENERGY, bool SWITCH, bool BY_TYPE, int ORDER>
 __device__ __forceinline__ PairAccumulator<COPIES, ENERGY, SWITCH> close_rest(const PairParams& p, const ForceArgs& a,
                                                                               const EwaldTable<COPIES>& table, int pair) {
-    PairAccumulator<COPIES, ENERGY, SWITCH> rest;
+    using Sums = PairAccumulator<COPIES, ENERGY, SWITCH>;
+    Sums rest;
     int first;
     const int atoms = pair_atoms(a.rows.quad, pair, first), last = first + atoms - 1;
     const int4 pa = a.pq[first], pb = a.pq[last];
     const F2 q = mul(both(p.kq), BY_TYPE ? f2(p.type_charge[pa.w], p.type_charge[pb.w]) : f2(a.qf[first], a.qf[last]));
-    const int mid = a.rows.row_int[pair], end = a.rows.row_end[pair], ghosts = (mid + 3) & ~3;
+    const int mid = a.rows.row_int[pair], end = a.rows.row_end[pair], ghosts = whole_groups<ORDER>(mid);
     const int k0 = a.phase == DSMD_PHASE_BOUNDARY ? ghosts : 0, k1 = a.phase == DSMD_PHASE_INTERIOR ? mid : end;
-    const unsigned* words = a.rows.rows + row_base(static_cast<unsigned>(pair), a.rows.stride);
+    const unsigned* words = a.rows.rows + row_base<ORDER>(static_cast<unsigned>(pair), a.rows.stride);
 #pragma unroll 1
     for (int k = k0 + (threadIdx.x & 31); k < k1; k += 32) {
         if (k >= mid && k < ghosts) continue;
-        const unsigned e = words[row_offset(k)];
+        const unsigned e = words[row_offset<ORDER>(k)];
         const int4 pj = __ldg(&a.pq[e]);
-        rest.add_close_rest(p, table, pa, pb, pj, mul(q, both(BY_TYPE ? p.type_charge[pj.w] : __ldg(&a.qf[e]))));
+        F2 dx, dy, dz;
+        const F2 r2 = Sums::distance(p, pa, pb, pj, dx, dy, dz);
+        rest.add_close_rest(p, table, dx, dy, dz, r2, mul(q, both(BY_TYPE ? p.type_charge[pj.w] : __ldg(&a.qf[e]))));
+    }
+    if ((threadIdx.x & 31) == 0 && atoms > 1 && a.phase != DSMD_PHASE_BOUNDARY && !(a.rows.row_special[pair] & kRowOwnExcluded)) {
+        F2 dx, dy, dz;
+        const F2 r2 = Sums::own_distance(p, pa, pb, dx, dy, dz);
+        rest.add_close_rest(p, table, dx, dy, dz, r2, mul(q, BY_TYPE ? f2(p.type_charge[pb.w], p.type_charge[pa.w]) : f2(a.qf[last], a.qf[first])));
     }
     rest.over_warp();
     return rest;
 }
 
-// Forces on the atoms of one pair row, worked on by `lanes` lanes of a warp, which take the row's chunks of four entries in
-// turn; this lane's share of the sums. The next chunk of entries and the partners of the current one are in flight before
+// The row that thread t of a force kernel works on (-1: none) and its place among the lanes of the row.
+__device__ __forceinline__ int row_of_thread(const ForceArgs& a, int t) {
+    const int slot = t >> a.lane_shift;
+    return slot < a.n_pairs ? (a.pair_list ? a.pair_list[slot] : a.first_pair + slot) : -1;
+}
+
+// t again, as a number that the compiler takes for another one: what follows from it is worked out (and read) anew instead of
+// being kept in registers across the loop over a row's entries.
+__device__ __forceinline__ int afresh(int t) {
+    asm volatile("" : "+r"(t));
+    return t;
+}
+
+// Forces on the atoms of one pair row, worked on by 2^lane_shift lanes of a warp, which take the row's chunks of four entries in
+// turn; the row's sums, in all its lanes. The next chunk of entries and the partners of the current one are in flight before
 // any arithmetic starts; the list is streamed with an evict-first hint so that the positions stay in L2.
 // Every listed pair is evaluated from the side of each of its owned atoms (a full list), so forces need no scatter and no
 // atomics and the order of the sums is fixed (bitwise reproducible). Energy and virial take half of every directed entry;
 // an owned-ghost pair is then counted half on each rank, as the reference's list kernel does
 // (src/force_calculator_cuda.cu:1784-1789).
-template <int COPIES, bool ENERGY, int TYPES, bool SWITCH, bool QTYPE>
+template <int COPIES, bool ENERGY, int TYPES, bool SWITCH, bool QTYPE, int ORDER>
 __device__ __forceinline__ void row_forces(const PairParams& p, const ForceArgs& a, const PairTables<COPIES, ENERGY, TYPES, QTYPE>& tables,
-                                           int pair, int sub, int lanes, int first, int atoms, float (&sum_a)[3], float (&sum_b)[3],
-                                           double (&v)[6]) {
+                                           int t, float (&sum_a)[3], float (&sum_b)[3], double (&v)[6]) {
     constexpr bool COULOMB = COPIES > 0, few = TYPES == kFewTypes, many = TYPES == kManyTypes, by_type = COULOMB && QTYPE;
-    const int nt = p.ntypes;
+    constexpr bool two_types = TYPES == kTwoTypes;
+    const int nt = p.ntypes, lanes = 1 << a.lane_shift, sub = t & (lanes - 1);
     const EwaldTable<COPIES>& table = tables.ewald;
     PairAccumulator<COPIES, ENERGY, SWITCH> acc;
     bool close = false;   // the row has a pair below the Ewald table
+    bool two = false;     // the row has two atoms
+    int first = 0;
+    const int pair = row_of_thread(a, t), atoms = pair >= 0 ? pair_atoms(a.rows.quad, pair, first) : 0;
     if (atoms > 0) {
         const int4 pa = a.pq[first], pb = a.pq[first + atoms - 1];
-        const int mid = a.rows.row_int[pair], end = a.rows.row_end[pair];
         const unsigned special = a.rows.row_special[pair];
-        const unsigned* words = a.rows.rows + row_base(static_cast<unsigned>(pair), a.rows.stride);
-        const uint4* row = reinterpret_cast<const uint4*>(words);
+        const uint4* row = reinterpret_cast<const uint4*>(a.rows.rows + row_base<ORDER>(static_cast<unsigned>(pair), a.rows.stride)) + (sub & ((1 << ORDER) - 1));
         F2 q{0};
         PairTerms one{};
         const int row3 = (pa.w * nt + pb.w) * nt;
@@ -346,12 +390,21 @@ __device__ __forceinline__ void row_forces(const PairParams& p, const ForceArgs&
             one.att = both(lj.y);
             if (by_type) one.qq = mul(q, both(tables.charge[0]));
         }
+        // two types: what either asks for, in registers
+        PairTerms of_type[2];
+        if (two_types)
+            for (int k = 0; k < 2; ++k) {
+                const float2 la = p.lj[pa.w * 2 + k], lb = p.lj[pb.w * 2 + k];
+                of_type[k].rep = f2(la.x, lb.x);
+                of_type[k].att = f2(la.y, lb.y);
+            }
         const auto take = [&](unsigned e, int4& pos, float& charge) {
             pos = __ldg(&a.pq[e]);
             if (COULOMB && !by_type) charge = __ldg(&a.qf[e]);
         };
         const auto terms = [&](int type, float charge) {
             PairTerms k = one;
+            if (two_types) k = type ? of_type[1] : of_type[0];
             if (few) {
                 const ulonglong2 lj = tables.lj3[row3 + type];
                 k.rep.v = lj.x;
@@ -367,92 +420,103 @@ __device__ __forceinline__ void row_forces(const PairParams& p, const ForceArgs&
             if (COULOMB && !by_type) k.qq = mul(q, both(charge));
             return k;
         };
-        const int part_begin = a.phase == DSMD_PHASE_BOUNDARY ? 1 : 0;
-        const int part_end = a.phase == DSMD_PHASE_INTERIOR || end <= mid ? 1 : 2;
-        acc.least = (special & kRowCareful) ? 0.0f : 3.0e38f;
-        for (int part = part_begin; part < part_end && !(special & kRowCareful); ++part) {
-            int c = (part == 0 ? 0 : (mid + 3) >> 2) + sub;
-            const int c_end = ((part == 0 ? mid : end) + 3) >> 2;
-            const auto add = [&](const int4& pos, float charge) {
-                acc.template add_partner<false>(p, table, pa, pb, pos, terms(pos.w, charge), 0u);
-            };
-            if (c >= c_end) continue;
-            uint4 e = __ldcs(row + static_cast<size_t>(c) * 32);
-            if (TYPES == kOneType && !COULOMB && !ENERGY) {   // two partners are worked on while the next two are on their way
-                int4 p_x, p_y, p_z, p_w;
-                float none;
-                take(e.x, p_x, none);
-                take(e.y, p_y, none);
-                for (; c < c_end; c += lanes) {
-                    take(e.z, p_z, none);
-                    take(e.w, p_w, none);
-                    if (c + lanes < c_end) e = __ldcs(row + static_cast<size_t>(c + lanes) * 32);
-                    add(p_x, 0.f);
-                    add(p_y, 0.f);
-                    take(e.x, p_x, none);
-                    take(e.y, p_y, none);
-                    add(p_z, 0.f);
-                    add(p_w, 0.f);
-                }
-            } else {
-                for (; c < c_end; c += lanes) {
-                    int4 p_x, p_y, p_z, p_w;
-                    float q_x, q_y, q_z, q_w;
-                    take(e.x, p_x, q_x);
-                    take(e.y, p_y, q_y);
-                    take(e.z, p_z, q_z);
-                    take(e.w, p_w, q_w);
-                    if (c + lanes < c_end) e = __ldcs(row + static_cast<size_t>(c + lanes) * 32);
-                    add(p_x, q_x);
-                    add(p_y, q_y);
-                    add(p_z, q_z);
-                    add(p_w, q_w);
-                }
-            }
+        const auto add = [&](const int4& pos, float charge) {
+            acc.template add_partner<false>(p, table, pa, pb, pos, terms(pos.w, charge), 0u);
+        };
+        // Chunks of entries, in groups of as many as lie side by side: those of owned partners, of ghosts, or all (what lies between
+        // the two kinds are atoms out of reach).
+        int c = sub, c_end;
+        {
+            const int mid = a.rows.row_int[pair], end = a.rows.row_end[pair];
+            if (a.phase == DSMD_PHASE_BOUNDARY) c += whole_groups<ORDER>(mid) >> 2;
+            c_end = whole_groups<ORDER>(a.phase == DSMD_PHASE_INTERIOR ? mid : max(mid, end)) >> 2;
         }
-        // What needs care, an entry per lane: the two atoms themselves (each is the other's partner), excluded partners, and
-        // all entries of a row with a pair that coincides (there is none in a sane system).
+        if (special & kRowCareful) c_end = 0;
+        uint4 e{};
+        if (c < c_end) e = __ldcs(row + (c >> ORDER) * size_t(32));
+        {   // the two atoms themselves: each is the other's partner
+            two = atoms > 1;
+            const bool own = two && a.phase != DSMD_PHASE_BOUNDARY && !(special & (kRowOwnExcluded | kRowCareful));
+            float q_a = 0.0f, q_b = 0.0f;
+            if (COULOMB && !by_type) { q_a = a.qf[first]; q_b = a.qf[first + atoms - 1]; }
+            acc.add_own(p, table, pa, pb, terms(pb.w, q_b), terms(pa.w, q_a), own && sub == 0);
+        }
+        for (; c < c_end; c += lanes) {
+            int4 p_x, p_y, p_z, p_w;
+            float q_x, q_y, q_z, q_w;
+            take(e.x, p_x, q_x);
+            take(e.y, p_y, q_y);
+            take(e.z, p_z, q_z);
+            take(e.w, p_w, q_w);
+            if (c + lanes < c_end) e = __ldcs(row + ((c + lanes) >> ORDER) * size_t(32));
+            add(p_x, q_x);
+            add(p_y, q_y);
+            add(p_z, q_z);
+            add(p_w, q_w);
+        }
+        // What needs care, an entry per lane: excluded partners, and all entries of a row with a pair that coincides (there is
+        // none in a sane system), the two atoms' own with them.
         const unsigned row_lanes = (lanes == 32 ? 0xFFFFFFFFu : (1u << lanes) - 1u) << (threadIdx.x & 31 & -lanes);
         // (one vote per row as a rule)
-        bool again = __any_sync(row_lanes, acc.least < (COULOMB ? kEwaldFirst : 1e-10f));
+        bool suspect;
+        if (!COULOMB && !ENERGY) {   // r^2 < 1e-10: r^-8 is infinite, and so, or no number, is what any parameters make of it
+            float s[6];
+            parts(acc.ax, s[0], s[1]);
+            parts(acc.ay, s[2], s[3]);
+            parts(acc.az, s[4], s[5]);
+            suspect = !(fabsf(s[0] + s[1]) + fabsf(s[2] + s[3]) + fabsf(s[4] + s[5]) < 3.0e38f);
+        } else {
+            suspect = acc.least < (COULOMB ? kEwaldFirst : 1e-10f);
+        }
+        bool again = __any_sync(row_lanes, suspect || (special & kRowCareful));
         if (COULOMB && again) {
-            again = __any_sync(row_lanes, acc.least < 1e-10f);
+            again = __any_sync(row_lanes, acc.least < 1e-10f || (special & kRowCareful));
             close = !again;
         }
-        if (again) acc = PairAccumulator<COPIES, ENERGY, SWITCH>();
-        const int ex_own = special & kRowCountMask, ex_all = ex_own + static_cast<int>((special >> kRowCountBits) & kRowCountMask);
-        const int x0 = a.phase == DSMD_PHASE_BOUNDARY ? ex_own : 0, x1 = a.phase == DSMD_PHASE_INTERIOR ? ex_own : ex_all;
-        const int n_own = atoms > 1 && a.phase != DSMD_PHASE_BOUNDARY && !(special & kRowOwnExcluded) ? 2 : 0;
-        const int n_first = part_begin == 0 ? mid : 0, n_second = part_end == 2 ? end - ((mid + 3) & ~3) : 0;
-        const int n_care = n_own + (x1 - x0) + (again ? n_first + n_second : 0);
+        if (again || (special & ((kRowCountMask << kRowCountBits) | kRowCountMask))) {
+            const int t2 = afresh(t), pair = row_of_thread(a, t2);
+            int first;
+            const int atoms = pair_atoms(a.rows.quad, pair, first);
+            const int mid = a.rows.row_int[pair], end = max(mid, a.rows.row_end[pair]), ghosts = whole_groups<ORDER>(mid);
+            const unsigned* words = a.rows.rows + row_base<ORDER>(static_cast<unsigned>(pair), a.rows.stride);
+            if (again) acc = PairAccumulator<COPIES, ENERGY, SWITCH>();
+            const bool interior = a.phase != DSMD_PHASE_BOUNDARY, boundary = a.phase != DSMD_PHASE_INTERIOR;
+            const int ex_own = special & kRowCountMask, ex_all = ex_own + static_cast<int>((special >> kRowCountBits) & kRowCountMask);
+            const int x0 = interior ? 0 : ex_own, x1 = boundary ? ex_all : ex_own;
+            const int n_own = again && atoms > 1 && interior && !(special & kRowOwnExcluded) ? 2 : 0;
+            const int n_first = interior ? mid : 0, n_second = boundary ? max(end - ghosts, 0) : 0;
+            const int n_care = n_own + (x1 - x0) + (again ? n_first + n_second : 0);
 #pragma unroll 1
-        for (int i = sub; i < n_care; i += lanes) {
-            const int x = i - n_own, k = x - (x1 - x0);
-            unsigned e = static_cast<unsigned>(first + i);
-            if (x >= 0) e = words[row_offset(k < 0 ? a.rows.stride - 1 - (x0 + x) : (k < n_first ? k : ((mid + 3) & ~3) + k - n_first))];
-            int4 pj;
-            float qj = 0.0f;
-            take(e & kIndexMask, pj, qj);
-            acc.template add_partner<true>(p, table, pa, pb, pj, terms(pj.w, qj), e);
+            for (int i = t2 & (lanes - 1); i < n_care; i += lanes) {
+                const int x = i - n_own, k = x - (x1 - x0);
+                unsigned e = static_cast<unsigned>(first + i);
+                if (x >= 0) e = words[row_offset<ORDER>(k < 0 ? a.rows.stride - 1 - (x0 + x) : (k < n_first ? k : ghosts + k - n_first))];
+                int4 pj;
+                float qj = 0.0f;
+                take(e & kIndexMask, pj, qj);
+                acc.template add_partner<true>(p, table, pa, pb, pj, terms(pj.w, qj), e);
+            }
         }
     }
     // Rows with a pair below the Ewald table, one after the other by the whole warp, an entry per lane. A warp has such a row now
     // and then (a box of 648,000 water atoms, started from jittered places, has 15 such pairs), and one lane on its own would keep
     // the others, and in a grid of one round the device, waiting for hundreds of entries: 1.56 ms for that box with the row done
-    // again by its lane, 1.14 this way, 1.53 with a row per atom and a branch per pair. A box without such pairs
-    // takes 1.12 ms (1.11 with the row done again: another schedule of the loop; with per-atom charges it is 1.11 against 1.13,
-    // with energy sums 1.49 against 1.51).
-    // Noting the rows and going over them every 32 rows, or a function that is not inlined: 1.12 to 1.16 and 1.10 to 1.14 ms, and the
-    // parameters by address cost the plain Lennard-Jones form 7 %.
+    // again by its lane, 1.14 this way, when a box without such pairs took 1.12 (1.53 with a row per atom and a branch per pair).
     if (COULOMB)
         for (unsigned todo = __ballot_sync(0xFFFFFFFFu, close && sub == 0); todo; todo &= todo - 1) {
             const int leader = __ffs(todo) - 1;
-            const auto rest = close_rest<COPIES, ENERGY, SWITCH, by_type>(p, a, table, __shfl_sync(0xFFFFFFFFu, pair, leader));
+            const int its_row = row_of_thread(a, afresh(t));
+            const auto rest = close_rest<COPIES, ENERGY, SWITCH, by_type, ORDER>(p, a, table, __shfl_sync(0xFFFFFFFFu, its_row, leader));
             if ((threadIdx.x & 31) == leader) acc.add_sums(rest);
         }
-    if (atoms > 0) {
-        if (ENERGY) acc.take_energies(atoms > 1, v);   // a lone atom's sums are in both lanes
-        acc.take_forces(sum_a, sum_b);
+    if (ENERGY) acc.take_energies(two, v);   // a lone atom's sums are in both lanes; no atom: zeros
+    acc.take_forces(sum_a, sum_b);
+    for (int o = lanes >> 1; o > 0; o >>= 1) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            sum_a[k] += __shfl_xor_sync(0xFFFFFFFFu, sum_a[k], o);
+            sum_b[k] += __shfl_xor_sync(0xFFFFFFFFu, sum_b[k], o);
+        }
     }
 }
 
@@ -460,27 +524,18 @@ __device__ __forceinline__ void row_forces(const PairParams& p, const ForceArgs&
 // the type that arrives with its position, instead of a second gather from global memory.
 // With Coulomb the blocks stay and take further rows in turn, so that the Ewald tables are laid out once per block; with
 // energy sums, so that the last block has few partial sums to add up.
-template <int COPIES, bool ENERGY, int TYPES, bool SWITCH, bool QTYPE>
+template <int COPIES, bool ENERGY, int TYPES, bool SWITCH, bool QTYPE, int ORDER>
 __global__ void __launch_bounds__((kPairThreads<COPIES, TYPES>), (kPairBlocks<COPIES, TYPES, ENERGY>)) k_pair(PairParams p, ForceArgs a) {
     extern __shared__ float4 smem[];
     if (!ENERGY && dsmd::gate_closed(a.st, a.gate2)) return;
     const PairTables<COPIES, ENERGY, TYPES, QTYPE> tables(p, smem);
-    const int lanes = 1 << a.lane_shift;
     double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};   // energy, virial and its diagonal, pairs
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; (t & ~31) >> a.lane_shift < a.n_pairs; t += gridDim.x * blockDim.x) {
-        const int slot = t >> a.lane_shift, sub = t & (lanes - 1);
-        const int pair = slot < a.n_pairs ? (a.pair_list ? a.pair_list[slot] : a.first_pair + slot) : -1;
+        float sum_a[3], sum_b[3];
+        row_forces<COPIES, ENERGY, TYPES, SWITCH, QTYPE, ORDER>(p, a, tables, t, sum_a, sum_b, v);
+        const int t2 = afresh(t), pair = row_of_thread(a, t2), sub = t2 & ((1 << a.lane_shift) - 1);
         int first = 0;
         const int atoms = pair >= 0 ? pair_atoms(a.rows.quad, pair, first) : 0;
-        float sum_a[3] = {0.f, 0.f, 0.f}, sum_b[3] = {0.f, 0.f, 0.f};
-        row_forces<COPIES, ENERGY, TYPES, SWITCH, QTYPE>(p, a, tables, pair, sub, lanes, first, atoms, sum_a, sum_b, v);
-        for (int o = lanes >> 1; o > 0; o >>= 1) {
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                sum_a[k] += __shfl_xor_sync(0xFFFFFFFFu, sum_a[k], o);
-                sum_b[k] += __shfl_xor_sync(0xFFFFFFFFu, sum_b[k], o);
-            }
-        }
         if (sub == 0 && atoms > 0) {
             double* const out[3] = {a.fx, a.fy, a.fz};
 #pragma unroll
@@ -503,28 +558,21 @@ __global__ void __launch_bounds__((kPairThreads<COPIES, TYPES>), (kPairBlocks<CO
 // The force pass of a step and what follows it up to the next force pass, for loops in which nobody reads forces or
 // velocities in between: v += kick f / m, x += dt v, fixed-point positions of the next step (into the other buffer: rows
 // still read this one's), displacement check. A separate pass would read and write the forces and read everything else again
-// (172 bytes per atom, 0.11 ms at 4,000,000 atoms); here the traffic (124 bytes) hides behind the force arithmetic, and a
-// small system's step is one launch.
-template <int TYPES, bool SWITCH>
+// (172 bytes per atom, 0.11 ms at 4,000,000 atoms beside 0.356 for the forces; this kernel 0.455, the blocks' ends being little
+// hidden by other blocks' force arithmetic), and a small system's step is one launch.
+template <int TYPES, bool SWITCH, int ORDER>
 __global__ void __launch_bounds__((kPairThreads<0, TYPES>), (kPairBlocks<0, TYPES, false>))
 k_step(PairParams p, ForceArgs a, Grid g, StepArgs at, DisplacementReport report) {
     extern __shared__ float4 smem[];
     if (dsmd::gate_closed(report.st, report.gate2)) return;
     const PairTables<0, false, TYPES, false> tables(p, smem);
-    const int lanes = 1 << a.lane_shift, t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int pair = t >> a.lane_shift, sub = t & (lanes - 1);
-    int first = 0;
-    const int atoms = pair < a.n_pairs ? pair_atoms(a.rows.quad, pair, first) : 0;
-    float sum_a[3] = {0.f, 0.f, 0.f}, sum_b[3] = {0.f, 0.f, 0.f};
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    float sum_a[3], sum_b[3];
     double unused[6];
-    row_forces<0, false, TYPES, SWITCH, false>(p, a, tables, pair, sub, lanes, first, atoms, sum_a, sum_b, unused);
-    for (int o = lanes >> 1; o > 0; o >>= 1) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            sum_a[k] += __shfl_xor_sync(0xFFFFFFFFu, sum_a[k], o);
-            sum_b[k] += __shfl_xor_sync(0xFFFFFFFFu, sum_b[k], o);
-        }
-    }
+    row_forces<0, false, TYPES, SWITCH, false, ORDER>(p, a, tables, t, sum_a, sum_b, unused);
+    const int t2 = afresh(t), pair = row_of_thread(a, t2), sub = t2 & ((1 << a.lane_shift) - 1);
+    int first = 0;
+    const int atoms = pair >= 0 ? pair_atoms(a.rows.quad, pair, first) : 0;
     // The atoms' turn: an atom per thread, neighbours side by side. (Two atoms by the lanes that hold their sums is four times
     // the instructions where rows have many lanes: 24.5 us per step of 32,000 atoms, 20.7 us this way.)
     __shared__ float s_force[2 * kPairThreads<0, TYPES>][3];
@@ -571,13 +619,13 @@ k_step(PairParams p, ForceArgs a, Grid g, StepArgs at, DisplacementReport report
 
 namespace dsmd {
 
-template <int COPIES, bool ENERGY>
+template <int COPIES, bool ENERGY, int ORDER>
 cudaError_t launch_pair(const PairParams& p, const ForceArgs& a, bool sw, unsigned blocks, cudaStream_t s) {
     const auto launch = [&](auto types, auto switched, auto qtype) {
         constexpr int TYPES = decltype(types)::value;
         constexpr bool SWITCH = decltype(switched)::value, QTYPE = decltype(qtype)::value;
         const size_t smem = PairTables<COPIES, ENERGY, TYPES, QTYPE>::bytes(p.ntypes, p.ewald_intervals);
-        const auto kernel = k_pair<COPIES, ENERGY, TYPES, SWITCH, QTYPE>;
+        const auto kernel = k_pair<COPIES, ENERGY, TYPES, SWITCH, QTYPE, ORDER>;
         if (smem > 48 * 1024) {
             const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
             if (e != cudaSuccess) return e;
@@ -591,8 +639,25 @@ cudaError_t launch_pair(const PairParams& p, const ForceArgs& a, bool sw, unsign
     };
     const auto by_switch = [&](auto types) { return sw ? by_charge(types, std::true_type()) : by_charge(types, std::false_type()); };
     if (p.ntypes == 1) return by_switch(std::integral_constant<int, kOneType>());
+    if (COPIES == 0 && p.ntypes == 2) return by_switch(std::integral_constant<int, COPIES == 0 ? kTwoTypes : kFewTypes>());
     if (p.ntypes <= kFewTypesMost) return by_switch(std::integral_constant<int, kFewTypes>());
     return by_switch(std::integral_constant<int, kManyTypes>());
+}
+
+template <int ORDER>
+cudaError_t launch_step(const PairParams& p, const ForceArgs& a, const Grid& g, const StepArgs& at, const DisplacementReport& report, bool sw,
+                        unsigned blocks, cudaStream_t s) {
+    const auto launch = [&](auto types) {
+        constexpr int TYPES = decltype(types)::value;
+        const size_t smem = PairTables<0, false, TYPES, false>::bytes(p.ntypes, 0);
+        const auto kernel = sw ? k_step<TYPES, true, ORDER> : k_step<TYPES, false, ORDER>;
+        kernel<<<blocks, kPairThreads<0, TYPES>, smem, s>>>(p, a, g, at, report);
+        return cudaGetLastError();
+    };
+    if (p.ntypes == 1) return launch(std::integral_constant<int, kOneType>());
+    if (p.ntypes == 2) return launch(std::integral_constant<int, kTwoTypes>());
+    if (p.ntypes <= kFewTypesMost) return launch(std::integral_constant<int, kFewTypes>());
+    return launch(std::integral_constant<int, kManyTypes>());
 }
 
 }  // namespace dsmd

@@ -79,7 +79,7 @@ struct ExcludedRange {
 // NEAR: the quad is compact against the box, so that the image of a candidate nearest to the first atom is the nearest
 // to all four: one fixed-point difference and conversion per candidate, the other atoms by their float offsets from the
 // first. Otherwise every atom takes its own fixed-point difference (exact for any placement).
-template <bool NEAR, bool EXCL>
+template <bool NEAR, bool EXCL, int ORDER>
 __device__ __forceinline__ void test_candidates(const Grid& g, QuadSearch& q, int n, const int* __restrict__ s_slot,
                                                 const int4* __restrict__ pq, const int* __restrict__ gid, const ExclusionTable& excl,
                                                 const ExcludedRange& s_excluded) {
@@ -146,8 +146,8 @@ __device__ __forceinline__ void test_candidates(const Grid& g, QuadSearch& q, in
                 const unsigned x0 = __ballot_sync(0xFFFFFFFFu, hit0 && flags0), x1 = __ballot_sync(0xFFFFFFFFu, hit1 && flags1);
                 const int p0 = static_cast<int>((q.special0 & kRowCountMask) + __popc(x0 & lt_mask));
                 const int p1 = static_cast<int>((q.special1 & kRowCountMask) + __popc(x1 & lt_mask));
-                if (hit0 && flags0 && p0 < q.stride) q.row0[row_offset(q.stride - 1 - p0)] = static_cast<unsigned>(s) | flags0;
-                if (hit1 && flags1 && p1 < q.stride) q.row1[row_offset(q.stride - 1 - p1)] = static_cast<unsigned>(s) | flags1;
+                if (hit0 && flags0 && p0 < q.stride) q.row0[row_offset<ORDER>(q.stride - 1 - p0)] = static_cast<unsigned>(s) | flags0;
+                if (hit1 && flags1 && p1 < q.stride) q.row1[row_offset<ORDER>(q.stride - 1 - p1)] = static_cast<unsigned>(s) | flags1;
                 q.special0 += __popc(x0);
                 q.special1 += __popc(x1);
                 if (__any_sync(0xFFFFFFFFu, hit0 && flags0 && own0)) q.special0 |= kRowOwnExcluded;
@@ -160,14 +160,14 @@ __device__ __forceinline__ void test_candidates(const Grid& g, QuadSearch& q, in
         hit1 = hit1 && !own1;
         const unsigned m0 = __ballot_sync(0xFFFFFFFFu, hit0), m1 = __ballot_sync(0xFFFFFFFFu, hit1);
         const int k0 = q.count0 + __popc(m0 & lt_mask), k1 = q.count1 + __popc(m1 & lt_mask);
-        if (hit0 && k0 < q.stride) q.row0[row_offset(k0)] = static_cast<unsigned>(s);
-        if (hit1 && k1 < q.stride) q.row1[row_offset(k1)] = static_cast<unsigned>(s);
+        if (hit0 && k0 < q.stride) q.row0[row_offset<ORDER>(k0)] = static_cast<unsigned>(s);
+        if (hit1 && k1 < q.stride) q.row1[row_offset<ORDER>(k1)] = static_cast<unsigned>(s);
         q.count0 += __popc(m0);
         q.count1 += __popc(m1);
     }
 }
 
-template <bool EXCL>
+template <bool EXCL, int ORDER>
 __global__ void __launch_bounds__(kBuildThreads, 8)
 k_build_rows(Grid g, int n_owned, int n_total, int n_quads, const int4* __restrict__ pq, const int* __restrict__ gid,
              ExclusionTable excl, const int* __restrict__ cell_start, const int* __restrict__ ghost_near_lo,
@@ -210,8 +210,8 @@ k_build_rows(Grid g, int n_owned, int n_total, int n_quads, const int4* __restri
     // a pair inside the rounding band is listed whether or not it lies inside the list radius (the export decides in fp64)
     q.hi_band = g.r2_list + g.band_rows;
     q.stride = out.stride;
-    q.row0 = out.rows + row_base(2 * quad, out.stride);
-    q.row1 = q.row0 + 4;   // the rows of a quad are neighbours
+    q.row0 = out.rows + row_base<ORDER>(2 * quad, out.stride);
+    q.row1 = q.row0 + (4 << ORDER);   // the rows of a quad are neighbours
     q.count0 = q.count1 = 0;
     q.special0 = q.special1 = 0u;
     q.far0 = q.far1 = -1;
@@ -335,20 +335,23 @@ k_build_rows(Grid g, int n_owned, int n_total, int n_quads, const int4* __restri
                 for (k = max(k0, len0); k < k1; ++k) to[k] = s1 + (k - len0);
             __syncwarp();
             const int n = min(total - base, kCandidates);
-            if (compact) test_candidates<true, EXCL>(g, q, n, slots, pq, gid, excl, s_excluded);
-            else test_candidates<false, EXCL>(g, q, n, slots, pq, gid, excl, s_excluded);
+            if (compact) test_candidates<true, EXCL, ORDER>(g, q, n, slots, pq, gid, excl, s_excluded);
+            else test_candidates<false, EXCL, ORDER>(g, q, n, slots, pq, gid, excl, s_excluded);
         }
         if (n_atoms <= 2) { q.count1 = 0; q.special1 = 0u; }
         if (seg == 0) { interior0 = q.count0; interior1 = q.count1; interior_special0 = q.special0; interior_special1 = q.special1; }
-        // Fill up the last chunk. Where the search has met no atom to fill it with, the row's own first atom does: the force kernel
+        // Fill up the last group. Where the search has met no atom to fill it with, the row's own first atom does: the force kernel
         // sees r^2 = 0 and counts the row's entries (as it does from the start if no such atom turns up at all: kRowCareful).
-        const int c = lane < 4 ? q.count0 : q.count1, far = lane < 4 ? q.far0 : q.far1;
-        const int k = (c & ~3) + (lane & 3);
-        if (lane < 8 && k >= c && (c & 3) && k < out.stride)
-            (lane < 4 ? q.row0 : q.row1)[row_offset(k)] = static_cast<unsigned>(far < 0 ? q.first + (lane < 4 ? 0 : 2) : far);
+        constexpr int group = 4 << ORDER;
+        static_assert(2 * group <= 32, "a lane per place of the last group of either row");
+        const bool second = lane >= group;
+        const int c = second ? q.count1 : q.count0, far = second ? q.far1 : q.far0;
+        const int k = c / group * group + lane % group;
+        if (lane < 2 * group && k >= c && c % group && k < out.stride)
+            (second ? q.row1 : q.row0)[row_offset<ORDER>(k)] = static_cast<unsigned>(far < 0 ? q.first + (second ? 2 : 0) : far);
         if (seg == 0 && n_seg == 2) {
-            q.count0 = (q.count0 + 3) & ~3;
-            q.count1 = (q.count1 + 3) & ~3;
+            q.count0 = whole_groups<ORDER>(q.count0);
+            q.count1 = whole_groups<ORDER>(q.count1);
         }
     }
     if (lane < 2) {
@@ -356,12 +359,12 @@ k_build_rows(Grid g, int n_owned, int n_total, int n_quads, const int4* __restri
         const unsigned special = lane ? q.special1 : q.special0, special_own = lane ? interior_special1 : interior_special0;
         const unsigned n_special = special & kRowCountMask, n_own = special_own & kRowCountMask;
         // a ghost pass without hits leaves the row as it was
-        const bool ghosts = n_seg == 2 && count > ((interior + 3) & ~3);
+        const bool ghosts = n_seg == 2 && count > whole_groups<ORDER>(interior);
         out.row_end[2 * quad + lane] = min(ghosts ? count : interior, out.stride);
         out.row_int[2 * quad + lane] = min(interior, out.stride);
         out.row_special[2 * quad + lane] = n_own | ((n_special - n_own) << kRowCountBits) | (special & kRowOwnExcluded) |
                                            ((lane ? q.far1 : q.far0) < 0 ? kRowCareful : 0u);
-        const int need = ((count + 3) & ~3) + static_cast<int>(n_special);   // whole chunks, and the ones apart behind them
+        const int need = whole_groups<ORDER>(count) + static_cast<int>(n_special);   // whole groups, and the ones apart behind them
         if (need > out.stride) atomicMax(&st->need_stride, static_cast<unsigned>(need));
         // pairs with a ghost partner, collected for the boundary pass of the force kernel (the order of the collection
         // does not matter: every pair's sums are its own threads')
@@ -376,7 +379,7 @@ k_build_rows(Grid g, int n_owned, int n_total, int n_quads, const int4* __restri
 // A warp per row, an entry per lane for both atoms, rows in turn. What bounds it: scattered reads of the partners' three doubles.
 // 4,000,000 Lennard-Jones atoms: 2.7 ms to count, 2.7 to write (a thread per row 3.5 and 8.3); 3,993 of water 0.05 ms each (1.5).
 constexpr int kMemberThreads = 256;
-template <bool WRITE>
+template <bool WRITE, int ORDER>
 __global__ void __launch_bounds__(kMemberThreads) k_list_members(Grid g, int n_pairs, RowArrays in, const double* __restrict__ x,
                                const double* __restrict__ y, const double* __restrict__ z, unsigned long long* __restrict__ per_atom,
                                unsigned long long* __restrict__ stats, int* __restrict__ out_i, int* __restrict__ out_j,
@@ -392,16 +395,16 @@ __global__ void __launch_bounds__(kMemberThreads) k_list_members(Grid g, int n_p
         const unsigned special = in.row_special[pair];
         const int special_own = special & kRowCountMask, special_all = special_own + ((special >> kRowCountBits) & kRowCountMask);
         const int total = end + special_all + (atoms > 1 && !(special & kRowOwnExcluded) ? 1 : 0);
-        const unsigned* row = in.rows + row_base(static_cast<unsigned>(pair), in.stride);
+        const unsigned* row = in.rows + row_base<ORDER>(static_cast<unsigned>(pair), in.stride);
         const int last = first + atoms - 1;
         const double at_atom[2][3] = {{x[first], y[first], z[first]}, {x[last], y[last], z[last]}};
         unsigned long long at[2] = {WRITE ? per_atom[first] : 0ull, WRITE && atoms > 1 ? per_atom[first + 1] : 0ull};
         for (int base = 0; base < total; base += 32) {
             const int k = base + lane, nth = k - end;   // the entries, then those at the row's end, then the pair's other atom
-            const bool there = k < total && !(k >= mid && k < min((mid + 3) & ~3, end));
+            const bool there = k < total && !(k >= mid && k < min(whole_groups<ORDER>(mid), end));
             const bool other = nth >= special_all;
             const bool owned = nth < 0 ? k < mid : (nth < special_own || other);
-            const unsigned e = !there || other ? 0u : row[row_offset(nth < 0 ? k : in.stride - 1 - nth)];
+            const unsigned e = !there || other ? 0u : row[row_offset<ORDER>(nth < 0 ? k : in.stride - 1 - nth)];
             const int partner = static_cast<int>(e & kIndexMask);
             double pj[3] = {0.0, 0.0, 0.0};
             if (there && !other) { pj[0] = x[partner]; pj[1] = y[partner]; pj[2] = z[partner]; }

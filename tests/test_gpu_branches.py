@@ -9,12 +9,13 @@ from oracle import cpu_oracle as co
 pytestmark = pytest.mark.gpu
 
 
-# atoms, box, cutoff, skin, types, Coulomb, exclusions: lone atoms and two; rows of one to four atoms; one, few and more than
-# eight types; Ewald tables in one copy (short rows) and in eight (rows of 240 and more)
+# atoms, box, cutoff, skin, types, Coulomb, exclusions: lone atoms and two; rows of one to four atoms; one, two, few and more than
+# eight types; Ewald tables in one copy (short rows) and in eight (rows of 240 and more, which have their entries in another order)
 ROWS = [
     (1, 20.0, 4.0, 0.5, 1, False, False), (2, 20.0, 4.0, 0.5, 1, True, False), (37, 20.0, 4.0, 0.5, 3, False, False),
     (333, 20.0, 4.0, 0.5, 8, True, True), (334, 20.0, 4.0, 0.5, 9, True, True), (600, 16.0, 3.0, 0.3, 9, False, True),
-    (2500, 25.0, 6.0, 0.5, 2, True, True), (2500, 25.0, 6.0, 0.5, 1, False, False),
+    (2500, 25.0, 6.0, 0.5, 2, True, True), (2500, 25.0, 6.0, 0.5, 1, False, False), (600, 16.0, 3.0, 0.3, 2, False, True),
+    (2500, 25.0, 6.0, 0.5, 2, False, True), (2503, 25.0, 6.0, 0.5, 9, False, True),
 ]
 
 
@@ -88,6 +89,31 @@ def test_atoms_that_coincide(cuda_device, n, L, rc, nt, coulomb):
     assert abs(got["pe"] - scalars["pe"]) <= 1e-5 * max(abs(scalars["pe"]), 1.0)
     assert got["pairs_in_cutoff"] == scalars["pairs_in_cutoff"]
     ctx.close()
+
+
+@pytest.mark.parametrize("n,rc", [(600, 4.0), (2500, 6.0)])
+def test_charges_switched_on_and_off_under_one_list(cuda_device, n, rc):
+    """The forms with and without Ewald read the rows of a list that either of them was built for (short rows, long rows)."""
+    rng = np.random.default_rng(n)
+    side = int(np.ceil(n ** (1 / 3)))
+    sites = np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij"), -1).reshape(-1, 3)[rng.permutation(side ** 3)[:n]]
+    pos, box, charge = (sites + 0.5 + rng.uniform(-0.2, 0.2, (n, 3))) * (25.0 / side), np.full(3, 25.0), rng.uniform(-0.5, 0.5, n)
+    pairs = co.pairs(*pos.T, n, box, search=rc + 0.5)
+    c6, c12 = co.lj_tables([[0.3]], [[1.0]])
+    for build_with in (False, True):
+        ctx = capi.Context(n)
+        ctx.set_box(box)
+        ctx.set_pair_params([[0.3]], [[1.0]], rc, 0.5)
+        ctx.set_coulomb(build_with)
+        ctx.upload(pos, charge=charge)
+        ctx.build_neighbor_list()
+        for coulomb in (build_with, not build_with, build_with):
+            ctx.set_coulomb(coulomb)
+            ctx.compute_forces()
+            want, _ = co.forces(*pos.T, n, box, pairs, c6, c12, rc, charge=charge, types=np.zeros(n, np.int32), do_coulomb=coulomb,
+                                alpha=co.ewald_alpha(rc) if coulomb else 0.0)
+            assert np.abs(ctx.forces_by_gid(n) - want).max() <= 2e-5 * np.abs(want).max()
+        ctx.close()
 
 
 @pytest.mark.parametrize("free", [False, True])

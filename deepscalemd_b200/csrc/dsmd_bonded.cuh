@@ -49,6 +49,7 @@ constexpr int kNoSlot = 0x7F7F7F7F;   // what a byte-wise fill of the map with 0
 constexpr double kCoulombConstant = 332.0636;   // kcal/mol A / e^2, the reference's constant
 
 __global__ void k_bonded_slot_map(int n_total, const int* __restrict__ gid, int n_global, int* __restrict__ slot_of) {
+    if (!dsmd::after_previous()) return;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n_total) return;
     const int g = gid[s];
@@ -109,11 +110,15 @@ __device__ __forceinline__ void put(double* __restrict__ contrib, int place, dou
 
 // One thread per term, the four kinds one after the other in the index space; a term that is skipped writes zeros.
 // SUMS: also scalars = {PE, W, Wxx, Wyy, Wzz}; not within a loop of steps, where the next evaluation would overwrite them.
+// beside: the launch before is the force kernel, which has waited for all before itself and touches nothing that is read or written
+// here: this kernel runs beside it and waits for its end only when its own work is done, so that whoever waits for this kernel has
+// waited for both. Step of 63,504 chain atoms: 38.7 us, 43.0 one after the other.
 template <bool SUMS>
 __global__ void __launch_bounds__(kBondedThreads) k_bonded_terms(BondedTable t, const double* __restrict__ x, const double* __restrict__ y,
                                const double* __restrict__ z, const double* __restrict__ charge,
                                double* __restrict__ contrib, double* __restrict__ partials, unsigned* __restrict__ ticket,
-                               double* __restrict__ scalars, unsigned* __restrict__ missing) {
+                               double* __restrict__ scalars, unsigned* __restrict__ missing, bool beside) {
+    if (!beside && !dsmd::after_previous()) return;
     const long long id = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     double sums[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
     const long long first_angle = t.n_bonds, first_torsion = first_angle + t.n_angles;
@@ -267,9 +272,11 @@ __global__ void __launch_bounds__(kBondedThreads) k_bonded_terms(BondedTable t, 
         put(contrib, place[1], -f[0], -f[1], -f[2]);
     }
     if (SUMS) sum_over_grid<5>(sums, partials, ticket, scalars, false);
+    if (beside) dsmd::after_previous();
 }
 
 __global__ void k_bonded_gather(int n_owned, BondedForces b, double* __restrict__ fx, double* __restrict__ fy, double* __restrict__ fz) {
+    if (!dsmd::after_previous()) return;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n_owned) return;
     double f[3];

@@ -42,7 +42,7 @@ struct Grid {
 struct Status {
     unsigned int need_stride;      // largest neighbour count seen (list rows that overflowed)
     unsigned int out_of_domain;    // atoms outside the mapped range or NaN
-    unsigned int unused;
+    unsigned int sort_outside;     // atoms outside the mapped range or NaN, as the sort of a list build found them
     unsigned int timeout;
     unsigned long long max_disp2;  // bits of the largest squared displacement (double, non-negative)
     unsigned long long select_count;

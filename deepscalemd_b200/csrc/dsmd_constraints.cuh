@@ -46,6 +46,7 @@ __device__ __forceinline__ void half_box_image(double d[3], const ClusterTable& 
 }
 
 __global__ void k_slot_of_gid(int n, const int* __restrict__ gid, int n_global, int* __restrict__ slot_of) {
+    if (!dsmd::after_previous()) return;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const int g = gid[s];
@@ -53,6 +54,7 @@ __global__ void k_slot_of_gid(int n, const int* __restrict__ gid, int n_global, 
 }
 
 __global__ void k_cluster_slots(int n, const int* __restrict__ atom_gid, const int* __restrict__ slot_of_gid, int* __restrict__ slot) {
+    if (!dsmd::after_previous()) return;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k < n) slot[k] = atom_gid[k] < 0 ? -1 : slot_of_gid[atom_gid[k]];
 }
@@ -283,6 +285,7 @@ template <class Shape, bool FINISH, bool START>
 __global__ void __launch_bounds__(128) k_constrained(ClusterTable t, Grid g, AtomArrays at, double half_kick, double dt, double tolerance,
                                                      int max_iterations, double prefactor, double* __restrict__ partials, unsigned* __restrict__ ticket,
                                                      double* __restrict__ virial, DisplacementReport report) {
+    if (!dsmd::after_previous()) return;
     if (START && dsmd::gate_closed(report.st, report.gate2)) return;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     double wsum[3] = {0.0, 0.0, 0.0}, worst2 = 0.0;

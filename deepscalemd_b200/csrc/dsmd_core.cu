@@ -23,6 +23,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -30,7 +31,9 @@
 #include "dsmd_cells.cuh"
 #include "dsmd_common.cuh"
 #include "dsmd_force.cuh"
+#include "dsmd_launch.cuh"
 #include "dsmd_report.cuh"
+#include "dsmd_scan.cuh"
 #include "dsmd_sums.cuh"
 #include "ewald_table.hpp"
 
@@ -89,6 +92,7 @@ struct Brick {
 // Cells are numbered [0, ncells) for owned atoms, [ncells, 2 ncells) for ghosts; atoms to be removed (only in a sort without
 // ghosts) count as cell ncells, behind every other.
 __global__ void k_cell_begin(int cells, int* __restrict__ cell_count, Status* st) {   // st: to be cleared as well, or null
+    if (!dsmd::after_previous()) return;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < cells; k += gridDim.x * blockDim.x) cell_count[k] = 0;
     if (st && blockIdx.x == 0 && threadIdx.x == 0) *st = Status{};
 }
@@ -96,6 +100,7 @@ __global__ void k_cell_begin(int cells, int* __restrict__ cell_count, Status* st
 __global__ void k_cell_keys(Grid g, Brick brick, int first, int n_owned, int n_total, const double* __restrict__ x,
                             const double* __restrict__ y, const double* __restrict__ z, unsigned* __restrict__ key,
                             int* __restrict__ arrival, int* __restrict__ cell_count, Status* st) {
+    if (!dsmd::after_previous()) return;
     const int s = first + blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n_total) return;
     const double p[3] = {x[s], y[s], z[s]};
@@ -103,7 +108,7 @@ __global__ void k_cell_keys(Grid g, Brick brick, int first, int n_owned, int n_t
     const unsigned fx = dsmd::to_fixed(p[0], 0, g, bad);
     const unsigned fy = dsmd::to_fixed(p[1], 1, g, bad);
     const unsigned fz = dsmd::to_fixed(p[2], 2, g, bad);
-    if (bad) atomicAdd(&st->out_of_domain, 1u);
+    if (bad) atomicAdd(&st->sort_outside, 1u);
     const unsigned cx = dsmd::cell_of(fx, g.wrap[0], g.nc[0]);
     const unsigned cy = dsmd::cell_of(fy, g.wrap[1], g.nc[1]);
     const unsigned cz = dsmd::cell_of(fz, g.wrap[2], g.nc[2]);
@@ -131,6 +136,7 @@ __global__ void k_reorder(Grid g, int first, int n_owned, int n_total, unsigned 
                           const int* __restrict__ gid_src, int* __restrict__ type_dst, int* __restrict__ gid_dst,
                           int4* __restrict__ pq, float* __restrict__ qf, double* __restrict__ xref,
                           double* __restrict__ yref, double* __restrict__ zref, int* __restrict__ ghost_slot) {
+    if (!dsmd::after_previous()) return;
     const int t = first + blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n_total) return;
     const int from = list[t];
@@ -167,6 +173,7 @@ __global__ void k_reorder(Grid g, int first, int n_owned, int n_total, unsigned 
 // (already in place) need not be copied across: one thread per ghost, all per-atom arrays.
 __global__ void k_copy_back(int first, int count, RealArrays from, RealArrays to, const int* __restrict__ type_from,
                             const int* __restrict__ gid_from, int* __restrict__ type_to, int* __restrict__ gid_to) {
+    if (!dsmd::after_previous()) return;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= count) return;
     const int s = first + t;
@@ -176,12 +183,22 @@ __global__ void k_copy_back(int first, int count, RealArrays from, RealArrays to
     gid_to[s] = gid_from[s];
 }
 
-// The end of a list build: its status goes to the host (out_of_domain, dropped, need_stride, boundary_pairs) and, unless the
-// host is going to report an error, starts again at zero, the displacement word with it.
-__global__ void k_build_done(Status* st, unsigned expect_dropped, Mail* mail, unsigned long long seq) {
-    const double out[4] = {static_cast<double>(st->out_of_domain), static_cast<double>(st->dropped), static_cast<double>(st->need_stride),
+// The end of a list build: its status goes to the host (atoms outside, dropped, need_stride, boundary_pairs), and the status words
+// start again at zero, the displacement word with them; or, where the host is going to report an error, keep what it says.
+// A build that failed, or has to be done again with longer rows, closes the gate of the launches queued behind it.
+__global__ void k_build_done(Status* st, unsigned expect_dropped, unsigned stride, Mail* mail, unsigned long long seq) {
+    if (!dsmd::after_previous()) return;
+    const double out[4] = {static_cast<double>(st->sort_outside), static_cast<double>(st->dropped), static_cast<double>(st->need_stride),
                            static_cast<double>(st->boundary_pairs)};
-    if (st->out_of_domain == 0u && st->dropped == expect_dropped) *st = Status{};
+    Status next{};
+    if (st->sort_outside != 0u || st->dropped != expect_dropped) {
+        next = *st;
+        next.out_of_domain = next.sort_outside;
+        next.max_disp2 = 0ull;
+        next.constraint_failed = 0u;
+    }
+    if (st->sort_outside != 0u || st->dropped != expect_dropped || st->need_stride > stride) next.gate = __longlong_as_double(0x7FF0000000000000ll);
+    *st = next;
     post(mail, out, 4, seq);
 }
 
@@ -189,6 +206,7 @@ __global__ void k_build_done(Status* st, unsigned expect_dropped, Mail* mail, un
 // none), hi_begin = the first x cell of its upper half that holds one (nc[0]: none). One warp per (y, z) row.
 __global__ void k_ghost_row_extent(Grid g, const int* __restrict__ ghost_cell_start, int* __restrict__ lo_end,
                                    int* __restrict__ hi_begin) {
+    if (!dsmd::after_previous()) return;
     const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (row >= g.nc[1] * g.nc[2]) return;
@@ -213,6 +231,7 @@ __global__ void k_ghost_row_extent(Grid g, const int* __restrict__ ghost_cell_st
 // pass of the list build altogether.
 __global__ void k_ghost_rows_near(Grid g, const int* __restrict__ lo_end, const int* __restrict__ hi_begin,
                                   int* __restrict__ near_lo, int* __restrict__ near_hi) {
+    if (!dsmd::after_previous()) return;
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
     if (row >= g.nc[1] * g.nc[2]) return;
     const int yc0 = row % g.nc[1], zc0 = row / g.nc[1];
@@ -269,6 +288,7 @@ struct ClusterMembers {
 __global__ void k_vv2(int n, double half_dt_c, double* __restrict__ vx, double* __restrict__ vy,
                       double* __restrict__ vz, const double* __restrict__ fx, const double* __restrict__ fy,
                       const double* __restrict__ fz, const double* __restrict__ mass, ClusterMembers skip) {
+    if (!dsmd::after_previous()) return;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n || skip.has(s)) return;
     const double a = half_dt_c / mass[s];
@@ -280,6 +300,7 @@ __global__ void k_vv2(int n, double half_dt_c, double* __restrict__ vx, double* 
 // What an upload leaves out: zero velocities, forces and charges, unit masses, type 0, ids in order (null: given by the
 // caller).
 __global__ void k_upload_defaults(int n, RealArrays r, int* type, int* gid) {
+    if (!dsmd::after_previous()) return;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
 #pragma unroll
@@ -291,6 +312,7 @@ __global__ void k_upload_defaults(int n, RealArrays r, int* type, int* gid) {
 
 // [n][3] rows, read from pinned host memory, to three arrays.
 __global__ void k_split_rows(int n, const double* __restrict__ rows, double* __restrict__ x, double* __restrict__ y, double* __restrict__ z) {
+    if (!dsmd::after_previous()) return;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < 3 * n; k += gridDim.x * blockDim.x) {
         const int s = k / 3, a = k - 3 * s;
         (a == 0 ? x : (a == 1 ? y : z))[s] = rows[k];
@@ -301,6 +323,7 @@ __global__ void k_split_rows(int n, const double* __restrict__ rows, double* __r
 // src/thermostat_kernels.cu:68-76): v *= factor.
 __global__ void k_scale_velocities(int n, double factor, double* __restrict__ vx, double* __restrict__ vy,
                                    double* __restrict__ vz) {
+    if (!dsmd::after_previous()) return;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     vx[s] *= factor;
@@ -311,6 +334,7 @@ __global__ void k_scale_velocities(int n, double factor, double* __restrict__ vx
 __global__ void k_kinetic(int n, const double* __restrict__ vx, const double* __restrict__ vy,
                           const double* __restrict__ vz, const double* __restrict__ mass, double* partials, unsigned* ticket,
                           double* out, Mail* mail, unsigned long long seq) {
+    if (!dsmd::after_previous()) return;
     double v[1] = {0.0};
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x)
         v[0] += 0.5 * mass[s] * (vx[s] * vx[s] + vy[s] * vy[s] + vz[s] * vz[s]);
@@ -338,6 +362,7 @@ __global__ void k_pack(Grid g, int first, int count, int n_owned, double* __rest
                        const double* __restrict__ xref, const double* __restrict__ yref,
                        const double* __restrict__ zref, int4* __restrict__ pq, double dt, double kick_c,
                        ClusterMembers skip, BondedForces bonded, DisplacementReport report) {
+    if (!dsmd::after_previous()) return;
     if (dsmd::gate_closed(report.st, report.gate2)) return;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int s = first + t;
@@ -521,6 +546,9 @@ struct dsmd_ctx {
     int* arrival = nullptr;        // its place among the atoms of the cell as they came
     int* list = nullptr;           // the cells' atoms as they came
     int* cell_count = nullptr;
+    bool counts_zero = false;      // the counts are zero, as every sort leaves them
+    bool sort_words_zero = false;  // the status words that a sort counts in are zero, as every list build leaves them
+    int* scan_sums = nullptr;      // [kScanBlocksMost]
     int* ghost_slot = nullptr;
     // the host-buffer force call as a pipeline (dsmd_forces_host): first slot of every z layer of cells as of the last
     // build, two copy streams, one event pair per piece
@@ -762,6 +790,7 @@ int ensure_cells(dsmd_ctx* c) {
         c->cell_start = c->cell_count = nullptr;
         DSMD_CUDA(c, cudaMalloc(&c->cell_start, sizeof(int) * need));
         DSMD_CUDA(c, cudaMalloc(&c->cell_count, sizeof(int) * need));
+        c->counts_zero = false;
         c->cell_capacity = need;
     }
     return DSMD_OK;
@@ -861,47 +890,74 @@ int ensure_partials(dsmd_ctx* c, int64_t blocks) {
     return DSMD_OK;
 }
 
+// What a sort does about the status words.
+enum class StatusWords {
+    kClear,       // all of them to zero, first
+    kAreZero,     // those that the sort counts in are zero since the last list build, the others are nobody's concern until the build's end
+    kKeep,        // a sort before this one has counted in them
+};
+
 // Sorts slots [first, n_total) by cell and gathers everything into the other buffer set. bounds (owned-only sorts): atoms
-// outside the brick sort behind every cell and fall off the end.
-int sort_range(dsmd_ctx* c, int64_t first, cudaStream_t s, bool clear, const Brick* bounds = nullptr, bool forces = true) {
+// outside the brick sort behind every cell and fall off the end. quads: to be worked out as well, or null.
+int sort_range(dsmd_ctx* c, int64_t first, cudaStream_t s, StatusWords words, const Brick* bounds = nullptr, bool forces = true,
+               const QuadArgs* quads = nullptr) {
     const int64_t n = c->n_total - first;
     const int from = c->cur, to = 1 - c->cur;
-    if (clear) c->disp_seq = 0;   // reports of displacement checks are void
+    if (words != StatusWords::kKeep) c->disp_seq = 0;   // reports of displacement checks are void
+    const bool clear = words == StatusWords::kClear || (words == StatusWords::kAreZero && !c->sort_words_zero);
+    c->sort_words_zero = false;
+    const unsigned quad_blocks = quads ? blocks_for(static_cast<int64_t>(quads->rows) * 32, kThreads) : 0;
     if (n > 0) {
         Brick brick{};
         if (bounds) { brick = *bounds; brick.drop = 1; }
         const int in = static_cast<int>(c->n_total), i0 = static_cast<int>(first);
         // cells this sort is about: the owned ones, the ghosts', or both; and one behind them
         const int cell0 = first > 0 ? c->grid.ncells : 0, cells = (c->n_total > c->n_owned ? 2 : 1) * c->grid.ncells + 2 - cell0;
-        k_cell_begin<<<std::min<unsigned>(blocks_for(cells, kThreads), kDeviceSms * 8), kThreads, 0, s>>>(cells, c->cell_count + cell0,
-                                                                                                        clear ? c->status : nullptr);
+        if (!c->counts_zero || clear) {
+            const int all = c->counts_zero ? 0 : static_cast<int>(c->cell_capacity);
+            dsmd::launch_next(k_cell_begin, std::min<unsigned>(blocks_for(std::max(all, 1), kThreads), kDeviceSms * 8), kThreads, 0, s, all,
+                              c->cell_count, clear ? c->status : nullptr);
+            DSMD_LAUNCHED(c);
+        }
+        c->counts_zero = false;
+        dsmd::launch_next(k_cell_keys, blocks_for(n, kThreads), kThreads, 0, s, c->grid, brick, i0, static_cast<int>(c->n_owned), in,
+                          c->real[from][0], c->real[from][1], c->real[from][2], c->key, c->arrival, c->cell_count, c->status);
         DSMD_LAUNCHED(c);
-        k_cell_keys<<<blocks_for(n, kThreads), kThreads, 0, s>>>(
-            c->grid, brick, i0, static_cast<int>(c->n_owned), in, c->real[from][0], c->real[from][1], c->real[from][2], c->key,
-            c->arrival, c->cell_count, c->status);
+        if (cells <= dsmd::kScanMost) {
+            const int launched = dsmd::launch_cell_scan(cells, i0, c->cell_count + cell0, c->scan_sums, c->cell_start + cell0, s);
+            if (launched == 2) ++c->launches;
+            DSMD_LAUNCHED(c);
+        } else {
+            size_t need = 0;
+            cub::DeviceScan::ExclusiveScan(nullptr, need, c->cell_count, c->cell_start, cuda::std::plus<int>(), i0, cells, s);
+            { const int rc = ensure_cub_temp(c, need); if (rc) return rc; }
+            DSMD_CUDA(c, cub::DeviceScan::ExclusiveScan(c->cub_temp, need, c->cell_count + cell0, c->cell_start + cell0,
+                                                        cuda::std::plus<int>(), i0, cells, s));
+        }
+        const unsigned place_blocks = blocks_for(n, kThreads);
+        dsmd::launch_next(k_place, place_blocks + quad_blocks, kThreads, 0, s, static_cast<int>(place_blocks), i0, in, c->key, c->arrival, c->cell_start,
+                          c->list, cells, c->cell_count + cell0, quads ? *quads : QuadArgs{});
         DSMD_LAUNCHED(c);
-        size_t need = 0;
-        cub::DeviceScan::ExclusiveScan(nullptr, need, c->cell_count, c->cell_start, cuda::std::plus<int>(), i0, cells, s);
-        { const int rc = ensure_cub_temp(c, need); if (rc) return rc; }
-        DSMD_CUDA(c, cub::DeviceScan::ExclusiveScan(c->cub_temp, need, c->cell_count + cell0, c->cell_start + cell0,
-                                                    cuda::std::plus<int>(), i0, cells, s));
-        dsmd::k_cell_place<<<blocks_for(n, kThreads), kThreads, 0, s>>>(i0, in, c->key, c->arrival, c->cell_start, c->list);
-        DSMD_LAUNCHED(c);
+        c->counts_zero = true;
         const auto reorder = forces ? k_reorder<true> : k_reorder<false>;
-        reorder<<<blocks_for(n, kThreads), kThreads, 0, s>>>(
-            c->grid, i0, static_cast<int>(c->n_owned), in, brick.drop ? static_cast<unsigned>(c->grid.ncells) : 0xFFFFFFFFu, c->key, c->list, c->cell_start, arrays_of(c, from), arrays_of(c, to),
-            c->type[from], c->gid[from], c->type[to], c->gid[to], c->pq, c->qf, c->ref[0], c->ref[1], c->ref[2], c->ghost_slot);
+        dsmd::launch_next(reorder, blocks_for(n, kThreads), kThreads, 0, s, c->grid, i0, static_cast<int>(c->n_owned), in,
+                          brick.drop ? static_cast<unsigned>(c->grid.ncells) : 0xFFFFFFFFu, c->key, c->list, c->cell_start, arrays_of(c, from),
+                          arrays_of(c, to), c->type[from], c->gid[from], c->type[to], c->gid[to], c->pq, c->qf, c->ref[0], c->ref[1], c->ref[2],
+                          c->ghost_slot);
         DSMD_LAUNCHED(c);
-    } else if (clear) {
-        DSMD_CUDA(c, cudaMemsetAsync(c->status, 0, sizeof(Status), s));
+    } else {
+        if (clear) DSMD_CUDA(c, cudaMemsetAsync(c->status, 0, sizeof(Status), s));
+        if (quads) {
+            dsmd::launch_next(k_place, quad_blocks, kThreads, 0, s, 0, 0, 0, c->key, c->arrival, c->cell_start, c->list, 0, c->cell_count, *quads);
+            DSMD_LAUNCHED(c);
+        }
     }
     if (first > 0) {
         // a ghost-only sort: the owned atoms are in place in the current set, the sorted ghosts come back to it (far
         // fewer bytes than carrying the owned atoms across, and one launch instead of thirteen copies)
         if (n > 0) {
-            k_copy_back<<<blocks_for(n, kThreads), kThreads, 0, s>>>(static_cast<int>(first), static_cast<int>(n),
-                                                                    arrays_of(c, to), arrays_of(c, from), c->type[to],
-                                                                    c->gid[to], c->type[from], c->gid[from]);
+            dsmd::launch_next(k_copy_back, blocks_for(n, kThreads), kThreads, 0, s, static_cast<int>(first), static_cast<int>(n),
+                              arrays_of(c, to), arrays_of(c, from), c->type[to], c->gid[to], c->type[from], c->gid[from]);
             DSMD_LAUNCHED(c);
         }
     } else {
@@ -970,6 +1026,7 @@ int dsmd_create(int device, int64_t capacity, dsmd_ctx** out) {
     DSMD_CUDA(c, cudaMalloc(&c->key, sizeof(unsigned) * capacity));
     DSMD_CUDA(c, cudaMalloc(&c->arrival, sizeof(int) * capacity));
     DSMD_CUDA(c, cudaMalloc(&c->list, sizeof(int) * capacity));
+    DSMD_CUDA(c, cudaMalloc(&c->scan_sums, sizeof(int) * dsmd::kScanBlocksMost));
     DSMD_CUDA(c, cudaMalloc(&c->qf, sizeof(float) * capacity));
     for (int a = 0; a < 3; ++a) DSMD_CUDA(c, cudaMalloc(&c->ref[a], sizeof(double) * capacity));
     DSMD_CUDA(c, cudaMalloc(&c->ghost_slot, sizeof(int) * capacity));
@@ -1001,7 +1058,7 @@ void dsmd_destroy(dsmd_ctx* c) {
         for (int f = 0; f < kNumReal; ++f) cudaFree(c->real[set][f]);
         cudaFree(c->type[set]); cudaFree(c->gid[set]); 
     }
-    cudaFree(c->pq); cudaFree(c->pq_next); cudaFree(c->key); cudaFree(c->arrival); cudaFree(c->list); cudaFree(c->cell_count); cudaFree(c->qf); cudaFree(c->type_charge);
+    cudaFree(c->pq); cudaFree(c->pq_next); cudaFree(c->key); cudaFree(c->arrival); cudaFree(c->list); cudaFree(c->scan_sums); cudaFree(c->cell_count); cudaFree(c->qf); cudaFree(c->type_charge);
     for (int a = 0; a < 3; ++a) cudaFree(c->ref[a]);
     cudaFree(c->ghost_slot); cudaFree(c->cell_start); cudaFree(c->ghost_rows);
     cudaFree(c->rows); cudaFree(c->quad); cudaFree(c->row_end); cudaFree(c->row_int); cudaFree(c->row_special); cudaFree(c->boundary_pairs);
@@ -1143,7 +1200,7 @@ static int upload_rest(dsmd_ctx* c, int64_t n_owned, int64_t n_total, const doub
     if (type) DSMD_CUDA(c, cudaMemcpyAsync(c->type[c->cur], type, sizeof(int) * n_total, cudaMemcpyHostToDevice, s));
     if (gid) DSMD_CUDA(c, cudaMemcpyAsync(c->gid[c->cur], gid, sizeof(int) * n_total, cudaMemcpyHostToDevice, s));
     if (n_total > 0) {
-        k_upload_defaults<<<blocks_for(n_total, kThreads), kThreads, 0, s>>>(static_cast<int>(n_total), missing, type ? nullptr : c->type[c->cur],
+        dsmd::launch_next(k_upload_defaults, blocks_for(n_total, kThreads), kThreads, 0, s, static_cast<int>(n_total), missing, type ? nullptr : c->type[c->cur],
                                                                             gid ? nullptr : c->gid[c->cur]);
         DSMD_LAUNCHED(c);
     }
@@ -1179,7 +1236,7 @@ static int upload_columns(dsmd_ctx* c, const double* rows, int64_t n, double* co
             DSMD_CUDA(c, cudaEventSynchronize(c->stage_free[b]));
         }
         std::memcpy(c->stage[b], rows + 3 * first, sizeof(double) * 3 * m);
-        k_split_rows<<<std::min<unsigned>(blocks_for(3 * m, kThreads), kDeviceSms), kThreads, 0, s>>>(m, c->stage[b], to[0] + first, to[1] + first,
+        dsmd::launch_next(k_split_rows, std::min<unsigned>(blocks_for(3 * m, kThreads), kDeviceSms), kThreads, 0, s, m, c->stage[b], to[0] + first, to[1] + first,
                                                                                                   to[2] + first);
         DSMD_LAUNCHED(c);
         DSMD_CUDA(c, cudaEventRecord(c->stage_free[b], s));
@@ -1251,7 +1308,7 @@ static int sort_owned_impl(dsmd_ctx* c, const Brick* bounds, int64_t n_outside, 
     { const int rc = ensure_cells(c); if (rc) return rc; }
     const int64_t keep_total = c->n_total;
     c->n_total = c->n_owned;   // sort the owned segment alone
-    const int rc = sort_range(c, 0, s, true, n_outside > 0 ? bounds : nullptr);
+    const int rc = sort_range(c, 0, s, StatusWords::kClear, n_outside > 0 ? bounds : nullptr);
     c->n_total = keep_total;
     if (rc) return rc;
     c->n_owned -= n_outside;
@@ -1261,7 +1318,7 @@ static int sort_owned_impl(dsmd_ctx* c, const Brick* bounds, int64_t n_outside, 
     c->expect_dropped = n_outside;
     if (!check_now) return DSMD_OK;   // the status words stay and are read with the list build's
     { const int rc2 = read_status(c, s); if (rc2) return rc2; }
-    if (c->h_status->out_of_domain)
+    if (c->h_status->sort_outside)
         return fail(c, DSMD_ERR_OUT_OF_DOMAIN, "an atom lies outside the subdomain + halo, or has a NaN position");
     if (c->h_status->dropped != static_cast<unsigned>(n_outside))
         return fail(c, DSMD_ERR_STATE, "sort: the number of atoms outside the brick differs from the caller's count");
@@ -1285,21 +1342,16 @@ int dsmd_sort_owned_in_brick(dsmd_ctx* c, const double lo[3], const double hi[3]
     return sort_owned_impl(c, &bounds, n_outside, false, static_cast<cudaStream_t>(stream));
 }
 
-// forces: the force arrays move with the atoms.
-static int build_list(dsmd_ctx* c, bool forces, cudaStream_t s) {
+// forces: the force arrays move with the atoms. queue_next (or null): called once everything is launched and before the host waits for the
+// build's report; what it launches must do nothing behind a closed gate. If the build has to be done again, or fails, the gate
+// was closed, and it is called again, or take_back instead.
+static int build_list(dsmd_ctx* c, bool forces, cudaStream_t s, const std::function<int()>& queue_next = nullptr,
+                      const std::function<void()>& take_back = nullptr) {
     DSMD_CUDA(c, cudaSetDevice(c->device));
     if (c->n_owned <= 0) return fail(c, DSMD_ERR_STATE, "no atoms uploaded");
     if (!c->grid_valid) { const int rc = make_grid(c); if (rc) return rc; }
     { const int rc = ensure_cells(c); if (rc) return rc; }
-    // 1. bin + sort + reorder (everything, or only the ghosts when the owned segment was sorted just before: the
-    //    status words of that sort are then still unread and are kept)
-    const int64_t first = c->owned_sorted_only ? c->n_owned : 0;
-    const int64_t expect_dropped = c->owned_sorted_only ? c->expect_dropped : 0;
-    const bool clear = !c->owned_sorted_only;
-    c->owned_sorted_only = false;
-    c->expect_dropped = 0;
-    if (first == 0 || c->n_total > first) { const int rc = sort_range(c, first, s, clear, nullptr, forces); if (rc) return rc; }
-    // 2. list rows
+    // what the list needs room for
     int row_entries = c->stride;
     if (c->stride == 0) {
         double volume = 1.0;
@@ -1318,7 +1370,7 @@ static int build_list(dsmd_ctx* c, bool forces, cudaStream_t s) {
         DSMD_CUDA(c, cudaMalloc(&c->ghost_rows, sizeof(int) * 4 * rows));
         c->ghost_rows_capacity = 4 * rows;
     }
-    {   // slab boundaries for the pipelined host-buffer call; k_quads writes them
+    {   // slab boundaries for the pipelined host-buffer call; written with the quads
         const int layers = c->grid.nc[2];
         if (layers + 1 > c->layer_capacity) {
             if (c->h_layer_start) cudaFreeHost(c->h_layer_start);
@@ -1328,47 +1380,63 @@ static int build_list(dsmd_ctx* c, bool forces, cudaStream_t s) {
             c->layer_capacity = layers + 1;
         }
     }
+    { const int rc = lay_out_rows(c, row_entries); if (rc) return rc; }
+    // 1. bin + sort + reorder (everything, or only the ghosts when the owned segment was sorted just before: the
+    //    status words of that sort are then still unread and are kept), and the quads
+    const int64_t first = c->owned_sorted_only ? c->n_owned : 0;
+    const int64_t expect_dropped = c->owned_sorted_only ? c->expect_dropped : 0;
+    const StatusWords words = c->owned_sorted_only ? StatusWords::kKeep : StatusWords::kAreZero;
+    c->owned_sorted_only = false;
+    c->expect_dropped = 0;
+    c->layer_tag = static_cast<unsigned>(++c->seq);
+    const QuadArgs quads{c->grid.nc[0], c->grid.nc[1], static_cast<int>(rows), static_cast<int>(c->n_owned), c->quad, c->h_layer_start, c->layer_tag};
+    { const int rc = sort_range(c, first, s, words, nullptr, forces, &quads); if (rc) return rc; }
+    // 2. list rows
     if (c->n_total > c->n_owned) {
-        k_ghost_row_extent<<<blocks_for(rows * 32, kThreads), kThreads, 0, s>>>(c->grid, c->cell_start + c->grid.ncells,
-                                                                               c->ghost_rows, c->ghost_rows + rows);
+        dsmd::launch_next(k_ghost_row_extent, blocks_for(rows * 32, kThreads), kThreads, 0, s, c->grid, c->cell_start + c->grid.ncells, c->ghost_rows,
+                          c->ghost_rows + rows);
         DSMD_LAUNCHED(c);
-        k_ghost_rows_near<<<blocks_for(rows, kThreads), kThreads, 0, s>>>(c->grid, c->ghost_rows, c->ghost_rows + rows,
-                                                                         c->ghost_rows + 2 * rows, c->ghost_rows + 3 * rows);
+        dsmd::launch_next(k_ghost_rows_near, blocks_for(rows, kThreads), kThreads, 0, s, c->grid, c->ghost_rows, c->ghost_rows + rows,
+                          c->ghost_rows + 2 * rows, c->ghost_rows + 3 * rows);
         DSMD_LAUNCHED(c);
     }
+    const bool was_valid = c->list_valid;
+    const auto failed = [&](int rc) {
+        c->list_valid = was_valid;
+        return rc;
+    };
     for (int attempt = 0; attempt < 4; ++attempt) {
-        { const int rc = lay_out_rows(c, row_entries); if (rc) return rc; }
+        if (attempt > 0) { const int rc = lay_out_rows(c, row_entries); if (rc) return failed(rc); }
         const ExclusionTable ex{c->excl_off, c->excl_partner, static_cast<int>(c->excl_n_global)};
-        if (attempt == 0) {
-            c->layer_tag = static_cast<unsigned>(++c->seq);
-            k_quads<<<blocks_for(rows * 32, kThreads), kThreads, 0, s>>>(c->grid.nc[0], c->grid.nc[1], static_cast<int>(rows),
-                                                                        static_cast<int>(c->n_owned), c->cell_start, c->quad, c->h_layer_start, c->layer_tag);
-            DSMD_LAUNCHED(c);
-        }
         const unsigned blocks = blocks_for(c->n_quads * 32, kBuildThreads);
         const auto build = ex.offsets ? (long_rows(c) ? k_build_rows<true, kLongOrder> : k_build_rows<true, 0>)
                                       : (long_rows(c) ? k_build_rows<false, kLongOrder> : k_build_rows<false, 0>);
-        build<<<blocks, kBuildThreads, 0, s>>>(c->grid, static_cast<int>(c->n_owned), static_cast<int>(c->n_total), static_cast<int>(c->n_quads),
-                                               c->pq, c->gid[c->cur], ex, c->cell_start, c->ghost_rows + 2 * rows, c->ghost_rows + 3 * rows,
-                                               rows_of(c), c->boundary_pairs, c->status);
+        dsmd::launch_next(build, blocks, kBuildThreads, 0, s, c->grid, static_cast<int>(c->n_owned), static_cast<int>(c->n_total),
+                          static_cast<int>(c->n_quads), c->pq, c->gid[c->cur], ex, c->cell_start, c->ghost_rows + 2 * rows, c->ghost_rows + 3 * rows,
+                          rows_of(c), c->boundary_pairs, c->status);
         DSMD_LAUNCHED(c);
-        k_build_done<<<1, 1, 0, s>>>(c->status, attempt == 0 ? static_cast<unsigned>(expect_dropped) : 0u, c->mail + kMailBuild, ++c->seq);
+        const unsigned long long seq = ++c->seq;
+        dsmd::launch_next(k_build_done, 1, 1, 0, s, c->status, attempt == 0 ? static_cast<unsigned>(expect_dropped) : 0u, static_cast<unsigned>(c->stride),
+                          c->mail + kMailBuild, seq);
         DSMD_LAUNCHED(c);
-        { const int rc = wait_mail(c, kMailBuild, 4, c->seq, s); if (rc) return rc; }
-        const Mail& report = c->mail[kMailBuild];
         c->disp_seq = 0;   // the displacement word starts again at zero
-        if (report.value(0) != 0.0)
-            return fail(c, DSMD_ERR_OUT_OF_DOMAIN, "an atom lies outside the subdomain + halo, or has a NaN position");
-        if (attempt == 0 && report.value(1) != static_cast<double>(expect_dropped))
-            return fail(c, DSMD_ERR_STATE, "sort: the number of atoms outside the brick differs from the caller's count");
+        ++c->build_epoch;
+        c->list_valid = true;
+        if (queue_next) { const int rc = queue_next(); if (rc) return rc; }
+        { const int rc = wait_mail(c, kMailBuild, 4, seq, s); if (rc) return failed(rc); }
+        const Mail& report = c->mail[kMailBuild];
+        const bool outside = report.value(0) != 0.0, miscounted = attempt == 0 && report.value(1) != static_cast<double>(expect_dropped);
+        const bool overflowed = report.value(2) > c->stride;
+        if ((outside || miscounted || overflowed) && take_back) take_back();
+        if (outside) return failed(fail(c, DSMD_ERR_OUT_OF_DOMAIN, "an atom lies outside the subdomain + halo, or has a NaN position"));
+        if (miscounted) return failed(fail(c, DSMD_ERR_STATE, "sort: the number of atoms outside the brick differs from the caller's count"));
         c->n_boundary = static_cast<int64_t>(report.value(3));
-        if (report.value(2) <= c->stride) break;
+        c->sort_words_zero = true;
+        if (!overflowed) break;
         // a row overflowed: grow and build again
         row_entries = static_cast<int>(report.value(2) * 1.1) + 8;
-        if (attempt == 3) return fail(c, DSMD_ERR_CAPACITY, "neighbour rows kept overflowing");
+        if (attempt == 3) return failed(fail(c, DSMD_ERR_CAPACITY, "neighbour rows kept overflowing"));
     }
-    ++c->build_epoch;
-    c->list_valid = true;
     return DSMD_OK;
 }
 
@@ -1450,8 +1518,8 @@ static int pack_impl(dsmd_ctx* c, int64_t first, int64_t count, bool integrate, 
     const DisplacementReport report = displacement_report(c, first == 0 && count >= c->n_owned, s);
     double** r = c->real[c->cur];
     const auto kernel = !integrate ? k_pack<false, false> : (bonded ? k_pack<true, true> : k_pack<true, false>);
-    kernel<<<blocks_for(count, kThreads), kThreads, 0, s>>>(
-        c->grid, static_cast<int>(first), static_cast<int>(count), static_cast<int>(c->n_owned), r[0], r[1], r[2], r[3], r[4], r[5],
+    // (a part of the atoms follows a copy on another stream: nothing to overlap with)
+    dsmd::launch_next_if(first == 0 && count >= c->n_owned, kernel, blocks_for(count, kThreads), kThreads, 0, s, c->grid, static_cast<int>(first), static_cast<int>(count), static_cast<int>(c->n_owned), r[0], r[1], r[2], r[3], r[4], r[5],
         r[6], r[7], r[8], r[9], c->type[c->cur], c->ref[0], c->ref[1], c->ref[2], c->pq, dt, kick * dt * f2a, skip,
         bonded ? *bonded : BondedForces{}, report);
     DSMD_LAUNCHED(c);
@@ -1556,7 +1624,7 @@ static int compute_forces_impl(dsmd_ctx* c, int phase, int want_energy, int64_t 
                                                        : (e ? dsmd::launch_pair<0, true, 0> : dsmd::launch_pair<0, false, 0>))
                             : copies == 1 ? (e ? dsmd::launch_pair<1, true, 0> : dsmd::launch_pair<1, false, 0>)
                                           : (e ? dsmd::launch_pair<kEwaldCopiesMost, true, kLongOrder> : dsmd::launch_pair<kEwaldCopiesMost, false, kLongOrder>);
-        DSMD_CUDA(c, launch(p, a, sw, blocks, s));
+        DSMD_CUDA(c, launch(p, a, sw, blocks, !ranged, s));
         ++c->launches;
     }
     return DSMD_OK;
@@ -1618,11 +1686,11 @@ ClusterTable cluster_table(const dsmd_ctx* c) {
 // Where the clusters' atoms are since the last sort.
 int ensure_slot_map(dsmd_ctx* c, cudaStream_t s) {
     if (c->slot_map_valid) return DSMD_OK;
-    k_slot_of_gid<<<blocks_for(c->n_owned, kThreads), kThreads, 0, s>>>(static_cast<int>(c->n_owned), c->gid[c->cur],
+    dsmd::launch_next(k_slot_of_gid, blocks_for(c->n_owned, kThreads), kThreads, 0, s, static_cast<int>(c->n_owned), c->gid[c->cur],
                                                                          static_cast<int>(c->cons_n_global), c->slot_of_gid);
     DSMD_LAUNCHED(c);
     const int n = c->n_clusters * kClusterAtoms;
-    k_cluster_slots<<<blocks_for(n, kThreads), kThreads, 0, s>>>(n, c->cl_gid, c->slot_of_gid, c->cl_slot);
+    dsmd::launch_next(k_cluster_slots, blocks_for(n, kThreads), kThreads, 0, s, n, c->cl_gid, c->slot_of_gid, c->cl_slot);
     DSMD_LAUNCHED(c);
     c->slot_map_valid = true;
     return DSMD_OK;
@@ -1636,7 +1704,7 @@ int launch_constrained(dsmd_ctx* c, bool finish, bool start, double half_kick, d
     const auto launch = [&](auto shape) {
         const auto kernel = finish && start ? k_constrained<decltype(shape), true, true>
                                             : (finish ? k_constrained<decltype(shape), true, false> : k_constrained<decltype(shape), false, true>);
-        kernel<<<blocks, 128, 0, s>>>(cluster_table(c), c->grid, at, half_kick, dt, c->cons_tolerance, c->cons_max_iterations, prefactor,
+        dsmd::launch_next(kernel, blocks, 128, 0, s, cluster_table(c), c->grid, at, half_kick, dt, c->cons_tolerance, c->cons_max_iterations, prefactor,
                                       c->partials, c->tickets + 3, d_virial3, report);
     };
     if (c->cl_shape == 1) launch(TriangleCluster());
@@ -1657,7 +1725,7 @@ int constrained_halves(dsmd_ctx* c, bool finish, bool start, double dt, double f
     const ClusterMembers members{c->cl_member, static_cast<int>(c->cons_n_global), c->gid[c->cur]};
     if (start) return pack_impl(c, 0, c->n_owned, true, dt, f2a, s, finish ? 1.0 : 0.5, members);
     double** r = c->real[c->cur];
-    k_vv2<<<blocks_for(c->n_owned, kThreads), kThreads, 0, s>>>(static_cast<int>(c->n_owned), half_kick, r[3], r[4], r[5], r[6], r[7], r[8],
+    dsmd::launch_next(k_vv2, blocks_for(c->n_owned, kThreads), kThreads, 0, s, static_cast<int>(c->n_owned), half_kick, r[3], r[4], r[5], r[6], r[7], r[8],
                                                                r[9], members);
     DSMD_LAUNCHED(c);
     return DSMD_OK;
@@ -1795,7 +1863,7 @@ int dsmd_integrate(dsmd_ctx* c, int half, double dt, double f2a, void* stream) {
     if (constrained) return constrained_halves(c, half == 2, half == 1, dt, f2a, s);
     if (half == 1) return pack_impl(c, 0, c->n_owned, true, dt, f2a, s);
     double** r = c->real[c->cur];
-    k_vv2<<<blocks_for(c->n_owned, kThreads), kThreads, 0, s>>>(static_cast<int>(c->n_owned), 0.5 * dt * f2a, r[3], r[4],
+    dsmd::launch_next(k_vv2, blocks_for(c->n_owned, kThreads), kThreads, 0, s, static_cast<int>(c->n_owned), 0.5 * dt * f2a, r[3], r[4],
                                                                r[5], r[6], r[7], r[8], r[9], ClusterMembers{});
     DSMD_LAUNCHED(c);
     return DSMD_OK;
@@ -1915,17 +1983,18 @@ int dsmd_set_bonded(dsmd_ctx* c, int64_t n_global, int64_t n_bonds, const int32_
     return DSMD_OK;
 }
 
-// The terms' contributions into their scratch array.
-static int bonded_terms(dsmd_ctx* c, bool sums, cudaStream_t s) {
+// The terms' contributions into their scratch array. behind_forces: the launch before is the force kernel at the same positions.
+static int bonded_terms(dsmd_ctx* c, bool sums, bool behind_forces, cudaStream_t s) {
     dsmd_ctx::Bonded& b = c->bonded;
     if (b.terms() == 0) return DSMD_OK;
     if (!c->list_valid) return fail(c, DSMD_ERR_STATE, "no neighbour list built yet (bonded terms find their atoms through the sorted arrays)");
     if (b.map_epoch != c->build_epoch) {   // the sort of a list build moved the atoms
         DSMD_CUDA(c, cudaMemsetAsync(b.slot_of_gid, 0x7F, sizeof(int) * b.n_global, s));   // 0x7F7F7F7F: beyond any slot
-        k_bonded_slot_map<<<blocks_for(c->n_total, kThreads), kThreads, 0, s>>>(static_cast<int>(c->n_total), c->gid[c->cur],
+        dsmd::launch_next(k_bonded_slot_map, blocks_for(c->n_total, kThreads), kThreads, 0, s, static_cast<int>(c->n_total), c->gid[c->cur],
                                                                                static_cast<int>(b.n_global), b.slot_of_gid);
         DSMD_LAUNCHED(c);
         b.map_epoch = c->build_epoch;
+        behind_forces = false;
     }
     BondedTable t{};
     t.place = b.place;
@@ -1940,8 +2009,8 @@ static int bonded_terms(dsmd_ctx* c, bool sums, cudaStream_t s) {
     for (int a = 0; a < 3; ++a) { t.box[a] = c->box[a]; t.periodic[a] = c->periodic[a]; }
     double** r = c->real[c->cur];
     const auto kernel = sums ? k_bonded_terms<true> : k_bonded_terms<false>;
-    kernel<<<static_cast<unsigned>(b.blocks), kBondedThreads, 0, s>>>(t, r[0], r[1], r[2], r[10], b.contrib, b.partials, c->tickets + 2,
-                                                                      b.scalars, b.missing);
+    dsmd::launch_next(kernel, static_cast<unsigned>(b.blocks), kBondedThreads, 0, s, t, r[0], r[1], r[2], r[10], b.contrib, b.partials, c->tickets + 2,
+                                                                      b.scalars, b.missing, behind_forces);
     DSMD_LAUNCHED(c);
     return DSMD_OK;
 }
@@ -1954,9 +2023,9 @@ int dsmd_compute_bonded(dsmd_ctx* c, void* stream) {
     if (!c) return DSMD_ERR_INVALID;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (c->bonded.terms() == 0) return DSMD_OK;
-    { const int rc = bonded_terms(c, true, s); if (rc) return rc; }
+    { const int rc = bonded_terms(c, true, false, s); if (rc) return rc; }
     double** r = c->real[c->cur];
-    k_bonded_gather<<<blocks_for(c->n_owned, kThreads), kThreads, 0, s>>>(static_cast<int>(c->n_owned), bonded_forces(c), r[6], r[7], r[8]);
+    dsmd::launch_next(k_bonded_gather, blocks_for(c->n_owned, kThreads), kThreads, 0, s, static_cast<int>(c->n_owned), bonded_forces(c), r[6], r[7], r[8]);
     DSMD_LAUNCHED(c);
     return DSMD_OK;
 }
@@ -1985,7 +2054,7 @@ int dsmd_kinetic_energy(dsmd_ctx* c, double* out, void* stream) {
     const int64_t blocks = std::min<int64_t>(blocks_for(c->n_owned, kThreads), kDeviceSms * 8);
     { const int rc = ensure_partials(c, blocks); if (rc) return rc; }
     double** r = c->real[c->cur];
-    k_kinetic<<<static_cast<unsigned>(blocks), kThreads, 0, s>>>(static_cast<int>(c->n_owned), r[3], r[4], r[5], r[9],
+    dsmd::launch_next(k_kinetic, static_cast<unsigned>(blocks), kThreads, 0, s, static_cast<int>(c->n_owned), r[3], r[4], r[5], r[9],
                                                                  c->partials, c->tickets + 1, c->scalars + 6, c->mail + kMailKinetic, ++c->seq);
     DSMD_LAUNCHED(c);
     DSMD_CUDA(c, cudaStreamSynchronize(s));
@@ -1999,7 +2068,7 @@ int dsmd_scale_velocities(dsmd_ctx* c, double factor, void* stream) {
     if (c->n_owned == 0) return DSMD_OK;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     double** r = c->real[c->cur];
-    k_scale_velocities<<<blocks_for(c->n_owned, kThreads), kThreads, 0, s>>>(static_cast<int>(c->n_owned), factor, r[3], r[4],
+    dsmd::launch_next(k_scale_velocities, blocks_for(c->n_owned, kThreads), kThreads, 0, s, static_cast<int>(c->n_owned), factor, r[3], r[4],
                                                                              r[5]);
     DSMD_LAUNCHED(c);
     return DSMD_OK;
@@ -2058,7 +2127,7 @@ int dsmd_run_nve(dsmd_ctx* c, int64_t n_steps, double dt, double f2a, double hi_
         } else {
             rc = dsmd_compute_forces(c, DSMD_PHASE_FULL, 0, s);
             if (bonded) {   // the bonded contributions go straight into the pass over the atoms
-                if (!rc) rc = bonded_terms(c, false, s);
+                if (!rc) rc = bonded_terms(c, false, true, s);
                 const BondedForces terms = bonded_forces(c);
                 if (!rc) rc = pack_impl(c, 0, c->n_owned, true, dt, f2a, s, 1.0, {}, &terms);
             } else {
@@ -2076,7 +2145,7 @@ int dsmd_run_nve(dsmd_ctx* c, int64_t n_steps, double dt, double f2a, double hi_
         const unsigned long long check = c->disp_seq;   // the displacement check of the positions that are current now
         const bool last = step + 1 == n_steps;
         ++since_build;
-        bool rebuild = every > 0 && since_build >= every, advanced = false;
+        bool rebuild = every > 0 && since_build >= every, advanced = false, built_ahead = false;
         if (!lagged) {
             // unless a rebuild is due or this is the end, the next kernels are queued before the host looks at the check
             if (ahead_of_check && !rebuild && !last) {
@@ -2110,8 +2179,12 @@ int dsmd_run_nve(dsmd_ctx* c, int64_t n_steps, double dt, double f2a, double hi_
             if (predicted * predicted > limit2) rebuild = true;
         }
         if (rebuild) {
-            const int rc = build_list(c, false, s);   // forces are evaluated next
+            // Forces are evaluated next, as a rule queued behind the build before the host hears of it.
+            const bool queue = ahead_of_check && !last && limit2 < dsmd::kGateOpen;
+            const int rc = queue ? build_list(c, false, s, [&] { return advance(limit2); }, [&] { if (fused) std::swap(c->pq, c->pq_next); })
+                                 : build_list(c, false, s);
             if (rc) return rc;
+            built_ahead = queue;
             ++rebuilds;
             since_build = 0;
             d_prev = d_prev2 = 0.0;
@@ -2121,7 +2194,7 @@ int dsmd_run_nve(dsmd_ctx* c, int64_t n_steps, double dt, double f2a, double hi_
             { const int rc = dsmd_compute_forces(c, DSMD_PHASE_FULL, 0, s); if (rc) return rc; }
             { const int rc = dsmd_compute_bonded(c, s); if (rc) return rc; }
             { const int rc = dsmd_integrate(c, 2, dt, f2a, s); if (rc) return rc; }
-        } else if (!advanced || rebuild) {
+        } else if (!built_ahead && (!advanced || rebuild)) {
             const int rc = advance(HUGE_VAL);
             if (rc) return rc;
         }

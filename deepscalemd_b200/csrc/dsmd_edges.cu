@@ -22,7 +22,9 @@
 #include "../../include/dsmd_b200.h"
 #include "dsmd_cells.cuh"
 #include "dsmd_common.cuh"
+#include "dsmd_launch.cuh"
 #include "dsmd_report.cuh"
+#include "dsmd_scan.cuh"
 
 using dsmd::Grid;
 
@@ -44,6 +46,7 @@ struct EdgeStatus {
 __global__ void k_edge_keys(Grid g, int n, const double* __restrict__ x, const double* __restrict__ y,
                             const double* __restrict__ z, unsigned* __restrict__ key, int* __restrict__ arrival,
                             int* __restrict__ cell_count, EdgeStatus* st) {
+    if (!dsmd::after_previous()) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     unsigned bad = 0;
@@ -92,6 +95,7 @@ __global__ void k_edge_gather(Grid g, int n, const unsigned* __restrict__ key, c
                               const double* __restrict__ z, const unsigned char* __restrict__ neighbour_ok,
                               const int* __restrict__ owner, int4* __restrict__ pq, float4* __restrict__ pf, int* __restrict__ wraps,
                               EdgeStatus* st) {
+    if (!dsmd::after_previous()) return;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     const int a = list[t];
@@ -111,6 +115,12 @@ __global__ void k_edge_gather(Grid g, int n, const unsigned* __restrict__ key, c
         wraps[s] = w;
         if (w != (kWrapBias | (kWrapBias << kWrapBits) | (kWrapBias << (2 * kWrapBits)))) st->outside_box = 1u;
     }
+}
+
+__global__ void k_edge_place(int n, const unsigned* __restrict__ key, const int* __restrict__ arrival, const int* __restrict__ cell_start,
+                             int* __restrict__ list, int cells, int* __restrict__ cell_count) {
+    if (!dsmd::after_previous()) return;
+    dsmd::cell_place(blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, 0, n, key, arrival, cell_start, list, cells, cell_count);
 }
 
 struct SearchArgs {
@@ -198,8 +208,7 @@ __device__ __forceinline__ void finish_search(const SearchArgs& a, int count) {
     if (threadIdx.x == 0) {
         const double out[4] = {static_cast<double>(carry), static_cast<double>(__ldcg(&a.st->out_of_bounds)),
                                static_cast<double>(__ldcg(&a.st->need_stride)), static_cast<double>(__ldcg(&a.st->outside_box))};
-        a.st->ticket = 0u;
-        a.st->need_stride = 0u;
+        *a.st = EdgeStatus{};   // for the next build; one that has to search again remembers the other words
         dsmd::post(a.mail, out, 4, a.seq);
     }
 }
@@ -216,6 +225,7 @@ constexpr int kAtATime = 3;                    // candidates in flight per threa
 // band are marked and decided in fp64 afterwards. 1,000,000 atoms, 100 candidates and 26 hits each: 0.28 ms (0.35 ms before).
 template <bool PERIODIC>
 __global__ void __launch_bounds__(kSearchThreads) k_edge_search(Grid g, SearchArgs a) {
+    if (!dsmd::after_previous()) return;
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     int count = 0;
     const int4 pi = a.pq[min(p, a.n - 1)];
@@ -300,6 +310,7 @@ constexpr int kWarpCandidates = 512;     // numbered at a time
 
 template <bool PERIODIC>
 __global__ void __launch_bounds__(kSearchThreads) k_edge_search_warp(Grid g, SearchArgs a) {
+    if (!dsmd::after_previous()) return;
     __shared__ int s_slots[kSearchThreads / 32][kWarpCandidates];
     const int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     int* slots = s_slots[threadIdx.x >> 5];
@@ -420,6 +431,7 @@ __global__ void __launch_bounds__(kFillThreads) k_edge_fill(int n, long long n_e
                             const double* __restrict__ shift_x, const double* __restrict__ shift_y,
                             const double* __restrict__ shift_z, long long* __restrict__ edges,
                             double* __restrict__ shift) {
+    if (!dsmd::after_previous()) return;
     __shared__ FlatSlice f;
     __shared__ int centres[32];
     // the three shift components of 32 edges are 96 consecutive doubles of the output
@@ -473,6 +485,7 @@ __global__ void __launch_bounds__(kFillThreads, 14) k_edge_fill_compact(
     Grid g, int n, int stride, int group_shift, const int4* __restrict__ pq, const int* __restrict__ wraps,
     const unsigned* __restrict__ rows, const int* __restrict__ counts, const long long* __restrict__ group_start,
     int* __restrict__ src, int* __restrict__ dst, signed char* __restrict__ shift, float* __restrict__ vec) {
+    if (!dsmd::after_previous()) return;
     __shared__ FlatSlice f;
     __shared__ int4 centres[32];
     __shared__ int centre_wraps[32];
@@ -557,6 +570,7 @@ __global__ void __launch_bounds__(kFillThreads, 14) k_edge_fill_compact(
 __global__ void __launch_bounds__(kThreads) k_edge_bounds(int n, const double* __restrict__ x, const double* __restrict__ y,
                                                           const double* __restrict__ z, double* __restrict__ partials, unsigned* ticket,
                                                           dsmd::Mail* mail, unsigned long long seq) {
+    if (!dsmd::after_previous()) return;
     __shared__ double sh[kThreads / 32][6];
     const auto over_block = [&](double (&v)[6]) {
         for (int k = 0; k < 6; ++k)
@@ -648,6 +662,7 @@ __device__ __forceinline__ int nth_set_bit(unsigned mask, int n) {
 __global__ void k_image_masks(ImageLattice L, int n, const double* __restrict__ x, const double* __restrict__ y,
                               const double* __restrict__ z, unsigned long long* __restrict__ masks,
                               long long* __restrict__ counts) {
+    if (!dsmd::after_previous()) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const unsigned mx = axis_mask(L, 0, wrapped_coord(L, 0, x[i]));
@@ -662,6 +677,7 @@ __global__ void k_image_masks(ImageLattice L, int n, const double* __restrict__ 
 // Images of the whole system, reported to the host.
 __global__ void k_image_total(int n, const long long* __restrict__ counts, const long long* __restrict__ first_image, dsmd::Mail* mail,
                               unsigned long long seq) {
+    if (!dsmd::after_previous()) return;
     const double total[1] = {static_cast<double>(first_image[n - 1] + counts[n - 1])};
     dsmd::post(mail, total, 1, seq);
 }
@@ -674,6 +690,7 @@ __global__ void k_image_fill(ImageLattice L, int n, long long n_images, const do
                              double* __restrict__ out_x, double* __restrict__ out_y, double* __restrict__ out_z,
                              int* __restrict__ out_type, int* __restrict__ out_owner, double* __restrict__ off_x,
                              double* __restrict__ off_y, double* __restrict__ off_z) {
+    if (!dsmd::after_previous()) return;
     const long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
     if (t >= n + n_images) return;
     int owner;
@@ -721,6 +738,7 @@ __global__ void k_image_fold(int n_out, int n, int with_images, const double* __
                              const double* __restrict__ fy, const double* __restrict__ fz,
                              const long long* __restrict__ first_image, const long long* __restrict__ counts,
                              double* __restrict__ tx, double* __restrict__ ty, double* __restrict__ tz) {
+    if (!dsmd::after_previous()) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_out) return;
     double sx = fx[i], sy = fy[i], sz = fz[i];
@@ -743,6 +761,7 @@ __global__ void __launch_bounds__(kThreads) k_virial(long long n, const double* 
                                                      const double* __restrict__ z, const double* __restrict__ fx,
                                                      const double* __restrict__ fy, const double* __restrict__ fz,
                                                      double* __restrict__ partials, unsigned* ticket, dsmd::Mail* mail, unsigned long long seq) {
+    if (!dsmd::after_previous()) return;
     __shared__ double sh[kThreads / 32][3];
     const auto over_block = [&](double (&v)[3]) {   // the total in thread 0
         for (int a = 0; a < 3; ++a)
@@ -780,6 +799,7 @@ __global__ void __launch_bounds__(kThreads) k_virial(long long n, const double* 
 __global__ void k_mark_receivers(int n, const double* __restrict__ x, const double* __restrict__ y,
                                  const double* __restrict__ z, double lx, double ly, double lz, double hx, double hy,
                                  double hz, double reach2, unsigned char* __restrict__ ok) {
+    if (!dsmd::after_previous()) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double dx = fmax(fmax(lx - x[i], x[i] - hx), 0.0);
@@ -813,6 +833,8 @@ struct dsmd_edges {
     int* arrival = nullptr;                 size_t cap_arrival = 0;   // its place among the cell's atoms as they came
     int* list = nullptr;                    size_t cap_list = 0;      // the cells' atoms as they came
     int* cell_count = nullptr;              size_t cap_cell_count = 0;   // behind kStatusWords words of EdgeStatus
+    bool counts_zero = false;               // counts and status are zero, as every search leaves them
+    int* scan_sums = nullptr;               // [kScanBlocksMost]
     int4* pq = nullptr;                     size_t cap_pq = 0;
     float4* pf = nullptr;                   size_t cap_pf = 0;
     int* wraps = nullptr;                   size_t cap_wraps = 0;     // per sorted slot, periodic form
@@ -972,21 +994,28 @@ int edge_search(dsmd_edges* e, const Grid& g, const double* d_x, const double* d
     EDGE_ALLOC(e, grow(e->pq, e->cap_pq, un));
     EDGE_ALLOC(e, grow(e->pf, e->cap_pf, un));
     if (PERIODIC) EDGE_ALLOC(e, grow(e->wraps, e->cap_wraps, un));
+    if (table + kStatusWords > e->cap_cell_count) e->counts_zero = false;
     EDGE_ALLOC(e, grow(e->cell_count, e->cap_cell_count, table + kStatusWords));
     EDGE_ALLOC(e, grow(e->cell_start, e->cap_cells, table));
     EDGE_ALLOC(e, grow(e->counts, e->cap_counts, un));
     EDGE_ALLOC(e, grow(e->group_sum, e->cap_group_sum, static_cast<size_t>(groups)));
     EDGE_ALLOC(e, grow(e->group_start, e->cap_group_start, static_cast<size_t>(groups)));
-    size_t scan_bytes = 0;
     int* const cell_count = e->cell_count + kStatusWords;
-    cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, cell_count, e->cell_start, static_cast<int>(table), s);
-    EDGE_ALLOC(e, grow(e->temp, e->cap_temp, scan_bytes));
     EdgeStatus* const st = reinterpret_cast<EdgeStatus*>(e->cell_count);
-    EDGE_CUDA(e, cudaMemsetAsync(e->cell_count, 0, sizeof(int) * (table + kStatusWords), s));
-    k_edge_keys<<<blocks_for(n, kThreads), kThreads, 0, s>>>(g, in, d_x, d_y, d_z, e->key, e->arrival, cell_count, st);
-    EDGE_CUDA(e, cub::DeviceScan::ExclusiveSum(e->temp, scan_bytes, cell_count, e->cell_start, static_cast<int>(table), s));
-    dsmd::k_cell_place<<<blocks_for(n, kThreads), kThreads, 0, s>>>(0, in, e->key, e->arrival, e->cell_start, e->list);
-    k_edge_gather<<<blocks_for(n, kThreads), kThreads, 0, s>>>(g, in, e->key, e->list, e->cell_start, d_x, d_y, d_z,
+    if (!e->counts_zero) EDGE_CUDA(e, cudaMemsetAsync(e->cell_count, 0, sizeof(int) * e->cap_cell_count, s));
+    e->counts_zero = false;
+    dsmd::launch_next(k_edge_keys, blocks_for(n, kThreads), kThreads, 0, s, g, in, d_x, d_y, d_z, e->key, e->arrival, cell_count, st);
+    if (table <= static_cast<size_t>(dsmd::kScanMost)) {
+        const int launched = dsmd::launch_cell_scan(static_cast<int>(table), 0, cell_count, e->scan_sums, e->cell_start, s);
+        e->launches += std::max(launched, 0);
+    } else {
+        size_t scan_bytes = 0;
+        cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, cell_count, e->cell_start, static_cast<int>(table), s);
+        EDGE_ALLOC(e, grow(e->temp, e->cap_temp, scan_bytes));
+        EDGE_CUDA(e, cub::DeviceScan::ExclusiveSum(e->temp, scan_bytes, cell_count, e->cell_start, static_cast<int>(table), s));
+    }
+    dsmd::launch_next(k_edge_place, blocks_for(n, kThreads), kThreads, 0, s, in, e->key, e->arrival, e->cell_start, e->list, static_cast<int>(table), cell_count);
+    dsmd::launch_next(k_edge_gather, blocks_for(n, kThreads), kThreads, 0, s, g, in, e->key, e->list, e->cell_start, d_x, d_y, d_z,
                                                               row == 1 ? d_ok : nullptr, d_owner, e->pq, e->pf,
                                                               PERIODIC ? e->wraps : nullptr, st);
     e->launches += 3;
@@ -999,18 +1028,19 @@ int edge_search(dsmd_edges* e, const Grid& g, const double* d_x, const double* d
         EDGE_ALLOC(e, grow(e->rows, e->cap_rows, slices * static_cast<size_t>(e->stride) * 32));
         const SearchArgs a{in, static_cast<int>(n_centers), e->stride, float_band(g, cutoff), e->pq, e->pf, d_x, d_y, d_z, e->cell_start,
                            row == 0 ? d_ok : nullptr, e->rows, e->counts, e->group_sum, e->group_start, st, e->mail, ++e->seq};
-        if (by_warp) k_edge_search_warp<PERIODIC><<<groups, kSearchThreads, 0, s>>>(g, a);
-        else k_edge_search<PERIODIC><<<groups, kSearchThreads, 0, s>>>(g, a);
+        if (by_warp) dsmd::launch_next(k_edge_search_warp<PERIODIC>, groups, kSearchThreads, 0, s, g, a);
+        else dsmd::launch_next(k_edge_search<PERIODIC>, groups, kSearchThreads, 0, s, g, a);
         ++e->launches;
         EDGE_CUDA(e, cudaGetLastError());
         // the one wait of a build that does not overflow: edge count, bounds flag, row overflow
         EDGE_CUDA(e, dsmd::wait_report(e->mail, 4, e->seq, s));
+        e->counts_zero = true;
+        if (attempt == 0) e->outside_box = e->mail->value(3) != 0.0;
         if (e->mail->value(1) != 0.0)
             return efail(e, DSMD_ERR_OUT_OF_DOMAIN, "an atom lies outside the given box (or has a NaN position)");
         const int need = static_cast<int>(e->mail->value(2));
         if (need <= e->stride) {
             *n_edges = static_cast<int64_t>(e->mail->value(0));
-            e->outside_box = e->mail->value(3) != 0.0;
             return DSMD_OK;
         }
         e->stride = (static_cast<int>(need * 1.2) + 8 + 3) & ~3;
@@ -1031,6 +1061,7 @@ int dsmd_edges_create(int device, dsmd_edges** out) {
     *out = e;
     EDGE_CUDA(e, cudaSetDevice(device));
     EDGE_CUDA(e, cudaMalloc(&e->partials, sizeof(double) * 6 * kReduceBlocks));
+    EDGE_CUDA(e, cudaMalloc(&e->scan_sums, sizeof(int) * dsmd::kScanBlocksMost));
     EDGE_CUDA(e, cudaMalloc(&e->ticket, sizeof(unsigned)));
     EDGE_CUDA(e, cudaMemset(e->ticket, 0, sizeof(unsigned)));
     EDGE_CUDA(e, cudaMallocHost(&e->mail, sizeof(dsmd::Mail)));
@@ -1045,7 +1076,7 @@ void dsmd_edges_destroy(dsmd_edges* e) {
     cudaFree(e->pq); cudaFree(e->wraps); cudaFree(e->cell_start); cudaFree(e->rows); cudaFree(e->counts);
     cudaFree(e->group_sum); cudaFree(e->group_start); cudaFree(e->temp); cudaFree(e->edges); cudaFree(e->shift);
     cudaFree(e->c_src); cudaFree(e->c_dst); cudaFree(e->c_shift); cudaFree(e->c_vec); cudaFree(e->partials);
-    cudaFree(e->ticket); cudaFree(e->img_counts); cudaFree(e->img_offsets); cudaFree(e->img_masks);
+    cudaFree(e->ticket); cudaFree(e->scan_sums); cudaFree(e->img_counts); cudaFree(e->img_offsets); cudaFree(e->img_masks);
     if (e->mail) cudaFreeHost(e->mail);
     cudaFree(e->ext_type); cudaFree(e->ext_owner);
     for (int k = 0; k < 6; ++k) cudaFree(e->ext[k]);
@@ -1078,8 +1109,7 @@ int dsmd_edges_build(dsmd_edges* e, const double* d_x, const double* d_y, const 
     if (lo && hi) {
         for (int a = 0; a < 3; ++a) { box_lo[a] = lo[a]; box_hi[a] = hi[a]; }
     } else {   // bounding box on the device: one extra wait
-        k_edge_bounds<<<std::min<unsigned>(blocks_for(n, kThreads), kReduceBlocks), kThreads, 0, s>>>(
-            static_cast<int>(n), d_x, d_y, d_z, e->partials, e->ticket, e->mail, ++e->seq);
+        dsmd::launch_next(k_edge_bounds, std::min<unsigned>(blocks_for(n, kThreads), kReduceBlocks), kThreads, 0, s, static_cast<int>(n), d_x, d_y, d_z, e->partials, e->ticket, e->mail, ++e->seq);
         ++e->launches;
         EDGE_CUDA(e, cudaGetLastError());
         EDGE_CUDA(e, dsmd::wait_report(e->mail, 6, e->seq, s));
@@ -1101,7 +1131,7 @@ int dsmd_edges_build(dsmd_edges* e, const double* d_x, const double* d_y, const 
     if (E == 0) return DSMD_OK;
     EDGE_ALLOC(e, grow(e->edges, e->cap_edges, 2 * static_cast<size_t>(E)));
     if (images) EDGE_ALLOC(e, grow(e->shift, e->cap_shift, 3 * static_cast<size_t>(E)));
-    k_edge_fill<<<blocks_for(n, 32), kFillThreads, 0, s>>>(static_cast<int>(n), E, e->stride, e->group_shift, e->pq, e->rows, e->counts,
+    dsmd::launch_next(k_edge_fill, blocks_for(n, 32), kFillThreads, 0, s, static_cast<int>(n), E, e->stride, e->group_shift, e->pq, e->rows, e->counts,
                                                           e->group_start, static_cast<int>(n_centers), d_owner, d_shift_x,
                                                           d_shift_y, d_shift_z, e->edges, images ? e->shift : nullptr);
     ++e->launches;
@@ -1145,7 +1175,7 @@ int dsmd_edges_build_periodic(dsmd_edges* e, const double* d_x, const double* d_
     EDGE_ALLOC(e, grow(e->c_shift, e->cap_cshift, 3 * static_cast<size_t>(E)));
     EDGE_ALLOC(e, grow(e->c_vec, e->cap_cvec, 3 * static_cast<size_t>(E)));
     const auto fill = e->outside_box ? k_edge_fill_compact<true> : k_edge_fill_compact<false>;
-    fill<<<blocks_for(n, 32), kFillThreads, 0, s>>>(g, static_cast<int>(n), e->stride, e->group_shift, e->pq, e->wraps, e->rows, e->counts,
+    dsmd::launch_next(fill, blocks_for(n, 32), kFillThreads, 0, s, g, static_cast<int>(n), e->stride, e->group_shift, e->pq, e->wraps, e->rows, e->counts,
                                                    e->group_start, e->c_src, e->c_dst, e->c_shift, e->c_vec);
     ++e->launches;
     EDGE_CUDA(e, cudaGetLastError());
@@ -1180,11 +1210,11 @@ int dsmd_images_build(dsmd_edges* e, const double* d_x, const double* d_y, const
     size_t scan_bytes = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, e->img_counts, e->img_offsets, static_cast<int>(n), s);
     EDGE_ALLOC(e, grow(e->temp, e->cap_temp, scan_bytes));
-    k_image_masks<<<blocks_for(n, kThreads), kThreads, 0, s>>>(lattice, static_cast<int>(n), d_x, d_y, d_z, e->img_masks,
+    dsmd::launch_next(k_image_masks, blocks_for(n, kThreads), kThreads, 0, s, lattice, static_cast<int>(n), d_x, d_y, d_z, e->img_masks,
                                                               e->img_counts);
     EDGE_CUDA(e, cub::DeviceScan::ExclusiveSum(e->temp, scan_bytes, e->img_counts, e->img_offsets, static_cast<int>(n), s));
     // the image count comes to the host: the one synchronisation (MLIPStep::prepare does the same, src/MLIPStep.cu:254-255)
-    k_image_total<<<1, 1, 0, s>>>(static_cast<int>(n), e->img_counts, e->img_offsets, e->mail, ++e->seq);
+    dsmd::launch_next(k_image_total, 1, 1, 0, s, static_cast<int>(n), e->img_counts, e->img_offsets, e->mail, ++e->seq);
     EDGE_CUDA(e, cudaGetLastError());
     EDGE_CUDA(e, dsmd::wait_report(e->mail, 1, e->seq, s));
     const int64_t n_images = static_cast<int64_t>(e->mail->value(0));
@@ -1193,7 +1223,7 @@ int dsmd_images_build(dsmd_edges* e, const double* d_x, const double* d_y, const
     for (int k = 0; k < 6; ++k) EDGE_ALLOC(e, grow(e->ext[k], e->cap_ext[k], static_cast<size_t>(total)));
     EDGE_ALLOC(e, grow(e->ext_type, e->cap_ext_type, static_cast<size_t>(total)));
     EDGE_ALLOC(e, grow(e->ext_owner, e->cap_ext_owner, static_cast<size_t>(total)));
-    k_image_fill<<<blocks_for(total, kThreads), kThreads, 0, s>>>(lattice, static_cast<int>(n), n_images, d_x, d_y, d_z, d_type,
+    dsmd::launch_next(k_image_fill, blocks_for(total, kThreads), kThreads, 0, s, lattice, static_cast<int>(n), n_images, d_x, d_y, d_z, d_type,
                                                                  e->img_masks, e->img_offsets, e->ext[0], e->ext[1], e->ext[2],
                                                                  e->ext_type, e->ext_owner, e->ext[3], e->ext[4], e->ext[5]);
     e->launches += 3;
@@ -1211,7 +1241,7 @@ int dsmd_images_fold_forces(dsmd_edges* e, const double* d_fx, const double* d_f
     if (n_out < 0 || n_out > e->n_img_src) n_out = e->n_img_src;
     if (n_out == 0) return DSMD_OK;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    k_image_fold<<<blocks_for(n_out, kThreads), kThreads, 0, s>>>(static_cast<int>(n_out), static_cast<int>(e->n_img_src),
+    dsmd::launch_next(k_image_fold, blocks_for(n_out, kThreads), kThreads, 0, s, static_cast<int>(n_out), static_cast<int>(e->n_img_src),
                                                                  with_images, d_fx, d_fy, d_fz, e->img_offsets, e->img_counts,
                                                                  d_tx, d_ty, d_tz);
     ++e->launches;
@@ -1227,7 +1257,7 @@ int dsmd_virial_from_forces(dsmd_edges* e, const double* d_x, const double* d_y,
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     EDGE_CUDA(e, cudaSetDevice(e->device));
     const int blocks = static_cast<int>(std::min<int64_t>(kReduceBlocks, (n + kThreads - 1) / kThreads));
-    k_virial<<<blocks, kThreads, 0, s>>>(n, d_x, d_y, d_z, d_fx, d_fy, d_fz, e->partials, e->ticket, e->mail, ++e->seq);
+    dsmd::launch_next(k_virial, blocks, kThreads, 0, s, n, d_x, d_y, d_z, d_fx, d_fy, d_fz, e->partials, e->ticket, e->mail, ++e->seq);
     ++e->launches;
     EDGE_CUDA(e, cudaGetLastError());
     EDGE_CUDA(e, dsmd::wait_report(e->mail, 4, e->seq, s));
@@ -1256,7 +1286,7 @@ int dsmd_mark_receivers(dsmd_edges* e, const double* d_x, const double* d_y, con
     if (!e || !lo || !hi || n < 0 || (n > 0 && (!d_x || !d_y || !d_z || !d_ok))) return DSMD_ERR_INVALID;
     if (n == 0) return DSMD_OK;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    k_mark_receivers<<<blocks_for(n, kThreads), kThreads, 0, s>>>(static_cast<int>(n), d_x, d_y, d_z, lo[0], lo[1], lo[2],
+    dsmd::launch_next(k_mark_receivers, blocks_for(n, kThreads), kThreads, 0, s, static_cast<int>(n), d_x, d_y, d_z, lo[0], lo[1], lo[2],
                                                                  hi[0], hi[1], hi[2], reach * reach, d_ok);
     ++e->launches;
     EDGE_CUDA(e, cudaGetLastError());

@@ -88,10 +88,10 @@ constexpr int kPairThreads = COPIES == kEwaldCopiesMost ? 512 : (COPIES == 0 && 
 template <int COPIES, int TYPES, bool ENERGY>
 constexpr int kPairBlocks = ENERGY || COPIES == kEwaldCopiesMost ? 1 : (COPIES > 0 ? 5 : (TYPES == kOneType ? 16 : 6));
 
-// Both return what the launch returned. sw: with the switching function. ENERGY: with energy sums. ORDER: of the rows' entries
+// Both return what the launch returned. sw: with the switching function. overlap: dsmd_launch.cuh. ENERGY: with energy sums. ORDER: of the rows' entries
 // (dsmd_row_layout.cuh).
 template <int COPIES, bool ENERGY, int ORDER>
-cudaError_t launch_pair(const PairParams& p, const ForceArgs& a, bool sw, unsigned blocks, cudaStream_t s);
+cudaError_t launch_pair(const PairParams& p, const ForceArgs& a, bool sw, unsigned blocks, bool overlap, cudaStream_t s);
 template <int ORDER>
 cudaError_t launch_step(const PairParams& p, const ForceArgs& a, const Grid& g, const StepArgs& at, const DisplacementReport& report,
                         bool sw, unsigned blocks, cudaStream_t s);

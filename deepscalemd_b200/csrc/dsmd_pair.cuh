@@ -5,6 +5,7 @@
 
 #include "../../include/dsmd_b200.h"
 #include "dsmd_f32x2.cuh"
+#include "dsmd_launch.cuh"
 #include "dsmd_force.cuh"
 #include "dsmd_row_layout.cuh"
 #include "dsmd_sums.cuh"
@@ -527,8 +528,8 @@ __device__ __forceinline__ void row_forces(const PairParams& p, const ForceArgs&
 template <int COPIES, bool ENERGY, int TYPES, bool SWITCH, bool QTYPE, int ORDER>
 __global__ void __launch_bounds__((kPairThreads<COPIES, TYPES>), (kPairBlocks<COPIES, TYPES, ENERGY>)) k_pair(PairParams p, ForceArgs a) {
     extern __shared__ float4 smem[];
-    if (!ENERGY && dsmd::gate_closed(a.st, a.gate2)) return;
-    const PairTables<COPIES, ENERGY, TYPES, QTYPE> tables(p, smem);
+    const PairTables<COPIES, ENERGY, TYPES, QTYPE> tables(p, smem);   // parameters: no kernel writes them
+    if (!dsmd::after_previous() || (!ENERGY && dsmd::gate_closed(a.st, a.gate2))) return;
     double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};   // energy, virial and its diagonal, pairs
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; (t & ~31) >> a.lane_shift < a.n_pairs; t += gridDim.x * blockDim.x) {
         float sum_a[3], sum_b[3];
@@ -564,8 +565,8 @@ template <int TYPES, bool SWITCH, int ORDER>
 __global__ void __launch_bounds__((kPairThreads<0, TYPES>), (kPairBlocks<0, TYPES, false>))
 k_step(PairParams p, ForceArgs a, Grid g, StepArgs at, DisplacementReport report) {
     extern __shared__ float4 smem[];
-    if (dsmd::gate_closed(report.st, report.gate2)) return;
-    const PairTables<0, false, TYPES, false> tables(p, smem);
+    const PairTables<0, false, TYPES, false> tables(p, smem);   // parameters: no kernel writes them
+    if (!dsmd::after_previous() || dsmd::gate_closed(report.st, report.gate2)) return;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     float sum_a[3], sum_b[3];
     double unused[6];
@@ -620,7 +621,7 @@ k_step(PairParams p, ForceArgs a, Grid g, StepArgs at, DisplacementReport report
 namespace dsmd {
 
 template <int COPIES, bool ENERGY, int ORDER>
-cudaError_t launch_pair(const PairParams& p, const ForceArgs& a, bool sw, unsigned blocks, cudaStream_t s) {
+cudaError_t launch_pair(const PairParams& p, const ForceArgs& a, bool sw, unsigned blocks, bool overlap, cudaStream_t s) {
     const auto launch = [&](auto types, auto switched, auto qtype) {
         constexpr int TYPES = decltype(types)::value;
         constexpr bool SWITCH = decltype(switched)::value, QTYPE = decltype(qtype)::value;
@@ -630,8 +631,7 @@ cudaError_t launch_pair(const PairParams& p, const ForceArgs& a, bool sw, unsign
             const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
             if (e != cudaSuccess) return e;
         }
-        kernel<<<blocks, kPairThreads<COPIES, TYPES>, smem, s>>>(p, a);
-        return cudaGetLastError();
+        return launch_next_if(overlap, kernel, blocks, kPairThreads<COPIES, TYPES>, smem, s, p, a);
     };
     const auto by_charge = [&](auto types, auto switched) {   // charges by type: only the kernels with Coulomb have this form
         if (COPIES > 0 && p.type_charge) return launch(types, switched, std::integral_constant<bool, (COPIES > 0)>());
@@ -651,8 +651,7 @@ cudaError_t launch_step(const PairParams& p, const ForceArgs& a, const Grid& g, 
         constexpr int TYPES = decltype(types)::value;
         const size_t smem = PairTables<0, false, TYPES, false>::bytes(p.ntypes, 0);
         const auto kernel = sw ? k_step<TYPES, true, ORDER> : k_step<TYPES, false, ORDER>;
-        kernel<<<blocks, kPairThreads<0, TYPES>, smem, s>>>(p, a, g, at, report);
-        return cudaGetLastError();
+        return launch_next(kernel, blocks, kPairThreads<0, TYPES>, smem, s, p, a, g, at, report);
     };
     if (p.ntypes == 1) return launch(std::integral_constant<int, kOneType>());
     if (p.ntypes == 2) return launch(std::integral_constant<int, kTwoTypes>());

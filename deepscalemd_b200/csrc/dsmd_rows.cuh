@@ -7,24 +7,39 @@ namespace {
 
 constexpr int kBuildThreads = 128;
 
-// The quads of every cell row (one warp per row): the numbers between two rows' bases that no atoms fill are kNoQuad.
-// layer_start (pinned host memory): first slot of every z layer of cells, and the end, by which a caller cuts the sorted
+struct QuadArgs {
+    int nx, ny, rows, n_owned;
+    unsigned* quad;
+    volatile unsigned long long* layer_start;   // pinned host memory, see below
+    unsigned tag;
+};
+
+// The quads of cell row `row` (a warp): the numbers between two rows' bases that no atoms fill are kNoQuad.
+// layer_start: first slot of every z layer of cells, and the end, by which a caller cuts the sorted
 // atoms into slabs; with `tag` in the same word, so that the host sees of each whether it has arrived.
-__global__ void k_quads(int nx, int ny, int rows, int n_owned, const int* __restrict__ cell_start, unsigned* __restrict__ quad,
-                        volatile unsigned long long* layer_start, unsigned tag) {
-    const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (row >= rows) return;
-    const int begin = min(cell_start[static_cast<size_t>(row) * nx], n_owned);
-    const int end = row + 1 < rows ? min(cell_start[static_cast<size_t>(row + 1) * nx], n_owned) : n_owned;
+__device__ __forceinline__ void row_quads(const QuadArgs& a, int row, const int* __restrict__ cell_start) {
+    const int lane = threadIdx.x & 31;
+    if (row >= a.rows) return;
+    const int begin = min(cell_start[static_cast<size_t>(row) * a.nx], a.n_owned);
+    const int end = row + 1 < a.rows ? min(cell_start[static_cast<size_t>(row + 1) * a.nx], a.n_owned) : a.n_owned;
     const int q0 = row == 0 ? 0 : quad_base(begin, row), q1 = quad_base(end, row + 1);
     const int q_first = quad_base(begin, row);
-    const unsigned long long tagged = static_cast<unsigned long long>(tag) << 32;
-    if (lane == 0 && row % ny == 0) layer_start[row / ny] = tagged | static_cast<unsigned>(begin);
-    if (lane == 0 && row + 1 == rows) layer_start[rows / ny] = tagged | static_cast<unsigned>(end);
+    const unsigned long long tagged = static_cast<unsigned long long>(a.tag) << 32;
+    if (lane == 0 && row % a.ny == 0) a.layer_start[row / a.ny] = tagged | static_cast<unsigned>(begin);
+    if (lane == 0 && row + 1 == a.rows) a.layer_start[a.rows / a.ny] = tagged | static_cast<unsigned>(end);
     for (int q = q0 + lane; q < q1; q += 32) {
         const int s = begin + 4 * (q - q_first);
-        quad[q] = (q >= q_first && s < end) ? static_cast<unsigned>(s) * 4u + static_cast<unsigned>(min(end - s, 4) - 1) : kNoQuad;
+        a.quad[q] = (q >= q_first && s < end) ? static_cast<unsigned>(s) * 4u + static_cast<unsigned>(min(end - s, 4) - 1) : kNoQuad;
     }
+}
+
+// Behind the scan of a sort: atoms into the cells' lists (the first place_blocks blocks), quads (the others).
+__global__ void k_place(int place_blocks, int first, int end, const unsigned* __restrict__ key, const int* __restrict__ arrival,
+                        const int* __restrict__ cell_start, int* __restrict__ list, int cells, int* __restrict__ cell_count, QuadArgs quads) {
+    if (!dsmd::after_previous()) return;
+    const int block = static_cast<int>(blockIdx.x) - place_blocks;
+    if (block < 0) dsmd::cell_place(blockIdx.x * blockDim.x + threadIdx.x, place_blocks * blockDim.x, first, end, key, arrival, cell_start, list, cells, cell_count);
+    else row_quads(quads, (block * static_cast<int>(blockDim.x) + static_cast<int>(threadIdx.x)) >> 5, cell_start);
 }
 
 struct ExclusionTable {
@@ -172,6 +187,7 @@ __global__ void __launch_bounds__(kBuildThreads, 8)
 k_build_rows(Grid g, int n_owned, int n_total, int n_quads, const int4* __restrict__ pq, const int* __restrict__ gid,
              ExclusionTable excl, const int* __restrict__ cell_start, const int* __restrict__ ghost_near_lo,
              const int* __restrict__ ghost_near_hi, RowArrays out, int* __restrict__ boundary_pairs, Status* st) {
+    if (!dsmd::after_previous()) return;
     __shared__ int s_slots[kBuildThreads / 32][kCandidates];
     __shared__ __align__(16) ExcludedRange s_ranges[EXCL ? kBuildThreads / 32 : 1];
     const int quad = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;

@@ -248,3 +248,50 @@ def test_loop_equals_step_by_step(cuda_device, n_cells, nt, lagged):
         ends.append(out)
         ctx.close()
     assert np.abs(ends[0] - ends[1]).max() <= 1e-4
+
+
+# cell tables of one block of the scan, of eight and a few more (sums of blocks), of more than it takes (the library's scan)
+@pytest.mark.parametrize("L,cells", [(14.0, 2916), (28.0, 27436), (38.0, 78732), (60.0, 296352), (126.0, 2819876)])
+def test_lists_over_cell_tables_of_every_size(cuda_device, L, cells):
+    n = 1500 if L > 14.0 else 700
+    rng = np.random.default_rng(cells)
+    pos, box = rng.uniform(0.0, L, (n, 3)), np.full(3, L)
+    ctx = capi.Context(20000)
+    ctx.set_box(box)
+    ctx.set_pair_params([[1.0]], [[1.0]], 2.5, 0.3)
+    for _ in range(2):   # the second build finds the counts as the first one left them
+        ctx.upload(pos)
+        ctx.build_neighbor_list()
+        assert ctx.list_stats()["cells"] == cells
+        i, j = ctx.list_pairs()[:2]
+        gid = ctx.download("global_id", n)
+        got = np.sort(np.stack([gid[np.asarray(i)], gid[np.asarray(j)]], 1), axis=1)
+        want = np.sort(co.pairs(*pos.T, n, box, search=2.8), axis=1)
+        got, want = np.unique(got, axis=0), np.unique(want, axis=0)
+        assert np.array_equal(got, want)
+        pos = rng.uniform(0.0, L, (n, 3))
+    ctx.close()
+
+
+def test_rebuild_with_longer_rows_inside_the_loop(cuda_device):
+    """Atoms without forces that fall towards the middle of the box: the loop queues a step behind each list build, and where
+    the rows turn out too short the step must not have happened."""
+    n, L, dt, steps = 4000, 40.0, 0.01, 60
+    rng = np.random.default_rng(7)
+    pos = rng.uniform(0.0, L, (n, 3))
+    vel = (L / 2 - pos) * 1.4
+    ctx = capi.Context(n)
+    ctx.set_box(np.full(3, L))
+    ctx.set_pair_params([[0.0]], [[1.0]], 2.5, 0.6)
+    ctx.upload(pos, vel=vel)
+    ctx.build_neighbor_list()
+    ctx.compute_forces()
+    short = ctx.list_stats()["row_stride"]
+    ctx.run_nve(steps, dt)
+    assert ctx.list_stats()["row_stride"] > short
+    gid = ctx.download("global_id", n)
+    out = np.empty((n, 3))
+    out[gid] = np.stack([ctx.download(k, n) for k in "xyz"], axis=1)
+    d = out - (pos + vel * dt * steps)
+    assert np.abs(d - L * np.round(d / L)).max() <= 1e-9
+    ctx.close()

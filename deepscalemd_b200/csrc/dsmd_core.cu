@@ -63,7 +63,6 @@ constexpr int kLongRow = 240;                         // entries (with the row's
 constexpr int64_t kRowsAlways = 4096;                 // cell rows that any system may have: 2 MB of list rows
 constexpr int kXRefine = 4;    // x cells per cell width of the y and z axes (tighter row windows in the list build)
 enum { kMailDisplacement = 0, kMailKinetic = 4, kMailScalars = 5, kMailBuild = 6, kMailSlots = 7 };   // report slots
-constexpr int kStageAtoms = 16384;
 constexpr unsigned kLinkBlocks = 64;      // blocks of kernels that read or write host memory: enough to fill the link
 // Host-buffer calls: below kPipelineLeast atoms one pass with kernels that read and write the host's memory (131,072 atoms
 // 0.18 ms, slabs 0.25; 262,144 atoms 0.37, slabs 0.36), above it four to eight slabs (1,000,000 atoms 0.86 ms with 4 or 6,
@@ -310,12 +309,15 @@ __global__ void k_upload_defaults(int n, RealArrays r, int* type, int* gid) {
     if (gid) gid[s] = s;
 }
 
-// [n][3] rows, read from pinned host memory, to three arrays.
-__global__ void k_split_rows(int n, const double* __restrict__ rows, double* __restrict__ x, double* __restrict__ y, double* __restrict__ z) {
+// [n][3] rows, n words of them in each of three arrays, to three columns.
+__global__ void k_split_rows(int n, const double* __restrict__ rows0, const double* __restrict__ rows1, const double* __restrict__ rows2,
+                             double* __restrict__ x, double* __restrict__ y, double* __restrict__ z) {
     if (!dsmd::after_previous()) return;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < 3 * n; k += gridDim.x * blockDim.x) {
-        const int s = k / 3, a = k - 3 * s;
-        (a == 0 ? x : (a == 1 ? y : z))[s] = rows[k];
+    const auto word = [&](long long k) { return k < n ? rows0[k] : (k < 2ll * n ? rows1[k - n] : rows2[k - 2ll * n]); };
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
+        x[s] = word(3ll * s);
+        y[s] = word(3ll * s + 1);
+        z[s] = word(3ll * s + 2);
     }
 }
 
@@ -602,8 +604,6 @@ struct dsmd_ctx {
     int disp_pending = -1;                // slot queued by the previous lagged query
     long long build_epoch = 0;            // bumped by every list build (new reference positions)
     cudaEvent_t disp_event[2] = {};
-    double* stage[2] = {};          // pinned: rows of kStageAtoms atoms on their way to the device, in turn
-    cudaEvent_t stage_free[2] = {};
     unsigned char* flag = nullptr;
     unsigned long long* offsets64 = nullptr;
     bool list_valid = false;
@@ -1081,8 +1081,6 @@ void dsmd_destroy(dsmd_ctx* c) {
     for (int k = 0; k < 2; ++k) {
         cudaFreeHost(c->h_disp[k]);
         if (c->disp_event[k]) cudaEventDestroy(c->disp_event[k]);
-        if (c->stage[k]) cudaFreeHost(c->stage[k]);
-        if (c->stage_free[k]) cudaEventDestroy(c->stage_free[k]);
     }
     delete c;
 }
@@ -1224,23 +1222,19 @@ int dsmd_upload(dsmd_ctx* c, int64_t n_owned, int64_t n_total, const double* x, 
     return upload_rest(c, n_owned, n_total, src, false, type, gid, s);
 }
 
-// [n][3] host rows (any memory) to three device arrays, through two pinned buffers: the host copies a piece while the device
-// reads the one before.
-static int upload_columns(dsmd_ctx* c, const double* rows, int64_t n, double* const* to, cudaStream_t s) {
-    for (int64_t first = 0, k = 0; first < n; first += kStageAtoms, ++k) {
-        const int b = static_cast<int>(k & 1), m = static_cast<int>(std::min<int64_t>(kStageAtoms, n - first));
-        if (!c->stage[b]) {
-            DSMD_CUDA(c, cudaMallocHost(&c->stage[b], sizeof(double) * 3 * kStageAtoms));
-            DSMD_CUDA(c, cudaEventCreateWithFlags(&c->stage_free[b], cudaEventDisableTiming));
-        } else {
-            DSMD_CUDA(c, cudaEventSynchronize(c->stage_free[b]));
-        }
-        std::memcpy(c->stage[b], rows + 3 * first, sizeof(double) * 3 * m);
-        dsmd::launch_next(k_split_rows, std::min<unsigned>(blocks_for(3 * m, kThreads), kDeviceSms), kThreads, 0, s, m, c->stage[b], to[0] + first, to[1] + first,
-                                                                                                  to[2] + first);
-        DSMD_LAUNCHED(c);
-        DSMD_CUDA(c, cudaEventRecord(c->stage_free[b], s));
-    }
+// [n][3] host rows (any memory) to three device arrays, through three others of the same size. The runtime's copy out of pageable
+// memory returns when the memory may be used again, and moves 24 GB/s (2.6 MB in 110 us); a copy of our own into pinned buffers that
+// a kernel reads moved 15 (170 us).
+static int upload_columns(dsmd_ctx* c, const double* rows, int64_t n, double* const* to, double* const* scratch, cudaStream_t s) {
+    if (n == 0) return DSMD_OK;
+    for (int k = 0; k < 3; ++k)
+        DSMD_CUDA(c, cudaMemcpyAsync(scratch[k], rows + k * n, sizeof(double) * n, cudaMemcpyHostToDevice, s));
+    dsmd::launch_next(k_split_rows, std::min<unsigned>(blocks_for(n, kThreads), kDeviceSms * 8), kThreads, 0, s, static_cast<int>(n), scratch[0],
+                      scratch[1], scratch[2], to[0], to[1], to[2]);
+    DSMD_LAUNCHED(c);
+    cudaPointerAttributes memory{};
+    if (cudaPointerGetAttributes(&memory, rows) != cudaSuccess) cudaGetLastError();   // not known to the runtime: pageable
+    else if (memory.type != cudaMemoryTypeUnregistered) DSMD_CUDA(c, cudaStreamSynchronize(s));   // the copy has only been queued
     return DSMD_OK;
 }
 
@@ -1250,8 +1244,8 @@ int dsmd_upload_rows(dsmd_ctx* c, int64_t n_owned, int64_t n_total, const double
     if (n_total > c->capacity) return fail(c, DSMD_ERR_CAPACITY, "more atoms than the context's capacity");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     DSMD_CUDA(c, cudaSetDevice(c->device));
-    { const int rc = upload_columns(c, pos, n_total, c->real[c->cur], s); if (rc) return rc; }
-    if (vel) { const int rc = upload_columns(c, vel, n_total, c->real[c->cur] + DSMD_VX, s); if (rc) return rc; }
+    { const int rc = upload_columns(c, pos, n_total, c->real[c->cur], c->real[1 - c->cur], s); if (rc) return rc; }
+    if (vel) { const int rc = upload_columns(c, vel, n_total, c->real[c->cur] + DSMD_VX, c->real[1 - c->cur] + DSMD_VX, s); if (rc) return rc; }
     const double* const src[kNumReal] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, mass, charge};
     return upload_rest(c, n_owned, n_total, src, vel != nullptr, type, gid, s);
 }

@@ -68,8 +68,10 @@ __device__ __forceinline__ double list_distance2(const Grid& g, const double (&p
 // packed behind each other by ballot.
 // What bounds it: instruction issue; 8 to 9 rounds of 32 candidates per quad of a Lennard-Jones liquid (130 of the 250
 // candidates lie inside the list radius of one of the four atoms), about 60 for water. A thread-per-atom walk of the same
-// windows spent 340 warp instructions per atom at 20 of 32 active lanes. Rebuild of 4,000,000 Lennard-Jones atoms 1.79 ms, of
-// 1,048,575 of the mixture 0.59, of 648,000 of water 1.87 (thread per atom: 2.58, 1.02, 5.97 ms).
+// windows spent 340 warp instructions per atom at 20 of 32 active lanes. In small systems the reads of a round: they are under way
+// a round ahead. Rebuild of 4,000,000 Lennard-Jones atoms 1.79 ms, of 1,048,575 of the mixture 0.585, of 648,000 of water 1.83, of
+// 3,993 0.069 (without reading ahead 1.80, 0.595, 1.88, 0.073; thread per atom: 2.58, 1.02, 5.97 ms). Blocks per SM: eight with
+// exclusions (seven 1.89 ms for water), seven without (eight 0.603 ms for the mixture).
 constexpr int kCandidates = 512;   // candidates numbered at a time (per warp, in shared memory)
 
 struct QuadSearch {
@@ -101,12 +103,19 @@ __device__ __forceinline__ void test_candidates(const Grid& g, QuadSearch& q, in
     const int lane = threadIdx.x & 31;
     const unsigned lt_mask = (1u << lane) - 1u;
     const unsigned own_first = static_cast<unsigned>(min(q.n_atoms, 2)), own_second = static_cast<unsigned>(max(q.n_atoms - 2, 0));
-    int s_next = lane < n ? s_slot[lane] : q.first;   // a round ahead
+    // the next round's candidate is on its way while this one is tested, and its slot a round before that
+    int s_next = lane < n ? s_slot[lane] : q.first;
+    int4 c_next = __ldg(&pq[s_next]);
+    int g_next = EXCL ? __ldg(&gid[s_next]) : 0;
+    int s_after = lane + 32 < n ? s_slot[lane + 32] : q.first;
     for (int t = lane; t - lane < n; t += 32) {
         const bool valid = t < n;
-        const int s = s_next;
-        const int4 c = __ldg(&pq[s]);
-        s_next = t + 32 < n ? s_slot[t + 32] : q.first;
+        const int s = s_next, gj = g_next;
+        const int4 c = c_next;
+        s_next = s_after;
+        c_next = __ldg(&pq[s_next]);
+        if (EXCL) g_next = __ldg(&gid[s_next]);
+        s_after = t + 64 < n ? s_slot[t + 64] : q.first;
         float r[4];
         if (NEAR) {
             const F2 rx = both(dsmd::fixed_delta(c.x, q.x, g.scale[0]));
@@ -140,7 +149,6 @@ __device__ __forceinline__ void test_candidates(const Grid& g, QuadSearch& q, in
         if (EXCL) {
             // a candidate inside the range of ids that one of the four atoms excludes (molecules are numbered together: few
             // are) is looked up in the atom's table row; the row's end holds those that are excluded for one of its atoms
-            const int gj = __ldg(&gid[s]);
             const int4 lo = *reinterpret_cast<const int4*>(s_excluded.lo);
             const uint4 span = *reinterpret_cast<const uint4*>(s_excluded.span);
             const bool look = static_cast<unsigned>(gj - lo.x) <= span.x || static_cast<unsigned>(gj - lo.y) <= span.y ||
@@ -183,7 +191,7 @@ __device__ __forceinline__ void test_candidates(const Grid& g, QuadSearch& q, in
 }
 
 template <bool EXCL, int ORDER>
-__global__ void __launch_bounds__(kBuildThreads, 8)
+__global__ void __launch_bounds__(kBuildThreads, EXCL ? 8 : 7)
 k_build_rows(Grid g, int n_owned, int n_total, int n_quads, const int4* __restrict__ pq, const int* __restrict__ gid,
              ExclusionTable excl, const int* __restrict__ cell_start, const int* __restrict__ ghost_near_lo,
              const int* __restrict__ ghost_near_hi, RowArrays out, int* __restrict__ boundary_pairs, Status* st) {

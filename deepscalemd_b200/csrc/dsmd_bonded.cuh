@@ -91,12 +91,20 @@ struct BondedForces {
     const double* contrib;
 };
 
-__device__ __forceinline__ void bonded_force(const BondedForces& b, int s, double (&f)[3]) {
-    f[0] = f[1] = f[2] = 0.0;
+struct BondedRange {
+    long long begin, end;
+};
+
+__device__ __forceinline__ BondedRange bonded_range(const BondedForces& b, int s) {
     const int g = b.gid[s];
-    if (g < 0 || g >= b.n_global) return;
-    const double* c = b.contrib + 3ll * b.entries_of[g];
-    const double* end = b.contrib + 3ll * b.entries_of[g + 1];
+    if (g < 0 || g >= b.n_global) return BondedRange{0, 0};
+    return BondedRange{b.entries_of[g], b.entries_of[g + 1]};
+}
+
+__device__ __forceinline__ void bonded_force(const BondedForces& b, const BondedRange& range, double (&f)[3]) {
+    f[0] = f[1] = f[2] = 0.0;
+    const double* c = b.contrib + 3ll * range.begin;
+    const double* end = b.contrib + 3ll * range.end;
 #pragma unroll 4
     for (; c < end; c += 3) {
         f[0] += c[0]; f[1] += c[1]; f[2] += c[2];
@@ -280,7 +288,7 @@ __global__ void k_bonded_gather(int n_owned, BondedForces b, double* __restrict_
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n_owned) return;
     double f[3];
-    bonded_force(b, s, f);
+    bonded_force(b, bonded_range(b, s), f);
     fx[s] += f[0]; fy[s] += f[1]; fz[s] += f[2];
 }
 

@@ -281,18 +281,19 @@ struct AtomArrays {
 // FINISH: v += half_kick f / m, RATTLE; START: v += half_kick f / m, x += dt v, SHAKE, fixed point, displacement check (of
 // the drifted position and of the corrected one). virial (may be null): the diagonal of the constraint virial of RATTLE,
 // -2 / (force_to_accel dt) * sum over corrections of k r_a^2 (`prefactor`).
+// behind_forces: the launch before is the force kernel, which has waited for all before itself and writes nothing but forces: the atoms'
+// state is read while it ends.
 template <class Shape, bool FINISH, bool START>
 __global__ void __launch_bounds__(128) k_constrained(ClusterTable t, Grid g, AtomArrays at, double half_kick, double dt, double tolerance,
                                                      int max_iterations, double prefactor, double* __restrict__ partials, unsigned* __restrict__ ticket,
-                                                     double* __restrict__ virial, DisplacementReport report) {
-    if (!dsmd::after_previous()) return;
-    if (START && dsmd::gate_closed(report.st, report.gate2)) return;
+                                                     double* __restrict__ virial, DisplacementReport report, bool behind_forces) {
+    if (!behind_forces && !dsmd::after_previous()) return;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     double wsum[3] = {0.0, 0.0, 0.0}, worst2 = 0.0;
+    Cluster<Shape> c;
+    c.n = 0;
+    double a[Shape::atoms][3];   // half_kick f / m
     if (k < t.n_clusters) {
-        Cluster<Shape> c;
-        c.n = 0;
-        double a[Shape::atoms][3];   // half_kick f / m
 #pragma unroll
         for (int m = 0; m < Shape::atoms; ++m) {
             const int s = t.atom_slot[k * kClusterAtoms + m];
@@ -301,9 +302,20 @@ __global__ void __launch_bounds__(128) k_constrained(ClusterTable t, Grid g, Ato
             c.n = m + 1;
             c.p[m][0] = at.x[s]; c.p[m][1] = at.y[s]; c.p[m][2] = at.z[s];
             c.v[m][0] = at.vx[s]; c.v[m][1] = at.vy[s]; c.v[m][2] = at.vz[s];
-            c.w[m] = 1.0 / at.mass[s];
+            const double mass = at.mass[s];
+            c.w[m] = 1.0 / mass;
+            a[m][0] = half_kick / mass;
+        }
+    }
+    if (behind_forces && !dsmd::after_previous()) return;
+    if (START && dsmd::gate_closed(report.st, report.gate2)) return;
+    if (k < t.n_clusters) {
+#pragma unroll
+        for (int m = 0; m < Shape::atoms; ++m) {
+            const int s = c.slot[m];
+            if (!Shape::known && s < 0) continue;
             if (half_kick != 0.0) {
-                const double h = half_kick / at.mass[s];
+                const double h = a[m][0];
                 a[m][0] = h * at.fx[s]; a[m][1] = h * at.fy[s]; a[m][2] = h * at.fz[s];
             } else {
                 a[m][0] = a[m][1] = a[m][2] = 0.0;

@@ -355,7 +355,8 @@ namespace {
 // INTEGRATE: kick and drift before the pack (v += kick_c f / m, x += dt v): the first velocity-Verlet half with
 // kick_c = dt/2 (times the force-to-acceleration factor), or, with kick_c = dt, the second half of the previous step and
 // the first half of this one in one pass (both use the same forces).
-// BONDED: the forces of the bonded terms are not in the force arrays yet.
+// BONDED: the forces of the bonded terms are not in the force arrays yet; the launches before are the force kernel and the bonded terms
+// beside it, which write nothing but forces and have waited for all before them: the atoms' state is read while they end.
 template <bool INTEGRATE, bool BONDED>
 __global__ void k_pack(Grid g, int first, int count, int n_owned, double* __restrict__ x, double* __restrict__ y,
                        double* __restrict__ z, double* __restrict__ vx, double* __restrict__ vy,
@@ -364,18 +365,30 @@ __global__ void k_pack(Grid g, int first, int count, int n_owned, double* __rest
                        const double* __restrict__ xref, const double* __restrict__ yref,
                        const double* __restrict__ zref, int4* __restrict__ pq, double dt, double kick_c,
                        ClusterMembers skip, BondedForces bonded, DisplacementReport report) {
-    if (!dsmd::after_previous()) return;
-    if (dsmd::gate_closed(report.st, report.gate2)) return;
+    if (!BONDED && !dsmd::after_previous()) return;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int s = first + t;
     double d2 = 0.0;
+    double state[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};   // BONDED: x, y, z, kick_c / mass, vx, vy, vz
+    BondedRange range{};
+    if (BONDED) {   // while the forces before end
+        if (t < count) {
+            state[0] = x[s]; state[1] = y[s]; state[2] = z[s];
+            state[3] = kick_c / mass[s];
+            state[4] = vx[s]; state[5] = vy[s]; state[6] = vz[s];
+            range = bonded_range(bonded, s);
+        }
+        if (!dsmd::after_previous()) return;
+    }
+    if (dsmd::gate_closed(report.st, report.gate2)) return;
     if (t < count && !skip.has(s)) {
-        double px = x[s], py = y[s], pz = z[s];
+        double px = BONDED ? state[0] : x[s], py = BONDED ? state[1] : y[s], pz = BONDED ? state[2] : z[s];
         if (INTEGRATE) {
-            const double a = kick_c / mass[s];
+            const double a = BONDED ? state[3] : kick_c / mass[s];
             double f[3] = {0.0, 0.0, 0.0};
-            if (BONDED) bonded_force(bonded, s, f);
-            const double ux = vx[s] + a * (fx[s] + f[0]), uy = vy[s] + a * (fy[s] + f[1]), uz = vz[s] + a * (fz[s] + f[2]);
+            if (BONDED) bonded_force(bonded, range, f);
+            const double ux = (BONDED ? state[4] : vx[s]) + a * (fx[s] + f[0]), uy = (BONDED ? state[5] : vy[s]) + a * (fy[s] + f[1]),
+                         uz = (BONDED ? state[6] : vz[s]) + a * (fz[s] + f[2]);
             vx[s] = ux; vy[s] = uy; vz[s] = uz;
             px += dt * ux; py += dt * uy; pz += dt * uz;
             x[s] = px; y[s] = py; z[s] = pz;
@@ -603,6 +616,8 @@ struct dsmd_ctx {
     long long disp_epoch[2] = {-1, -1};   // list build each read-back slot was measured under
     int disp_pending = -1;                // slot queued by the previous lagged query
     long long build_epoch = 0;            // bumped by every list build (new reference positions)
+    long long settled_epoch = -1;         // list build, and stream, of the last force launch (list_settled)
+    cudaStream_t settled_stream = nullptr;
     cudaEvent_t disp_event[2] = {};
     unsigned char* flag = nullptr;
     unsigned long long* offsets64 = nullptr;
@@ -1567,6 +1582,15 @@ int dsmd_max_displacement_sq_lagged(dsmd_ctx* c, double* out, void* stream) {
     return DSMD_OK;
 }
 
+// Whether the force launch about to be made in `s` may read the list before the launch before it has ended: a force launch in the same
+// stream came between the build and this one, and has itself waited for the build. (Never in a graph, whose edges are its own.)
+static bool list_settled(dsmd_ctx* c, cudaStream_t s) {
+    const bool settled = !c->captured && c->settled_epoch == c->build_epoch && c->settled_stream == s;
+    c->settled_epoch = c->build_epoch;
+    c->settled_stream = s;
+    return settled;
+}
+
 static PairParams pair_params(const dsmd_ctx* c) {
     PairParams p{};
     for (int a = 0; a < 3; ++a) p.scale[a] = c->grid.scale[a];
@@ -1609,7 +1633,7 @@ static int compute_forces_impl(dsmd_ctx* c, int phase, int want_energy, int64_t 
     double** r = c->real[c->cur];
     const ForceArgs a{c->pq, c->qf, rows_of(c), phase, phase == DSMD_PHASE_BOUNDARY ? c->boundary_pairs : nullptr,
                       static_cast<int>(ranged ? first : 0), static_cast<int>(pairs), c->lane_shift, r[DSMD_FX], r[DSMD_FY], r[DSMD_FZ], c->partials,
-                      c->tickets, c->scalars, report ? c->mail + kMailScalars : nullptr, report ? ++c->seq : 0, c->status, c->gate2};
+                      c->tickets, c->scalars, report ? c->mail + kMailScalars : nullptr, report ? ++c->seq : 0, c->status, c->gate2, list_settled(c, s)};
     if (e && pairs > 0) c->scalars_seq = a.seq;
     if (pairs > 0) {   // else nothing to add to the forces; the energy sums of a boundary pass stay as the interior pass left them
         const unsigned blocks = static_cast<unsigned>(pair_blocks(c, pairs, e));
@@ -1631,7 +1655,7 @@ static int force_step(dsmd_ctx* c, double dt, double f2a, cudaStream_t s) {
     const int64_t pairs = 2 * c->n_quads;
     double** r = c->real[c->cur];
     const ForceArgs a{c->pq, c->qf, rows_of(c), DSMD_PHASE_FULL, nullptr, 0, static_cast<int>(pairs), c->lane_shift,
-                      nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, c->status, c->gate2};
+                      nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, c->status, c->gate2, list_settled(c, s)};
     const StepArgs at{r[0], r[1], r[2], r[3], r[4], r[5], r[9], c->ref[0], c->ref[1], c->ref[2], c->pq_next, dt, dt * f2a};
     const unsigned blocks = static_cast<unsigned>(pair_blocks(c, pairs, false));
     const DisplacementReport report = displacement_report(c, true, s);
@@ -1690,7 +1714,8 @@ int ensure_slot_map(dsmd_ctx* c, cudaStream_t s) {
     return DSMD_OK;
 }
 
-int launch_constrained(dsmd_ctx* c, bool finish, bool start, double half_kick, double dt, double prefactor, double* d_virial3, cudaStream_t s) {
+int launch_constrained(dsmd_ctx* c, bool finish, bool start, double half_kick, double dt, double prefactor, double* d_virial3, bool behind_forces,
+                       cudaStream_t s) {
     double** r = c->real[c->cur];
     const AtomArrays at{r[0], r[1], r[2], r[3], r[4], r[5], r[6], r[7], r[8], r[9], c->type[c->cur], c->ref[0], c->ref[1], c->ref[2], c->pq};
     const unsigned blocks = blocks_for(c->n_clusters, 128);
@@ -1699,7 +1724,7 @@ int launch_constrained(dsmd_ctx* c, bool finish, bool start, double half_kick, d
         const auto kernel = finish && start ? k_constrained<decltype(shape), true, true>
                                             : (finish ? k_constrained<decltype(shape), true, false> : k_constrained<decltype(shape), false, true>);
         dsmd::launch_next(kernel, blocks, 128, 0, s, cluster_table(c), c->grid, at, half_kick, dt, c->cons_tolerance, c->cons_max_iterations, prefactor,
-                                      c->partials, c->tickets + 3, d_virial3, report);
+                                      c->partials, c->tickets + 3, d_virial3, report, behind_forces);
     };
     if (c->cl_shape == 1) launch(TriangleCluster());
     else if (c->cl_shape == 2) launch(BondCluster());
@@ -1710,10 +1735,12 @@ int launch_constrained(dsmd_ctx* c, bool finish, bool start, double half_kick, d
 
 // The velocity-Verlet halves of a system with constraints: the second half of a step with RATTLE (finish), the first half
 // with SHAKE (start), or both in one pass (a second half and the first half of the next step, the same forces).
-int constrained_halves(dsmd_ctx* c, bool finish, bool start, double dt, double f2a, cudaStream_t s) {
+// behind_forces: the launch before was the force kernel, in the same stream.
+int constrained_halves(dsmd_ctx* c, bool finish, bool start, double dt, double f2a, bool behind_forces, cudaStream_t s) {
+    behind_forces = behind_forces && c->slot_map_valid;
     { const int rc = ensure_slot_map(c, s); if (rc) return rc; }
     const double half_kick = 0.5 * dt * f2a;
-    const int rc = launch_constrained(c, finish, start, half_kick, dt, 0.0, nullptr, s);
+    const int rc = launch_constrained(c, finish, start, half_kick, dt, 0.0, nullptr, behind_forces, s);
     if (rc || c->cl_atoms == c->n_owned) return rc;
     // the free atoms
     const ClusterMembers members{c->cl_member, static_cast<int>(c->cons_n_global), c->gid[c->cur]};
@@ -1728,7 +1755,7 @@ int constrained_halves(dsmd_ctx* c, bool finish, bool start, double dt, double f
 int rattle_impl(dsmd_ctx* c, double dt, double f2a, double* d_virial3, cudaStream_t s) {
     { const int rc = ensure_slot_map(c, s); if (rc) return rc; }
     if (d_virial3) { const int rc = ensure_partials(c, blocks_for(c->n_clusters, 128)); if (rc) return rc; }
-    return launch_constrained(c, true, false, 0.0, dt, -2.0 / (f2a * dt), d_virial3, s);
+    return launch_constrained(c, true, false, 0.0, dt, -2.0 / (f2a * dt), d_virial3, false, s);
 }
 
 }  // namespace
@@ -1854,7 +1881,7 @@ int dsmd_integrate(dsmd_ctx* c, int half, double dt, double f2a, void* stream) {
         if (constrained) return fail(c, DSMD_ERR_STATE, "the merged half steps are not available with constraints");
         return pack_impl(c, 0, c->n_owned, true, dt, f2a, s, 1.0);
     }
-    if (constrained) return constrained_halves(c, half == 2, half == 1, dt, f2a, s);
+    if (constrained) return constrained_halves(c, half == 2, half == 1, dt, f2a, false, s);
     if (half == 1) return pack_impl(c, 0, c->n_owned, true, dt, f2a, s);
     double** r = c->real[c->cur];
     dsmd::launch_next(k_vv2, blocks_for(c->n_owned, kThreads), kThreads, 0, s, static_cast<int>(c->n_owned), 0.5 * dt * f2a, r[3], r[4],
@@ -2126,7 +2153,7 @@ int dsmd_run_nve(dsmd_ctx* c, int64_t n_steps, double dt, double f2a, double hi_
                 if (!rc) rc = pack_impl(c, 0, c->n_owned, true, dt, f2a, s, 1.0, {}, &terms);
             } else {
                 if (!rc) rc = dsmd_compute_bonded(c, s);
-                if (!rc) rc = constrained ? constrained_halves(c, true, true, dt, f2a, s) : dsmd_integrate(c, 3, dt, f2a, s);
+                if (!rc) rc = constrained ? constrained_halves(c, true, true, dt, f2a, c->bonded.terms() == 0, s) : dsmd_integrate(c, 3, dt, f2a, s);
             }
         }
         c->gate2 = HUGE_VAL;

@@ -68,6 +68,7 @@ struct ForceArgs {
     unsigned long long seq;
     const Status* st;
     double gate2;            // see gate_closed
+    bool list_settled;       // the list was complete before the launch before this one began: it may be read without waiting
 };
 
 struct StepArgs {

@@ -357,6 +357,38 @@ __device__ __forceinline__ int afresh(int t) {
     return t;
 }
 
+// What a lane knows of its row from the list alone.
+struct RowHead {
+    int pair, first, atoms;   // no atoms: no row
+    int c, c_end;             // this lane's first chunk of entries, one past the row's last
+    unsigned special;
+    uint4 e;                  // the first chunk
+};
+
+template <int ORDER>
+__device__ __forceinline__ const uint4* row_chunks(const ForceArgs& a, int pair, int sub) {
+    return reinterpret_cast<const uint4*>(a.rows.rows + row_base<ORDER>(static_cast<unsigned>(pair), a.rows.stride)) + (sub & ((1 << ORDER) - 1));
+}
+
+template <int ORDER>
+__device__ __forceinline__ RowHead open_row(const ForceArgs& a, int t) {
+    const int sub = t & ((1 << a.lane_shift) - 1);
+    RowHead h{};
+    h.pair = row_of_thread(a, t);
+    if (h.pair < 0) return h;
+    h.atoms = pair_atoms(a.rows.quad, h.pair, h.first);
+    const int mid = a.rows.row_int[h.pair], end = a.rows.row_end[h.pair];
+    h.special = a.rows.row_special[h.pair];
+    // Chunks of entries, in groups of as many as lie side by side: those of owned partners, of ghosts, or all (what lies between
+    // the two kinds are atoms out of reach).
+    h.c = sub;
+    if (a.phase == DSMD_PHASE_BOUNDARY) h.c += whole_groups<ORDER>(mid) >> 2;
+    h.c_end = whole_groups<ORDER>(a.phase == DSMD_PHASE_INTERIOR ? mid : max(mid, end)) >> 2;
+    if (h.special & kRowCareful) h.c_end = 0;
+    if (h.c < h.c_end) h.e = __ldcs(row_chunks<ORDER>(a, h.pair, sub) + (h.c >> ORDER) * size_t(32));
+    return h;
+}
+
 // Forces on the atoms of one pair row, worked on by 2^lane_shift lanes of a warp, which take the row's chunks of four entries in
 // turn; the row's sums, in all its lanes. The next chunk of entries and the partners of the current one are in flight before
 // any arithmetic starts; the list is streamed with an evict-first hint so that the positions stay in L2.
@@ -366,7 +398,7 @@ __device__ __forceinline__ int afresh(int t) {
 // (src/force_calculator_cuda.cu:1784-1789).
 template <int COPIES, bool ENERGY, int TYPES, bool SWITCH, bool QTYPE, int ORDER>
 __device__ __forceinline__ void row_forces(const PairParams& p, const ForceArgs& a, const PairTables<COPIES, ENERGY, TYPES, QTYPE>& tables,
-                                           int t, float (&sum_a)[3], float (&sum_b)[3], double (&v)[6]) {
+                                           int t, const RowHead& head, float (&sum_a)[3], float (&sum_b)[3], double (&v)[6]) {
     constexpr bool COULOMB = COPIES > 0, few = TYPES == kFewTypes, many = TYPES == kManyTypes, by_type = COULOMB && QTYPE;
     constexpr bool two_types = TYPES == kTwoTypes;
     const int nt = p.ntypes, lanes = 1 << a.lane_shift, sub = t & (lanes - 1);
@@ -374,12 +406,11 @@ __device__ __forceinline__ void row_forces(const PairParams& p, const ForceArgs&
     PairAccumulator<COPIES, ENERGY, SWITCH> acc;
     bool close = false;   // the row has a pair below the Ewald table
     bool two = false;     // the row has two atoms
-    int first = 0;
-    const int pair = row_of_thread(a, t), atoms = pair >= 0 ? pair_atoms(a.rows.quad, pair, first) : 0;
+    const int first = head.first, atoms = head.atoms;
     if (atoms > 0) {
         const int4 pa = a.pq[first], pb = a.pq[first + atoms - 1];
-        const unsigned special = a.rows.row_special[pair];
-        const uint4* row = reinterpret_cast<const uint4*>(a.rows.rows + row_base<ORDER>(static_cast<unsigned>(pair), a.rows.stride)) + (sub & ((1 << ORDER) - 1));
+        const unsigned special = head.special;
+        const uint4* row = row_chunks<ORDER>(a, head.pair, sub);
         F2 q{0};
         PairTerms one{};
         const int row3 = (pa.w * nt + pb.w) * nt;
@@ -424,17 +455,9 @@ __device__ __forceinline__ void row_forces(const PairParams& p, const ForceArgs&
         const auto add = [&](const int4& pos, float charge) {
             acc.template add_partner<false>(p, table, pa, pb, pos, terms(pos.w, charge), 0u);
         };
-        // Chunks of entries, in groups of as many as lie side by side: those of owned partners, of ghosts, or all (what lies between
-        // the two kinds are atoms out of reach).
-        int c = sub, c_end;
-        {
-            const int mid = a.rows.row_int[pair], end = a.rows.row_end[pair];
-            if (a.phase == DSMD_PHASE_BOUNDARY) c += whole_groups<ORDER>(mid) >> 2;
-            c_end = whole_groups<ORDER>(a.phase == DSMD_PHASE_INTERIOR ? mid : max(mid, end)) >> 2;
-        }
-        if (special & kRowCareful) c_end = 0;
-        uint4 e{};
-        if (c < c_end) e = __ldcs(row + (c >> ORDER) * size_t(32));
+        int c = head.c;
+        const int c_end = head.c_end;
+        uint4 e = head.e;
         {   // the two atoms themselves: each is the other's partner
             two = atoms > 1;
             const bool own = two && a.phase != DSMD_PHASE_BOUNDARY && !(special & (kRowOwnExcluded | kRowCareful));
@@ -529,11 +552,15 @@ template <int COPIES, bool ENERGY, int TYPES, bool SWITCH, bool QTYPE, int ORDER
 __global__ void __launch_bounds__((kPairThreads<COPIES, TYPES>), (kPairBlocks<COPIES, TYPES, ENERGY>)) k_pair(PairParams p, ForceArgs a) {
     extern __shared__ float4 smem[];
     const PairTables<COPIES, ENERGY, TYPES, QTYPE> tables(p, smem);   // parameters: no kernel writes them
+    const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
+    RowHead head{};
+    if (a.list_settled) head = open_row<ORDER>(a, t0);   // while the launch before this one ends
     if (!dsmd::after_previous() || (!ENERGY && dsmd::gate_closed(a.st, a.gate2))) return;
     double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};   // energy, virial and its diagonal, pairs
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; (t & ~31) >> a.lane_shift < a.n_pairs; t += gridDim.x * blockDim.x) {
+    for (int t = t0; (t & ~31) >> a.lane_shift < a.n_pairs; t += gridDim.x * blockDim.x) {
+        if (t != t0 || !a.list_settled) head = open_row<ORDER>(a, t);
         float sum_a[3], sum_b[3];
-        row_forces<COPIES, ENERGY, TYPES, SWITCH, QTYPE, ORDER>(p, a, tables, t, sum_a, sum_b, v);
+        row_forces<COPIES, ENERGY, TYPES, SWITCH, QTYPE, ORDER>(p, a, tables, t, head, sum_a, sum_b, v);
         const int t2 = afresh(t), pair = row_of_thread(a, t2), sub = t2 & ((1 << a.lane_shift) - 1);
         int first = 0;
         const int atoms = pair >= 0 ? pair_atoms(a.rows.quad, pair, first) : 0;
@@ -566,11 +593,14 @@ __global__ void __launch_bounds__((kPairThreads<0, TYPES>), (kPairBlocks<0, TYPE
 k_step(PairParams p, ForceArgs a, Grid g, StepArgs at, DisplacementReport report) {
     extern __shared__ float4 smem[];
     const PairTables<0, false, TYPES, false> tables(p, smem);   // parameters: no kernel writes them
-    if (!dsmd::after_previous() || dsmd::gate_closed(report.st, report.gate2)) return;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    RowHead head{};
+    if (a.list_settled) head = open_row<ORDER>(a, t);   // while the launch before this one ends
+    if (!dsmd::after_previous() || dsmd::gate_closed(report.st, report.gate2)) return;
+    if (!a.list_settled) head = open_row<ORDER>(a, t);
     float sum_a[3], sum_b[3];
     double unused[6];
-    row_forces<0, false, TYPES, SWITCH, false, ORDER>(p, a, tables, t, sum_a, sum_b, unused);
+    row_forces<0, false, TYPES, SWITCH, false, ORDER>(p, a, tables, t, head, sum_a, sum_b, unused);
     const int t2 = afresh(t), pair = row_of_thread(a, t2), sub = t2 & ((1 << a.lane_shift) - 1);
     int first = 0;
     const int atoms = pair >= 0 ? pair_atoms(a.rows.quad, pair, first) : 0;

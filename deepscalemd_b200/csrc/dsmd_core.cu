@@ -59,6 +59,10 @@ constexpr int kDeviceSms = 148;                       // of a B200
 // with twice as many 17.4, 20.7, 27.2 and 33.4 us, with half as many 12.0, 14.1, 19.2 and 33.3 us.
 constexpr int64_t kPairLanesWanted = kDeviceSms * 512;
 constexpr int64_t kPairLanesWantedEwald = kDeviceSms * 768;   // one and a half rounds of one block of 512 each
+// Atoms up to which the last block of a displacement check reports it; beyond, a launch of its own does, and no block waits for its
+// writes to arrive before it takes its ticket and makes room for the next. Steps of 130,000, 260,000, 1,000,000 and 4,000,000
+// Lennard-Jones atoms: 22.8, 39.8, 118 and 441 us, with tickets 23.9, 42.3, 121 and 455; of 64,000 a launch is dearer than the tickets.
+constexpr int64_t kTicketMost = 100000;
 constexpr int kLongRow = 240;                         // entries (with the row's spare room): about 150 partners per atom
 constexpr int64_t kRowsAlways = 4096;                 // cell rows that any system may have: 2 MB of list rows
 constexpr int kXRefine = 4;    // x cells per cell width of the y and z axes (tighter row windows in the list build)
@@ -180,6 +184,11 @@ __global__ void k_copy_back(int first, int count, RealArrays from, RealArrays to
     for (int f = 0; f < kNumReal; ++f) to.p[f][s] = from.p[f][s];
     type_to[s] = type_from[s];
     gid_to[s] = gid_from[s];
+}
+
+__global__ void k_post_displacement(DisplacementReport r) {
+    if (!dsmd::after_previous() || dsmd::gate_closed(r.st, r.gate2)) return;
+    post_displacement(r);
 }
 
 // The end of a list build: its status goes to the host (atoms outside, dropped, need_stride, boundary_pairs), and the status words
@@ -1002,7 +1011,15 @@ DisplacementReport displacement_report(dsmd_ctx* c, bool all_atoms, cudaStream_t
     if (!all_atoms || !reports_count(c, s)) return DisplacementReport{c->status, nullptr, nullptr, 0, c->gate2};
     c->disp_seq = ++c->seq;
     const int slot = static_cast<int>(c->seq & 3);
-    return DisplacementReport{c->status, c->tickets + 4 + slot, c->mail + kMailDisplacement + slot, c->seq, c->gate2};
+    return DisplacementReport{c->status, c->n_owned > kTicketMost ? nullptr : c->tickets + 4 + slot, c->mail + kMailDisplacement + slot, c->seq, c->gate2};
+}
+
+// Behind the launch that was given `report`.
+int displacement_posted(dsmd_ctx* c, const DisplacementReport& report, cudaStream_t s) {
+    if (!report.mail || report.ticket) return DSMD_OK;
+    dsmd::launch_next(k_post_displacement, 1, 1, 0, s, report);
+    DSMD_LAUNCHED(c);
+    return DSMD_OK;
 }
 
 int read_status(dsmd_ctx* c, cudaStream_t s) {
@@ -1532,7 +1549,7 @@ static int pack_impl(dsmd_ctx* c, int64_t first, int64_t count, bool integrate, 
         r[6], r[7], r[8], r[9], c->type[c->cur], c->ref[0], c->ref[1], c->ref[2], c->pq, dt, kick * dt * f2a, skip,
         bonded ? *bonded : BondedForces{}, report);
     DSMD_LAUNCHED(c);
-    return DSMD_OK;
+    return displacement_posted(c, report, s);
 }
 
 int dsmd_pack_positions(dsmd_ctx* c, int64_t first, int64_t count, void* stream) {
@@ -1663,7 +1680,7 @@ static int force_step(dsmd_ctx* c, double dt, double f2a, cudaStream_t s) {
     DSMD_CUDA(c, launch(p, a, c->grid, at, report, c->switch_distance > 0.0, blocks, s));
     ++c->launches;
     std::swap(c->pq, c->pq_next);
-    return DSMD_OK;
+    return displacement_posted(c, report, s);
 }
 
 int dsmd_compute_forces(dsmd_ctx* c, int phase, int want_energy, void* stream) {
@@ -1730,7 +1747,7 @@ int launch_constrained(dsmd_ctx* c, bool finish, bool start, double half_kick, d
     else if (c->cl_shape == 2) launch(BondCluster());
     else launch(AnyCluster());
     DSMD_LAUNCHED(c);
-    return DSMD_OK;
+    return displacement_posted(c, report, s);
 }
 
 // The velocity-Verlet halves of a system with constraints: the second half of a step with RATTLE (finish), the first half

@@ -23,7 +23,7 @@ struct RowArrays {
 // Who writes where when a displacement check ends.
 struct DisplacementReport {
     Status* st;
-    unsigned* ticket;      // blocks that have finished
+    unsigned* ticket;      // blocks that have finished, or null: see report_displacement
     Mail* mail;            // or null: no report
     unsigned long long seq;
     double gate2;          // see gate_closed

@@ -586,7 +586,7 @@ __global__ void __launch_bounds__((kPairThreads<COPIES, TYPES>), (kPairBlocks<CO
 // The force pass of a step and what follows it up to the next force pass, for loops in which nobody reads forces or
 // velocities in between: v += kick f / m, x += dt v, fixed-point positions of the next step (into the other buffer: rows
 // still read this one's), displacement check. A separate pass would read and write the forces and read everything else again
-// (172 bytes per atom, 0.11 ms at 4,000,000 atoms beside 0.356 for the forces; this kernel 0.455, the blocks' ends being little
+// (172 bytes per atom, 0.11 ms at 4,000,000 atoms beside 0.356 for the forces; this kernel 0.441, the blocks' ends being little
 // hidden by other blocks' force arithmetic), and a small system's step is one launch.
 template <int TYPES, bool SWITCH, int ORDER>
 __global__ void __launch_bounds__((kPairThreads<0, TYPES>), (kPairBlocks<0, TYPES, false>))

@@ -9,11 +9,25 @@ using dsmd::DisplacementReport;
 using dsmd::Mail;
 using dsmd::post;
 
-// The block's largest squared displacement goes into the status word; the last block of the grid reports the word.
+// The status word with the largest squared displacement goes to the host and becomes the gate of the launches behind.
+__device__ __forceinline__ void post_displacement(const DisplacementReport& r) {   // one thread
+    const double out[2] = {__longlong_as_double(static_cast<long long>(__ldcg(&r.st->max_disp2))), static_cast<double>(__ldcg(&r.st->out_of_domain))};
+    r.st->gate = out[1] != 0.0 ? __longlong_as_double(0x7FF0000000000000ll) : out[0];
+    post(r.mail, out, 2, r.seq);
+}
+
+// The block's largest squared displacement goes into the status word. With a ticket the last block of the grid reports the word.
+// Without one (large grids) nothing waits for anything: every warp adds its own, if it is larger than what it reads there, and a
+// launch behind this one reports the word (k_post_displacement).
 __device__ __forceinline__ void report_displacement(double v, const DisplacementReport& r) {
     for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
-    __shared__ double warp_max[32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (!r.ticket) {
+        const unsigned long long bits = static_cast<unsigned long long>(__double_as_longlong(v));
+        if (lane == 0 && v > 0.0 && bits > __ldcg(&r.st->max_disp2)) atomicMax(&r.st->max_disp2, bits);
+        return;
+    }
+    __shared__ double warp_max[32];
     if (lane == 0) warp_max[w] = v;
     __syncthreads();
     if (w == 0) {
@@ -21,16 +35,11 @@ __device__ __forceinline__ void report_displacement(double v, const Displacement
         for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
         if (lane == 0) {
             if (v > 0.0) atomicMax(&r.st->max_disp2, static_cast<unsigned long long>(__double_as_longlong(v)));
-            if (r.mail) {
+            __threadfence();
+            if (atomicAdd(r.ticket, 1u) == gridDim.x - 1) {
                 __threadfence();
-                if (atomicAdd(r.ticket, 1u) == gridDim.x - 1) {
-                    __threadfence();
-                    const double out[2] = {__longlong_as_double(static_cast<long long>(__ldcg(&r.st->max_disp2))),
-                                           static_cast<double>(__ldcg(&r.st->out_of_domain))};
-                    *r.ticket = 0u;
-                    r.st->gate = out[1] != 0.0 ? __longlong_as_double(0x7FF0000000000000ll) : out[0];
-                    post(r.mail, out, 2, r.seq);
-                }
+                *r.ticket = 0u;
+                post_displacement(r);
             }
         }
     }

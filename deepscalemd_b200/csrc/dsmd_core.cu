@@ -55,9 +55,12 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kDeviceSms = 148;                       // of a B200
-// Lanes that keep them busy. Steps of 12,000, 32,000, 64,000 and 130,000 Lennard-Jones atoms: 12.9, 16.1, 18.5 and 28.2 us;
-// with twice as many 17.4, 20.7, 27.2 and 33.4 us, with half as many 12.0, 14.1, 19.2 and 33.3 us.
-constexpr int64_t kPairLanesWanted = kDeviceSms * 512;
+// Lanes that keep them busy, below which a row gets twice as many: half of those that an SM holds of the force kernel, 1,024 with one
+// type. Steps of 12,000, 32,000, 64,000 and 130,000 Lennard-Jones atoms: 10.7, 13.4, 16.4 and 22.0 us; with twice as many lanes 14.7,
+// 18.3, 24.6 and 27.5, with half as many 11.0, 15.0, 21.5 and 27.4. With more types an SM holds 768, and from four lanes per row on
+// half of them do: mixture of 16,000, 30,000, 60,000 and 100,000 atoms 13.0, 16.6, 24.3 and 26.2 us (512 at any number of lanes: 15.8, 20.1,
+// 24.3, 26.2; 384: 13.0, 16.6, 25.5, 26.2).
+constexpr int64_t pair_lanes_wanted(int types, int shift) { return kDeviceSms * (types == 1 || shift < 2 ? 512 : 384); }
 constexpr int64_t kPairLanesWantedEwald = kDeviceSms * 768;   // one and a half rounds of one block of 512 each
 // Atoms up to which the last block of a displacement check reports it; beyond, a launch of its own does, and no block waits for its
 // writes to arrive before it takes its ticket and makes room for the next. Steps of 130,000, 260,000, 1,000,000 and 4,000,000
@@ -874,9 +877,9 @@ RowArrays rows_of(const dsmd_ctx* c) { return RowArrays{c->quad, c->rows, c->str
 // gives the same bits as a pass over all of them.
 int pair_lane_shift(const dsmd_ctx* c) {
     const int64_t pairs = std::min(2 * c->n_quads, c->n_owned);   // as many rows at most have atoms
-    const int64_t wanted = ewald_copies(c) == kEwaldCopiesMost ? kPairLanesWantedEwald : kPairLanesWanted;
+    const auto wanted = [&](int shift) { return ewald_copies(c) == kEwaldCopiesMost ? kPairLanesWantedEwald : pair_lanes_wanted(c->ntypes, shift); };
     int shift = long_rows(c) ? kLongOrder : 0;
-    while (shift < 5 && (pairs << shift) < wanted && (8 << shift) <= c->stride) ++shift;
+    while (shift < 5 && (pairs << shift) < wanted(shift) && (8 << shift) <= c->stride) ++shift;
     return shift;
 }
 

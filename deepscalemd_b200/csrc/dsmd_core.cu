@@ -55,17 +55,17 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kDeviceSms = 148;                       // of a B200
-// Lanes that keep them busy, below which a row gets twice as many: half of those that an SM holds of the force kernel, 1,024 with one
-// type. Steps of 12,000, 32,000, 64,000 and 130,000 Lennard-Jones atoms: 10.7, 13.4, 16.4 and 22.0 us; with twice as many lanes 14.7,
-// 18.3, 24.6 and 27.5, with half as many 11.0, 15.0, 21.5 and 27.4. With more types an SM holds 768, and from four lanes per row on
-// half of them do: mixture of 16,000, 30,000, 60,000 and 100,000 atoms 13.0, 16.6, 24.3 and 26.2 us (512 at any number of lanes: 15.8, 20.1,
-// 24.3, 26.2; 384: 13.0, 16.6, 25.5, 26.2).
-constexpr int64_t pair_lanes_wanted(int types, int shift) { return kDeviceSms * (types == 1 || shift < 2 ? 512 : 384); }
+// Lanes that keep them busy, below which a row gets twice as many: half of those that an SM holds of the plain force kernel (1,024)
+// before rows are shared at all, a third where a row's set-up is paid by several lanes. Steps of 16,000, 32,000, 64,000, 90,000 and
+// 130,000 Lennard-Jones atoms: 9.3, 11.3, 15.3, 17.7 and 22.0 us; with 512 throughout 9.6, 12.2, 15.1, 17.7 and 22.0, with 1,024 13.7, 15.7, 21.3,
+// 23.7 and 27.6, with 256 9.3, 11.3, 14.8, 22.1 and 27.4. Of 30,000, 60,000 and 90,000 of the mixture: 13.0, 19.0 and 22.2; with 512 16.2, 22.3 and 22.3.
+constexpr int64_t pair_lanes_wanted(int shift) { return kDeviceSms * (shift == 0 ? 512 : 352); }
 constexpr int64_t kPairLanesWantedEwald = kDeviceSms * 768;   // one and a half rounds of one block of 512 each
-// Atoms up to which the last block of a displacement check reports it; beyond, a launch of its own does, and no block waits for its
-// writes to arrive before it takes its ticket and makes room for the next. Steps of 130,000, 260,000, 1,000,000 and 4,000,000
-// Lennard-Jones atoms: 22.8, 39.8, 118 and 441 us, with tickets 23.9, 42.3, 121 and 455; of 64,000 a launch is dearer than the tickets.
-constexpr int64_t kTicketMost = 100000;
+// Threads of a launch up to which its last block reports the displacement check; beyond, a launch of its own does, and no block waits
+// for its writes to arrive before it takes its ticket (one word for all) and makes room for the next. Steps of 1,500 (24,000
+// threads), 5,000, 20,000, 75,000, 260,000 and 4,000,000 Lennard-Jones atoms: 7.3, 7.4, 9.8, 17.0, 39.8 and 441 us, with tickets 6.9, 9.1, 13.1,
+// 23.6, 42.3 and 455.
+constexpr int64_t kTicketThreadsMost = 25000;
 constexpr int kLongRow = 240;                         // entries (with the row's spare room): about 150 partners per atom
 constexpr int64_t kRowsAlways = 4096;                 // cell rows that any system may have: 2 MB of list rows
 constexpr int kXRefine = 4;    // x cells per cell width of the y and z axes (tighter row windows in the list build)
@@ -877,7 +877,7 @@ RowArrays rows_of(const dsmd_ctx* c) { return RowArrays{c->quad, c->rows, c->str
 // gives the same bits as a pass over all of them.
 int pair_lane_shift(const dsmd_ctx* c) {
     const int64_t pairs = std::min(2 * c->n_quads, c->n_owned);   // as many rows at most have atoms
-    const auto wanted = [&](int shift) { return ewald_copies(c) == kEwaldCopiesMost ? kPairLanesWantedEwald : pair_lanes_wanted(c->ntypes, shift); };
+    const auto wanted = [&](int shift) { return ewald_copies(c) == kEwaldCopiesMost ? kPairLanesWantedEwald : pair_lanes_wanted(shift); };
     int shift = long_rows(c) ? kLongOrder : 0;
     while (shift < 5 && (pairs << shift) < wanted(shift) && (8 << shift) <= c->stride) ++shift;
     return shift;
@@ -1009,12 +1009,12 @@ bool reports_count(dsmd_ctx* c, cudaStream_t s) {
 // The report of a displacement check about to be launched: of all owned atoms, or none (a part says little, and parts may
 // run side by side on several streams). Slot and ticket follow from the launch's number: the MD loop has a check unread while
 // the next one is under way, and their numbers differ by one (only a list build takes numbers in between, and it voids the check).
-DisplacementReport displacement_report(dsmd_ctx* c, bool all_atoms, cudaStream_t s) {
+DisplacementReport displacement_report(dsmd_ctx* c, bool all_atoms, int64_t threads, cudaStream_t s) {
     c->disp_seq = 0;
     if (!all_atoms || !reports_count(c, s)) return DisplacementReport{c->status, nullptr, nullptr, 0, c->gate2};
     c->disp_seq = ++c->seq;
     const int slot = static_cast<int>(c->seq & 3);
-    return DisplacementReport{c->status, c->n_owned > kTicketMost ? nullptr : c->tickets + 4 + slot, c->mail + kMailDisplacement + slot, c->seq, c->gate2};
+    return DisplacementReport{c->status, threads > kTicketThreadsMost ? nullptr : c->tickets + 4 + slot, c->mail + kMailDisplacement + slot, c->seq, c->gate2};
 }
 
 // Behind the launch that was given `report`.
@@ -1544,7 +1544,7 @@ int dsmd_list_export(dsmd_ctx* c, int32_t* d_i, int32_t* d_j, uint8_t* d_flags, 
 static int pack_impl(dsmd_ctx* c, int64_t first, int64_t count, bool integrate, double dt, double f2a, cudaStream_t s,
                      double kick = 0.5, const ClusterMembers& skip = {}, const BondedForces* bonded = nullptr) {
     if (count <= 0) return DSMD_OK;
-    const DisplacementReport report = displacement_report(c, first == 0 && count >= c->n_owned, s);
+    const DisplacementReport report = displacement_report(c, first == 0 && count >= c->n_owned, count, s);
     double** r = c->real[c->cur];
     const auto kernel = !integrate ? k_pack<false, false> : (bonded ? k_pack<true, true> : k_pack<true, false>);
     // (a part of the atoms follows a copy on another stream: nothing to overlap with)
@@ -1678,7 +1678,7 @@ static int force_step(dsmd_ctx* c, double dt, double f2a, cudaStream_t s) {
                       nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, c->status, c->gate2, list_settled(c, s)};
     const StepArgs at{r[0], r[1], r[2], r[3], r[4], r[5], r[9], c->ref[0], c->ref[1], c->ref[2], c->pq_next, dt, dt * f2a};
     const unsigned blocks = static_cast<unsigned>(pair_blocks(c, pairs, false));
-    const DisplacementReport report = displacement_report(c, true, s);
+    const DisplacementReport report = displacement_report(c, true, pairs << c->lane_shift, s);
     const auto launch = long_rows(c) ? dsmd::launch_step<kLongOrder> : dsmd::launch_step<0>;
     DSMD_CUDA(c, launch(p, a, c->grid, at, report, c->switch_distance > 0.0, blocks, s));
     ++c->launches;
@@ -1739,7 +1739,7 @@ int launch_constrained(dsmd_ctx* c, bool finish, bool start, double half_kick, d
     double** r = c->real[c->cur];
     const AtomArrays at{r[0], r[1], r[2], r[3], r[4], r[5], r[6], r[7], r[8], r[9], c->type[c->cur], c->ref[0], c->ref[1], c->ref[2], c->pq};
     const unsigned blocks = blocks_for(c->n_clusters, 128);
-    const DisplacementReport report = start ? displacement_report(c, c->cl_atoms == c->n_owned, s) : DisplacementReport{c->status, nullptr, nullptr, 0, HUGE_VAL};
+    const DisplacementReport report = start ? displacement_report(c, c->cl_atoms == c->n_owned, c->n_clusters, s) : DisplacementReport{c->status, nullptr, nullptr, 0, HUGE_VAL};
     const auto launch = [&](auto shape) {
         const auto kernel = finish && start ? k_constrained<decltype(shape), true, true>
                                             : (finish ? k_constrained<decltype(shape), true, false> : k_constrained<decltype(shape), false, true>);

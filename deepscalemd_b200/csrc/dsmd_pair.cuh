@@ -535,7 +535,7 @@ __device__ __forceinline__ void row_forces(const PairParams& p, const ForceArgs&
         }
     if (ENERGY) acc.take_energies(two, v);   // a lone atom's sums are in both lanes; no atom: zeros
     acc.take_forces(sum_a, sum_b);
-    for (int o = lanes >> 1; o > 0; o >>= 1) {
+    for (int o = 1; o < lanes; o <<= 1) {   // (neighbouring chunks first)
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             sum_a[k] += __shfl_xor_sync(0xFFFFFFFFu, sum_a[k], o);

@@ -31,7 +31,7 @@ L2_BYTES = 126e6
 WORKLOAD_NAME = "LJ NVE 4,000,000 atoms (FCC 100^3, rho*=0.8442, T*=1.44, rc=2.5, skin=0.3, dt=0.005)"
 SETTLE_STEPS = 12              # untimed MD steps of the set-up: they take the run through its first list rebuild (and, on several
                                # GPUs, the first migration), so that no first-use cost lands in the timed steps
-NCU_PAIR_TRAFFIC_BYTES_PER_ATOM = 119.2e6 / 500_000   # measured DRAM bytes per launch / atoms (rows of the list + positions)
+NCU_PAIR_TRAFFIC_BYTES_PER_ATOM = 118.8e6 / 500_000   # measured DRAM bytes per launch / atoms (rows of the list + positions)
 
 
 def measured_peaks():
@@ -466,7 +466,7 @@ def single_gpu(args):
         "peak_source": "measured in this run (independent FMA chains on every SM); no fp32 CUDA-core figure in MEASURED_PEAKS.json",
         "peak_nominal": sms * 128 * 2 * clocks_max_ghz(0) * 1e-3,   # TFLOP/s: SMs x 128 fp32 lanes x 2 flops x max SM clock
         # dram__bytes_read + dram__bytes_write of one k_pair launch, from the ncu capture of the 500,000-atom case
-        # (profiles/k_pair_k_build_rows_lj_500k_ncu_full.md: 119.2 MB) scaled by the atom count
+        # (profiles/k_pair_k_build_rows_lj_500k_ncu_full.md: 118.8 MB) scaled by the atom count
         "traffic": NCU_PAIR_TRAFFIC_BYTES_PER_ATOM * s.n,
         "algorithmic_bytes_per_launch": pair_bytes, "algorithmic_flops_per_launch": pair_flops,
         "hbm": {"achieved": pk["gbs"], "peak": hbm_peak, "unit": "GB/s", "frac": pk["frac_hbm"],

@@ -1662,7 +1662,8 @@ static int compute_forces_impl(dsmd_ctx* c, int phase, int want_energy, int64_t 
                                                        : (e ? dsmd::launch_pair<0, true, 0> : dsmd::launch_pair<0, false, 0>))
                             : copies == 1 ? (e ? dsmd::launch_pair<1, true, 0> : dsmd::launch_pair<1, false, 0>)
                                           : (e ? dsmd::launch_pair<kEwaldCopiesMost, true, kLongOrder> : dsmd::launch_pair<kEwaldCopiesMost, false, kLongOrder>);
-        DSMD_CUDA(c, launch(p, a, sw, blocks, !ranged, s));
+        // (ranges and boundary passes follow work of other streams: nothing to overlap with)
+        DSMD_CUDA(c, launch(p, a, sw, blocks, !ranged && phase != DSMD_PHASE_BOUNDARY, s));
         ++c->launches;
     }
     return DSMD_OK;

@@ -295,3 +295,46 @@ def test_rebuild_with_longer_rows_inside_the_loop(cuda_device):
     d = out - (pos + vel * dt * steps)
     assert np.abs(d - L * np.round(d / L)).max() <= 1e-9
     ctx.close()
+
+
+# the last block reports the check up to 25,000 threads, a launch behind it beyond
+@pytest.mark.parametrize("n", [1000, 24999, 25001])
+def test_displacement_checks_reported_by_block_and_by_launch(cuda_device, n):
+    rng = np.random.default_rng(n)
+    L = 60.0
+    pos, vel, box = rng.uniform(0.0, L, (n, 3)), rng.normal(size=(n, 3)), np.full(3, L)
+    ctx = capi.Context(n)
+    ctx.set_box(box)
+    ctx.set_pair_params([[0.0]], [[1.0]], 2.0, 0.5)
+    ctx.upload(pos, vel=vel)
+    ctx.build_neighbor_list()
+    ctx.compute_forces()
+    for k in range(1, 4):   # each check stands for itself and for the largest so far
+        ctx.integrate(1, 0.01)
+        want = ((k * 0.01 * vel) ** 2).sum(1).max()
+        assert abs(ctx.max_displacement_sq() - want) <= 1e-9 * want
+    ctx.close()
+
+
+@pytest.mark.parametrize("pinned", [False, True])
+@pytest.mark.parametrize("n", [1, 3, 4097, 50000])
+def test_uploaded_rows_are_the_callers_again_at_once(cuda_device, n, pinned):
+    import torch
+    rng = np.random.default_rng(n)
+    rows = [rng.uniform(0.0, 20.0, (n, 3)) for _ in range(2)]
+    given = [torch.from_numpy(r.copy()).pin_memory().numpy() if pinned else r.copy() for r in rows]
+    ctx = capi.Context(n + 5)
+    ctx.set_box(np.full(3, 20.0))
+    ctx.set_pair_params([[1.0]], [[1.0]], 2.0, 0.5)
+    for _ in range(2):   # the second upload goes through the set of arrays that the first one's sort left behind
+        for g, r in zip(given, rows):
+            g[:] = r
+        ctx.upload(given[0], vel=given[1])
+        for g in given:
+            g[:] = -1.0
+        if n > 1:
+            ctx.build_neighbor_list()
+        gid = ctx.download("global_id", n)
+        for names, want in (("xyz", rows[0]), (("vx", "vy", "vz"), rows[1])):
+            assert np.array_equal(np.stack([ctx.download(k, n) for k in names], axis=1), want[gid])
+    ctx.close()

@@ -1004,10 +1004,13 @@ int edge_search(dsmd_edges* e, const Grid& g, const double* d_x, const double* d
     EdgeStatus* const st = reinterpret_cast<EdgeStatus*>(e->cell_count);
     if (!e->counts_zero) EDGE_CUDA(e, cudaMemsetAsync(e->cell_count, 0, sizeof(int) * e->cap_cell_count, s));
     e->counts_zero = false;
+    // (every launch is looked at before the next one is made: that one indexes with what it writes)
     dsmd::launch_next(k_edge_keys, blocks_for(n, kThreads), kThreads, 0, s, g, in, d_x, d_y, d_z, e->key, e->arrival, cell_count, st);
+    EDGE_CUDA(e, cudaGetLastError());
     if (table <= static_cast<size_t>(dsmd::kScanMost)) {
         const int launched = dsmd::launch_cell_scan(static_cast<int>(table), 0, cell_count, e->scan_sums, e->cell_start, s);
-        e->launches += std::max(launched, 0);
+        EDGE_CUDA(e, cudaGetLastError());
+        e->launches += launched;
     } else {
         size_t scan_bytes = 0;
         cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, cell_count, e->cell_start, static_cast<int>(table), s);
@@ -1015,9 +1018,10 @@ int edge_search(dsmd_edges* e, const Grid& g, const double* d_x, const double* d
         EDGE_CUDA(e, cub::DeviceScan::ExclusiveSum(e->temp, scan_bytes, cell_count, e->cell_start, static_cast<int>(table), s));
     }
     dsmd::launch_next(k_edge_place, blocks_for(n, kThreads), kThreads, 0, s, in, e->key, e->arrival, e->cell_start, e->list, static_cast<int>(table), cell_count);
+    EDGE_CUDA(e, cudaGetLastError());
     dsmd::launch_next(k_edge_gather, blocks_for(n, kThreads), kThreads, 0, s, g, in, e->key, e->list, e->cell_start, d_x, d_y, d_z,
-                                                              row == 1 ? d_ok : nullptr, d_owner, e->pq, e->pf,
-                                                              PERIODIC ? e->wraps : nullptr, st);
+                      row == 1 ? d_ok : nullptr, d_owner, e->pq, e->pf, PERIODIC ? e->wraps : nullptr, st);
+    EDGE_CUDA(e, cudaGetLastError());
     e->launches += 3;
     if (e->stride == 0) {
         const double expect = density_hint * 4.18879020479 * g.r2_list_d * std::sqrt(g.r2_list_d);

@@ -1373,9 +1373,9 @@ int dsmd_sort_owned_in_brick(dsmd_ctx* c, const double lo[3], const double hi[3]
 
 // forces: the force arrays move with the atoms. queue_next (or null): called once everything is launched and before the host waits for the
 // build's report; what it launches must do nothing behind a closed gate. If the build has to be done again, or fails, the gate
-// was closed, and it is called again, or take_back instead.
-static int build_list(dsmd_ctx* c, bool forces, cudaStream_t s, const std::function<int()>& queue_next = nullptr,
-                      const std::function<void()>& take_back = nullptr) {
+// was closed, and what it swapped is put back; in the first case it is called again. After an error behind the first launch there
+// is no list: the atoms may have been sorted, and rows rewritten.
+static int build_list(dsmd_ctx* c, bool forces, cudaStream_t s, const std::function<int()>& queue_next = nullptr) {
     DSMD_CUDA(c, cudaSetDevice(c->device));
     if (c->n_owned <= 0) return fail(c, DSMD_ERR_STATE, "no atoms uploaded");
     if (!c->grid_valid) { const int rc = make_grid(c); if (rc) return rc; }
@@ -1409,6 +1409,7 @@ static int build_list(dsmd_ctx* c, bool forces, cudaStream_t s, const std::funct
             c->layer_capacity = layers + 1;
         }
     }
+    c->list_valid = false;
     { const int rc = lay_out_rows(c, row_entries); if (rc) return rc; }
     // 1. bin + sort + reorder (everything, or only the ghosts when the owned segment was sorted just before: the
     //    status words of that sort are then still unread and are kept), and the quads
@@ -1429,13 +1430,19 @@ static int build_list(dsmd_ctx* c, bool forces, cudaStream_t s, const std::funct
                           c->ghost_rows + 2 * rows, c->ghost_rows + 3 * rows);
         DSMD_LAUNCHED(c);
     }
-    const bool was_valid = c->list_valid;
+    int4* const places[2] = {c->pq, c->pq_next};
+    const auto take_back = [&] {   // what was queued behind the build
+        c->list_valid = false;
+        c->disp_seq = 0;
+        c->pq = places[0];
+        c->pq_next = places[1];
+    };
     const auto failed = [&](int rc) {
-        c->list_valid = was_valid;
+        take_back();
         return rc;
     };
     for (int attempt = 0; attempt < 4; ++attempt) {
-        if (attempt > 0) { const int rc = lay_out_rows(c, row_entries); if (rc) return failed(rc); }
+        if (attempt > 0) { const int rc = lay_out_rows(c, row_entries); if (rc) return rc; }
         const ExclusionTable ex{c->excl_off, c->excl_partner, static_cast<int>(c->excl_n_global)};
         const unsigned blocks = blocks_for(c->n_quads * 32, kBuildThreads);
         const auto build = ex.offsets ? (long_rows(c) ? k_build_rows<true, kLongOrder> : k_build_rows<true, 0>)
@@ -1450,21 +1457,21 @@ static int build_list(dsmd_ctx* c, bool forces, cudaStream_t s, const std::funct
         DSMD_LAUNCHED(c);
         c->disp_seq = 0;   // the displacement word starts again at zero
         ++c->build_epoch;
-        c->list_valid = true;
-        if (queue_next) { const int rc = queue_next(); if (rc) return rc; }
+        c->list_valid = true;   // for what is queued behind it
+        if (queue_next) { const int rc = queue_next(); if (rc) return failed(rc); }
         { const int rc = wait_mail(c, kMailBuild, 4, seq, s); if (rc) return failed(rc); }
         const Mail& report = c->mail[kMailBuild];
         const bool outside = report.value(0) != 0.0, miscounted = attempt == 0 && report.value(1) != static_cast<double>(expect_dropped);
         const bool overflowed = report.value(2) > c->stride;
-        if ((outside || miscounted || overflowed) && take_back) take_back();
-        if (outside) return failed(fail(c, DSMD_ERR_OUT_OF_DOMAIN, "an atom lies outside the subdomain + halo, or has a NaN position"));
-        if (miscounted) return failed(fail(c, DSMD_ERR_STATE, "sort: the number of atoms outside the brick differs from the caller's count"));
+        if (outside || miscounted || overflowed) take_back();
+        if (outside) return fail(c, DSMD_ERR_OUT_OF_DOMAIN, "an atom lies outside the subdomain + halo, or has a NaN position");
+        if (miscounted) return fail(c, DSMD_ERR_STATE, "sort: the number of atoms outside the brick differs from the caller's count");
         c->n_boundary = static_cast<int64_t>(report.value(3));
         c->sort_words_zero = true;
         if (!overflowed) break;
         // a row overflowed: grow and build again
         row_entries = static_cast<int>(report.value(2) * 1.1) + 8;
-        if (attempt == 3) return failed(fail(c, DSMD_ERR_CAPACITY, "neighbour rows kept overflowing"));
+        if (attempt == 3) return fail(c, DSMD_ERR_CAPACITY, "neighbour rows kept overflowing");
     }
     return DSMD_OK;
 }
@@ -2198,8 +2205,11 @@ int dsmd_run_nve(dsmd_ctx* c, int64_t n_steps, double dt, double f2a, double hi_
             double d2 = 0.0;
             const int rc = reported(check, d2);
             if (rc) {
-                // an atom outside closed the gate: the kernel queued above left its buffer of positions unwritten
-                if (advanced && fused && limit2 < dsmd::kGateOpen) std::swap(c->pq, c->pq_next);
+                // an atom outside closed the gate: the kernel queued above left its buffer of positions unwritten, and reports nothing
+                if (advanced && limit2 < dsmd::kGateOpen) {
+                    if (fused) std::swap(c->pq, c->pq_next);
+                    c->disp_seq = 0;
+                }
                 return rc;
             }
             if (d2 > limit2) rebuild = true;
@@ -2223,7 +2233,7 @@ int dsmd_run_nve(dsmd_ctx* c, int64_t n_steps, double dt, double f2a, double hi_
         if (rebuild) {
             // Forces are evaluated next, as a rule queued behind the build before the host hears of it.
             const bool queue = ahead_of_check && !last && limit2 < dsmd::kGateOpen;
-            const int rc = queue ? build_list(c, false, s, [&] { return advance(limit2); }, [&] { if (fused) std::swap(c->pq, c->pq_next); })
+            const int rc = queue ? build_list(c, false, s, [&] { return advance(limit2); })
                                  : build_list(c, false, s);
             if (rc) return rc;
             built_ahead = queue;

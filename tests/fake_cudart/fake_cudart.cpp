@@ -24,7 +24,7 @@ std::string refused;                           // launches of kernels with this 
 int refuse_after = 0;                          // ... from this one on
 cudaError_t last = cudaSuccess;
 unsigned need_stride = 0;                      // what list builds find
-bool outside = false;                          // an atom outside, found by list builds
+bool outside = false, check_outside = false;   // an atom outside, found by list builds and by displacement checks
 bool gate_closed = false;
 int copies_until_failure = -1;
 std::set<std::pair<const char*, const char*>> pinned_ranges;
@@ -36,6 +36,13 @@ void post(dsmd::Mail* mail, const double* v, int n, unsigned long long seq) {
         mail->word[2 * k] = (bits >> 32 << 32) | (seq & 0xFFFFFFFFull);
         mail->word[2 * k + 1] = (bits << 32) | (seq & 0xFFFFFFFFull);
     }
+}
+
+void report_check(const dsmd::DisplacementReport& r) {
+    if (gate_closed && r.gate2 < dsmd::kGateOpen) return;
+    const double out[2] = {0.0, check_outside ? 1.0 : 0.0};
+    gate_closed = check_outside;
+    post(r.mail, out, 2, r.seq);
 }
 
 cudaError_t launch(const std::string& name, void** args) {
@@ -50,13 +57,10 @@ cudaError_t launch(const std::string& name, void** args) {
         gate_closed = outside || out[2] > stride;
         post(*static_cast<dsmd::Mail**>(args[3]), out, 4, *static_cast<unsigned long long*>(args[4]));
     } else if (name.find("k_post_displacement") != std::string::npos) {
-        const auto& r = *static_cast<dsmd::DisplacementReport*>(args[0]);
-        const double out[2] = {0.0, 0.0};
-        if (!(gate_closed && r.gate2 < dsmd::kGateOpen)) post(r.mail, out, 2, r.seq);
+        report_check(*static_cast<dsmd::DisplacementReport*>(args[0]));
     } else if (name.find("k_pack") != std::string::npos) {
         const auto& r = *static_cast<dsmd::DisplacementReport*>(args[23]);
-        const double out[2] = {0.0, 0.0};
-        if (r.ticket && !(gate_closed && r.gate2 < dsmd::kGateOpen)) post(r.mail, out, 2, r.seq);
+        if (r.ticket) report_check(r);
     }
     return cudaSuccess;
 }
@@ -72,12 +76,13 @@ void fake_reset() {
     refuse_after = 0;
     last = cudaSuccess;
     need_stride = 0;
-    outside = gate_closed = false;
+    outside = check_outside = gate_closed = false;
     copies_until_failure = -1;
     pinned_ranges.clear();
 }
 void fake_refuse(const char* name, int after) { refused = name; refuse_after = after; }
 void fake_build_finds(unsigned stride, int atoms_outside) { need_stride = stride; outside = atoms_outside != 0; }   // ~0: always a longer row
+void fake_check_finds(int atoms_outside) { check_outside = atoms_outside != 0; }
 void fake_pin(const char* p, size_t bytes) { pinned_ranges.insert({p, p + bytes}); }
 void fake_fail_copy(int after) { copies_until_failure = after; }
 int fake_log_size() { return static_cast<int>(log_.size()); }
@@ -155,8 +160,7 @@ cudaError_t launch_pair(const PairParams&, const ForceArgs&, bool, unsigned, boo
 template <int ORDER>
 cudaError_t launch_step(const PairParams&, const ForceArgs&, const Grid&, const StepArgs&, const DisplacementReport& r, bool, unsigned, cudaStream_t) {
     const cudaError_t e = launch("k_step", nullptr);
-    const double out[2] = {0.0, 0.0};
-    if (e == cudaSuccess && r.ticket && !(gate_closed && r.gate2 < kGateOpen)) post(r.mail, out, 2, r.seq);
+    if (e == cudaSuccess && r.ticket) report_check(r);
     return e;
 }
 

@@ -12,7 +12,7 @@ from deepscalemd_b200 import build
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(ROOT, "deepscalemd_b200", "csrc")
-CUDA_ERROR, CAPACITY, STATE = 2, 5, 6
+CUDA_ERROR, OUT_OF_DOMAIN, CAPACITY, STATE = 2, 4, 5, 6
 i64, f64, ptr = ctypes.c_int64, ctypes.c_double, ctypes.c_void_p
 
 
@@ -66,3 +66,74 @@ def test_edge_search_ends_at_the_first_refused_launch(lib, kernel, later, n, L):
     lib.dsmd_edges_build_periodic(edges, *(ptr(a.ctypes.data) for a in x), i64(n), ptr(box.ctypes.data), f64(5.0), ctypes.byref(n_edges), None)
     assert any("k_edge_gather" in line for line in log(lib))
     lib.dsmd_edges_destroy(edges)
+
+
+# -- list builds that fail ----------------------------------------------------------------------------------------------
+class System:
+    def __init__(self, lib, n=4000, L=16.8):
+        self.lib, self.n, self.h = lib, n, ptr()
+        assert lib.dsmd_create(0, i64(n), ctypes.byref(self.h)) == 0
+        box, periodic, zero = np.full(3, L), (ctypes.c_int * 3)(1, 1, 1), np.zeros(3)
+        assert lib.dsmd_set_box(self.h, *(ptr(a.ctypes.data) for a in (box,)), periodic, ptr(zero.ctypes.data), ptr(zero.ctypes.data), f64(0.0)) == 0
+        one = np.ones(1)
+        assert lib.dsmd_set_pair_params(self.h, ctypes.c_int(1), ptr(one.ctypes.data), ptr(one.ctypes.data), f64(2.5), f64(0.3), f64(-1.0)) == 0
+        self.rows = np.random.default_rng(2).uniform(0.0, L, (n, 3))
+        assert lib.dsmd_upload_rows(self.h, i64(n), i64(n), ptr(self.rows.ctypes.data), None, None, None, None, None, None) == 0
+
+    def build(self):
+        return self.lib.dsmd_build_neighbor_list(self.h, None)
+
+    def forces(self):
+        return self.lib.dsmd_compute_forces(self.h, ctypes.c_int(0), ctypes.c_int(0), None)
+
+    def run(self, steps, every):
+        return self.lib.dsmd_run_nve(self.h, i64(steps), f64(0.001), f64(1.0), f64(0.5), ctypes.c_int(every), ctypes.c_int(0), None, None, None)
+
+    def displacement(self):
+        return self.lib.dsmd_max_displacement_sq(self.h, ctypes.byref(f64()), None)
+
+
+@pytest.fixture
+def system(lib):
+    s = System(lib)
+    assert s.build() == 0 and s.forces() == 0
+    yield s
+    lib.dsmd_destroy(s.h)
+
+
+def assert_no_list_until_rebuilt(s):
+    assert s.forces() == STATE
+    assert s.displacement() != CUDA_ERROR   # no wait for a check that a closed gate kept from reporting
+    s.lib.fake_reset()
+    assert s.build() == 0 and s.forces() == 0 and s.run(5, 2) == 0
+
+
+@pytest.mark.parametrize("in_loop", [False, True])
+@pytest.mark.parametrize("stride,outside,code", [(0xFFFFFFFF, 0, CAPACITY), (0, 1, OUT_OF_DOMAIN)])
+def test_a_failed_build_leaves_no_list(lib, system, in_loop, stride, outside, code):
+    """Rows that keep overflowing, an atom outside: the atoms have been sorted and the rows rewritten."""
+    lib.fake_build_finds(ctypes.c_uint(stride), outside)
+    assert (system.run(6, 2) if in_loop else system.build()) == code
+    assert_no_list_until_rebuilt(system)
+
+
+@pytest.mark.parametrize("kernel", ["k_cell_keys", "k_cell_starts", "k_place", "k_reorder", "k_build_rows", "k_build_done"])
+def test_a_build_with_a_refused_launch_leaves_no_list(lib, system, kernel):
+    lib.fake_refuse(kernel.encode(), 0)
+    assert system.build() == CUDA_ERROR
+    assert_no_list_until_rebuilt(system)
+
+
+@pytest.mark.parametrize("kernel", ["k_step", "k_post_displacement"])
+def test_a_step_refused_behind_a_build_leaves_no_list(lib, system, kernel):
+    lib.fake_refuse(kernel.encode(), 1)   # the first one is in front of the build
+    assert system.run(6, 2) == CUDA_ERROR
+    lines = log(lib)
+    assert "k_build_done" in "".join(lines[-3:]) and "refused" in lines[-1]
+    assert_no_list_until_rebuilt(system)
+
+
+def test_a_check_that_finds_an_atom_outside_can_be_asked_again(lib, system):
+    lib.fake_check_finds(1)
+    assert system.run(6, 0) == OUT_OF_DOMAIN
+    assert system.displacement() != CUDA_ERROR

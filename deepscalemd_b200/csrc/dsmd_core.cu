@@ -69,6 +69,10 @@ constexpr int64_t kTicketThreadsMost = 25000;
 constexpr int kLongRow = 240;                         // entries (with the row's spare room): about 150 partners per atom
 constexpr int64_t kRowsAlways = 4096;                 // cell rows that any system may have: 2 MB of list rows
 constexpr int kXRefine = 4;    // x cells per cell width of the y and z axes (tighter row windows in the list build)
+// Rows (of positions and of velocities together) up to which an upload goes through pinned memory of the context, so that it returns
+// while what is queued in the stream is still at work. 1,000 atoms 25 us (by the runtime 40), 8,000 36 (35), 16,000 47 (46), 32,000 73
+// (66); with velocities 1,000 31 (65), 8,000 47 (56), 16,000 72 (83).
+constexpr int64_t kStageRows = 32768;
 enum { kMailDisplacement = 0, kMailKinetic = 4, kMailScalars = 5, kMailBuild = 6, kMailSlots = 7 };   // report slots
 constexpr unsigned kLinkBlocks = 64;      // blocks of kernels that read or write host memory: enough to fill the link
 // Host-buffer calls: below kPipelineLeast atoms one pass with kernels that read and write the host's memory (131,072 atoms
@@ -321,15 +325,13 @@ __global__ void k_upload_defaults(int n, RealArrays r, int* type, int* gid) {
     if (gid) gid[s] = s;
 }
 
-// [n][3] rows, n words of them in each of three arrays, to three columns.
+// [n][3] rows, n words of them in each of three arrays (device memory, or pinned host memory), to three columns.
 __global__ void k_split_rows(int n, const double* __restrict__ rows0, const double* __restrict__ rows1, const double* __restrict__ rows2,
                              double* __restrict__ x, double* __restrict__ y, double* __restrict__ z) {
     if (!dsmd::after_previous()) return;
-    const auto word = [&](long long k) { return k < n ? rows0[k] : (k < 2ll * n ? rows1[k - n] : rows2[k - 2ll * n]); };
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
-        x[s] = word(3ll * s);
-        y[s] = word(3ll * s + 1);
-        z[s] = word(3ll * s + 2);
+    for (long long k = blockIdx.x * blockDim.x + threadIdx.x; k < 3ll * n; k += gridDim.x * blockDim.x) {
+        const int s = static_cast<int>(k / 3), a = static_cast<int>(k - 3ll * s);
+        (a == 0 ? x : (a == 1 ? y : z))[s] = k < n ? rows0[k] : (k < 2ll * n ? rows1[k - n] : rows2[k - 2ll * n]);
     }
 }
 
@@ -631,6 +633,8 @@ struct dsmd_ctx {
     long long settled_epoch = -1;         // list build, and stream, of the last force launch (list_settled)
     cudaStream_t settled_stream = nullptr;
     cudaEvent_t disp_event[2] = {};
+    double* stage = nullptr;              // pinned: rows on their way to the device (kStageRows)
+    cudaEvent_t stage_free = nullptr;
     unsigned char* flag = nullptr;
     unsigned long long* offsets64 = nullptr;
     bool list_valid = false;
@@ -1117,6 +1121,8 @@ void dsmd_destroy(dsmd_ctx* c) {
         cudaFreeHost(c->h_disp[k]);
         if (c->disp_event[k]) cudaEventDestroy(c->disp_event[k]);
     }
+    if (c->stage) cudaFreeHost(c->stage);
+    if (c->stage_free) cudaEventDestroy(c->stage_free);
     delete c;
 }
 
@@ -1257,20 +1263,59 @@ int dsmd_upload(dsmd_ctx* c, int64_t n_owned, int64_t n_total, const double* x, 
     return upload_rest(c, n_owned, n_total, src, false, type, gid, s);
 }
 
-// [n][3] host rows (any memory) to three device arrays, through three others of the same size. The runtime's copy out of pageable
-// memory returns when the memory may be used again, and moves 24 GB/s (2.6 MB in 110 us); a copy of our own into pinned buffers that
-// a kernel reads moved 15 (170 us).
-static int upload_columns(dsmd_ctx* c, const double* rows, int64_t n, double* const* to, double* const* scratch, cudaStream_t s) {
-    if (n == 0) return DSMD_OK;
-    for (int k = 0; k < 3; ++k)
-        DSMD_CUDA(c, cudaMemcpyAsync(scratch[k], rows + k * n, sizeof(double) * n, cudaMemcpyHostToDevice, s));
-    dsmd::launch_next(k_split_rows, std::min<unsigned>(blocks_for(n, kThreads), kDeviceSms * 8), kThreads, 0, s, static_cast<int>(n), scratch[0],
-                      scratch[1], scratch[2], to[0], to[1], to[2]);
+static int split_rows(dsmd_ctx* c, const double* rows0, const double* rows1, const double* rows2, int64_t n, double* const* to, cudaStream_t s) {
+    dsmd::launch_next(k_split_rows, std::min<unsigned>(blocks_for(3 * n, kThreads), kDeviceSms * 8), kThreads, 0, s, static_cast<int>(n), rows0, rows1,
+                      rows2, to[0], to[1], to[2]);
     DSMD_LAUNCHED(c);
-    cudaPointerAttributes memory{};
-    if (cudaPointerGetAttributes(&memory, rows) != cudaSuccess) cudaGetLastError();   // not known to the runtime: pageable
-    else if (memory.type != cudaMemoryTypeUnregistered) DSMD_CUDA(c, cudaStreamSynchronize(s));   // the copy has only been queued
     return DSMD_OK;
+}
+
+// Rows of any memory into pinned memory of the context, kStageRows at a time, from where a kernel takes them in its turn. used: rows
+// of it that kernels of this call have been given.
+static int stage_rows(dsmd_ctx* c, const double* rows, int64_t n, double* const* to, int64_t& used, cudaStream_t s) {
+    const int64_t most = std::min(kStageRows, 2 * c->capacity);
+    if (!c->stage) {
+        DSMD_CUDA(c, cudaEventCreateWithFlags(&c->stage_free, cudaEventDisableTiming));
+        DSMD_CUDA(c, cudaMallocHost(&c->stage, sizeof(double) * 3 * most));
+    }
+    for (int64_t first = 0; first < n;) {
+        if (used == 0 || used == most) {   // the rows of another call, or of this one's beginning, are still there
+            DSMD_CUDA(c, cudaEventSynchronize(c->stage_free));
+            used = 0;
+        }
+        const int64_t m = std::min(most - used, n - first);
+        double* const at = c->stage + 3 * used;
+        std::memcpy(at, rows + 3 * first, sizeof(double) * 3 * m);
+        double* const columns[3] = {to[0] + first, to[1] + first, to[2] + first};
+        const int rc = split_rows(c, at, at + m, at + 2 * m, m, columns, s);
+        DSMD_CUDA(c, cudaEventRecord(c->stage_free, s));
+        if (rc) return rc;
+        used += m;
+        first += m;
+    }
+    return DSMD_OK;
+}
+
+// [n][3] host rows (any memory) to three device arrays. Few rows are staged: the host waits for nothing but the upload before. More are
+// copied by the runtime, through three arrays of the same size: from pageable memory 17 to 24 GB/s (100,000 atoms 0.16 ms,
+// 400,000 0.57; staged 0.20 and 0.69), but it waits for what is queued in the stream. It takes a copy by where it starts: out
+// of pageable memory it has read all of it when it returns; out of memory that it knows it only queues the copy (queued: the
+// caller of the upload is to get the rows back when that is over), and refuses it if part of it is not known. Those rows are staged.
+static int upload_columns(dsmd_ctx* c, const double* rows, int64_t n, double* const* to, double* const* scratch, bool few, int64_t& used, bool& queued,
+                          cudaStream_t s) {
+    if (few) return stage_rows(c, rows, n, to, used, s);
+    for (int k = 0; k < 3; ++k) {
+        cudaPointerAttributes memory{};
+        if (cudaPointerGetAttributes(&memory, rows + k * n) != cudaSuccess) cudaGetLastError();   // not known to the runtime: pageable
+        else if (memory.type != cudaMemoryTypeUnregistered) queued = true;
+        const cudaError_t e = cudaMemcpyAsync(scratch[k], rows + k * n, sizeof(double) * n, cudaMemcpyHostToDevice, s);
+        if (e == cudaErrorInvalidValue && queued) {
+            cudaGetLastError();
+            return stage_rows(c, rows, n, to, used, s);
+        }
+        DSMD_CUDA(c, e);
+    }
+    return split_rows(c, scratch[0], scratch[1], scratch[2], n, to, s);
 }
 
 int dsmd_upload_rows(dsmd_ctx* c, int64_t n_owned, int64_t n_total, const double* pos, const double* vel, const double* mass,
@@ -1279,10 +1324,20 @@ int dsmd_upload_rows(dsmd_ctx* c, int64_t n_owned, int64_t n_total, const double
     if (n_total > c->capacity) return fail(c, DSMD_ERR_CAPACITY, "more atoms than the context's capacity");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     DSMD_CUDA(c, cudaSetDevice(c->device));
-    { const int rc = upload_columns(c, pos, n_total, c->real[c->cur], c->real[1 - c->cur], s); if (rc) return rc; }
-    if (vel) { const int rc = upload_columns(c, vel, n_total, c->real[c->cur] + DSMD_VX, c->real[1 - c->cur] + DSMD_VX, s); if (rc) return rc; }
+    const bool few = n_total * (vel ? 2 : 1) <= kStageRows;
+    bool queued = false;
+    int64_t used = 0;
+    int rc = DSMD_OK;
+    if (n_total > 0) rc = upload_columns(c, pos, n_total, c->real[c->cur], c->real[1 - c->cur], few, used, queued, s);
+    if (n_total > 0 && !rc && vel)
+        rc = upload_columns(c, vel, n_total, c->real[c->cur] + DSMD_VX, c->real[1 - c->cur] + DSMD_VX, few, used, queued, s);
     const double* const src[kNumReal] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, mass, charge};
-    return upload_rest(c, n_owned, n_total, src, vel != nullptr, type, gid, s);
+    if (!rc) rc = upload_rest(c, n_owned, n_total, src, vel != nullptr, type, gid, s);
+    if (queued) {
+        const cudaError_t e = cudaStreamSynchronize(s);
+        if (!rc) DSMD_CUDA(c, e);
+    }
+    return rc;
 }
 
 int dsmd_upload_positions(dsmd_ctx* c, const double* x, const double* y, const double* z, void* stream) {

@@ -100,7 +100,7 @@ int dsmd_upload(dsmd_ctx* ctx, int64_t n_owned, int64_t n_total, const double* x
                 const int32_t* type, const int32_t* gid, void* stream);
 
 /* The same with positions and velocities (may be NULL) as rows of three, in any host memory: copied before the call
- * returns. */
+ * returns. Up to 32,768 rows of both together the call does not wait for what is queued in `stream`; larger ones do. */
 int dsmd_upload_rows(dsmd_ctx* ctx, int64_t n_owned, int64_t n_total, const double* pos, const double* vel, const double* mass,
                      const double* charge, const int32_t* type, const int32_t* gid, void* stream);
 

@@ -113,9 +113,13 @@ cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) { std::
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
     if (copies_until_failure >= 0 && copies_until_failure-- == 0) {
         log_.push_back("failed copy");
-        return last = cudaErrorInvalidValue;
+        return last = cudaErrorUnknown;
     }
-    log_.push_back("copy");
+    for (const auto& r : pinned_ranges)   // as the runtime does: by where the copy starts
+        if (s >= r.first && s < r.second) {
+            if (static_cast<const char*>(s) + n > r.second) return last = cudaErrorInvalidValue;
+            log_.push_back("queued copy");
+        }
     std::memcpy(d, s, n);
     return cudaSuccess;
 }

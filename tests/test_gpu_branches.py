@@ -338,3 +338,61 @@ def test_uploaded_rows_are_the_callers_again_at_once(cuda_device, n, pinned):
         for names, want in (("xyz", rows[0]), (("vx", "vy", "vz"), rows[1])):
             assert np.array_equal(np.stack([ctx.download(k, n) for k in names], axis=1), want[gid])
     ctx.close()
+
+
+@pytest.mark.parametrize("n,vel", [(1000, False), (16384, True), (32768, False)])
+@pytest.mark.parametrize("pinned", [False, True])
+def test_few_rows_are_uploaded_without_waiting_for_the_stream(cuda_device, n, vel, pinned):
+    import ctypes
+    import torch
+    rng = np.random.default_rng(n)
+    given = [torch.from_numpy(rng.uniform(0.0, 20.0, (n, 3))) for _ in range(2)]
+    given = [(g.pin_memory() if pinned else g).numpy() for g in given]
+    want = [g.copy() for g in given]
+    ctx = capi.Context(n)
+    stream = torch.cuda.Stream()
+
+    def upload():
+        pos, velocities = (ctypes.c_void_p(g.ctypes.data) for g in given)
+        assert ctx.lib.dsmd_upload_rows(ctx.h, ctypes.c_int64(n), ctypes.c_int64(n), pos, velocities if vel else None, None, None, None, None,
+                                        ctypes.c_void_p(stream.cuda_stream)) == 0
+
+    upload()   # allocations
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        torch.cuda._sleep(200_000_000)   # 0.1 s
+    upload()
+    assert not stream.query()
+    for g in given:
+        g[:] = -1.0
+    torch.cuda.synchronize()
+    for names, rows in (("xyz", want[0]), (("vx", "vy", "vz"), want[1] if vel else np.zeros((n, 3)))):
+        assert np.array_equal(np.stack([ctx.download(k, n) for k in names], axis=1), rows)
+    ctx.close()
+
+
+@pytest.mark.parametrize("first,last", [(0.4, 0.6), (0.0, 0.5), (0.5, 1.0), (0.0, 1.0)])
+def test_rows_of_memory_registered_in_part(cuda_device, first, last):
+    import ctypes
+    import mmap
+    import torch
+    n = 60000
+    memory = mmap.mmap(-1, 24 * n)   # whole pages
+    rows = np.frombuffer(memory, np.float64).reshape(n, 3)
+    want = np.random.default_rng(5).uniform(0.0, 20.0, (n, 3))
+    rows[:] = want
+    lo, hi = int(first * rows.nbytes) // 4096 * 4096, rows.nbytes if last == 1.0 else int(last * rows.nbytes) // 4096 * 4096
+    runtime = torch.cuda.cudart()
+    assert int(runtime.cudaHostRegister(rows.ctypes.data + lo, hi - lo, 0)) == 0
+    ctx = capi.Context(n)
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        torch.cuda._sleep(20_000_000)
+    assert ctx.lib.dsmd_upload_rows(ctx.h, ctypes.c_int64(n), ctypes.c_int64(n), ctypes.c_void_p(rows.ctypes.data), None, None, None, None, None,
+                                    ctypes.c_void_p(stream.cuda_stream)) == 0
+    rows[:] = -1.0
+    torch.cuda.synchronize()
+    assert int(runtime.cudaHostUnregister(rows.ctypes.data + lo)) == 0
+    assert np.array_equal(np.stack([ctx.download(k, n) for k in "xyz"], axis=1), want)
+    ctx.close()

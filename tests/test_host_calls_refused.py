@@ -137,3 +137,37 @@ def test_a_check_that_finds_an_atom_outside_can_be_asked_again(lib, system):
     lib.fake_check_finds(1)
     assert system.run(6, 0) == OUT_OF_DOMAIN
     assert system.displacement() != CUDA_ERROR
+
+
+# -- uploads of rows ----------------------------------------------------------------------------------------------------
+def upload(s, pos, vel=None):
+    return s.lib.dsmd_upload_rows(s.h, i64(len(pos)), i64(len(pos)), ptr(pos.ctypes.data), ptr(vel.ctypes.data) if vel is not None else None, None,
+                                  None, None, None, None)
+
+
+@pytest.mark.parametrize("first,last", [(400, 600), (0, 1000), (0, 500), (500, 1000), (666, 667), (999, 1000)])   # registered: thousandths of the buffer
+def test_rows_in_memory_registered_in_part(lib, first, last):
+    """The runtime only queues a copy that starts in memory that it knows, and refuses it if the memory ends before; the call promises
+    the rows back, of any memory."""
+    n = 50000
+    s = System(lib, n, 40.0)
+    pos = np.random.default_rng(3).uniform(0.0, 40.0, (n, 3))
+    lib.fake_reset()
+    lib.fake_pin(ptr(pos.ctypes.data + pos.nbytes // 1000 * first), ctypes.c_size_t(pos.nbytes // 1000 * (last - first)))
+    assert upload(s, pos) == 0
+    lines = log(lib)
+    queued = [k for k, line in enumerate(lines) if line == "queued copy"]
+    assert not queued or "wait" in lines[queued[-1]:]
+    lib.dsmd_destroy(s.h)
+
+
+@pytest.mark.parametrize("fails", [1, 2, 4])
+def test_rows_are_waited_for_when_a_later_copy_fails(lib, fails):
+    s = System(lib, 50000, 40.0)
+    pos = np.random.default_rng(4).uniform(0.0, 40.0, (50000, 3))
+    lib.fake_reset()
+    lib.fake_pin(ptr(pos.ctypes.data), ctypes.c_size_t(pos.nbytes))
+    lib.fake_fail_copy(fails)
+    assert upload(s, pos, pos) == CUDA_ERROR
+    assert log(lib)[-1] == "wait"
+    lib.dsmd_destroy(s.h)

@@ -1011,11 +1011,11 @@ bool reports_count(dsmd_ctx* c, cudaStream_t s) {
 }
 
 // The report of a displacement check about to be launched: of all owned atoms, or none (a part says little, and parts may
-// run side by side on several streams). Slot and ticket follow from the launch's number: the MD loop has a check unread while
+// run side by side on several streams; nor where the caller has the word, which is then what counts). Slot and ticket follow from the launch's number: the MD loop has a check unread while
 // the next one is under way, and their numbers differ by one (only a list build takes numbers in between, and it voids the check).
 DisplacementReport displacement_report(dsmd_ctx* c, bool all_atoms, int64_t threads, cudaStream_t s) {
     c->disp_seq = 0;
-    if (!all_atoms || !reports_count(c, s)) return DisplacementReport{c->status, nullptr, nullptr, 0, c->gate2};
+    if (!all_atoms || !reports_count(c, s) || c->word_shared) return DisplacementReport{c->status, nullptr, nullptr, 0, c->gate2};
     c->disp_seq = ++c->seq;
     const int slot = static_cast<int>(c->seq & 3);
     return DisplacementReport{c->status, threads > kTicketThreadsMost ? nullptr : c->tickets + 4 + slot, c->mail + kMailDisplacement + slot, c->seq, c->gate2};
@@ -2197,13 +2197,16 @@ int dsmd_run_nve(dsmd_ctx* c, int64_t n_steps, double dt, double f2a, double hi_
     int since_build = 0;
     double d_prev = 0.0, d_prev2 = 0.0;    // displacement (not squared) seen one and two steps ago (lagged mode)
     unsigned long long pending = 0;        // the last displacement check whose report has not been looked at
-    // the loop reads the reports of its own launches only, whatever was captured before
+    // the loop reads the reports of its own launches only, whatever was captured before and whoever has the displacement word
     struct Reporting {
         dsmd_ctx* c;
-        bool captured;
-        ~Reporting() { c->captured |= captured; }
-    } reporting{c, c->captured};
-    c->captured = false;
+        bool captured, word_shared;
+        ~Reporting() {
+            c->captured |= captured;
+            c->word_shared = word_shared;
+        }
+    } reporting{c, c->captured, c->word_shared};
+    c->captured = c->word_shared = false;
     const auto reported = [&](unsigned long long seq, double& d2) {
         d2 = 0.0;
         if (!seq) return static_cast<int>(DSMD_OK);   // no atoms, no check

@@ -1,5 +1,5 @@
 """The library's host code over a stand-in for the CUDA runtime (tests/fake_cudart): what a call does when a launch or a copy
-behind it is refused, and what its caller may do next."""
+behind it is refused, and what its caller may do next; and which launches it makes."""
 import ctypes
 import os
 import subprocess
@@ -170,4 +170,27 @@ def test_rows_are_waited_for_when_a_later_copy_fails(lib, fails):
     lib.fake_fail_copy(fails)
     assert upload(s, pos, pos) == CUDA_ERROR
     assert log(lib)[-1] == "wait"
+    lib.dsmd_destroy(s.h)
+
+
+# -- launches -----------------------------------------------------------------------------------------------------------
+def test_no_report_of_a_check_whose_word_the_caller_has(lib):
+    """Whoever has the displacement word's address reads it there (the loop over several GPUs): nothing is launched, or waited for
+    within a kernel, for a report that nobody looks at; the loop of one GPU still reads its own."""
+    s = System(lib, 30000, 33.0)
+    assert s.build() == 0 and s.forces() == 0
+
+    def launches_of_a_step():
+        lib.fake_reset()
+        assert lib.dsmd_integrate(s.h, ctypes.c_int(1), f64(0.001), f64(1.0), None) == 0
+        return [line for line in log(lib) if line.startswith("launch")]
+
+    assert [("k_pack" in line, "k_post_displacement" in line) for line in launches_of_a_step()] == [(True, False), (False, True)]
+    word = ptr()
+    assert lib.dsmd_displacement_word(s.h, ctypes.byref(word)) == 0
+    for _ in range(2):
+        lines = launches_of_a_step()
+        assert len(lines) == 1 and "k_pack" in lines[0]
+        assert s.displacement() == 0
+        assert s.run(4, 2) == 0 and any("k_post_displacement" in line for line in log(lib))
     lib.dsmd_destroy(s.h)

@@ -48,7 +48,7 @@ constexpr int kBondedThreads = 128;
 constexpr int kNoSlot = 0x7F7F7F7F;   // what a byte-wise fill of the map with 0x7F leaves: beyond any slot
 constexpr double kCoulombConstant = 332.0636;   // kcal/mol A / e^2, the reference's constant
 
-__global__ void k_bonded_slot_map(int n_total, const int* __restrict__ gid, int n_global, int* __restrict__ slot_of) {
+__global__ void k_bonded_slot_map(int n_total, const int* gid, int n_global, int* __restrict__ slot_of) {
     if (!dsmd::after_previous()) return;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n_total) return;
@@ -122,8 +122,8 @@ __device__ __forceinline__ void put(double* __restrict__ contrib, int place, dou
 // here: this kernel runs beside it and waits for its end only when its own work is done, so that whoever waits for this kernel has
 // waited for both. Step of 63,504 chain atoms: 38.7 us, 43.0 one after the other.
 template <bool SUMS>
-__global__ void __launch_bounds__(kBondedThreads) k_bonded_terms(BondedTable t, const double* __restrict__ x, const double* __restrict__ y,
-                               const double* __restrict__ z, const double* __restrict__ charge,
+__global__ void __launch_bounds__(kBondedThreads) k_bonded_terms(BondedTable t, const double* x, const double* y,
+                               const double* z, const double* charge,
                                double* __restrict__ contrib, double* __restrict__ partials, unsigned* __restrict__ ticket,
                                double* __restrict__ scalars, unsigned* __restrict__ missing, bool beside) {
     if (!beside && !dsmd::after_previous()) return;

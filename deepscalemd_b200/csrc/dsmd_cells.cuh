@@ -15,15 +15,15 @@ namespace dsmd {
 
 // Thread t of `threads`. Atoms [first, end); key, arrival by atom, list by slot. And the counts of `cells` cells, which the scan has
 // read, go back to zero for the next sort.
-__device__ __forceinline__ void cell_place(int t, int threads, int first, int end, const unsigned* __restrict__ key, const int* __restrict__ arrival,
-                                           const int* __restrict__ cell_start, int* __restrict__ list, int cells, int* __restrict__ cell_count) {
+__device__ __forceinline__ void cell_place(int t, int threads, int first, int end, const unsigned* key, const int* arrival,
+                                           const int* cell_start, int* __restrict__ list, int cells, int* __restrict__ cell_count) {
     const int i = first + t;
     if (i < end) list[cell_start[key[i]] + arrival[i]] = i;
     for (int k = t; k < cells; k += threads) cell_count[k] = 0;
 }
 
 // Final slot of the atom `a` of cell `cell`.
-__device__ __forceinline__ int cell_slot(int a, unsigned cell, const int* __restrict__ cell_start, const int* __restrict__ list) {
+__device__ __forceinline__ int cell_slot(int a, unsigned cell, const int* cell_start, const int* list) {
     const int begin = cell_start[cell], end = cell_start[cell + 1];
     int slot = begin;
     for (int k = begin; k < end; ++k) slot += list[k] < a ? 1 : 0;

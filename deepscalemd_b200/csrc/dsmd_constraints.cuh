@@ -45,7 +45,7 @@ __device__ __forceinline__ void half_box_image(double d[3], const ClusterTable& 
         }
 }
 
-__global__ void k_slot_of_gid(int n, const int* __restrict__ gid, int n_global, int* __restrict__ slot_of) {
+__global__ void k_slot_of_gid(int n, const int* gid, int n_global, int* __restrict__ slot_of) {
     if (!dsmd::after_previous()) return;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
@@ -53,7 +53,7 @@ __global__ void k_slot_of_gid(int n, const int* __restrict__ gid, int n_global, 
     if (g >= 0 && g < n_global) slot_of[g] = s;
 }
 
-__global__ void k_cluster_slots(int n, const int* __restrict__ atom_gid, const int* __restrict__ slot_of_gid, int* __restrict__ slot) {
+__global__ void k_cluster_slots(int n, const int* atom_gid, const int* slot_of_gid, int* __restrict__ slot) {
     if (!dsmd::after_previous()) return;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k < n) slot[k] = atom_gid[k] < 0 ? -1 : slot_of_gid[atom_gid[k]];

@@ -107,8 +107,8 @@ __global__ void k_cell_begin(int cells, int* __restrict__ cell_count, Status* st
     if (st && blockIdx.x == 0 && threadIdx.x == 0) *st = Status{};
 }
 
-__global__ void k_cell_keys(Grid g, Brick brick, int first, int n_owned, int n_total, const double* __restrict__ x,
-                            const double* __restrict__ y, const double* __restrict__ z, unsigned* __restrict__ key,
+__global__ void k_cell_keys(Grid g, Brick brick, int first, int n_owned, int n_total, const double* x,
+                            const double* y, const double* z, unsigned* __restrict__ key,
                             int* __restrict__ arrival, int* __restrict__ cell_count, Status* st) {
     if (!dsmd::after_previous()) return;
     const int s = first + blockIdx.x * blockDim.x + threadIdx.x;
@@ -141,9 +141,9 @@ __global__ void k_cell_keys(Grid g, Brick brick, int first, int n_owned, int n_t
 // ghost slot map. FORCES: the force arrays too (a loop that evaluates forces next does not need them). unranked: the cell of
 // atoms that are about to be removed, any number of them in any order, or a number that no cell has.
 template <bool FORCES>
-__global__ void k_reorder(Grid g, int first, int n_owned, int n_total, unsigned unranked, const unsigned* __restrict__ key,
-                          const int* __restrict__ list, const int* __restrict__ cell_start, RealArrays src, RealArrays dst, const int* __restrict__ type_src,
-                          const int* __restrict__ gid_src, int* __restrict__ type_dst, int* __restrict__ gid_dst,
+__global__ void k_reorder(Grid g, int first, int n_owned, int n_total, unsigned unranked, const unsigned* key,
+                          const int* list, const int* cell_start, RealArrays src, RealArrays dst, const int* type_src,
+                          const int* gid_src, int* __restrict__ type_dst, int* __restrict__ gid_dst,
                           int4* __restrict__ pq, float* __restrict__ qf, double* __restrict__ xref,
                           double* __restrict__ yref, double* __restrict__ zref, int* __restrict__ ghost_slot) {
     if (!dsmd::after_previous()) return;
@@ -181,8 +181,8 @@ __global__ void k_reorder(Grid g, int first, int n_owned, int n_total, unsigned 
 
 // A ghost-only sort gathers the ghosts into the other buffer set; this brings them back, so that the owned atoms
 // (already in place) need not be copied across: one thread per ghost, all per-atom arrays.
-__global__ void k_copy_back(int first, int count, RealArrays from, RealArrays to, const int* __restrict__ type_from,
-                            const int* __restrict__ gid_from, int* __restrict__ type_to, int* __restrict__ gid_to) {
+__global__ void k_copy_back(int first, int count, RealArrays from, RealArrays to, const int* type_from,
+                            const int* gid_from, int* __restrict__ type_to, int* __restrict__ gid_to) {
     if (!dsmd::after_previous()) return;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= count) return;
@@ -219,7 +219,7 @@ __global__ void k_build_done(Status* st, unsigned expect_dropped, unsigned strid
 
 // Where the ghosts of a cell row sit: lo_end = one past the last x cell of the row's lower half that holds a ghost (0:
 // none), hi_begin = the first x cell of its upper half that holds one (nc[0]: none). One warp per (y, z) row.
-__global__ void k_ghost_row_extent(Grid g, const int* __restrict__ ghost_cell_start, int* __restrict__ lo_end,
+__global__ void k_ghost_row_extent(Grid g, const int* ghost_cell_start, int* __restrict__ lo_end,
                                    int* __restrict__ hi_begin) {
     if (!dsmd::after_previous()) return;
     const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -244,7 +244,7 @@ __global__ void k_ghost_row_extent(Grid g, const int* __restrict__ ghost_cell_st
 // The same over the rows a centre of row (yc, zc) searches (stencil reach in y and z, wrapping where the axis does): an
 // owned atom whose x window stays inside [near_lo, near_hi) of its row cannot have a ghost partner and skips the ghost
 // pass of the list build altogether.
-__global__ void k_ghost_rows_near(Grid g, const int* __restrict__ lo_end, const int* __restrict__ hi_begin,
+__global__ void k_ghost_rows_near(Grid g, const int* lo_end, const int* hi_begin,
                                   int* __restrict__ near_lo, int* __restrict__ near_hi) {
     if (!dsmd::after_previous()) return;
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
@@ -301,8 +301,8 @@ struct ClusterMembers {
 };
 
 __global__ void k_vv2(int n, double half_dt_c, double* __restrict__ vx, double* __restrict__ vy,
-                      double* __restrict__ vz, const double* __restrict__ fx, const double* __restrict__ fy,
-                      const double* __restrict__ fz, const double* __restrict__ mass, ClusterMembers skip) {
+                      double* __restrict__ vz, const double* fx, const double* fy,
+                      const double* fz, const double* mass, ClusterMembers skip) {
     if (!dsmd::after_previous()) return;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n || skip.has(s)) return;
@@ -326,7 +326,7 @@ __global__ void k_upload_defaults(int n, RealArrays r, int* type, int* gid) {
 }
 
 // [n][3] rows, n words of them in each of three arrays (device memory, or pinned host memory), to three columns.
-__global__ void k_split_rows(int n, const double* __restrict__ rows0, const double* __restrict__ rows1, const double* __restrict__ rows2,
+__global__ void k_split_rows(int n, const double* rows0, const double* rows1, const double* rows2,
                              double* __restrict__ x, double* __restrict__ y, double* __restrict__ z) {
     if (!dsmd::after_previous()) return;
     for (long long k = blockIdx.x * blockDim.x + threadIdx.x; k < 3ll * n; k += gridDim.x * blockDim.x) {
@@ -347,8 +347,8 @@ __global__ void k_scale_velocities(int n, double factor, double* __restrict__ vx
     vz[s] *= factor;
 }
 
-__global__ void k_kinetic(int n, const double* __restrict__ vx, const double* __restrict__ vy,
-                          const double* __restrict__ vz, const double* __restrict__ mass, double* partials, unsigned* ticket,
+__global__ void k_kinetic(int n, const double* vx, const double* vy,
+                          const double* vz, const double* mass, double* partials, unsigned* ticket,
                           double* out, Mail* mail, unsigned long long seq) {
     if (!dsmd::after_previous()) return;
     double v[1] = {0.0};
@@ -374,10 +374,10 @@ namespace {
 template <bool INTEGRATE, bool BONDED>
 __global__ void k_pack(Grid g, int first, int count, int n_owned, double* __restrict__ x, double* __restrict__ y,
                        double* __restrict__ z, double* __restrict__ vx, double* __restrict__ vy,
-                       double* __restrict__ vz, const double* __restrict__ fx, const double* __restrict__ fy,
-                       const double* __restrict__ fz, const double* __restrict__ mass, const int* __restrict__ type,
-                       const double* __restrict__ xref, const double* __restrict__ yref,
-                       const double* __restrict__ zref, int4* __restrict__ pq, double dt, double kick_c,
+                       double* __restrict__ vz, const double* fx, const double* fy,
+                       const double* fz, const double* mass, const int* type,
+                       const double* xref, const double* yref,
+                       const double* zref, int4* __restrict__ pq, double dt, double kick_c,
                        ClusterMembers skip, BondedForces bonded, DisplacementReport report) {
     if (!BONDED && !dsmd::after_previous()) return;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -396,7 +396,8 @@ __global__ void k_pack(Grid g, int first, int count, int n_owned, double* __rest
     }
     if (dsmd::gate_closed(report.st, report.gate2)) return;
     if (t < count && !skip.has(s)) {
-        double px = BONDED ? state[0] : x[s], py = BONDED ? state[1] : y[s], pz = BONDED ? state[2] : z[s];
+        // (without INTEGRATE nothing is written there: __ldcg keeps the reads from the read-only path)
+        double px = BONDED ? state[0] : __ldcg(x + s), py = BONDED ? state[1] : __ldcg(y + s), pz = BONDED ? state[2] : __ldcg(z + s);
         if (INTEGRATE) {
             const double a = BONDED ? state[3] : kick_c / mass[s];
             double f[3] = {0.0, 0.0, 0.0};

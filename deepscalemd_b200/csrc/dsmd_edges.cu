@@ -43,8 +43,8 @@ struct EdgeStatus {
     unsigned int ticket;
 };
 
-__global__ void k_edge_keys(Grid g, int n, const double* __restrict__ x, const double* __restrict__ y,
-                            const double* __restrict__ z, unsigned* __restrict__ key, int* __restrict__ arrival,
+__global__ void k_edge_keys(Grid g, int n, const double* x, const double* y,
+                            const double* z, unsigned* __restrict__ key, int* __restrict__ arrival,
                             int* __restrict__ cell_count, EdgeStatus* st) {
     if (!dsmd::after_previous()) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -90,10 +90,10 @@ __device__ __forceinline__ float place_of(int fixed, float scale) { return __uin
 
 // Sorted atoms in two forms, fixed-point and float (w = the caller's atom index, kPruned: not wanted as a neighbour), and
 // their wrap counts (periodic form only). A thread takes the atom at its place of the cell lists.
-__global__ void k_edge_gather(Grid g, int n, const unsigned* __restrict__ key, const int* __restrict__ list,
-                              const int* __restrict__ cell_start, const double* __restrict__ x, const double* __restrict__ y,
-                              const double* __restrict__ z, const unsigned char* __restrict__ neighbour_ok,
-                              const int* __restrict__ owner, int4* __restrict__ pq, float4* __restrict__ pf, int* __restrict__ wraps,
+__global__ void k_edge_gather(Grid g, int n, const unsigned* key, const int* list,
+                              const int* cell_start, const double* x, const double* y,
+                              const double* z, const unsigned char* neighbour_ok,
+                              const int* owner, int4* __restrict__ pq, float4* __restrict__ pf, int* __restrict__ wraps,
                               EdgeStatus* st) {
     if (!dsmd::after_previous()) return;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -117,7 +117,7 @@ __global__ void k_edge_gather(Grid g, int n, const unsigned* __restrict__ key, c
     }
 }
 
-__global__ void k_edge_place(int n, const unsigned* __restrict__ key, const int* __restrict__ arrival, const int* __restrict__ cell_start,
+__global__ void k_edge_place(int n, const unsigned* key, const int* arrival, const int* cell_start,
                              int* __restrict__ list, int cells, int* __restrict__ cell_count) {
     if (!dsmd::after_previous()) return;
     dsmd::cell_place(blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, 0, n, key, arrival, cell_start, list, cells, cell_count);
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(kSearchThreads) k_edge_search(Grid g, SearchAr
                     for (; s < end; s += kAtATime) {   // loads first, and no branch but the stores'
                         float4 pj[kAtATime];
 #pragma unroll
-                        for (int u = 0; u < kAtATime; ++u) pj[u] = __ldg(&a.pf[min(s + u, end - 1)]);
+                        for (int u = 0; u < kAtATime; ++u) pj[u] = a.pf[min(s + u, end - 1)];
 #pragma unroll
                         for (int u = 0; u < kAtATime; ++u) {
                             const float dx = pj[u].x - sx, ey = pj[u].y - sy, ez = pj[u].z - sz;
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(kSearchThreads) k_edge_search_warp(Grid g, Sea
             const int n = min(total - base, kWarpCandidates);
             for (int t = lane; t - lane < n; t += 32) {
                 const int s = t < n ? slots[t] : p;
-                const int4 pj = __ldg(&a.pq[s]);
+                const int4 pj = a.pq[s];
                 const float dx = dsmd::fixed_delta(pj.x, pi.x, g.scale[0]);
                 const float ey = dsmd::fixed_delta(pj.y, pi.y, g.scale[1]);
                 const float ez = dsmd::fixed_delta(pj.z, pi.z, g.scale[2]);
@@ -389,8 +389,8 @@ struct FlatSlice {
 };
 
 // Where the slice's edges start, and the prefix sums of its atoms' counts.
-__device__ __forceinline__ void open_slice(FlatSlice& f, int n, int group_shift, const int* __restrict__ counts,
-                                           const long long* __restrict__ group_start) {
+__device__ __forceinline__ void open_slice(FlatSlice& f, int n, int group_shift, const int* counts,
+                                           const long long* group_start) {
     if (threadIdx.x < 32) {
         const int lane = threadIdx.x, p0 = blockIdx.x * 32, p = p0 + lane;
         const int cnt = p < n ? counts[p] : 0;
@@ -411,7 +411,7 @@ __device__ __forceinline__ void open_slice(FlatSlice& f, int n, int group_shift,
 }
 
 // Flat positions [from, from + kFlat) of the slice.
-__device__ __forceinline__ void lay_flat(FlatSlice& f, int from, int stride, const unsigned* __restrict__ rows) {
+__device__ __forceinline__ void lay_flat(FlatSlice& f, int from, int stride, const unsigned* rows) {
     const int lane = threadIdx.x & 31, begin = f.prefix[lane], cnt = f.prefix[lane + 1] - begin;
     const unsigned* slice = rows + static_cast<size_t>(blockIdx.x) * stride * 32 + lane;
     const int k1 = min(cnt, from + kFlat - begin);
@@ -425,11 +425,11 @@ __device__ __forceinline__ void lay_flat(FlatSlice& f, int from, int stride, con
 }
 
 // Interface form.
-__global__ void __launch_bounds__(kFillThreads) k_edge_fill(int n, long long n_edges, int stride, int group_shift, const int4* __restrict__ pq,
-                            const unsigned* __restrict__ rows, const int* __restrict__ counts,
-                            const long long* __restrict__ group_start, int n_centers, const int* __restrict__ owner,
-                            const double* __restrict__ shift_x, const double* __restrict__ shift_y,
-                            const double* __restrict__ shift_z, long long* __restrict__ edges,
+__global__ void __launch_bounds__(kFillThreads) k_edge_fill(int n, long long n_edges, int stride, int group_shift, const int4* pq,
+                            const unsigned* rows, const int* counts,
+                            const long long* group_start, int n_centers, const int* owner,
+                            const double* shift_x, const double* shift_y,
+                            const double* shift_z, long long* __restrict__ edges,
                             double* __restrict__ shift) {
     if (!dsmd::after_previous()) return;
     __shared__ FlatSlice f;
@@ -482,8 +482,8 @@ __global__ void __launch_bounds__(kFillThreads) k_edge_fill(int n, long long n_e
 // neighbours; 0.19 ms (0.28 ms before). 14 blocks per SM: registers for 14 cost nothing and hide the start of a slice.
 template <bool WRAPS>
 __global__ void __launch_bounds__(kFillThreads, 14) k_edge_fill_compact(
-    Grid g, int n, int stride, int group_shift, const int4* __restrict__ pq, const int* __restrict__ wraps,
-    const unsigned* __restrict__ rows, const int* __restrict__ counts, const long long* __restrict__ group_start,
+    Grid g, int n, int stride, int group_shift, const int4* pq, const int* wraps,
+    const unsigned* rows, const int* counts, const long long* group_start,
     int* __restrict__ src, int* __restrict__ dst, signed char* __restrict__ shift, float* __restrict__ vec) {
     if (!dsmd::after_previous()) return;
     __shared__ FlatSlice f;
@@ -514,8 +514,8 @@ __global__ void __launch_bounds__(kFillThreads, 14) k_edge_fill_compact(
         const auto fetch = [&](int t) {
             if (t < from || t >= upto) return;
             const int slot = f.entry[t - from];
-            pj_next = __ldg(&pq[slot]);
-            if (WRAPS) wj_next = __ldg(&wraps[slot]);
+            pj_next = pq[slot];
+            if (WRAPS) wj_next = wraps[slot];
         };
         fetch(t0 + lane);
         for (; t0 < upto; t0 += kFillThreads) {
@@ -567,8 +567,8 @@ __global__ void __launch_bounds__(kFillThreads, 14) k_edge_fill_compact(
 
 // Smallest and largest coordinate per axis, reported to the host: x, y, z least, x, y, z most. NaN coordinates do not count
 // (they are found when the atoms are put into cells).
-__global__ void __launch_bounds__(kThreads) k_edge_bounds(int n, const double* __restrict__ x, const double* __restrict__ y,
-                                                          const double* __restrict__ z, double* __restrict__ partials, unsigned* ticket,
+__global__ void __launch_bounds__(kThreads) k_edge_bounds(int n, const double* x, const double* y,
+                                                          const double* z, double* __restrict__ partials, unsigned* ticket,
                                                           dsmd::Mail* mail, unsigned long long seq) {
     if (!dsmd::after_previous()) return;
     __shared__ double sh[kThreads / 32][6];
@@ -659,8 +659,8 @@ __device__ __forceinline__ int nth_set_bit(unsigned mask, int n) {
 }
 
 // Per atom: the three shift masks packed into one word, and how many images that makes.
-__global__ void k_image_masks(ImageLattice L, int n, const double* __restrict__ x, const double* __restrict__ y,
-                              const double* __restrict__ z, unsigned long long* __restrict__ masks,
+__global__ void k_image_masks(ImageLattice L, int n, const double* x, const double* y,
+                              const double* z, unsigned long long* __restrict__ masks,
                               long long* __restrict__ counts) {
     if (!dsmd::after_previous()) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -675,7 +675,7 @@ __global__ void k_image_masks(ImageLattice L, int n, const double* __restrict__ 
 }
 
 // Images of the whole system, reported to the host.
-__global__ void k_image_total(int n, const long long* __restrict__ counts, const long long* __restrict__ first_image, dsmd::Mail* mail,
+__global__ void k_image_total(int n, const long long* counts, const long long* first_image, dsmd::Mail* mail,
                               unsigned long long seq) {
     if (!dsmd::after_previous()) return;
     const double total[1] = {static_cast<double>(first_image[n - 1] + counts[n - 1])};
@@ -684,9 +684,9 @@ __global__ void k_image_total(int n, const long long* __restrict__ counts, const
 
 // One thread per output slot: slots [0, n) are the wrapped atoms, slot n + m is image number m of the whole system, which
 // belongs to the last atom whose first image number is <= m.
-__global__ void k_image_fill(ImageLattice L, int n, long long n_images, const double* __restrict__ x,
-                             const double* __restrict__ y, const double* __restrict__ z, const int* __restrict__ type,
-                             const unsigned long long* __restrict__ masks, const long long* __restrict__ first_image,
+__global__ void k_image_fill(ImageLattice L, int n, long long n_images, const double* x,
+                             const double* y, const double* z, const int* type,
+                             const unsigned long long* masks, const long long* first_image,
                              double* __restrict__ out_x, double* __restrict__ out_y, double* __restrict__ out_z,
                              int* __restrict__ out_type, int* __restrict__ out_owner, double* __restrict__ off_x,
                              double* __restrict__ off_y, double* __restrict__ off_z) {
@@ -734,9 +734,9 @@ __global__ void k_image_fill(ImageLattice L, int n, long long n_images, const do
 // target[i] += f[i] + the forces on the images of atom i, added in slot order (MLIPStep::add_forces,
 // src/MLIPStep.cu:108-124, 373-381), for the first n_out of the n atoms. with_images == 0: the images were edge shifts,
 // not atoms the model saw, and carry no force.
-__global__ void k_image_fold(int n_out, int n, int with_images, const double* __restrict__ fx,
-                             const double* __restrict__ fy, const double* __restrict__ fz,
-                             const long long* __restrict__ first_image, const long long* __restrict__ counts,
+__global__ void k_image_fold(int n_out, int n, int with_images, const double* fx,
+                             const double* fy, const double* fz,
+                             const long long* first_image, const long long* counts,
                              double* __restrict__ tx, double* __restrict__ ty, double* __restrict__ tz) {
     if (!dsmd::after_previous()) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -757,9 +757,9 @@ __global__ void k_image_fold(int n_out, int n, int with_images, const double* __
 
 // Sum over atoms of r . F and of its three diagonal terms (MLIPStep::virial / virial_diag, src/MLIPStep.cu:126-148,
 // 383-432): per-block sums in a fixed order, which the block that finishes last adds up in a fixed order and reports.
-__global__ void __launch_bounds__(kThreads) k_virial(long long n, const double* __restrict__ x, const double* __restrict__ y,
-                                                     const double* __restrict__ z, const double* __restrict__ fx,
-                                                     const double* __restrict__ fy, const double* __restrict__ fz,
+__global__ void __launch_bounds__(kThreads) k_virial(long long n, const double* x, const double* y,
+                                                     const double* z, const double* fx,
+                                                     const double* fy, const double* fz,
                                                      double* __restrict__ partials, unsigned* ticket, dsmd::Mail* mail, unsigned long long seq) {
     if (!dsmd::after_previous()) return;
     __shared__ double sh[kThreads / 32][3];
@@ -796,8 +796,8 @@ __global__ void __launch_bounds__(kThreads) k_virial(long long n, const double* 
     }
 }
 
-__global__ void k_mark_receivers(int n, const double* __restrict__ x, const double* __restrict__ y,
-                                 const double* __restrict__ z, double lx, double ly, double lz, double hx, double hy,
+__global__ void k_mark_receivers(int n, const double* x, const double* y,
+                                 const double* z, double lx, double ly, double lz, double hx, double hy,
                                  double hz, double reach2, unsigned char* __restrict__ ok) {
     if (!dsmd::after_previous()) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;

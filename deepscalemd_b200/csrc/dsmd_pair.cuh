@@ -330,10 +330,10 @@ __device__ __forceinline__ PairAccumulator<COPIES, ENERGY, SWITCH> close_rest(co
     for (int k = k0 + (threadIdx.x & 31); k < k1; k += 32) {
         if (k >= mid && k < ghosts) continue;
         const unsigned e = words[row_offset<ORDER>(k)];
-        const int4 pj = __ldg(&a.pq[e]);
+        const int4 pj = a.pq[e];
         F2 dx, dy, dz;
         const F2 r2 = Sums::distance(p, pa, pb, pj, dx, dy, dz);
-        rest.add_close_rest(p, table, dx, dy, dz, r2, mul(q, both(BY_TYPE ? p.type_charge[pj.w] : __ldg(&a.qf[e]))));
+        rest.add_close_rest(p, table, dx, dy, dz, r2, mul(q, both(BY_TYPE ? p.type_charge[pj.w] : a.qf[e])));
     }
     if ((threadIdx.x & 31) == 0 && atoms > 1 && a.phase != DSMD_PHASE_BOUNDARY && !(a.rows.row_special[pair] & kRowOwnExcluded)) {
         F2 dx, dy, dz;
@@ -431,8 +431,8 @@ __device__ __forceinline__ void row_forces(const PairParams& p, const ForceArgs&
                 of_type[k].att = f2(la.y, lb.y);
             }
         const auto take = [&](unsigned e, int4& pos, float& charge) {
-            pos = __ldg(&a.pq[e]);
-            if (COULOMB && !by_type) charge = __ldg(&a.qf[e]);
+            pos = a.pq[e];
+            if (COULOMB && !by_type) charge = a.qf[e];
         };
         const auto terms = [&](int type, float charge) {
             PairTerms k = one;

@@ -64,7 +64,7 @@ __host__ __device__ inline int whole_groups(int k) {
 }
 
 // First atom and number of atoms (0, 1, 2) of a pair.
-__device__ __forceinline__ int pair_atoms(const unsigned* __restrict__ quad, int pair, int& first) {
+__device__ __forceinline__ int pair_atoms(const unsigned* quad, int pair, int& first) {
     const unsigned w = quad[pair >> 1];
     first = static_cast<int>(w >> 2) + 2 * (pair & 1);
     return w == kNoQuad ? 0 : min(max(static_cast<int>(w & 3u) + 1 - 2 * (pair & 1), 0), 2);

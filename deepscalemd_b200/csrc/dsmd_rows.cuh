@@ -17,7 +17,7 @@ struct QuadArgs {
 // The quads of cell row `row` (a warp): the numbers between two rows' bases that no atoms fill are kNoQuad.
 // layer_start: first slot of every z layer of cells, and the end, by which a caller cuts the sorted
 // atoms into slabs; with `tag` in the same word, so that the host sees of each whether it has arrived.
-__device__ __forceinline__ void row_quads(const QuadArgs& a, int row, const int* __restrict__ cell_start) {
+__device__ __forceinline__ void row_quads(const QuadArgs& a, int row, const int* cell_start) {
     const int lane = threadIdx.x & 31;
     if (row >= a.rows) return;
     const int begin = min(cell_start[static_cast<size_t>(row) * a.nx], a.n_owned);
@@ -34,8 +34,8 @@ __device__ __forceinline__ void row_quads(const QuadArgs& a, int row, const int*
 }
 
 // Behind the scan of a sort: atoms into the cells' lists (the first place_blocks blocks), quads (the others).
-__global__ void k_place(int place_blocks, int first, int end, const unsigned* __restrict__ key, const int* __restrict__ arrival,
-                        const int* __restrict__ cell_start, int* __restrict__ list, int cells, int* __restrict__ cell_count, QuadArgs quads) {
+__global__ void k_place(int place_blocks, int first, int end, const unsigned* key, const int* arrival,
+                        const int* cell_start, int* __restrict__ list, int cells, int* __restrict__ cell_count, QuadArgs quads) {
     if (!dsmd::after_previous()) return;
     const int block = static_cast<int>(blockIdx.x) - place_blocks;
     if (block < 0) dsmd::cell_place(blockIdx.x * blockDim.x + threadIdx.x, place_blocks * blockDim.x, first, end, key, arrival, cell_start, list, cells, cell_count);
@@ -97,24 +97,25 @@ struct ExcludedRange {
 // to all four: one fixed-point difference and conversion per candidate, the other atoms by their float offsets from the
 // first. Otherwise every atom takes its own fixed-point difference (exact for any placement).
 template <bool NEAR, bool EXCL, int ORDER>
-__device__ __forceinline__ void test_candidates(const Grid& g, QuadSearch& q, int n, const int* __restrict__ s_slot,
-                                                const int4* __restrict__ pq, const int* __restrict__ gid, const ExclusionTable& excl,
+__device__ __forceinline__ void test_candidates(const Grid& g, QuadSearch& q, int n, const int* s_slot,
+                                                const int4* pq, const int* gid, const ExclusionTable& excl,
                                                 const ExcludedRange& s_excluded) {
     const int lane = threadIdx.x & 31;
     const unsigned lt_mask = (1u << lane) - 1u;
     const unsigned own_first = static_cast<unsigned>(min(q.n_atoms, 2)), own_second = static_cast<unsigned>(max(q.n_atoms - 2, 0));
-    // the next round's candidate is on its way while this one is tested, and its slot a round before that
+    // the next round's candidate is on its way while this one is tested, and its slot a round before that (__ldca: ordinary loads, but
+    // the compiler need not keep their order with the stores of rows; 1.79 ms at 4,000,000 atoms, 1.83 with the order kept)
     int s_next = lane < n ? s_slot[lane] : q.first;
-    int4 c_next = __ldg(&pq[s_next]);
-    int g_next = EXCL ? __ldg(&gid[s_next]) : 0;
+    int4 c_next = __ldca(&pq[s_next]);
+    int g_next = EXCL ? __ldca(&gid[s_next]) : 0;
     int s_after = lane + 32 < n ? s_slot[lane + 32] : q.first;
     for (int t = lane; t - lane < n; t += 32) {
         const bool valid = t < n;
         const int s = s_next, gj = g_next;
         const int4 c = c_next;
         s_next = s_after;
-        c_next = __ldg(&pq[s_next]);
-        if (EXCL) g_next = __ldg(&gid[s_next]);
+        c_next = __ldca(&pq[s_next]);
+        if (EXCL) g_next = __ldca(&gid[s_next]);
         s_after = t + 64 < n ? s_slot[t + 64] : q.first;
         float r[4];
         if (NEAR) {
@@ -129,7 +130,7 @@ __device__ __forceinline__ void test_candidates(const Grid& g, QuadSearch& q, in
         } else {
 #pragma unroll
             for (int m = 0; m < 4; ++m) {
-                const int4 atom = __ldg(&pq[q.first + min(m, q.n_atoms - 1)]);
+                const int4 atom = __ldca(&pq[q.first + min(m, q.n_atoms - 1)]);
                 const float dx = dsmd::fixed_delta(c.x, atom.x, g.scale[0]);
                 const float dy = dsmd::fixed_delta(c.y, atom.y, g.scale[1]);
                 const float dz = dsmd::fixed_delta(c.z, atom.z, g.scale[2]);
@@ -192,9 +193,9 @@ __device__ __forceinline__ void test_candidates(const Grid& g, QuadSearch& q, in
 
 template <bool EXCL, int ORDER>
 __global__ void __launch_bounds__(kBuildThreads, EXCL ? 8 : 7)
-k_build_rows(Grid g, int n_owned, int n_total, int n_quads, const int4* __restrict__ pq, const int* __restrict__ gid,
-             ExclusionTable excl, const int* __restrict__ cell_start, const int* __restrict__ ghost_near_lo,
-             const int* __restrict__ ghost_near_hi, RowArrays out, int* __restrict__ boundary_pairs, Status* st) {
+k_build_rows(Grid g, int n_owned, int n_total, int n_quads, const int4* pq, const int* gid,
+             ExclusionTable excl, const int* cell_start, const int* ghost_near_lo,
+             const int* ghost_near_hi, RowArrays out, int* __restrict__ boundary_pairs, Status* st) {
     if (!dsmd::after_previous()) return;
     __shared__ int s_slots[kBuildThreads / 32][kCandidates];
     __shared__ __align__(16) ExcludedRange s_ranges[EXCL ? kBuildThreads / 32 : 1];

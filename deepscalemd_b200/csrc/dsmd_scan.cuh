@@ -20,7 +20,7 @@ constexpr int kScanBlocksMost = 256;
 constexpr int kScanMost = kScanItems * kScanBlocksMost;
 
 // Counts [first, first + kScanEach) of n, whether or not they lie on 16 bytes.
-__device__ __forceinline__ int scan_load(const int* __restrict__ counts, int first, int n, int (&v)[kScanEach]) {
+__device__ __forceinline__ int scan_load(const int* counts, int first, int n, int (&v)[kScanEach]) {
     if (first + kScanEach <= n && (reinterpret_cast<size_t>(counts) & 15) == 0) {
 #pragma unroll
         for (int q = 0; q < kScanEach; q += 4) {
@@ -49,7 +49,7 @@ __device__ __forceinline__ int scan_block_sum(int v) {
     return v;
 }
 
-static __global__ void __launch_bounds__(kScanThreads) k_cell_sums(int n, const int* __restrict__ counts, int* __restrict__ sums) {
+static __global__ void __launch_bounds__(kScanThreads) k_cell_sums(int n, const int* counts, int* __restrict__ sums) {
     if (!after_previous()) return;
     int v[kScanEach];
     const int all = scan_block_sum(scan_load(counts, blockIdx.x * kScanItems + threadIdx.x * kScanEach, n, v));
@@ -57,7 +57,7 @@ static __global__ void __launch_bounds__(kScanThreads) k_cell_sums(int n, const 
 }
 
 // starts[k] = init + counts[0] + ... + counts[k - 1] for k < n. sums: of the blocks' counts, or null.
-static __global__ void __launch_bounds__(kScanThreads) k_cell_starts(int n, int init, const int* __restrict__ counts, const int* __restrict__ sums,
+static __global__ void __launch_bounds__(kScanThreads) k_cell_starts(int n, int init, const int* counts, const int* sums,
                                                                      int* __restrict__ starts) {
     if (!after_previous()) return;
     __shared__ int s_warp[32];

@@ -396,3 +396,279 @@ def test_rows_of_memory_registered_in_part(cuda_device, first, last):
     assert int(runtime.cudaHostUnregister(rows.ctypes.data + lo)) == 0
     assert np.array_equal(np.stack([ctx.download(k, n) for k in "xyz"], axis=1), want)
     ctx.close()
+
+
+# types, Coulomb, exclusions, atoms at one place, pairs below the Ewald table
+LONG_ROWS_WITH_GHOSTS = [(1, False, False, False, False), (2, False, True, False, False), (9, False, False, True, False), (1, True, False, False, True),
+                         (2, True, True, False, False), (3, True, False, True, True)]
+
+
+@pytest.mark.parametrize("dims", [(2, 1, 1), (2, 2, 1)])
+@pytest.mark.parametrize("nt,coulomb,excl,coincide,close", LONG_ROWS_WITH_GHOSTS)
+def test_long_rows_with_ghosts(cuda_device, nt, coulomb, excl, coincide, close, dims):
+    """Rows of 240 entries and more (groups of 16 entries, four lanes and more per row) that end in ghosts: all at once, and first the
+    owned partners and then the ghosts, with and without sums, brick by brick against the undivided system."""
+    from deepscalemd_b200 import synthetic as syn
+    n, L, rc, skin = 3000, 26.0, 6.5, 0.5
+    rng = np.random.default_rng(nt + 10 * coulomb)
+    side = int(np.ceil(n ** (1 / 3)))
+    sites = np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij"), -1).reshape(-1, 3)[rng.permutation(side ** 3)[:n]]
+    pos, box = ((sites + 0.5 + rng.uniform(-0.2, 0.2, (n, 3))) * (L / side)) % L, np.full(3, L)
+    near = np.argsort(np.abs(pos[:, 0] - L / 2))   # of the face between the bricks
+    touched = np.zeros(n, bool)
+    if coincide:
+        pos[near[40:48]] = pos[near[:8]]
+        touched[near[:8]] = touched[near[40:48]] = True
+    if close:
+        a, b = near[100:108], near[140:148]
+        pos[a, 0] = L / 2 - rng.uniform(0.1, 0.3, 8)
+        pos[b] = pos[a] + [0.6, 0.0, 0.0]
+        touched[a] = touched[b] = True
+    types, charge = rng.integers(0, nt, n).astype(np.int32), rng.uniform(-0.5, 0.5, n) if coulomb else np.zeros(n)
+    eps, sig = np.full((nt, nt), 0.3), np.full((nt, nt), 0.5)
+    sig += 0.05 * np.add.outer(np.arange(nt), np.arange(nt)) / nt
+    pairs = co.pairs(*pos.T, n, box, search=rc + skin)
+    exclusions = pairs[:: 7] if excl else None
+    c6, c12 = co.lj_tables(eps, sig)
+    want, scalars = co.forces(*pos.T, n, box, pairs, c6, c12, rc, charge=charge, types=types, do_coulomb=coulomb,
+                              alpha=co.ewald_alpha(rc) if coulomb else 0.0, exclusions=exclusions)
+
+    def check(got, atom):
+        for mask in (touched[atom], ~touched[atom]):   # (what touches feels far more than the others)
+            if mask.any():
+                assert np.abs(got[mask] - want[atom[mask]]).max() <= 2e-5 * np.abs(want[atom[mask]]).max()
+
+    pe = counted = 0.0
+    halo = rc + skin + 0.2
+    for brick in syn.brick_decompose(pos, box, dims, halo):
+        own, src, img = brick["owned"], brick["ghost_src"], brick["ghost_image"]
+        place, atom = np.concatenate([pos[own], pos[src] + img * box]), np.concatenate([own, src])
+        ctx = capi.Context(len(atom))
+        ctx.set_box(box, (1, 1, 1), brick["lo"], brick["hi"], halo)
+        ctx.set_pair_params(eps, sig, rc, skin)
+        if coulomb:
+            ctx.set_coulomb(True)
+        if excl:
+            ctx.set_exclusions(n, exclusions)
+        ctx.upload(place, n_owned=len(own), types=types[atom], charge=charge[atom], gid=atom.astype(np.int32))
+        ctx.build_neighbor_list()
+        assert ctx.list_stats()["row_stride"] >= 240
+        i, j = ctx.list_pairs()[:2]
+        here = ctx.download("global_id", len(atom))
+        assert ctx.list_stats()["interior_entries"] == int((np.asarray(j) < len(own)).sum()) < len(j)
+        for energy in (False, True):
+            for phases in ((capi.PHASE_INTERIOR, capi.PHASE_BOUNDARY), (capi.PHASE_FULL,)):
+                for phase in phases:
+                    ctx.compute_forces(phase, want_energy=energy)
+                check(np.stack([ctx.download(k, len(own)) for k in ("fx", "fy", "fz")], axis=1), here[:len(own)])
+                if energy:
+                    sums = ctx.read_scalars()
+                    if len(phases) == 2:
+                        parts = sums
+        assert abs(parts["pe"] - sums["pe"]) <= 1e-6 * abs(sums["pe"]) and parts["pairs_in_cutoff"] == sums["pairs_in_cutoff"]
+        pe += sums["pe"]
+        counted += sums["pairs_in_cutoff"]
+        ctx.close()
+    # charges of either sign all but cancel in the sum: a rounding of single precision per term, of terms of up to 332 / 4 / 1.4
+    # at random signs, each counted twice at half
+    cancelled = 2.0 ** -24 * 60.0 * np.sqrt(2.0 * counted) if coulomb else 0.0
+    assert abs(pe - scalars["pe"]) <= 1e-5 * abs(scalars["pe"]) + cancelled
+    # a pair within a rounding of single precision of the cutoff counts or not: 2^-23 of 295,000 pairs, half as many again per unit of
+    # ln r^2, are 0.05 per system (one here lies 5e-9 inside)
+    assert abs(counted - scalars["pairs_in_cutoff"]) <= 1
+
+
+def after_steps(make, steps, dt, f2a=1.0, hi_frac=0.5, lagged=None, bonded=False):
+    """Places and velocities after some steps, by run_nve or (lagged None) through the single entry points; and the rebuilds."""
+    ctx, limit = make()
+    ctx.build_neighbor_list()
+    ctx.compute_forces()
+    if bonded:
+        ctx.compute_bonded()
+    rebuilds = 0
+    if lagged is not None:
+        rebuilds = ctx.run_nve(steps, dt, f2a, hi_frac, 0, lagged)["rebuilds"]
+    else:
+        for _ in range(steps):
+            ctx.integrate(1, dt, f2a)
+            if ctx.max_displacement_sq() > (hi_frac * limit) ** 2:
+                ctx.build_neighbor_list()
+                rebuilds += 1
+            ctx.compute_forces()
+            if bonded:
+                ctx.compute_bonded()
+            ctx.integrate(2, dt, f2a)
+    n = ctx.counts()[0]
+    gid = ctx.download("global_id", n)
+    out = np.empty((n, 6))
+    out[gid] = np.stack([ctx.download(k, n) for k in ("x", "y", "z", "vx", "vy", "vz")], axis=1)
+    stride = ctx.list_stats()["row_stride"]
+    ctx.close()
+    return out[:, :3], out[:, 3:], rebuilds, stride
+
+
+def assert_same_run(make, steps, dt, rebuilds_least, tolerance=1e-6, **kwargs):
+    """The loop sums the same forces in the same order as the single calls, over lists built at the same steps: what is left are
+    the roundings of two half kicks against one whole (2^-53), multiplied by the system's own divergence."""
+    want, got = after_steps(make, steps, dt, **kwargs), after_steps(make, steps, dt, lagged=False, **kwargs)
+    assert got[2] == want[2] >= rebuilds_least
+    for g, w in zip(got[:2], want[:2]):
+        assert np.abs(g - w).max() <= tolerance * np.abs(w).max()
+    return got
+
+
+def test_longer_rows_inside_the_loop_with_forces(cuda_device):
+    """Atoms that interact and fall towards the middle of the box: where the rows turn out too short, the step queued behind the list
+    build must not have happened, and the next one must read the places that it would have read."""
+    side, L = 14, 40.0
+    rng = np.random.default_rng(8)
+    pos = (np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij"), -1).reshape(-1, 3) + rng.uniform(-0.1, 0.1, (side ** 3, 3))) * 1.7 + 8.0
+    vel = (L / 2 - pos) * 0.6
+
+    def make():
+        ctx = capi.Context(len(pos))
+        ctx.set_box(np.full(3, L))
+        ctx.set_pair_params([[1.0]], [[0.8]], 2.5, 0.6)
+        ctx.upload(pos, vel=vel)
+        return ctx, 0.6
+
+    ctx, _ = make()
+    ctx.build_neighbor_list()
+    short = ctx.list_stats()["row_stride"]
+    ctx.close()
+    _, _, _, stride = assert_same_run(make, 120, 0.005, 3)
+    assert stride > short
+
+
+@pytest.mark.parametrize("side,free", [(12, False), (12, True), (38, False)])   # 38: more than 25,000 groups
+def test_loop_with_constraints_equals_step_by_step(cuda_device, side, free):
+    rng = np.random.default_rng(side)
+    sites = (np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij"), -1).reshape(-1, 3) + 0.5) * 2.2
+    u = rng.normal(size=sites.shape)
+    u *= 0.45 / np.linalg.norm(u, axis=1, keepdims=True)
+    groups = len(sites) * 2 // 3 if free else len(sites)
+    pos = np.concatenate([np.stack([sites[:groups] - u[:groups], sites[:groups] + u[:groups]], 1).reshape(-1, 3), sites[groups:]])
+    n, box = len(pos), np.full(3, side * 2.2)
+    mates = np.arange(2 * groups, dtype=np.int32).reshape(-1, 2)
+    vel = rng.normal(scale=1.2, size=(n, 3))
+    vel[:2 * groups] = np.repeat(vel[:groups], 2, axis=0)
+
+    def make():
+        ctx = capi.Context(n)
+        ctx.set_box(box)
+        ctx.set_pair_params([[1.0]], [[0.9]], 2.5, 0.4)
+        ctx.set_exclusions(n, mates)
+        ctx.set_constraints(n, np.concatenate([mates, np.full((groups, 1), 0.9)], axis=1))
+        ctx.upload(pos % box, vel=vel)
+        return ctx, 0.4
+
+    # SHAKE stops at a relative error of 1e-8 of the squared length, from places that differ by their roundings
+    assert_same_run(make, 60, 0.004, 2, tolerance=1e-5)
+
+
+def test_loop_with_constrained_water_equals_step_by_step(cuda_device):
+    from deepscalemd_b200 import synthetic as syn
+    s = syn.water_box(11, seed=5)
+
+    def make():
+        ctx = capi.Context(s.n)
+        ctx.set_box(s.box)
+        ctx.set_pair_params(s.eps, s.sig, s.cutoff, s.skin)
+        ctx.set_coulomb(True)
+        ctx.set_exclusions(s.n, s.exclusions)
+        ctx.set_constraints(s.n, s.constraints)
+        ctx.upload(s.pos, vel=s.vel, mass=s.mass, types=s.types, charge=s.charge)
+        return ctx, s.skin
+
+    assert_same_run(make, 60, 2.0, 2, tolerance=1e-5, f2a=4.184e-4, hi_frac=0.1)
+
+
+def test_loop_with_bonded_terms_equals_step_by_step(cuda_device):
+    from deepscalemd_b200 import synthetic as syn
+    s = syn.chain_fluid(4, 8, spacing=14.0, seed=12)   # (closer ones overlap)
+
+    def make():
+        ctx = capi.Context(s.n)
+        ctx.set_box(s.box)
+        ctx.set_pair_params(s.eps, s.sig, s.cutoff, s.skin)
+        ctx.set_coulomb(True)
+        ctx.set_exclusions(s.n, s.exclusions)
+        ctx.set_bonded(s.n, s.bonded)
+        ctx.upload(s.pos, vel=s.vel, mass=s.mass, types=s.types, charge=s.charge)
+        return ctx, s.skin
+
+    assert_same_run(make, 80, 0.5, 2, f2a=s.force_to_accel, hi_frac=0.1, bonded=True)
+
+
+def test_loop_of_many_threads_equals_step_by_step(cuda_device):
+    """More than 25,000 threads: checks reported by a launch of their own, behind the loop's kernel and behind the single calls'."""
+    from deepscalemd_b200 import synthetic as syn
+    s = syn.fcc_lj(20)
+
+    def make():
+        ctx = capi.Context(s.n)
+        ctx.set_box(s.box)
+        ctx.set_pair_params(s.eps, s.sig, s.cutoff, s.skin)
+        ctx.upload(s.pos, vel=s.vel)
+        return ctx, s.skin
+
+    assert_same_run(make, 40, 0.004, 2)
+
+
+@pytest.mark.parametrize("system", ["lj_864", "lj_32000", "water", "chains"])
+def test_captured_steps_equal_the_calls(cuda_device, system):
+    """A whole step captured into a graph (kernels that overlap become programmatic edges) and replayed, against the same calls."""
+    import torch
+    from deepscalemd_b200 import synthetic as syn
+    s = {"lj_864": lambda: syn.fcc_lj(6), "lj_32000": lambda: syn.fcc_lj(20), "water": lambda: syn.water_box(11, seed=6),
+         "chains": lambda: syn.chain_fluid(4, 8, spacing=14.0, seed=15)}[system]()
+    dt, f2a = {"water": (1.0, 4.184e-4), "chains": (0.5, getattr(s, "force_to_accel", 1.0))}.get(system, (0.002, 1.0))
+    ends = []
+    for captured in (False, True):
+        ctx = capi.Context(s.n)
+        ctx.set_box(s.box)
+        ctx.set_pair_params(s.eps, s.sig, s.cutoff, s.skin)
+        if s.coulomb:
+            ctx.set_coulomb(True)
+        if s.exclusions is not None:
+            ctx.set_exclusions(s.n, s.exclusions)
+        if system == "water":
+            ctx.set_constraints(s.n, s.constraints)
+        if system == "chains":
+            ctx.set_bonded(s.n, s.bonded)
+        ctx.upload(s.pos, vel=s.vel, mass=s.mass, types=s.types, charge=s.charge)
+        ctx.build_neighbor_list()
+        stream = torch.cuda.Stream()
+
+        def step():
+            ctx.integrate(1, dt, f2a, stream=stream)
+            ctx.compute_forces(stream=stream)
+            if system == "chains":
+                ctx.compute_bonded(stream=stream)
+            ctx.integrate(2, dt, f2a, stream=stream)
+
+        ctx.compute_forces(stream=stream)
+        if system == "chains":
+            ctx.compute_bonded(stream=stream)
+        step()   # allocations, and the maps from ids to slots
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        if captured:
+            with torch.cuda.graph(graph, stream=stream):
+                step()
+                step()
+        for _ in range(4):
+            if captured:
+                graph.replay()
+            else:
+                step()
+                step()
+        torch.cuda.synchronize()
+        moved = ctx.max_displacement_sq()
+        gid = ctx.download("global_id", s.n)
+        out = np.empty((s.n, 9))
+        out[gid] = np.stack([ctx.download(k, s.n) for k in ("x", "y", "z", "vx", "vy", "vz", "fx", "fy", "fz")], axis=1)
+        ends.append((out, moved))
+        del graph
+        ctx.close()
+    assert np.array_equal(ends[0][0], ends[1][0]) and ends[0][1] == ends[1][1] > 0.0

@@ -670,7 +670,7 @@ struct dsmd_ctx {
     bool slot_map_valid = false;
     double cons_tolerance = 1e-8;
     int cons_max_iterations = 500;
-    bool owned_sorted_only = false;
+    bool owned_sorted_only = false;   // the owned atoms lie as their last sort left them: a list build sorts the ghosts alone
     int64_t expect_dropped = 0;    // atoms the last owned-only sort was told to remove (checked with the build status)
     int64_t stat_entries = 0, stat_interior = 0;   // worked out when asked for (list_members)
     int stat_rechecked = 0;
@@ -1248,6 +1248,7 @@ static int upload_rest(dsmd_ctx* c, int64_t n_owned, int64_t n_total, const doub
     c->n_total = n_total;
     c->list_valid = false;
     c->slot_map_valid = false;
+    c->owned_sorted_only = false;
     return DSMD_OK;
 }
 
@@ -1347,6 +1348,7 @@ int dsmd_upload_positions(dsmd_ctx* c, const double* x, const double* y, const d
     const double* src[3] = {x, y, z};
     for (int a = 0; a < 3; ++a)
         DSMD_CUDA(c, cudaMemcpyAsync(c->real[c->cur][a], src[a], sizeof(double) * c->n_total, cudaMemcpyHostToDevice, s));
+    c->owned_sorted_only = false;
     return DSMD_OK;
 }
 
@@ -2455,6 +2457,7 @@ int dsmd_forces_host(dsmd_ctx* c, const double* x, const double* y, const double
     {
         const int rc = from.all && c->n_total > 0 ? pull_positions(c, from, 0, c->n_total, s) : dsmd_upload_positions(c, x, y, z, s);
         if (rc) return rc;
+        c->owned_sorted_only = false;
     }
     if (rebuild || !c->list_valid) {
         const int rc = dsmd_build_neighbor_list(c, s);

@@ -139,6 +139,19 @@ def test_a_check_that_finds_an_atom_outside_can_be_asked_again(lib, system):
     assert system.displacement() != CUDA_ERROR
 
 
+@pytest.mark.parametrize("positions_only", [False, True])
+def test_a_sort_of_the_owned_atoms_does_not_count_for_atoms_uploaded_since(lib, system, positions_only):
+    """A build behind dsmd_sort_owned sorts the ghosts alone: not if there are other atoms, or places, than were sorted."""
+    assert lib.dsmd_sort_owned(system.h, None) == 0
+    if positions_only:
+        assert lib.dsmd_upload_positions(system.h, *(ptr(a.ctypes.data) for a in np.ascontiguousarray(system.rows.T)), None) == 0
+    else:
+        assert upload(system, system.rows) == 0
+    lib.fake_reset()
+    assert system.build() == 0
+    assert any("k_cell_keys" in line for line in log(lib)) and any("k_reorder" in line for line in log(lib))
+
+
 # -- uploads of rows ----------------------------------------------------------------------------------------------------
 def upload(s, pos, vel=None):
     return s.lib.dsmd_upload_rows(s.h, i64(len(pos)), i64(len(pos)), ptr(pos.ctypes.data), ptr(vel.ctypes.data) if vel is not None else None, None,

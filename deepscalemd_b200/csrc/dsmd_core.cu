@@ -62,9 +62,15 @@ constexpr int kDeviceSms = 148;                       // of a B200
 constexpr int64_t pair_lanes_wanted(int shift) { return kDeviceSms * (shift == 0 ? 512 : 352); }
 constexpr int64_t kPairLanesWantedEwald = kDeviceSms * 768;   // one and a half rounds of one block of 512 each
 // Threads of a launch up to which its last block reports the displacement check; beyond, a launch of its own does, and no block waits
-// for its writes to arrive before it takes its ticket (one word for all) and makes room for the next. Steps of 1,500 (24,000
-// threads), 5,000, 20,000, 75,000, 260,000 and 4,000,000 Lennard-Jones atoms: 7.3, 7.4, 9.8, 17.0, 39.8 and 441 us, with tickets 6.9, 9.1, 13.1,
-// 23.6, 42.3 and 455.
+// for its writes to arrive before it takes its ticket (one word for all) and makes room for the next. A step, us, with tickets and
+// with the launch:
+//   k_step, blocks of 64 (18,000 threads at 2,048 atoms, 26,000 at 2,916, 35,000 at 4,000): 1,372 atoms 7.2 and 7.7, 2,048 7.9 and 7.4,
+//   2,916 7.7 and 8.1, 4,000 9.0 and 8.1, 5,324 9.9 and 8.8, 16,384 13.2 and 10.0, 32,000 15.4 and 11.3, 131,072 24.1 and 22.2, 256,000 41.7 and 38.6;
+//   k_pack, a thread per atom, blocks of 256 (step with the force kernel): 8,788 12.0 and 12.8, 16,384 14.8 and 15.3, 23,328 19.2 and 19.0,
+//   32,000 18.4 and 18.7, 55,296 23.7 and 22.4, 131,072 48.2 and 40.3, 256,000 73.3 and 68.5;
+//   k_constrained, a thread per group, blocks of 128 (step of water): 1,728 groups 30.8 and 30.6, 13,824 98.2 and 98.1, 216,000 1,032 and 1,033.
+// So the lines cross between 18,000 and 35,000 threads of the first and 23,000 and 55,000 of the second, and the third does not care. In
+// blocks they lie further apart, 290 to 550 and 90 to 220: a block of 256 holds more back while it waits.
 constexpr int64_t kTicketThreadsMost = 25000;
 constexpr int kLongRow = 240;                         // entries (with the row's spare room): about 150 partners per atom
 constexpr int64_t kRowsAlways = 4096;                 // cell rows that any system may have: 2 MB of list rows

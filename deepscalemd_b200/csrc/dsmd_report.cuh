@@ -1,4 +1,5 @@
-// Values that the host waits for leave a kernel through pinned host memory: the block that finishes last writes them, each
+// Values that the host waits for leave a kernel through pinned host memory: the block that finishes last writes them (or, for
+// displacement checks of large grids, a launch of one thread behind them: report_displacement), each
 // half of a value in one 64-bit word with the number of the launch, which the host polls (dsmd_ctx::mail). That saves the
 // copy behind the kernel and the wait for the copy; and, as every word says by itself whether it has arrived, the fence
 // between values and number (1.4 us each: it waits for the host's memory).

@@ -1,4 +1,4 @@
-// Largest displacement and sums over the blocks of a grid, reported to the host by the block that finishes last.
+// Largest displacement and sums over the blocks of a grid, reported to the host by the block that finishes last, or by a launch behind it.
 #pragma once
 
 #include "dsmd_force.cuh"
@@ -17,8 +17,8 @@ __device__ __forceinline__ void post_displacement(const DisplacementReport& r) {
 }
 
 // The block's largest squared displacement goes into the status word. With a ticket the last block of the grid reports the word.
-// Without one (large grids) nothing waits for anything: every warp adds its own, if it is larger than what it reads there, and a
-// launch behind this one reports the word (k_post_displacement).
+// Without one (large grids, or nobody to report to) nothing waits for anything: every warp adds its own, if it is larger than what it reads
+// there, and a launch behind this one reports the word (k_post_displacement), if there is to be a report.
 __device__ __forceinline__ void report_displacement(double v, const DisplacementReport& r) {
     for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;

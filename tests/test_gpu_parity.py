@@ -388,6 +388,31 @@ def test_nve_drift_is_no_worse_than_the_reference_over_10k_steps(cuda_device):
     ctx.close()
 
 
+def test_nve_drift_over_trajectories(cuda_device):
+    """The trend of one trajectory says little: over 400 starts of the 32,000-atom system the fitted trends have a mean of 0.9e-5 +- 0.3e-5
+    per atom and 10,000 steps and a spread of 5.4e-5 (a little more than a fit to white noise would have, 4.3e-5), so that one
+    in a hundred lies beyond the bound of the test above. The mean over eight, within three standard errors of such a mean."""
+    g = np.load(os.path.join(GOLDEN, "nve_lj_32000.npz"))
+    dt, every, samples = float(g["dt"]), int(g["every"]), int(g["steps"]) // int(g["every"])
+    t, trends = np.arange(samples + 1), []
+    for seed in range(1, 9):
+        s = syn.fcc_lj(20, seed=seed)
+        ctx = make_context(s)
+        ctx.build_neighbor_list()
+        ctx.compute_forces()
+        ctx.run_nve(int(g["equilibration"]), dt, 1.0, 0.5, 0, True)
+        trace = []
+        for k in range(samples + 1):
+            ctx.compute_forces(want_energy=True)
+            trace.append((ctx.read_scalars()["pe"] + ctx.kinetic_energy()) / s.n)
+            if k < samples:
+                ctx.run_nve(every, dt, 1.0, 0.5, 0, True)
+        trends.append(np.polyfit(t, trace, 1)[0] * samples)
+        ctx.close()
+    ref = np.polyfit(t, g["energy_per_atom"], 1)[0] * samples
+    assert abs(np.mean(trends)) <= abs(ref) + 3.0 * 5.4e-5 / np.sqrt(len(trends)), trends
+
+
 def test_nve_trajectory_tracks_the_oracle(cuda_device):
     """Twenty velocity-Verlet steps on the GPU and on the oracle's fp64 forces stay together to fp32-force accuracy."""
     s = syn.fcc_lj(5, seed=8)

@@ -161,12 +161,12 @@ __global__ void k_reorder(Grid g, int first, int n_owned, int n_total, unsigned 
 #pragma unroll
     for (int f = 0; f < kNumReal; ++f)
         if (FORCES || f < DSMD_FX || f > DSMD_FZ) r[f] = src.p[f][from];
+    const int ty = type_src[from], id = gid_src[from];   // (reads before the writes: for all the compiler knows it is the same memory)
 #pragma unroll
     for (int f = 0; f < kNumReal; ++f)
         if (FORCES || f < DSMD_FX || f > DSMD_FZ) dst.p[f][s] = r[f];
-    const int ty = type_src[from];
     type_dst[s] = ty;
-    gid_dst[s] = gid_src[from];
+    gid_dst[s] = id;
     unsigned bad = 0;
     int4 p;
     p.x = static_cast<int>(dsmd::to_fixed(r[0], 0, g, bad));
@@ -1305,8 +1305,8 @@ static int stage_rows(dsmd_ctx* c, const double* rows, int64_t n, double* const*
 }
 
 // [n][3] host rows (any memory) to three device arrays. Few rows are staged: the host waits for nothing but the upload before. More are
-// copied by the runtime, through three arrays of the same size: from pageable memory 17 to 24 GB/s (100,000 atoms 0.16 ms,
-// 400,000 0.57; staged 0.20 and 0.69), but it waits for what is queued in the stream. It takes a copy by where it starts: out
+// copied by the runtime, through three arrays of the same size (from pageable memory 100,000 atoms 0.16 ms,
+// 400,000 0.57; staged 0.20 and 0.69), but that waits for what is queued in the stream. The runtime takes a copy by where it starts: out
 // of pageable memory it has read all of it when it returns; out of memory that it knows it only queues the copy (queued: the
 // caller of the upload is to get the rows back when that is over), and refuses it if part of it is not known. Those rows are staged.
 static int upload_columns(dsmd_ctx* c, const double* rows, int64_t n, double* const* to, double* const* scratch, bool few, int64_t& used, bool& queued,

@@ -1675,11 +1675,15 @@ int dsmd_max_displacement_sq_lagged(dsmd_ctx* c, double* out, void* stream) {
 
 // Whether the force launch about to be made in `s` may read the list before the launch before it has ended: a force launch in the same
 // stream came between the build and this one, and has itself waited for the build. (Never in a graph, whose edges are its own.)
-static bool list_settled(dsmd_ctx* c, cudaStream_t s) {
-    const bool settled = !c->captured && c->settled_epoch == c->build_epoch && c->settled_stream == s;
+static bool list_settled(const dsmd_ctx* c, cudaStream_t s) {
+    return !c->captured && c->settled_epoch == c->build_epoch && c->settled_stream == s;
+}
+
+static void force_launched(dsmd_ctx* c, cudaStream_t s) {
+    ++c->launches;
+    if (c->captured) return;   // perhaps into a graph only
     c->settled_epoch = c->build_epoch;
     c->settled_stream = s;
-    return settled;
 }
 
 static PairParams pair_params(const dsmd_ctx* c) {
@@ -1735,7 +1739,7 @@ static int compute_forces_impl(dsmd_ctx* c, int phase, int want_energy, int64_t 
                                           : (e ? dsmd::launch_pair<kEwaldCopiesMost, true, kLongOrder> : dsmd::launch_pair<kEwaldCopiesMost, false, kLongOrder>);
         // (ranges and boundary passes follow work of other streams: nothing to overlap with)
         DSMD_CUDA(c, launch(p, a, sw, blocks, !ranged && phase != DSMD_PHASE_BOUNDARY, s));
-        ++c->launches;
+        force_launched(c, s);
     }
     return DSMD_OK;
 }
@@ -1753,7 +1757,7 @@ static int force_step(dsmd_ctx* c, double dt, double f2a, cudaStream_t s) {
     const DisplacementReport report = displacement_report(c, true, pairs << c->lane_shift, s);
     const auto launch = long_rows(c) ? dsmd::launch_step<kLongOrder> : dsmd::launch_step<0>;
     DSMD_CUDA(c, launch(p, a, c->grid, at, report, c->switch_distance > 0.0, blocks, s));
-    ++c->launches;
+    force_launched(c, s);
     std::swap(c->pq, c->pq_next);
     return displacement_posted(c, report, s);
 }

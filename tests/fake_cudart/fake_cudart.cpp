@@ -159,7 +159,9 @@ cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const
 namespace dsmd {
 
 template <int COPIES, bool ENERGY, int ORDER>
-cudaError_t launch_pair(const PairParams&, const ForceArgs&, bool, unsigned, bool, cudaStream_t) { return launch("k_pair", nullptr); }
+cudaError_t launch_pair(const PairParams&, const ForceArgs& a, bool, unsigned, bool, cudaStream_t) {
+    return launch(a.list_settled ? "k_pair early" : "k_pair", nullptr);
+}
 
 template <int ORDER>
 cudaError_t launch_step(const PairParams&, const ForceArgs&, const Grid&, const StepArgs&, const DisplacementReport& r, bool, unsigned, cudaStream_t) {

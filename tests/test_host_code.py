@@ -207,3 +207,22 @@ def test_no_report_of_a_check_whose_word_the_caller_has(lib):
         assert s.displacement() == 0
         assert s.run(4, 2) == 0 and any("k_post_displacement" in line for line in log(lib))
     lib.dsmd_destroy(s.h)
+
+
+@pytest.mark.parametrize("before", ["nothing", "no boundary pairs", "a refused launch", "another stream"])
+def test_the_list_is_read_early_only_behind_a_force_launch(lib, before):
+    """A force kernel reads the list before the launch before it has ended if a force launch of the same stream came between the list
+    build and it: one that was made."""
+    s = System(lib)
+    assert s.build() == 0
+    if before == "no boundary pairs":
+        assert lib.dsmd_compute_forces(s.h, ctypes.c_int(2), ctypes.c_int(0), None) == 0   # nothing to launch
+    if before == "a refused launch":
+        lib.fake_refuse(b"k_pair", 0)
+        assert s.forces() == CUDA_ERROR
+    if before == "another stream":
+        assert lib.dsmd_compute_forces(s.h, ctypes.c_int(0), ctypes.c_int(0), ptr(64)) == 0
+    lib.fake_reset()
+    assert s.forces() == 0 and s.forces() == 0
+    assert [line for line in log(lib) if "k_pair" in line] == ["launch k_pair", "launch k_pair early"]
+    lib.dsmd_destroy(s.h)
